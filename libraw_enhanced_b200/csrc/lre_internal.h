@@ -163,7 +163,10 @@ lre_status launch_axial_ca_banded(Context* c, const float* in, float* out, size_
 lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, size_t h, float radius,
                            float edge_thr, float chroma_thr, float strength, bool green,
                            float green_scale, const float* in_max_g = nullptr, float* out_max_g = nullptr);
-lre_status launch_detail_tonemap(Context* c, const float* in, float* out, size_t w, size_t h);
+// reference_order: the box sums in the reference's scan order, for callers to
+// whom the last bit of the result matters.
+lre_status launch_detail_tonemap(Context* c, const float* in, float* out, size_t w, size_t h,
+                                 bool reference_order = false);
 lre_status launch_micro_contrast(Context* c, const float* in, float* out, size_t w, size_t h,
                                  float threshold, float strength, float target, const float* mask);
 lre_status launch_lateral_ca(Context* c, const float* in, float* out, size_t w, size_t h, int cell,
