@@ -88,6 +88,8 @@ void lre_inject_fault(lre_ctx* ctx, int countdown);
 /* Bound of every device-side wait of the in-order sweeps (DCB, AAHD,
  * highlight recovery: a band waits for the band above to publish its
  * columns), in SM clock cycles; cycles <= 0 restores the default (~2 s).
+ * The passes run on independent blocks, which wait for nothing, and in order
+ * only where the blocks disagree; with a limit set they run in order always.
  * A wait that runs out sets an error flag, stops waiting and lets the kernel
  * finish; the call then returns LRE_ERR_TIMEOUT and the context stays
  * usable.  No counterpart in the reference (its loops run on the CPU). */

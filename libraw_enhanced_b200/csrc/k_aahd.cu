@@ -5,8 +5,8 @@
 // vertical interpolations, a 4-px zero margin), two int[3] YUV images, and a
 // byte direction map.  Here each channel of each direction is its own padded
 // plane in HBM ((W+8) x (H+8) floats): X (the native samples), R/G/B for
-// d = 0 (horizontal) and d = 1 (vertical), and the direction map held as
-// floats for the in-order refinement sweep.  The YUV images are never stored:
+// d = 0 (horizontal) and d = 1 (vertical), and the direction map held in
+// the bits of floats for the in-order refinement sweep.  The YUV images are never stored:
 // evaluate_ahd recomputes them from the gamma table where it needs them.
 //
 // Ordering.  make_ahd_greens, make_ahd_rb and evaluate_ahd read only values
@@ -58,7 +58,7 @@ struct Aahd {
   float maxv;
   float* X;        // native samples (after hide_hots: with hot sites replaced)
   float* P[2][3];  // [d][channel]
-  float* ND;       // direction map
+  float* ND;       // direction map (the flags as the bits of a float)
   float* stats;    // channel max [3], channel min [3]
   int* hot;        // count of sites hot against the original samples
   __device__ __forceinline__ unsigned fc(int i, int j) const { return fcol3((unsigned)i, (unsigned)j, filters); }
@@ -175,13 +175,15 @@ __global__ void k_aahd_hot_pretest(Aahd A) {
 // and r + 1 advance together, each row pair three columns behind the pair
 // above: (r - 2, c + 2) is then already rewritten and (r + 2, c - 2) not yet.
 struct OpHideHots {
-  static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing;
+  static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 2, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr bool UNROLL = false, STEP2 = false;
+  // padded coordinates; the 2x2 pattern makes the 4-px offset invisible
+  __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo& g) {
-    // padded coordinates; the 2x2 pattern makes the 4-px offset invisible
-    if (g.fc(r, c) == 1) return;
+  __device__ static void cell(const T& t, int, const Geo&) {
     float o;
-    if (hot_site([&](int dr, int dc) { return t(0, r + dr, c + dc); }, &o)) t(0, r, c) = o;
+    if (hot_site([&](int dr, int dc) { return t.get(0, dr, dc); }, &o)) t.set(0, o);
   }
 };
 
@@ -323,7 +325,7 @@ __global__ void k_aahd_evaluate(Aahd A) {
     if (totv < toth * 1.2f) nd |= kVer;
     if (toth < totv * 1.2f) nd |= kHor;
     if (nd == 0) nd = kHor | kVer;
-    A.ND[p] = (float)nd;
+    A.ND[p] = __int_as_float(nd);
   }
 }
 
@@ -334,32 +336,37 @@ __global__ void k_aahd_evaluate(Aahd A) {
 // image so the last odd column is reached.  Every neighbour read precedes or
 // follows the site exactly as in the row-major loops with skew 1.
 struct OpRefineDirs {
-  static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing;
+  static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr bool UNROLL = true, STEP2 = true;
+  // the walk acts at even image columns; rows two steps apart share their parity
+  __device__ static bool site(int, int c, const Geo&) { return ((c - kMargin) & 1) == 0; }
+  __device__ static int phase(int, const Geo&) { return kMargin & 1; }
   template <class T>
-  __device__ static void upd(const T& t, int r, int c) {
-    const int n = (int)t(0, r - 1, c), s = (int)t(0, r + 1, c), w = (int)t(0, r, c - 1), e = (int)t(0, r, c + 1);
-    int m = (int)t(0, r, c);
+  __device__ static void upd(const T& t) {
+    const int n = __float_as_int(t.get(0, -1, 0)), s = __float_as_int(t.get(0, 1, 0)),
+              w = __float_as_int(t.get(0, 0, -1)), e = __float_as_int(t.get(0, 0, 1));
+    int m = __float_as_int(t.get(0, 0, 0));
     const int nv = ((n & kVer) + (s & kVer) + (w & kVer) + (e & kVer)) / kVer;
     const int nh = ((n & kHor) + (s & kHor) + (w & kHor) + (e & kHor)) / kHor;
     const bool codir = (m & kVer) ? ((n & kVer) || (s & kVer)) : ((w & kHor) || (e & kHor));
     if ((m & kVer) && (nh > 2 && !codir)) m = kHor;
     if ((m & kHor) && (nv > 2 && !codir)) m = kVer;
-    t(0, r, c) = (float)m;
+    t.set(0, __int_as_float(m));
   }
   // g.W here is the padded width; image columns are [kMargin, g.W - kMargin).
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo& g) {
+  __device__ static void cell(const T& t, int c, const Geo& g) {
     const int j = c - kMargin;
-    if (j & 1) return;
-    if (c < g.W - kMargin) upd(t, r, c);
-    if (j >= 1) upd(t, r, c - 1);
+    if (c < g.W - kMargin) upd(t);
+    if (j >= 1) upd(t.off(-1));
   }
 };
 
 __global__ void k_aahd_combine(Aahd A, float* __restrict__ rgb) {
   AAHD_FOR_PIXELS(A) {
     const size_t p = A.pi(i, j);
-    const int d = ((int)A.ND[p] & kVer) ? 1 : 0;
+    const int d = (__float_as_int(A.ND[p]) & kVer) ? 1 : 0;
     float* o = rgb + ((size_t)i * A.W + j) * 3;
     o[0] = A.pl(d, 0)[p] / A.maxv;
     o[1] = A.pl(d, 1)[p] / A.maxv;
@@ -402,7 +409,8 @@ size_t padded_bytes(size_t w, size_t h) {
 
 size_t ws_bytes_aahd(size_t w, size_t h) {
   const size_t nb = 2 * ((h + 2 * kMargin + 31) / 32 + 1);
-  return 8 * padded_bytes(w, h) + 256 + (kSyncInts + nb) * sizeof(int) + 1024;
+  return 8 * padded_bytes(w, h) + 256 + (kSyncInts + nb) * sizeof(int) + 1024 +
+         blk_ws_bytes<OpHideHots, OpRefineDirs>(w + 2 * kMargin, h + 2 * kMargin);
 }
 
 lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rgb, size_t w, size_t h,
@@ -420,7 +428,9 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
   float* stats = reinterpret_cast<float*>(c->ws.take(256));
   const int nb_max = 2 * (int)((h + 2 * kMargin + 31) / 32 + 1);
   int* sync = reinterpret_cast<int*>(c->ws.take((kSyncInts + nb_max) * sizeof(int)));
-  if (!base || !stats || !sync) return fail(c, LRE_ERR_CUDA, "demosaic_bayer_aahd: workspace not reserved");
+  const size_t blk_len = blk_ws_bytes<OpHideHots, OpRefineDirs>(w + 2 * kMargin, h + 2 * kMargin);
+  void* blk_ws = c->ws.take(blk_len);
+  if (!base || !stats || !sync || !blk_ws) return fail(c, LRE_ERR_CUDA, "demosaic_bayer_aahd: workspace not reserved");
   auto plane = [&](int k) { return reinterpret_cast<float*>(base + (size_t)k * pb); };
   A.X = plane(0);
   for (int d = 0; d < 2; d++)
@@ -458,7 +468,9 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
     hh.c_lo = kMargin;
     hh.c_hi = (int)w + kMargin - 1;
     hh.skip_if_zero = A.hot;
-    LRE_TRY(sweep<OpHideHots>(c, hh, sync, nb_max, "aahd_hide_hots"));
+    // through the direction plane (unused so far, its margin zero like X's)
+    // and back: without hot sites nothing runs and X stays as it is
+    LRE_TRY(sweep<OpHideHots>(c, hh, &A.ND, true, blk_ws, blk_len, sync, nb_max, "aahd_hide_hots"));
   }
   AAHD_LAUNCH(k_aahd_greens, A);
   AAHD_LAUNCH(k_aahd_rb_hv, A);
@@ -471,7 +483,8 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
     rd.r_hi = (int)h + kMargin - 1;
     rd.c_lo = kMargin;
     rd.c_hi = (int)w + kMargin;  // one past the image: the last odd column
-    LRE_TRY(sweep<OpRefineDirs>(c, rd, sync, nb_max, "aahd_refine_dirs"));
+    LRE_TRY(sweep<OpRefineDirs>(c, rd, &A.X, false, blk_ws, blk_len, sync, nb_max, "aahd_refine_dirs"));
+    std::swap(A.ND, A.X);  // the samples are no longer needed
   }
   AAHD_LAUNCH(k_aahd_combine, A, rgb);
 #undef AAHD_LAUNCH

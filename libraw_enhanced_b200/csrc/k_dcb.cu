@@ -401,55 +401,71 @@ __global__ void k_dcb_pp_terms(const float* __restrict__ G, float* __restrict__ 
 // R and B do not change across the nyquist passes).  A site reads rows r +- 2
 // only, so rows r and r + 1 advance together.
 struct OpNyquist {
-  static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing;
+  static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 1, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr bool UNROLL = true, STEP2 = true;
+  __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
+  // sites with r + c of the non-green parity
+  __device__ static int phase(int r0, const Geo& g) { return (r0 & 1) ^ (g.fc(0, 0) == 1); }
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo& g) {
-    if (g.fc(r, c) == 1) return;
-    t(0, r, c) = dclip((t(0, r + 2, c) + t(0, r - 2, c) + t(0, r, c - 2) + t(0, r, c + 2)) / 4.0f + t(1, r, c) -
-                           t(2, r, c),
-                       g.maxv);
+  __device__ static void cell(const T& t, int, const Geo& g) {
+    t.set(0, dclip((t.get(0, 2, 0) + t.get(0, -2, 0) + t.get(0, 0, -2) + t.get(0, 0, 2)) / 4.0f + t.input(1) -
+                       t.input(2),
+                   g.maxv));
   }
 };
 
 // dcb_pp (:820-834), one channel (R or B) per warp: state the channel;
 // input K = G - mean8(G) (k_dcb_pp_terms; green does not change in the pass).
 struct OpPP {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr bool UNROLL = true, STEP2 = false;
+  __device__ static bool site(int, int, const Geo&) { return true; }
+  __device__ static int phase(int, const Geo&) { return 0; }
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo& g) {
-    const float x1 = (t(0, r, c - 1) + t(0, r, c + 1) + t(0, r - 1, c) + t(0, r + 1, c) + t(0, r - 1, c - 1) +
-                      t(0, r + 1, c + 1) + t(0, r - 1, c + 1) + t(0, r + 1, c - 1)) /
+  __device__ static void cell(const T& t, int, const Geo& g) {
+    const float x1 = (t.get(0, 0, -1) + t.get(0, 0, 1) + t.get(0, -1, 0) + t.get(0, 1, 0) + t.get(0, -1, -1) +
+                      t.get(0, 1, 1) + t.get(0, -1, 1) + t.get(0, 1, -1)) /
                      8.0f;
-    t(0, r, c) = dclip(x1 + t(1, r, c), g.maxv);
+    t.set(0, dclip(x1 + t.input(1), g.maxv));
   }
 };
 
 template <class T>
-__device__ __forceinline__ void clamp8(const T& t, int p, int r, int c, float v) {
-  const float n0 = t(p, r + 1, c + 1), n1 = t(p, r - 1, c + 1), n2 = t(p, r + 1, c - 1), n3 = t(p, r - 1, c - 1),
-              n4 = t(p, r, c - 1), n5 = t(p, r, c + 1), n6 = t(p, r - 1, c), n7 = t(p, r + 1, c);
+__device__ __forceinline__ void clamp8(const T& t, float v) {
+  const float n0 = t.get(0, 1, 1), n1 = t.get(0, -1, 1), n2 = t.get(0, 1, -1), n3 = t.get(0, -1, -1),
+              n4 = t.get(0, 0, -1), n5 = t.get(0, 0, 1), n6 = t.get(0, -1, 0), n7 = t.get(0, 1, 0);
   const float lo = smin(smin(smin(smin(smin(smin(smin(n0, n1), n2), n3), n4), n5), n6), n7);
   const float hi = smax(smax(smax(smax(smax(smax(smax(n0, n1), n2), n3), n4), n5), n6), n7);
-  t(p, r, c) = ulim(v, hi, lo);
+  t.set(0, ulim(v, hi, lo));
 }
 
 // dcb_refinement's closing clamp (:992-994): state G; input the pre-clamp value.
 struct OpRefine {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr bool UNROLL = true, STEP2 = true;
+  __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
+  // sites with r + c of the non-green parity
+  __device__ static int phase(int r0, const Geo& g) { return (r0 & 1) ^ (g.fc(0, 0) == 1); }
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo& g) {
-    if (g.fc(r, c) == 1) return;
-    clamp8(t, 0, r, c, t(1, r, c));
+  __device__ static void cell(const T& t, int, const Geo&) {
+    clamp8(t, t.input(1));
   }
 };
 
 // dcb_color_full's last loop (:898-913), one channel per warp: state R or B;
 // input that channel's CLIP(chroma + G).
 struct OpColorFull {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr bool UNROLL = true, STEP2 = false;
+  __device__ static bool site(int, int, const Geo&) { return true; }
+  __device__ static int phase(int, const Geo&) { return 0; }
   template <class T>
-  __device__ static void cell(const T& t, int r, int c, const Geo&) {
-    clamp8(t, 0, r, c, t(1, r, c));
+  __device__ static void cell(const T& t, int, const Geo&) {
+    clamp8(t, t.input(1));
   }
 };
 
@@ -461,7 +477,8 @@ bool bayer_2x2_layout(uint32_t filters) { return bayer_2x2(filters); }
 
 size_t ws_bytes_dcb(size_t w, size_t h) {
   const size_t nb = 2 * ((h + 31) / 32 + 1);
-  return 7 * plane_bytes(w, h) + ((w * h + 255) & ~size_t(255)) + (kSyncInts + nb) * sizeof(int) + 1024;
+  return 7 * plane_bytes(w, h) + ((w * h + 255) & ~size_t(255)) + (kSyncInts + nb) * sizeof(int) + 1024 +
+         blk_ws_bytes<OpNyquist, OpPP, OpRefine, OpColorFull>(w, h);
 }
 
 lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb, size_t w, size_t h,
@@ -481,7 +498,9 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
   uint8_t* M = reinterpret_cast<uint8_t*>(take((w * h + 255) & ~size_t(255)));
   const int nb_max = 2 * (int)((h + 31) / 32 + 1);
   int* sync = reinterpret_cast<int*>(take((kSyncInts + nb_max) * sizeof(int)));
-  if (!R || !G || !B || !P1 || !P2 || !P3 || !P4 || !M || !sync)
+  const size_t blk_len = blk_ws_bytes<OpNyquist, OpPP, OpRefine, OpColorFull>(w, h);
+  void* blk_ws = take(blk_len);
+  if (!R || !G || !B || !P1 || !P2 || !P3 || !P4 || !M || !sync || !blk_ws)
     return fail(c, LRE_ERR_CUDA, "demosaic_bayer_dcb: workspace not reserved");
 
   Geo g{(int)w, (int)h, filters, maximum_value};
@@ -517,10 +536,13 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
   if (iterations > 0) DCB_LAUNCH(k_dcb_nyq_terms, R, B, P1, P2, g);
   for (int it = 1; it <= iterations; it++) {
     SweepArgs ny = rect(sa, 2);
-    ny.plane[0] = G;
     ny.plane[1] = P1;
     ny.plane[2] = P2;
-    for (int k = 0; k < 3; k++) LRE_TRY(sweep<OpNyquist>(c, ny, sync, nb_max, "dcb_nyquist"));
+    for (int k = 0; k < 3; k++) {
+      ny.plane[0] = G;
+      LRE_TRY(sweep<OpNyquist>(c, ny, &P3, false, blk_ws, blk_len, sync, nb_max, "dcb_nyquist"));
+      std::swap(G, P3);
+    }
     DCB_LAUNCH(k_dcb_map, G, M, g);
     DCB_LAUNCH(k_dcb_correction, G, M, g);
   }
@@ -532,7 +554,10 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     pp.plane[1] = B;
     pp.plane[2] = P1;
     pp.plane[3] = P1;
-    LRE_TRY(sweep<OpPP>(c, pp, sync, nb_max, "dcb_pp"));
+    float* const out[2] = {P2, P3};
+    LRE_TRY(sweep<OpPP>(c, pp, out, false, blk_ws, blk_len, sync, nb_max, "dcb_pp"));
+    std::swap(R, P2);
+    std::swap(B, P3);
   }
   DCB_LAUNCH(k_dcb_map, G, M, g);
   DCB_LAUNCH(k_dcb_correction2, G, R, B, M, g);
@@ -547,7 +572,8 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     SweepArgs rf = rect(sa, 4);
     rf.plane[0] = G;
     rf.plane[1] = P1;
-    LRE_TRY(sweep<OpRefine>(c, rf, sync, nb_max, "dcb_refinement"));
+    LRE_TRY(sweep<OpRefine>(c, rf, &P2, false, blk_ws, blk_len, sync, nb_max, "dcb_refinement"));
+    std::swap(G, P2);
     DCB_LAUNCH(k_dcb_chroma_native, R, B, G, P4, g);
     DCB_LAUNCH(k_dcb_chroma, P4, P2, P3, g);
     DCB_LAUNCH(k_dcb_chroma_g, P2, P3, G, P1, P4, g);
@@ -556,7 +582,10 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     cf.plane[1] = B;
     cf.plane[2] = P1;
     cf.plane[3] = P4;
-    LRE_TRY(sweep<OpColorFull>(c, cf, sync, nb_max, "dcb_color_full"));
+    float* const out[2] = {P2, P3};
+    LRE_TRY(sweep<OpColorFull>(c, cf, out, false, blk_ws, blk_len, sync, nb_max, "dcb_color_full"));
+    std::swap(R, P2);
+    std::swap(B, P3);
   }
   DCB_LAUNCH(k_dcb_output, R, G, B, rgb, g);
 #undef DCB_LAUNCH

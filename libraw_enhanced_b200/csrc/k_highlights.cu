@@ -183,7 +183,7 @@ __global__ void k_hl_ratio_sums(const float* __restrict__ t_rg, const float* __r
 // pixels copy through); flag bit 2 marks white pixels.  scal[2] = max_val.
 __global__ void k_hl_pass2(const float* __restrict__ in, size_t n, HlParams P, uint8_t* __restrict__ flags,
                            float* __restrict__ R, float* __restrict__ G, float* __restrict__ B,
-                           float* __restrict__ hl, float* __restrict__ scal) {
+                           float* __restrict__ scal) {
   const float grf = scal[0], gbf = scal[1];
   float local_max = 0.f;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -202,91 +202,151 @@ __global__ void k_hl_pass2(const float* __restrict__ in, size_t n, HlParams P, u
     R[i] = p0;
     G[i] = p1;
     B[i] = p2;
-    hl[i] = (f & 1) ? 1.f : 0.f;
   }
   block_max_atomic(local_max, scal + 2);
+}
+
+// The neighbour terms of a pixel: its largest channel, and its G / RB ratio
+// where the pixel takes part in its neighbours' ratio means, -1 where not.
+__device__ __forceinline__ float loca_ratio(float n0, float n1, float n2, float nl, float thr) {
+  const float nrb = 0.5f * (n0 + n2);
+  if (nl < thr * 0.75f || nrb <= 1e-6f) return -1.f;
+  const float ratio = n1 / nrb;
+  return (ratio < 0.70f || ratio > 1.35f) ? -1.f : ratio;
 }
 
 // Loop 3 (:1259-1296): white pixels off the 1-px frame take the mean of their
 // 8 neighbours, all read before any is written (out of place).
 __global__ void k_hl_white(const float* __restrict__ R, const float* __restrict__ G, const float* __restrict__ B,
                            const uint8_t* __restrict__ flags, float* __restrict__ R2, float* __restrict__ G2,
-                           float* __restrict__ B2, int W, int H) {
+                           float* __restrict__ B2, float* __restrict__ cand, float* __restrict__ nl,
+                           float* __restrict__ rt, float* out, int W, int H, float thr) {
   const size_t n = (size_t)W * H;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(i / W), x = (int)(i % W);
     const float* src[3] = {R, G, B};
     float* dst[3] = {R2, G2, B2};
     const bool white = (flags[i] & 4) && x > 0 && x < W - 1 && y > 0 && y < H - 1;
+    float v[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
       const float* s = src[c];
-      dst[c][i] = white ? (s[i - W - 1] + s[i - W] + s[i - W + 1] + s[i - 1] + s[i + 1] + s[i + W - 1] + s[i + W] +
+      v[c] = white ? (s[i - W - 1] + s[i - W] + s[i - W + 1] + s[i - 1] + s[i + 1] + s[i + W - 1] + s[i + W] +
                            s[i + W + 1]) *
                               (1.f / 8.f)
-                        : s[i];
+                   : s[i];
+      dst[c][i] = v[c];
     }
+    // Loop 4 changes a highlight pixel only from its own value, and only when
+    // that value passes these two tests (:1307-1329), so they are decided
+    // here, once, for all pixels.
+    const float l = smax(v[0], smax(v[1], v[2]));
+    const float rb = 0.5f * (v[0] + v[2]);
+    nl[i] = l;
+    rt[i] = loca_ratio(v[0], v[1], v[2], l, thr);
+    out[i * 3] = v[0];
+    out[i * 3 + 1] = v[1];
+    out[i * 3 + 2] = v[2];
+    cand[i] = (flags[i] & 1) && !(l < thr * 0.90f) && !(rb <= v[1] * 1.04f) ? 1.f : 0.f;
   }
 }
 
-// Loop 4 (:1301-1377), in pixel order: state R, G, B; input the highlight
-// flag.  aux[0] = threshold, aux[1] = max_val.
+// A candidate's new value from its own value and its neighbours' terms, or
+// false where it keeps its value.  nl(dy, dx) and ratio(dy, dx) read the terms.
+template <class NL, class RT>
+__device__ __forceinline__ bool loca_lift(NL nl, RT ratio, float thr, float max_val, float& p0, float& p1, float& p2) {
+  float local_max = 0.0f, local_min = FLT_MAX;
+#pragma unroll
+  for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+    for (int dx = -1; dx <= 1; ++dx) {
+      const float n = nl(dy, dx);
+      local_max = smax(local_max, n);
+      local_min = smin(local_min, n);
+    }
+  if ((local_max - local_min) < 0.015f) return false;
+  const float l = smax(p0, smax(p1, p2));
+  const float rb = 0.5f * (p0 + p2);
+  // Unrolled, so each weight 1.0 / (1 + |dx| + |dy|) is the same correctly
+  // rounded double, folded at compile time.
+  double ratio_sum = 0.0, ratio_w = 0.0;
+#pragma unroll
+  for (int dy = -2; dy <= 2; ++dy)
+#pragma unroll
+    for (int dx = -2; dx <= 2; ++dx) {
+      const float q = ratio(dy, dx);
+      if (q == -1.f) continue;
+      const double w = 1.0 / (double)(1 + abs(dx) + abs(dy));
+      ratio_sum += q * w;
+      ratio_w += w;
+    }
+  const float local_ratio = (float)(ratio_w > 0.0 ? ratio_sum / ratio_w : 1.0);
+  const float desired_g = rb * sclamp(local_ratio, 0.95f, 1.08f);
+  const float g_missing = desired_g - p1;
+  if (g_missing <= 0.0f) return false;
+  const float sat_w = sclamp((l - thr) / smax(1e-6f, smax(1.0f, max_val) - thr), 0.0f, 1.0f);
+  const float edge_w = sclamp((local_max - local_min) / 0.08f, 0.0f, 1.0f);
+  const float alpha = sclamp(0.30f + 0.55f * sat_w * edge_w, 0.0f, 0.90f);
+  const float g_boost = alpha * smin(g_missing, (rb - p1) * 0.90f);
+  p1 += g_boost;
+  const float rb_residual = smax(0.0f, 0.5f * (p0 + p2) - p1);
+  if (rb_residual > 0.0f) {
+    const float trim = smin(rb_residual * alpha * 0.45f, 0.5f * (p0 + p2) * 0.12f);
+    p0 = smax(0.0f, p0 - trim);
+    p2 = smax(0.0f, p2 - trim);
+  }
+  p1 = smax(0.0f, p1);
+  return true;
+}
+
+// Loop 4 (:1301-1377), in pixel order: state R, G, B; input the candidate
+// flag (k_hl_white).  aux[0] = threshold, aux[1] = max_val.
 struct OpLoca {
   static constexpr int NS = 3, NP = 4, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, RING = 256;
+  __device__ static bool site(int, int, const Geo&) { return true; }
   template <class T>
-  __device__ static void cell(const T& t, int y, int x, const Geo& g) {
-    if (t(3, y, x) == 0.f) return;
-    const float thr = g.aux[0], max_val = g.aux[1];
-    float p0 = t(0, y, x), p1 = t(1, y, x), p2 = t(2, y, x);
-    const float l = smax(p0, smax(p1, p2));
-    if (l < thr * 0.90f) return;
-    float local_max = 0.0f, local_min = FLT_MAX;
-#pragma unroll
-    for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-      for (int dx = -1; dx <= 1; ++dx) {
-        const float nl = smax(t(0, y + dy, x + dx), smax(t(1, y + dy, x + dx), t(2, y + dy, x + dx)));
-        local_max = smax(local_max, nl);
-        local_min = smin(local_min, nl);
-      }
-    if ((local_max - local_min) < 0.015f) return;
-    const float rb = 0.5f * (p0 + p2);
-    if (rb <= p1 * 1.04f) return;
-    // Unrolled, so each weight 1.0 / (1 + |dx| + |dy|) is the same correctly
-    // rounded double, folded at compile time.
-    double ratio_sum = 0.0, ratio_w = 0.0;
-#pragma unroll
-    for (int dy = -2; dy <= 2; ++dy)
-#pragma unroll
-      for (int dx = -2; dx <= 2; ++dx) {
-        const float n0 = t(0, y + dy, x + dx), n1 = t(1, y + dy, x + dx), n2 = t(2, y + dy, x + dx);
-        const float nrb = 0.5f * (n0 + n2);
-        const float nl = smax(n0, smax(n1, n2));
-        if (nl < thr * 0.75f || nrb <= 1e-6f) continue;
-        const float ratio = n1 / nrb;
-        if (ratio < 0.70f || ratio > 1.35f) continue;
-        const double w = 1.0 / (double)(1 + abs(dx) + abs(dy));
-        ratio_sum += ratio * w;
-        ratio_w += w;
-      }
-    const float local_ratio = (float)(ratio_w > 0.0 ? ratio_sum / ratio_w : 1.0);
-    const float desired_g = rb * sclamp(local_ratio, 0.95f, 1.08f);
-    const float g_missing = desired_g - p1;
-    if (g_missing <= 0.0f) return;
-    const float sat_w = sclamp((l - thr) / smax(1e-6f, smax(1.0f, max_val) - thr), 0.0f, 1.0f);
-    const float edge_w = sclamp((local_max - local_min) / 0.08f, 0.0f, 1.0f);
-    const float alpha = sclamp(0.30f + 0.55f * sat_w * edge_w, 0.0f, 0.90f);
-    const float g_boost = alpha * smin(g_missing, (rb - p1) * 0.90f);
-    p1 += g_boost;
-    const float rb_residual = smax(0.0f, 0.5f * (p0 + p2) - p1);
-    if (rb_residual > 0.0f) {
-      const float trim = smin(rb_residual * alpha * 0.45f, 0.5f * (p0 + p2) * 0.12f);
-      p0 = smax(0.0f, p0 - trim);
-      p2 = smax(0.0f, p2 - trim);
+  __device__ static void cell(const T& t, int, const Geo& g) {
+    if (t.input(3) == 0.f) return;
+    const float thr = g.aux[0];
+    float p0 = t.get(0, 0, 0), p1 = t.get(1, 0, 0), p2 = t.get(2, 0, 0);
+    auto nl = [&](int dy, int dx) { return smax(t.get(0, dy, dx), smax(t.get(1, dy, dx), t.get(2, dy, dx))); };
+    auto rt = [&](int dy, int dx) {
+      return loca_ratio(t.get(0, dy, dx), t.get(1, dy, dx), t.get(2, dy, dx), nl(dy, dx), thr);
+    };
+    if (!loca_lift(nl, rt, thr, g.aux[1], p0, p1, p2)) return;
+    t.set(0, p0);
+    t.set(1, p1);
+    t.set(2, p2);
+  }
+};
+
+// The same loop for blocks.  A pixel's neighbours see only two terms of it,
+// so those are the state (two planes instead of three, and no division per
+// neighbour: each pixel's ratio is formed once).  The pixel's own RGB is read
+// from the planes where it is a candidate, and its result goes straight into
+// the interleaved image.
+struct OpLocaBlk {
+  static constexpr int NS = 2, NP = 3, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, BLK_WARPS = 6;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr bool UNROLL = false, STEP2 = false;
+  __device__ static bool site(int, int, const Geo&) { return true; }
+  template <class T>
+  __device__ static void cell(const T& t, int, const Geo& g) {
+    if (t.input(2) == 0.f) return;
+    const float thr = g.aux[0];
+    float p0 = __ldg(g.ex[0] + t.px), p1 = __ldg(g.ex[1] + t.px), p2 = __ldg(g.ex[2] + t.px);
+    if (loca_lift([&](int dy, int dx) { return t.get(0, dy, dx); }, [&](int dy, int dx) { return t.get(1, dy, dx); },
+                  thr, g.aux[1], p0, p1, p2)) {
+      const float n = smax(p0, smax(p1, p2));
+      t.set(0, n);
+      t.set(1, loca_ratio(p0, p1, p2, n, thr));
     }
-    p1 = smax(0.0f, p1);
-    t(0, y, x) = p0;
-    t(1, y, x) = p1;
-    t(2, y, x) = p2;
+    if (t.own) {  // also where it keeps its value: a repair may undo a first run's change
+      float* o = g.ex_out + t.px * 3;
+      o[0] = p0;
+      o[1] = p1;
+      o[2] = p2;
+    }
   }
 };
 
@@ -296,8 +356,11 @@ __global__ void k_hl_aux(float* scal, float thr) {
   scal[4] = scal[2];
 }
 
+// The in-order sweep's planes into the result, where it had to run.
 __global__ void k_hl_interleave(const float* __restrict__ R, const float* __restrict__ G,
-                                const float* __restrict__ B, float* __restrict__ out, size_t n) {
+                                const float* __restrict__ B, float* __restrict__ out, size_t n,
+                                const int* __restrict__ run_if) {
+  if (*run_if == 0) return;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     out[i * 3] = R[i];
     out[i * 3 + 1] = G[i];
@@ -313,8 +376,8 @@ size_t ws_bytes_highlights(size_t w, size_t h) {
   const size_t n = w * h;
   const size_t nb = (n + kHlBlock - 1) / kHlBlock;
   const size_t bands = (h + 31) / 32 + 1;
-  return 7 * plane(n) + ((n + 255) & ~size_t(255)) + 2 * ((nb + 1) * sizeof(int) + 256) + 256 +
-         (kSyncInts + bands) * sizeof(int) + 1024;
+  return 9 * plane(n) + ((n + 255) & ~size_t(255)) + 2 * ((nb + 1) * sizeof(int) + 256) + 256 +
+         (kSyncInts + bands) * sizeof(int) + 1024 + blk_ws_bytes<OpLocaBlk>(w, h);
 }
 
 lre_status launch_recover_highlights(Context* c, const float* in, float* out, size_t w, size_t h,
@@ -330,13 +393,17 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
   float* G2 = reinterpret_cast<float*>(c->ws.take(plane(n)));
   float* B2 = reinterpret_cast<float*>(c->ws.take(plane(n)));
   float* HL = reinterpret_cast<float*>(c->ws.take(plane(n)));
+  float* NL = reinterpret_cast<float*>(c->ws.take(plane(n)));
+  float* RT = reinterpret_cast<float*>(c->ws.take(plane(n)));
   uint8_t* flags = reinterpret_cast<uint8_t*>(c->ws.take((n + 255) & ~size_t(255)));
   int* counts = reinterpret_cast<int*>(c->ws.take((nb + 1) * sizeof(int) + 256));
   int* offs = reinterpret_cast<int*>(c->ws.take((nb + 1) * sizeof(int) + 256));
   float* scal = reinterpret_cast<float*>(c->ws.take(256));
   const int nb_max = (int)((h + 31) / 32 + 1);
   int* sync = reinterpret_cast<int*>(c->ws.take((kSyncInts + nb_max) * sizeof(int)));
-  if (!R || !G || !B || !R2 || !G2 || !B2 || !HL || !flags || !counts || !offs || !scal || !sync)
+  const size_t blk_len = blk_ws_bytes<OpLocaBlk>(w, h);
+  void* blk_ws = c->ws.take(blk_len);
+  if (!R || !G || !B || !R2 || !G2 || !B2 || !HL || !NL || !RT || !flags || !counts || !offs || !scal || !sync || !blk_ws)
     return fail(c, LRE_ERR_CUDA, "recover_highlights: workspace not reserved");
 
   HlParams P{};
@@ -363,9 +430,9 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
   k_hl_ratio_sums<<<1, 32, 0, s>>>(R2, G2, offs + nb, scal);
   LRE_TRY(ck("recover_highlights"));
   const unsigned g1 = grid_for(n, 256, c->sm_count * 8);
-  k_hl_pass2<<<g1, 256, 0, s>>>(in, n, P, flags, R, G, B, HL, scal);
+  k_hl_pass2<<<g1, 256, 0, s>>>(in, n, P, flags, R, G, B, scal);
   LRE_TRY(ck("recover_highlights"));
-  k_hl_white<<<g1, 256, 0, s>>>(R, G, B, flags, R2, G2, B2, (int)w, (int)h);
+  k_hl_white<<<g1, 256, 0, s>>>(R, G, B, flags, R2, G2, B2, HL, NL, RT, out, (int)w, (int)h, P.thr);
   LRE_TRY(ck("recover_highlights"));
   // loop 4 reads the threshold and max_val from the device
   k_hl_aux<<<1, 1, 0, s>>>(scal, P.thr);
@@ -383,8 +450,30 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
   sa.c_lo = 2;
   sa.c_hi = (int)w - 3;
   if (!d_err) LRE_CUDA_TRY(c, cudaMemsetAsync(err, 0, sizeof(int), s));
-  LRE_TRY(sweep<OpLoca>(c, sa, sync, nb_max, "recover_highlights_loca"));
-  k_hl_interleave<<<g1, 256, 0, s>>>(R2, G2, B2, out, n);
+  BlkArgs b{};
+  b.g = sa.g;
+  b.g.ex[0] = R2;
+  b.g.ex[1] = G2;
+  b.g.ex[2] = B2;
+  b.g.ex_out = out;
+  b.in[0] = NL;
+  b.in[1] = RT;
+  b.in[2] = HL;
+  b.out[0] = R;  // dead since loop 3
+  b.out[1] = G;
+  b.r_lo = sa.r_lo;
+  b.r_hi = sa.r_hi;
+  b.c_lo = sa.c_lo;
+  b.c_hi = sa.c_hi;
+  if (sa.r_hi < sa.r_lo || sa.c_hi < sa.c_lo) {  // no pixel is off the 2-px frame
+    if (d_max_val_out)
+      LRE_CUDA_TRY(c, cudaMemcpyAsync(d_max_val_out, scal + 2, sizeof(float), cudaMemcpyDeviceToDevice, s));
+    if (!d_err) LRE_CUDA_TRY(c, cudaStreamSynchronize(s));
+    return LRE_OK;
+  }
+  LRE_TRY(blk_sweep<OpLocaBlk>(c, b, blk_ws, blk_len, &sa.run_if, "recover_highlights_loca"));
+  LRE_TRY(sweep_in_order<OpLoca>(c, sa, sync, nb_max, "recover_highlights_loca"));
+  k_hl_interleave<<<g1, 256, 0, s>>>(R2, G2, B2, out, n, sa.run_if);
   LRE_TRY(ck("recover_highlights"));
   if (d_max_val_out) LRE_CUDA_TRY(c, cudaMemcpyAsync(d_max_val_out, scal + 2, sizeof(float), cudaMemcpyDeviceToDevice, s));
   if (d_err) return LRE_OK;  // the caller reads the flag after its own synchronisation

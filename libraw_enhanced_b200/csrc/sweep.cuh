@@ -19,15 +19,24 @@
 //     already running;
 //   * every wait is bounded: on time-out the kernel raises an error flag and
 //     stops waiting, and the host reports the failure.
+// That in-order form is the fallback: k_blk_sweep (below) runs the same ops on
+// independent blocks and checks that the result is the in-order one.
+//
 // An op supplies NS state planes + inputs (NP planes per warp), HALO, SKEW,
 // PAIR, NCH (independent channels run as separate warps), LAG (how many
 // columns behind its walk position a cell may still write), RING (ring
-// columns, a power of two) and a cell(t, r, c, g) that updates the site
-// (r, c) through the ring accessor t.
+// columns, a power of two), BLK_WARPS (warps of a block), BLK_ROWS and
+// BLK_COLS (a block's overlap), BLK_SKEW and BLK_PAIR (a block's own skew),
+// UNROLL (whether a block's group of steps is unrolled), STEP2 (a block visits
+// every second step only, from phase(r0, g) on), site(r, c, g) (whether the
+// pass visits the site) and cell(t, c, g), which updates the site that the
+// accessor t stands on.
 #pragma once
 
+#include <algorithm>
 #include <climits>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "lre_internal.h"
@@ -42,6 +51,8 @@ struct Geo {
   uint32_t filters;
   float maxv;
   const float* aux;  // optional device scalars an op reads (nullptr when unused)
+  const float* ex[3];  // optional planes an op reads at its own sites only
+  float* ex_out;       // and where it writes for the sites its block owns
   __device__ __forceinline__ unsigned fc(int r, int c) const { return fcol3((unsigned)r, (unsigned)c, filters); }
   __device__ __forceinline__ size_t at(int r, int c) const { return (size_t)r * W + c; }
 };
@@ -65,6 +76,7 @@ struct SweepArgs {
   int* err;
   int* progress;  // per band: columns < progress[b] of band b are final in HBM
   const int* skip_if_zero;  // optional: every band returns at once when *skip_if_zero == 0
+  const int* run_if;        // optional: likewise when *run_if == 0
   long long wait_cycles;    // bound of one wait for the band above (SM clock cycles)
   int hold_ticket;          // fault injection: this band never publishes (-1: none)
 };
@@ -83,6 +95,19 @@ struct Ring {
   __device__ __forceinline__ float& operator()(int p, int r, int c) const {
     return sweep_smem[p * PLANE + (r - rbase) * PITCH + (c & (RING - 1))];
   }
+};
+
+// One site of the ring as an op sees it: get(p, dr, dc) is state plane p at
+// (r + dr, c + dc), input(p) input plane p at the site, set(p, v) writes the
+// site, off(dc) is the site dc columns away.
+template <class R>
+struct RingCell {
+  R t;
+  int r, c;
+  __device__ __forceinline__ float get(int p, int dr, int dc) const { return t(p, r + dr, c + dc); }
+  __device__ __forceinline__ float input(int p) const { return t(p, r, c); }
+  __device__ __forceinline__ void set(int p, float v) const { t(p, r, c) = v; }
+  __device__ __forceinline__ RingCell off(int dc) const { return RingCell{t, r, c + dc}; }
 };
 
 // Row padding so the 32 lanes of a step hit 32 different banks: lane l
@@ -140,6 +165,7 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
   constexpr int SPAN = Op::SKEW * (31 / Op::PAIR);  // column lag of lane 31 behind lane 0
   static_assert((kAhead + 1) * GS + SPAN + 2 * HALO + Op::LAG <= Op::RING, "sweep ring too small for this op");
   if (a.skip_if_zero && *a.skip_if_zero == 0) return;
+  if (a.run_if && *a.run_if == 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lc = lane & 15, lr = lane >> 4;
   __shared__ int s_ticket;
   if (threadIdx.x == 0) s_ticket = atomicAdd(a.ticket, 1);
@@ -164,7 +190,7 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
 #pragma unroll 4
       for (int s = 0; s < GS; s++) {
         const int c = t0 + s - Op::SKEW * (lane / Op::PAIR);
-        if (row_on && c >= a.c_lo && c <= a.c_hi) Op::cell(t, r, c, a.g);
+        if (row_on && c >= a.c_lo && c <= a.c_hi && Op::site(r, c, a.g)) Op::cell(RingCell<R>{t, r, c}, c, a.g);
         __syncwarp();
       }
       group_barrier();
@@ -287,8 +313,431 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
   publish(flushed);
 }
 
+
+// ---------------------------------------------------------------- blocks
+// The same sweep on independent blocks, checked.
+//
+// A site's new value depends on values far above and to the left of it only
+// through a chain of sites each of which passes on a fraction of a change (an
+// average, a clamp that mostly does not bind).  So a block that starts
+// BLK_ROWS rows above and BLK_COLS steps left of the sites it owns, from the
+// pass's input values, arrives at its own sites with the in-order values, bit
+// for bit, although what it started from was wrong.  That is not assumed but
+// checked: each block keeps the values of the sites just outside its own that
+// its own sites read (HALO rows above, REACH steps left), and
+// k_blk_check compares them with what the owners of those sites produced.
+// Where all agree, every site is its op's value of its final predecessors and
+// its original successors, which is the in-order result (by induction in
+// row-major order from the first block, which starts at the frame).  A block
+// that disagrees runs once more from its neighbours' values (k_blk_sweep,
+// repair), is checked again, and if that disagrees too the in-order sweep
+// below runs on the untouched input.  The result is the in-order one always.
+//
+// Block geometry: BLK_WARPS warps of 32 rows walk the steps tau = c + SKEW *
+// (row / PAIR) of the block in groups of kBlkGroup, each warp one group behind
+// the warp above; a barrier per group.  The state planes live in a
+// shared-memory ring of kBlkRing steps indexed by tau (the skew is in the
+// index, so the ring needs no columns for it); the inputs, read at the site
+// only, in one group's buffer per warp.  With the group's steps unrolled,
+// every access of a cell is one instruction: the group's place in the ring is
+// in a register, the rest in the immediate.  What bounds it is the latency of
+// a warp's steps (shared memory, then a chain of dependent operations), so the
+// buffers are kept small enough for two blocks per SM.
+//
+// Why: the in-order form chains its 32-row bands through global memory and
+// leaves most SMs waiting; a sweep of 24 MP took 1.9 to 2.8 ms (44 ms for the
+// LoCA lift) whatever its arithmetic.  Blocks at 24 MP: nyquist 1930 -> 252 us,
+// pp 2810 -> 324, refinement 2360 -> 186, color_full 2800 -> 378, LoCA 44470
+// -> 1420 (with its terms as state); direction refinement at 12 MP 2210 ->
+// 104, hot pixels 2000 -> 205.  Staging through registers and keeping the
+// inputs in one group's buffer (two blocks per SM instead of one) was worth
+// 1.9x; 4-byte cp.async into a full ring of every plane had given 620 us for
+// nyquist.
+//
+// Overlap: an average of four updated neighbours passes on 3/7 of a change
+// per row and 1/1.5 per step (pp); from a difference of 2^18 ulps, 64 rows
+// and 96 steps leave fewer than 2^-20 ulps.  With 64 steps, one pp block in
+// about 2000 was repaired at 24 MP.
+constexpr int kBlkGroup = 8;    // steps per group
+constexpr int kBlkRing = 64;    // ring steps (power of two): groups g-2 .. g+5
+
+struct BlkArgs {
+  const float* in[4];  // state planes first, then read-only inputs (NCH = 2: as SweepArgs::plane)
+  float* out[4];       // where the state planes' result goes (every site of the plane)
+  Geo g;
+  int r_lo, r_hi, c_lo, c_hi;  // updated rectangle (inclusive)
+  int S, nbj, nbi;             // owned steps per block, blocks per row of blocks, rows of blocks
+  float* side;                 // per block: the kept outside values
+  int* bad;                    // [0], [1]: a block disagreed in the first / second check; [2..]: per block
+  const int* skip_if_zero;
+};
+
 template <class Op>
-lre_status sweep(Context* c, const SweepArgs& base, int* sync, int nb_max, const char* what) {
+struct Blk {
+  static constexpr int NW = Op::BLK_WARPS, ROWS = NW * 32, OWN = ROWS - Op::BLK_ROWS;
+  static constexpr int PITCH = kBlkRing + 1;  // odd: the 32 rows of a step are on 32 banks
+  static constexpr int PLANE = (ROWS + 2 * Op::HALO) * PITCH;
+  static constexpr int NI = Op::NP - Op::NS, IPITCH = kBlkGroup + 1, IPLANE = ROWS * IPITCH;
+  static constexpr int INPUTS = Op::NS * PLANE;  // where the input buffers start
+  static constexpr size_t BYTES = (size_t)(INPUTS + NI * IPLANE) * sizeof(float);
+  static constexpr int SKEW = Op::BLK_SKEW, PAIR = Op::BLK_PAIR;
+  // skew of a row relative to the block's first one (floor division)
+  __host__ __device__ static constexpr int skew(int lr) { return SKEW * (PAIR == 2 ? (lr >> 1) : lr); }
+  // columns read left of a site or above it reach this many steps back
+  static constexpr int REACH = Op::HALO * SKEW + Op::HALO + Op::LAG;
+  static_assert(REACH <= kBlkGroup + Op::LAG, "the ring keeps two groups behind");
+  static_assert(Op::BLK_ROWS % 32 == 0 && Op::BLK_COLS % kBlkGroup == 0 && OWN > 0, "row pairs and groups stay together");
+  // side buffer of one block: per state plane HALO rows of S + REACH steps,
+  // then OWN rows of REACH steps
+  static size_t side_floats(int S) { return (size_t)Op::NS * (Op::HALO * (S + REACH) + OWN * REACH); }
+};
+
+// The accessor of a block's cells.  b[q] is the ring place of group g - 2 + q
+// in this lane's row and s the step in the group, a constant after unrolling,
+// so the group a neighbour falls into is known at compile time.
+template <class Op>
+struct BlkCell {
+  unsigned b[5], in;
+  int s;
+  __device__ __forceinline__ unsigned at(int p, int dr, int dc) const {
+    using B = Blk<Op>;
+    const int dt = s + dc + B::SKEW * (B::PAIR == 2 ? dr / 2 : dr) + 2 * kBlkGroup;
+    return b[dt >> 3] + p * B::PLANE + dr * B::PITCH + (dt & 7);
+  }
+  __device__ __forceinline__ float get(int p, int dr, int dc) const { return sweep_smem[at(p, dr, dc)]; }
+  __device__ __forceinline__ float input(int p) const { return sweep_smem[in + (p - Op::NS) * Blk<Op>::IPLANE + s]; }
+  __device__ __forceinline__ void set(int p, float v) const { sweep_smem[at(p, 0, 0)] = v; }
+  __device__ __forceinline__ BlkCell off(int dc) const {
+    BlkCell o = *this;
+    o.s += dc;
+    return o;
+  }
+};
+// Without unrolling: the step is a run-time value.
+template <class Op>
+struct BlkCellAny {
+  unsigned row, in;  // this lane's row in the ring and in the input buffer
+  int lr, tau;
+  size_t px;  // the site's index in the image
+  bool own;   // the block owns the site
+  __device__ __forceinline__ unsigned at(int p, int dr, int dc) const {
+    using B = Blk<Op>;
+    const int dt = dc + (B::PAIR == 2 ? B::skew(lr + dr) - B::skew(lr) : B::SKEW * dr);
+    return row + p * B::PLANE + dr * B::PITCH + ((tau + dt) & (kBlkRing - 1));
+  }
+  __device__ __forceinline__ float get(int p, int dr, int dc) const { return sweep_smem[at(p, dr, dc)]; }
+  __device__ __forceinline__ float input(int p) const {
+    return sweep_smem[in + (p - Op::NS) * Blk<Op>::IPLANE + (tau & (kBlkGroup - 1))];
+  }
+  __device__ __forceinline__ void set(int p, float v) const { sweep_smem[at(p, 0, 0)] = v; }
+};
+
+template <class Op, bool REPAIR>
+__global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
+  using B = Blk<Op>;
+  constexpr int G = kBlkGroup, NP = Op::NP, NS = Op::NS, HALO = Op::HALO, NCH = Op::NCH, KR = Op::BLK_ROWS;
+  if (a.skip_if_zero && *a.skip_if_zero == 0) return;
+  const int ch = blockIdx.z, bi = blockIdx.y, bj = blockIdx.x;
+  const int blk = (ch * a.nbi + bi) * a.nbj + bj;
+  if (REPAIR && a.bad[2 + blk] == 0) return;
+  const int W = a.g.W, H = a.g.H;
+  const int own_r = bi * B::OWN, r0 = own_r - KR;
+  const int own_lo = B::skew(KR) + bj * a.S, own_hi = own_lo + a.S;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int l8 = lane & 7, l4 = lane >> 3;
+  const float* src[NP];
+  float* dst[NS];
+#pragma unroll
+  for (int p = 0; p < NP; p++)
+    src[p] = NCH == 1 ? a.in[p] : (p < NS ? (ch ? a.in[1] : a.in[0]) : (ch ? a.in[3] : a.in[2]));
+#pragma unroll
+  for (int p = 0; p < NS; p++) dst[p] = NCH == 1 ? a.out[p] : (ch ? a.out[1] : a.out[0]);
+  const int g_lo = (REPAIR ? own_lo : own_lo - Op::BLK_COLS) >> 3;  // first group walked
+  const int g_hi = (own_hi - 1 + Op::LAG) >> 3;                    // last one
+  const int ng = g_hi - g_lo + 1;
+
+  // Rows this warp stages: its 32, eight steps of rows k, k + 8, k + 16 and
+  // k + 24 per instruction (32 distinct banks), and, at the block's ends, the
+  // halo rows.  Loaded into registers in one phase and stored to shared memory
+  // at the start of the next: state for group g + 5, inputs for group g.
+  const int lr8 = warp * 32 + 8 * l4;  // even, so row lr8 + k has skew skew(lr8) + skew(k)
+  const int lrh = warp == 0 && l4 < HALO ? l4 - HALO : (warp == B::NW - 1 && l4 < HALO ? B::ROWS + l4 : INT_MAX);
+  const unsigned slr = (lr8 + HALO) * B::PITCH;
+  float v[8][NP], vh[NS];
+  // every row and column of group g inside the image (the same in every lane)
+  auto inside = [&](int g) {
+    return r0 + warp * 32 >= 0 && r0 + warp * 32 + 32 <= H && g * G - B::skew(warp * 32 + 31) >= 0 &&
+           g * G + G - B::skew(warp * 32) <= W;
+  };
+  // planes [P0, P1) of group g
+  auto load = [&](int g, auto p0, auto p1) {
+    constexpr int P0 = decltype(p0)::value, P1 = decltype(p1)::value;
+    const int tau = g * G + l8;
+    const int c0 = tau - B::skew(lr8);
+    const ptrdiff_t i0 = (ptrdiff_t)(r0 + lr8) * W + c0;
+    if (!REPAIR && inside(g)) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int p = P0; p < P1; p++) v[k][p] = __ldg(src[p] + i0 + ((ptrdiff_t)k * W - B::skew(k)));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int r = r0 + lr8 + k, c = c0 - B::skew(k);
+        const bool on = r >= 0 && r < H && c >= 0 && c < W;
+#pragma unroll
+        for (int p = P0; p < P1; p++) {
+          // a repair starts from what the neighbours before it produced
+          const float* q = REPAIR && p < NS && (lr8 + k < KR || tau < own_lo) ? dst[p] : src[p];
+          v[k][p] = on ? __ldcg(q + i0 + ((ptrdiff_t)k * W - B::skew(k))) : 0.f;
+        }
+      }
+    }
+    if (P0 == 0 && lrh != INT_MAX) {
+      const int r = r0 + lrh, c = tau - B::skew(lrh);
+      const bool on = r >= 0 && r < H && c >= 0 && c < W;
+#pragma unroll
+      for (int p = 0; p < NS; p++) {
+        const float* q = REPAIR && lrh < KR ? dst[p] : src[p];
+        vh[p] = on ? __ldcg(q + (ptrdiff_t)r * W + c) : 0.f;
+      }
+    }
+  };
+  auto store = [&](int g) {  // state planes
+    const unsigned tr = (g * G + l8) & (kBlkRing - 1);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int p = 0; p < NS; p++) sweep_smem[p * B::PLANE + slr + tr + k * B::PITCH] = v[k][p];
+    if (lrh != INT_MAX) {
+#pragma unroll
+      for (int p = 0; p < NS; p++) sweep_smem[p * B::PLANE + (lrh + HALO) * B::PITCH + tr] = vh[p];
+    }
+  };
+  auto store_inputs = [&]() {
+    const unsigned sl = B::INPUTS + lr8 * B::IPITCH + l8;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int p = NS; p < NP; p++) sweep_smem[sl + (p - NS) * B::IPLANE + k * B::IPITCH] = v[k][p];
+  };
+  const std::integral_constant<int, 0> z0{};
+  const std::integral_constant<int, NS> zs{};
+  const std::integral_constant<int, NP> zp{};
+
+  const int top_len = a.S + B::REACH;
+  float* side = a.side + (size_t)blk * (NS * (HALO * top_len + B::OWN * B::REACH));
+  // final values of group g: the owned ones to the result, the outside ones
+  // that owned sites read to the side buffer
+  auto flush = [&](int g) {
+    const int tau = g * G + l8;
+    const int c0 = tau - B::skew(lr8);
+    const ptrdiff_t i0 = (ptrdiff_t)(r0 + lr8) * W + c0;
+    const unsigned sl = slr + (tau & (kBlkRing - 1));
+    if (warp * 32 >= KR && g * G >= own_lo && g * G + G <= own_hi && inside(g)) {
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int p = 0; p < NS; p++)
+          dst[p][i0 + ((ptrdiff_t)k * W - B::skew(k))] = sweep_smem[p * B::PLANE + sl + k * B::PITCH];
+      return;
+    }
+    if (g * G + G <= own_lo - B::REACH || (warp * 32 + 32 <= KR - HALO)) return;
+    const bool own_c = tau >= own_lo && tau < own_hi;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++) {
+      const int lr = lr8 + k, r = r0 + lr, c = c0 - B::skew(k);
+      if (r < 0 || r >= H || c < 0 || c >= W) continue;
+      const unsigned q = sl + k * B::PITCH;
+      if (lr >= KR) {
+        if (own_c) {
+#pragma unroll
+          for (int p = 0; p < NS; p++) dst[p][(size_t)r * W + c] = sweep_smem[p * B::PLANE + q];
+        } else if (tau < own_lo && tau >= own_lo - B::REACH) {
+#pragma unroll
+          for (int p = 0; p < NS; p++)
+            side[NS * HALO * top_len + (p * B::OWN + lr - KR) * B::REACH + tau - (own_lo - B::REACH)] =
+                sweep_smem[p * B::PLANE + q];
+        }
+      } else if (lr >= KR - HALO && tau >= own_lo - B::REACH && tau < own_hi) {
+#pragma unroll
+        for (int p = 0; p < NS; p++)
+          side[(p * HALO + lr - (KR - HALO)) * top_len + tau - (own_lo - B::REACH)] = sweep_smem[p * B::PLANE + q];
+      }
+    }
+  };
+
+  for (int g = g_lo - 2; g <= g_lo + 4; g++) {
+    load(g, z0, zs);
+    store(g);
+  }
+  load(g_lo, zs, zp);
+  load(g_lo + 5, z0, zs);
+  __syncthreads();
+  if (REPAIR) {  // the outside values a repair starts from are the ones it uses
+    flush(g_lo - 2);
+    flush(g_lo - 1);
+  }
+  const int lr = warp * 32 + lane, r = r0 + lr;
+  const bool row_on = r >= a.r_lo && r <= a.r_hi && (!REPAIR || lr >= KR);
+  const unsigned srow = (lr + HALO) * B::PITCH, irow = B::INPUTS + lr * B::IPITCH;
+  for (int k = 0; k < ng + B::NW; k++) {
+    const int g = g_lo + k - warp;
+    if (k >= warp && k - warp < ng) {
+      store(g + 5);
+      store_inputs();
+      __syncwarp();
+      load(g + 1, zs, zp);
+      load(g + 6, z0, zs);
+      const int c0 = g * G - B::skew(lr);
+      if constexpr (Op::UNROLL) {
+        BlkCell<Op> t;
+        t.in = irow;
+#pragma unroll
+        for (int q = 0; q < 5; q++) t.b[q] = srow + (((g - 2 + q) * G) & (kBlkRing - 1));
+        // which steps the pass visits: all, or (STEP2) every second one
+        const int ph = Op::STEP2 ? Op::phase(r0, a.g) & 1 : 0;
+        auto steps = [&](auto all, auto first) {
+          constexpr bool ALL = decltype(all)::value;
+          constexpr int F = decltype(first)::value;
+#pragma unroll
+          for (int s = F; s < G; s += Op::STEP2 ? 2 : 1) {
+            t.s = s;
+            const int c = c0 + s;
+            if (ALL || (row_on && c >= a.c_lo && c <= a.c_hi)) Op::cell(t, c, a.g);
+            __syncwarp();
+          }
+        };
+        // every site of the group is updated (the same answer in every lane)
+        const bool all = !REPAIR && r0 + warp * 32 >= a.r_lo && r0 + warp * 32 + 31 <= a.r_hi &&
+                         g * G - B::skew(warp * 32 + 31) >= a.c_lo && g * G + G - 1 - B::skew(warp * 32) <= a.c_hi;
+        const std::true_type yes{};
+        const std::false_type no{};
+        const std::integral_constant<int, 0> f0{};
+        const std::integral_constant<int, Op::STEP2 ? 1 : 0> f1{};
+        if (all) {
+          if (ph) steps(yes, f1); else steps(yes, f0);
+        } else {
+          if (ph) steps(no, f1); else steps(no, f0);
+        }
+      } else {
+        const size_t px = (size_t)r * W + c0;
+#pragma unroll 1
+        for (int s = 0; s < G; s++) {
+          const int c = c0 + s, tau = g * G + s;
+          if (row_on && c >= a.c_lo && c <= a.c_hi && Op::site(r, c, a.g))
+            Op::cell(BlkCellAny<Op>{srow, irow, lr, tau, px + s, lr >= KR && tau >= own_lo && tau < own_hi}, c, a.g);
+          __syncwarp();
+        }
+      }
+      if (k > warp) flush(g - 1);
+    } else if (k - warp == ng) {
+      flush(g_hi);
+    }
+    __syncthreads();
+  }
+}
+
+// Compares every block's kept outside values with the owners' results.
+// ROUND 0 is the first check; ROUND 1 runs only where round 0 found a block
+// bad, after the repair.
+template <class Op, int ROUND>
+__global__ void __launch_bounds__(256) k_blk_check(BlkArgs a) {
+  using B = Blk<Op>;
+  constexpr int NS = Op::NS, HALO = Op::HALO, NCH = Op::NCH;
+  if (a.skip_if_zero && *a.skip_if_zero == 0) return;
+  if (ROUND == 1 && a.bad[0] == 0) return;
+  const int ch = blockIdx.z, bi = blockIdx.y, bj = blockIdx.x;
+  const int blk = (ch * a.nbi + bi) * a.nbj + bj;
+  const int own_r = bi * B::OWN, r0 = own_r - Op::BLK_ROWS;
+  const int own_lo = B::skew(Op::BLK_ROWS) + bj * a.S;
+  const int top_len = a.S + B::REACH;
+  const size_t per = NS * (HALO * top_len + B::OWN * B::REACH);
+  const float* side = a.side + (size_t)blk * per;
+  int bad = 0;
+  for (int e = threadIdx.x; e < (int)per; e += blockDim.x) {
+    int p, lr, tau;
+    if (e < NS * HALO * top_len) {
+      p = e / (HALO * top_len);
+      const int q = e - p * HALO * top_len;
+      lr = Op::BLK_ROWS - HALO + q / top_len;
+      tau = own_lo - B::REACH + q % top_len;
+    } else {
+      const int q = e - NS * HALO * top_len;
+      p = q / (B::OWN * B::REACH);
+      const int z = q - p * B::OWN * B::REACH;
+      lr = Op::BLK_ROWS + z / B::REACH;
+      tau = own_lo - B::REACH + z % B::REACH;
+    }
+    const int r = r0 + lr, c = tau - B::skew(lr);
+    if (r < a.r_lo || r > a.r_hi || c < a.c_lo || c > a.c_hi) continue;
+    const float* o = NCH == 1 ? (p == 0 ? a.out[0] : (p == 1 ? a.out[1] : a.out[2])) : (ch ? a.out[1] : a.out[0]);
+    bad |= __float_as_int(o[(size_t)r * a.g.W + c]) != __float_as_int(side[e]);
+  }
+  bad = __syncthreads_or(bad);
+  if (threadIdx.x == 0) {
+    if (ROUND == 0) a.bad[2 + blk] = bad;
+    if (bad) atomicExch(a.bad + ROUND, 1);
+    // an op that also writes behind its walk position is not repaired: a
+    // repair would update the last site of the block before it twice
+    if (bad && Op::LAG > 0) atomicExch(a.bad + 1, 1);
+  }
+}
+
+// out = in where the in-order sweep ran in place on `in` (run_if), or, for a
+// sweep whose result stays in its input planes, in = out where it did not.
+template <int NPL>
+__global__ void k_blk_copy(BlkArgs a, const int* run_if, int back) {
+  if (a.skip_if_zero && *a.skip_if_zero == 0) return;
+  if ((*run_if != 0) == (back != 0)) return;
+  const size_t n = (size_t)a.g.W * a.g.H;
+#pragma unroll
+  for (int p = 0; p < NPL; p++) {
+    const float* s = back ? a.out[p] : a.in[p];
+    float* d = back ? const_cast<float*>(a.in[p]) : a.out[p];
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) d[i] = s[i];
+  }
+}
+
+// Owned steps per block: what takes the fewest phases over all waves of
+// blocks (two per SM).  A wide block spends less on overlap, a narrow one
+// fills the last wave: at 24 MP (21 rows of blocks) 512 gives one wave of 84
+// phases, 256 two of 52.
+constexpr int kBlkSms = 148;  // the grid shape is also planned without a device
+template <class Op>
+void blk_grid(int W, int H, int* S, int* nbj, int* nbi) {
+  using B = Blk<Op>;
+  *nbi = (H + B::OWN - 1) / B::OWN;
+  const int steps = W + B::skew(B::ROWS - 1) - B::skew(Op::BLK_ROWS);
+  long long best = LLONG_MAX;
+  for (int t = 64; t <= 2048; t += 64) {
+    const long long n = (long long)((steps + t - 1) / t) * *nbi * Op::NCH;
+    const long long cost = (n + 2 * kBlkSms - 1) / (2 * kBlkSms) * ((t + Op::BLK_COLS) / kBlkGroup + B::NW);
+    if (cost < best) {
+      best = cost;
+      *S = t;
+    }
+  }
+  *nbj = (steps + *S - 1) / *S;
+}
+
+// Workspace of block sweeps of a w x h plane, whichever of the ops runs.
+template <class... Ops>
+size_t blk_ws_bytes(size_t w, size_t h) {
+  size_t m = 0;
+  auto one = [&](auto* op) {
+    using Op = std::remove_pointer_t<decltype(op)>;
+    int S, nbj, nbi;
+    blk_grid<Op>((int)w, (int)h, &S, &nbj, &nbi);
+    const size_t n = (size_t)nbj * nbi * Op::NCH;
+    m = std::max(m, n * Blk<Op>::side_floats(S) * sizeof(float) + (n + 2) * sizeof(int) + 1024);
+  };
+  (one(static_cast<Ops*>(nullptr)), ...);
+  return m;
+}
+
+template <class Op>
+lre_status sweep_in_order(Context* c, const SweepArgs& base, int* sync, int nb_max, const char* what) {
   if (base.r_hi < base.r_lo || base.c_hi < base.c_lo) return LRE_OK;
   using R = RingOf<Op>;
   const int nb = (base.r_hi - base.r_lo + 32) / 32 * Op::NCH;
@@ -305,6 +754,70 @@ lre_status sweep(Context* c, const SweepArgs& base, int* sync, int nb_max, const
   LRE_CUDA_TRY(c, cudaMemsetAsync(a.progress, 0, (size_t)nb * sizeof(int), c->stream));
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_gs_sweep<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::BYTES));
   k_gs_sweep<Op><<<nb, kSweepWarps * 32, R::BYTES, c->stream>>>(a);
+  count_launch(c);
+  return check_launch(c, what);
+}
+
+// The block sweep with its checks and the repair.  *run_if (device) is then
+// non-zero when the in-order sweep has to run instead.
+template <class Op>
+lre_status blk_sweep(Context* c, BlkArgs& b, void* ws, size_t ws_len, const int** run_if, const char* what) {
+  using B = Blk<Op>;
+  blk_grid<Op>(b.g.W, b.g.H, &b.S, &b.nbj, &b.nbi);
+  const size_t n = (size_t)b.nbj * b.nbi * Op::NCH;
+  if (n * B::side_floats(b.S) * sizeof(float) + (n + 2) * sizeof(int) > ws_len || b.nbi > 65535)
+    return fail(c, LRE_ERR_CUDA, std::string(what) + ": block table too small");
+  b.bad = reinterpret_cast<int*>(ws);
+  b.side = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + (((n + 2) * sizeof(int) + 255) & ~size_t(255)));
+  *run_if = b.bad + 1;
+  // fault injection and a wait limit are about the in-order sweep
+  const bool held = c->sweep_hold_band >= 0 || c->sweep_wait_cycles > 0;
+  LRE_CUDA_TRY(c, cudaMemsetAsync(b.bad, held ? 1 : 0, 2 * sizeof(int), c->stream));
+  if (held) return LRE_OK;
+  const dim3 grid((unsigned)b.nbj, (unsigned)b.nbi, Op::NCH);
+  auto k0 = k_blk_sweep<Op, false>;
+  auto k1 = k_blk_sweep<Op, true>;
+  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::BYTES));
+  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::BYTES));
+  k0<<<grid, B::NW * 32, B::BYTES, c->stream>>>(b);
+  k_blk_check<Op, 0><<<grid, 256, 0, c->stream>>>(b);
+  count_launch(c, 2);
+  if (Op::LAG == 0) {
+    k1<<<grid, B::NW * 32, B::BYTES, c->stream>>>(b);
+    k_blk_check<Op, 1><<<grid, 256, 0, c->stream>>>(b);
+    count_launch(c, 2);
+  }
+  return check_launch(c, what);
+}
+
+// The sweep of base.plane[0 .. NS * NCH) into out[0 .. NS * NCH) (whole
+// planes; the input planes are scratch afterwards).  keep: the result is to
+// end in the input planes instead.  ws: blk_ws_bytes of the plane.
+template <class Op>
+lre_status sweep(Context* c, const SweepArgs& base, float* const* out, bool keep, void* ws, size_t ws_len, int* sync,
+                 int nb_max, const char* what) {
+  constexpr int NPL = Op::NS * Op::NCH;
+  if (base.r_hi < base.r_lo || base.c_hi < base.c_lo) {  // nothing to update
+    if (!keep)
+      for (int p = 0; p < NPL; p++)
+        LRE_CUDA_TRY(c, cudaMemcpyAsync(out[p], base.plane[p], (size_t)base.g.W * base.g.H * sizeof(float),
+                                        cudaMemcpyDeviceToDevice, c->stream));
+    return LRE_OK;
+  }
+  BlkArgs b{};
+  for (int p = 0; p < 4; p++) b.in[p] = base.plane[p];
+  for (int p = 0; p < NPL; p++) b.out[p] = out[p];
+  b.g = base.g;
+  b.r_lo = base.r_lo;
+  b.r_hi = base.r_hi;
+  b.c_lo = base.c_lo;
+  b.c_hi = base.c_hi;
+  b.skip_if_zero = base.skip_if_zero;
+  SweepArgs a = base;
+  LRE_TRY(blk_sweep<Op>(c, b, ws, ws_len, &a.run_if, what));
+  LRE_TRY(sweep_in_order<Op>(c, a, sync, nb_max, what));
+  const unsigned cg = grid_for((size_t)b.g.W * b.g.H, 256, c->sm_count * 4);
+  k_blk_copy<NPL><<<cg, 256, 0, c->stream>>>(b, a.run_if, keep ? 1 : 0);
   count_launch(c);
   return check_launch(c, what);
 }
