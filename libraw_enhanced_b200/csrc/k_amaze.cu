@@ -24,9 +24,10 @@
 //     R/B-only quantities are stored half-indexed.  148 slabs (~95 MB) sit
 //     in L2.
 //   * cfa (read by nearly every stage) lives in shared memory (102 KB).
-//   * hvwt and pmwt live in shared memory (2 x 51 KB), so both Gauss-Seidel
-//     sweeps chase their row-to-row dependency through SMEM; the work that
-//     only needs a site's final weight runs in a parallel pass afterwards.
+//   * hvwt and pmwt live in shared memory (2 x 51 KB).  One warp runs their
+//     Gauss-Seidel sweeps from registers (weight_sweep) beside stages that do
+//     not read them: hvwt's beside stages 7 and 8, pmwt's beside stage 6's
+//     green.
 //   * Stage-3 chains run one chain per thread with the next step's operands
 //     loaded ahead of the dependent arithmetic.
 // Positions the reference reads without writing in the same tile read zeros
@@ -68,16 +69,16 @@ constexpr size_t kSmemBytes = 2 * HALF * 4 + TS2 * 4;            // hvwt + pmwt 
 
 // Lifetime map of the reference's planes onto the slab (F0..F5 full planes;
 // "a"/"b" = first/second half of a full plane):
-//   F0 vcd  (S2..S6)     -> a rbm, b rbp     (S8..S9)
+//   F0 vcd  (S2..S6)
 //   F1 hcd  (S2..S6)     -> a pmwt copy-out unused, b rbint (S9)
 //   F2 vcdalt (S2..S3)   -> a cddiffsq (S3..S5) then Dgrb0 (S6..S10), b rgbgreen@R/B (S6..S10)
 //   F3 hcdalt (S2..S3)   -> a Dgrb2h, b Dgrb2v (S6) -> a Dgrb1 (S9..S10)
-//   F4 dgintv (S2..S5)   -> a delp, b delm (S7..S8)
-//   F5 dginth (S2..S5)   -> a Dgrbsq1p, b Dgrbsq1m (S7..S8)
+//   F4 dgintv (S2..S5)   -> a rbm, b rbp     (S8..S9)
+//   F5 dginth (S2..S5)
 //   SMEM: cfa (fill..S10), hvwt (S4..S10), pmwt (S8..S9)
 struct Slab {
   float *cfa, *vcd, *hcd, *vcdalt, *hcdalt, *dgintv, *dginth;
-  float *rbm, *rbp, *rbint, *cddiffsq, *Dgrb0, *rgbg, *Dgrb2h, *Dgrb2v, *Dgrb1, *delp, *delm, *Dq1p, *Dq1m;
+  float *rbm, *rbp, *rbint, *cddiffsq, *Dgrb0, *rgbg, *Dgrb2h, *Dgrb2v, *Dgrb1;
   unsigned char *nyquist, *nyquist2;
 };
 
@@ -91,8 +92,8 @@ __device__ Slab make_slab(unsigned char* base, float* cfa_smem) {
   s.hcdalt = F + 3 * TS2;
   s.dgintv = F + 4 * TS2;
   s.dginth = F + 5 * TS2;
-  s.rbm = s.vcd;
-  s.rbp = s.vcd + HALF;
+  s.rbm = s.dgintv;
+  s.rbp = s.dgintv + HALF;
   s.rbint = s.hcd + HALF;
   s.cddiffsq = s.vcdalt;
   s.Dgrb0 = s.vcdalt;
@@ -100,10 +101,6 @@ __device__ Slab make_slab(unsigned char* base, float* cfa_smem) {
   s.Dgrb2h = s.hcdalt;
   s.Dgrb2v = s.hcdalt + HALF;
   s.Dgrb1 = s.hcdalt;
-  s.delp = s.dgintv;
-  s.delm = s.dgintv + HALF;
-  s.Dq1p = s.dginth;
-  s.Dq1m = s.dginth + HALF;
   s.nyquist = reinterpret_cast<unsigned char*>(F + kFull * TS2);
   s.nyquist2 = s.nyquist + HALF;
   return s;
@@ -196,6 +193,73 @@ __device__ __forceinline__ float s3_finish(float h, float c, float cm, float cp,
 // Directional variance of three consecutive chain values (:1380-1381).
 __device__ __forceinline__ float s3_var(float a, float b, float c) {
   return 3.f * (SQR(a) + SQR(b) + SQR(c)) - SQR(a + b + c);
+}
+
+// The Gauss-Seidel sweeps of stages 6 and 9 (:1456-1464, :1537-1542): each
+// R/B site of rows and columns [a, n - a) takes the mean of its four diagonal
+// neighbours' weights where that is farther from 0.5 than its own; row rr
+// reads row rr - 1 as already updated and row rr + 1 as it was.
+//
+// One warp runs it from registers: a lane holds three neighbouring sites of
+// the rows above, here and below, and a row costs one shuffle and about eight
+// dependent operations.  The other 31 warps meanwhile run stages that do not
+// read the weight.  (1024 threads with a barrier per row took 400 cycles a
+// row and nothing ran beside it: 58 k + 55 k of a tile's 600 k cycles.)
+// w is half-indexed: site (rr, cc) of a row with parity cc & 1 == par is
+// w[rr * TSH + (cc >> 1)].
+__device__ __forceinline__ void weight_sweep(float* w, int a, int rr1, int cc1, int par0) {
+  const int j0 = 3 * (threadIdx.x & 31);
+  auto row = [&](int rr, float (&v)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) v[i] = j0 + i < TSH ? w[rr * TSH + j0 + i] : 0.f;
+  };
+  float up[3], cur[3], dn[3];
+  row(a - 1, up);
+  row(a, cur);
+  row(a + 1, dn);
+  for (int rr = a; rr < rr1 - a; rr++) {
+    float nx[3];
+    row(min(rr + 2, TS - 1), nx);
+    const int par = (par0 ^ rr) & 1;
+    float ul[3], ur[3], dl[3], dr[3];
+    if (par == 0) {  // the diagonal neighbours of site j are sites j - 1 and j
+      ul[0] = __shfl_up_sync(0xffffffffu, up[2], 1);
+      dl[0] = __shfl_up_sync(0xffffffffu, dn[2], 1);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        if (i) {
+          ul[i] = up[i - 1];
+          dl[i] = dn[i - 1];
+        }
+        ur[i] = up[i];
+        dr[i] = dn[i];
+      }
+    } else {  // sites j and j + 1
+      ur[2] = __shfl_down_sync(0xffffffffu, up[0], 1);
+      dr[2] = __shfl_down_sync(0xffffffffu, dn[0], 1);
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        if (i < 2) {
+          ur[i] = up[i + 1];
+          dr[i] = dn[i + 1];
+        }
+        ul[i] = up[i];
+        dl[i] = dn[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int j = j0 + i, cc = 2 * j + par;
+      const float alt = 0.25f * (ul[i] + ur[i] + dl[i] + dr[i]);
+      if (cc >= a && cc < cc1 - a && fabsf(0.5f - cur[i]) < fabsf(0.5f - alt)) {
+        cur[i] = alt;
+        w[rr * TSH + j] = alt;
+      }
+      up[i] = cur[i];
+      cur[i] = dn[i];
+      dn[i] = nx[i];
+    }
+  }
 }
 
 __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
@@ -536,102 +600,21 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       }
       __syncthreads();
     }
-    // Gauss-Seidel sweep of hvwt in shared memory (row rr reads row rr-1
-    // already updated), then the per-site green / Dgrb2 in parallel.
-    {
+    // ---- S7/S8 diagonal R/B interpolation (:1483-1532); pmwt into SMEM.  The
+    // R/B gradient planes of stage 7 are formed from cfa where they are read.
+    // Warp 0 sweeps hvwt, which stage 8 does not read, at the same time.
+    const int par0 = (int)(fc_rt(A, 0, 2) & 1);  // column parity of row 0's R/B sites
+    if (tid < 32) {
+      weight_sweep(hvwt, 8, rr1, cc1, par0);
+    } else {
       const int a = 8;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int rr = a; rr < rr1 - a; rr++) {
-        for (int k = tid; k < per_row; k += nth) {
-          const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * k;
-          if (cc >= cc1 - a) continue;
-          const int idx = rr * TS + cc;
-          const float hvwtalt =
-              0.25f * (hvwt[(idx - m1) >> 1] + hvwt[(idx + p1) >> 1] + hvwt[(idx - p1) >> 1] + hvwt[(idx + m1) >> 1]);
-          const float cur = hvwt[idx >> 1];
-          hvwt[idx >> 1] = fabsf(0.5f - cur) < fabsf(0.5f - hvwtalt) ? hvwtalt : cur;
-        }
-        __syncthreads();
-      }
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
-        const int q_ = fdr.div(i), rr = a + q_;
-        const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
-        if (cc >= cc1 - a) continue;
-        const int idx = rr * TS + cc;
-        const float hv = hvwt[idx >> 1];
-        const float d0 = hv * S.vcd[idx] + (1.f - hv) * S.hcd[idx];
-        S.Dgrb0[idx >> 1] = d0;
-        const float g = cfa[idx] + d0;
-        S.rgbg[idx >> 1] = g;
-        const bool nq2 = S.nyquist2[idx >> 1] != 0;
-        // horizontal / vertical neighbours are G sites: their green is cfa
-        S.Dgrb2h[idx >> 1] = nq2 ? SQR(g - xdiv2f(cfa[idx - 1] + cfa[idx + 1])) : 0.f;
-        S.Dgrb2v[idx >> 1] = nq2 ? SQR(g - xdiv2f(cfa[idx - v1] + cfa[idx + v1])) : 0.f;
-      }
-      __syncthreads();
-    }
-    if (doNyquist) {
-      const int a = 8;
-      const int per_row = rb_count(a);
-      const FDiv fdr(per_row);
-      const float* D2h = S.Dgrb2h;
-      const float* D2v = S.Dgrb2v;
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
-        const int q_ = fdr.div(i), rr = a + q_;
-        const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
-        if (cc >= cc1 - a) continue;
-        const int idx = rr * TS + cc;
-        if (!S.nyquist2[idx >> 1]) continue;
-        const float gvarh =
-            epssq + (gquinc[0] * D2h[idx >> 1] +
-                     gquinc[1] * (D2h[(idx - m1) >> 1] + D2h[(idx + p1) >> 1] + D2h[(idx - p1) >> 1] + D2h[(idx + m1) >> 1]) +
-                     gquinc[2] * (D2h[(idx - v2) >> 1] + D2h[(idx - 2) >> 1] + D2h[(idx + 2) >> 1] + D2h[(idx + v2) >> 1]) +
-                     gquinc[3] * (D2h[(idx - m2) >> 1] + D2h[(idx + p2) >> 1] + D2h[(idx - p2) >> 1] + D2h[(idx + m2) >> 1]));
-        const float gvarv =
-            epssq + (gquinc[0] * D2v[idx >> 1] +
-                     gquinc[1] * (D2v[(idx - m1) >> 1] + D2v[(idx + p1) >> 1] + D2v[(idx - p1) >> 1] + D2v[(idx + m1) >> 1]) +
-                     gquinc[2] * (D2v[(idx - v2) >> 1] + D2v[(idx - 2) >> 1] + D2v[(idx + 2) >> 1] + D2v[(idx + v2) >> 1]) +
-                     gquinc[3] * (D2v[(idx - m2) >> 1] + D2v[(idx + p2) >> 1] + D2v[(idx - p2) >> 1] + D2v[(idx + m2) >> 1]));
-        const float d0 = (S.hcd[idx] * gvarv + S.vcd[idx] * gvarh) / (gvarv + gvarh);
-        S.Dgrb0[idx >> 1] = d0;
-        S.rgbg[idx >> 1] = cfa[idx] + d0;
-      }
-      __syncthreads();
-    }
-
-    // ---- S7 R/B gradients (:1483-1502)
-    const int per7 = (cc1 - 12 + 1) / 2;
-    const FDiv fd7(per7);
-    for (int i = tid; i < (rr1 - 12) * per7; i += nth) {
-      const int q_ = fd7.div(i);
-      const int rr = 6 + q_;
-      const int cc = 6 + 2 * (i - q_ * per7);
-      const int idx = rr * TS + cc;
-      if ((fc_rt(A, rr, 2) & 1) == 0) {
-        S.delp[idx >> 1] = fabsf(cfa[idx + p1] - cfa[idx - p1]);
-        S.delm[idx >> 1] = fabsf(cfa[idx + m1] - cfa[idx - m1]);
-        S.Dq1p[idx >> 1] = SQR(cfa[idx + 1] - cfa[idx + 1 - p1]) + SQR(cfa[idx + 1] - cfa[idx + 1 + p1]);
-        S.Dq1m[idx >> 1] = SQR(cfa[idx + 1] - cfa[idx + 1 - m1]) + SQR(cfa[idx + 1] - cfa[idx + 1 + m1]);
-      } else {
-        S.Dq1p[idx >> 1] = SQR(cfa[idx] - cfa[idx - p1]) + SQR(cfa[idx] - cfa[idx + p1]);
-        S.Dq1m[idx >> 1] = SQR(cfa[idx] - cfa[idx - m1]) + SQR(cfa[idx] - cfa[idx + m1]);
-        S.delp[idx >> 1] = fabsf(cfa[idx + 1 + p1] - cfa[idx + 1 - p1]);
-        S.delm[idx >> 1] = fabsf(cfa[idx + 1 + m1] - cfa[idx + 1 - m1]);
-      }
-    }
-    __syncthreads();
-
-    // ---- S8 diagonal R/B interpolation (:1504-1532); pmwt into SMEM
-    {
-      const int a = 8;
-      const int per_row = rb_count(a);
-      const FDiv fdr(per_row);
-      const float* delp = S.delp;
-      const float* delm = S.delm;
-      const float* Dq1m = S.Dq1m;
-      const float* Dq1p = S.Dq1p;
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      auto delm = [&](int x) { return fabsf(cfa[x + m1] - cfa[x - m1]); };  // at R/B sites
+      auto delp = [&](int x) { return fabsf(cfa[x + p1] - cfa[x - p1]); };
+      auto Dq1m = [&](int x) { return SQR(cfa[x] - cfa[x - m1]) + SQR(cfa[x] - cfa[x + m1]); };  // at G sites
+      auto Dq1p = [&](int x) { return SQR(cfa[x] - cfa[x - p1]) + SQR(cfa[x] - cfa[x + p1]); };
+      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -644,10 +627,10 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         const float rbnw = fabsf(1.f - crnw) < arthresh ? cfa[idx] * crnw : (cfa[idx - m1]) + xdiv2f(cfa[idx] - cfa[idx - m2]);
         const float rbne = fabsf(1.f - crne) < arthresh ? cfa[idx] * crne : (cfa[idx + p1]) + xdiv2f(cfa[idx] - cfa[idx + p2]);
         const float rbsw = fabsf(1.f - crsw) < arthresh ? cfa[idx] * crsw : (cfa[idx - p1]) + xdiv2f(cfa[idx] - cfa[idx - p2]);
-        const float wtse = eps + delm[idx1] + delm[(idx + m1) >> 1] + delm[(idx + m2) >> 1];
-        const float wtnw = eps + delm[idx1] + delm[(idx - m1) >> 1] + delm[(idx - m2) >> 1];
-        const float wtne = eps + delp[idx1] + delp[(idx + p1) >> 1] + delp[(idx + p2) >> 1];
-        const float wtsw = eps + delp[idx1] + delp[(idx - p1) >> 1] + delp[(idx - p2) >> 1];
+        const float wtse = eps + delm(idx) + delm(idx + m1) + delm(idx + m2);
+        const float wtnw = eps + delm(idx) + delm(idx - m1) + delm(idx - m2);
+        const float wtne = eps + delp(idx) + delp(idx + p1) + delp(idx + p2);
+        const float wtsw = eps + delp(idx) + delp(idx - p1) + delp(idx - p2);
         float rbm = (wtse * rbnw + wtnw * rbse) / (wtse + wtnw);
         float rbp = (wtne * rbsw + wtsw * rbne) / (wtne + wtsw);
         if (rbp < cfa[idx]) {
@@ -671,37 +654,76 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         S.rbm[idx1] = rbm;
         S.rbp[idx1] = rbp;
         const float rbvarm =
-            epssq + (gausseven[0] * (Dq1m[(idx - v1) >> 1] + Dq1m[(idx - 1) >> 1] + Dq1m[(idx + 1) >> 1] + Dq1m[(idx + v1) >> 1]) +
-                     gausseven[1] * (Dq1m[(idx - v2 - 1) >> 1] + Dq1m[(idx - v2 + 1) >> 1] + Dq1m[(idx - 2 - v1) >> 1] +
-                                     Dq1m[(idx + 2 - v1) >> 1] + Dq1m[(idx - 2 + v1) >> 1] + Dq1m[(idx + 2 + v1) >> 1] +
-                                     Dq1m[(idx + v2 - 1) >> 1] + Dq1m[(idx + v2 + 1) >> 1]));
+            epssq + (gausseven[0] * (Dq1m(idx - v1) + Dq1m(idx - 1) + Dq1m(idx + 1) + Dq1m(idx + v1)) +
+                     gausseven[1] * (Dq1m(idx - v2 - 1) + Dq1m(idx - v2 + 1) + Dq1m(idx - 2 - v1) +
+                                     Dq1m(idx + 2 - v1) + Dq1m(idx - 2 + v1) + Dq1m(idx + 2 + v1) +
+                                     Dq1m(idx + v2 - 1) + Dq1m(idx + v2 + 1)));
         const float rbvarp =
-            epssq + (gausseven[0] * (Dq1p[(idx - v1) >> 1] + Dq1p[(idx - 1) >> 1] + Dq1p[(idx + 1) >> 1] + Dq1p[(idx + v1) >> 1]) +
-                     gausseven[1] * (Dq1p[(idx - v2 - 1) >> 1] + Dq1p[(idx - v2 + 1) >> 1] + Dq1p[(idx - 2 - v1) >> 1] +
-                                     Dq1p[(idx + 2 - v1) >> 1] + Dq1p[(idx - 2 + v1) >> 1] + Dq1p[(idx + 2 + v1) >> 1] +
-                                     Dq1p[(idx + v2 - 1) >> 1] + Dq1p[(idx + v2 + 1) >> 1]));
+            epssq + (gausseven[0] * (Dq1p(idx - v1) + Dq1p(idx - 1) + Dq1p(idx + 1) + Dq1p(idx + v1)) +
+                     gausseven[1] * (Dq1p(idx - v2 - 1) + Dq1p(idx - v2 + 1) + Dq1p(idx - 2 - v1) +
+                                     Dq1p(idx + 2 - v1) + Dq1p(idx - 2 + v1) + Dq1p(idx + 2 + v1) +
+                                     Dq1p(idx + v2 - 1) + Dq1p(idx + v2 + 1)));
         pmwt[idx1] = rbvarm / (rbvarp + rbvarm);
       }
     }
     __syncthreads();
 
-    // ---- S9 (:1534-1592): Gauss-Seidel pmwt sweep in SMEM, then rbint
+    // ---- S6 green / Dgrb2 per site from the swept hvwt, then the Nyquist
+    // sites' green (:1456-1481), while warp 0 sweeps pmwt (:1534-1542)
+    if (tid < 32) {
+      weight_sweep(pmwt, 10, rr1, cc1, par0);
+    } else {
+      const int a = 8;
+      const int per_row = rb_count(a);
+      const FDiv fdr(per_row);
+      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
+        const int q_ = fdr.div(i), rr = a + q_;
+        const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
+        if (cc >= cc1 - a) continue;
+        const int idx = rr * TS + cc;
+        const float hv = hvwt[idx >> 1];
+        const float d0 = hv * S.vcd[idx] + (1.f - hv) * S.hcd[idx];
+        S.Dgrb0[idx >> 1] = d0;
+        const float g = cfa[idx] + d0;
+        S.rgbg[idx >> 1] = g;
+        const bool nq2 = S.nyquist2[idx >> 1] != 0;
+        // horizontal / vertical neighbours are G sites: their green is cfa
+        S.Dgrb2h[idx >> 1] = nq2 ? SQR(g - xdiv2f(cfa[idx - 1] + cfa[idx + 1])) : 0.f;
+        S.Dgrb2v[idx >> 1] = nq2 ? SQR(g - xdiv2f(cfa[idx - v1] + cfa[idx + v1])) : 0.f;
+      }
+      if (doNyquist) {
+        asm volatile("bar.sync 1, %0;" ::"n"(AMZ_THREADS - 32) : "memory");
+      const float* D2h = S.Dgrb2h;
+      const float* D2v = S.Dgrb2v;
+      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
+        const int q_ = fdr.div(i), rr = a + q_;
+        const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
+        if (cc >= cc1 - a) continue;
+        const int idx = rr * TS + cc;
+        if (!S.nyquist2[idx >> 1]) continue;
+        const float gvarh =
+            epssq + (gquinc[0] * D2h[idx >> 1] +
+                     gquinc[1] * (D2h[(idx - m1) >> 1] + D2h[(idx + p1) >> 1] + D2h[(idx - p1) >> 1] + D2h[(idx + m1) >> 1]) +
+                     gquinc[2] * (D2h[(idx - v2) >> 1] + D2h[(idx - 2) >> 1] + D2h[(idx + 2) >> 1] + D2h[(idx + v2) >> 1]) +
+                     gquinc[3] * (D2h[(idx - m2) >> 1] + D2h[(idx + p2) >> 1] + D2h[(idx - p2) >> 1] + D2h[(idx + m2) >> 1]));
+        const float gvarv =
+            epssq + (gquinc[0] * D2v[idx >> 1] +
+                     gquinc[1] * (D2v[(idx - m1) >> 1] + D2v[(idx + p1) >> 1] + D2v[(idx - p1) >> 1] + D2v[(idx + m1) >> 1]) +
+                     gquinc[2] * (D2v[(idx - v2) >> 1] + D2v[(idx - 2) >> 1] + D2v[(idx + 2) >> 1] + D2v[(idx + v2) >> 1]) +
+                     gquinc[3] * (D2v[(idx - m2) >> 1] + D2v[(idx + p2) >> 1] + D2v[(idx - p2) >> 1] + D2v[(idx + m2) >> 1]));
+        const float d0 = (S.hcd[idx] * gvarv + S.vcd[idx] * gvarh) / (gvarv + gvarh);
+        S.Dgrb0[idx >> 1] = d0;
+        S.rgbg[idx >> 1] = cfa[idx] + d0;
+      }
+    }
+    }
+    __syncthreads();
+
+    // ---- S9 (:1543-1592): rbint
     {
       const int a = 10;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int rr = a; rr < rr1 - a; rr++) {
-        for (int k = tid; k < per_row; k += nth) {
-          const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * k;
-          if (cc >= cc1 - a) continue;
-          const int idx = rr * TS + cc, idx1 = idx >> 1;
-          const float pmwtalt =
-              0.25f * (pmwt[(idx - m1) >> 1] + pmwt[(idx + p1) >> 1] + pmwt[(idx - p1) >> 1] + pmwt[(idx + m1) >> 1]);
-          const float pw = pmwt[idx1];
-          if (fabsf(0.5f - pw) < fabsf(0.5f - pmwtalt)) pmwt[idx1] = pmwtalt;
-        }
-        __syncthreads();
-      }
       for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
