@@ -64,8 +64,15 @@ __device__ __forceinline__ float xmul2f(float x) { return x + x; }
 __device__ __forceinline__ float xdiv2f(float x) { return x * 0.5f; }
 
 constexpr size_t kFull = 6;
-constexpr size_t kSlabBytes = kFull * TS2 * 4 + 2 * HALF + 256;  // + nyquist, nyquist2 bytes
+constexpr size_t kSlabBytes = kFull * TS2 * 4 + 256;
 constexpr size_t kSmemBytes = 2 * HALF * 4 + TS2 * 4;            // hvwt + pmwt + cfa
+constexpr int S3_ROW_WARPS = 10;          // 16 rows each: the 152 rows of a tile's stage 3
+constexpr int S3_LD = 19;                 // row pitch of a row warp's buffer: 18 columns
+constexpr int S3_BUF = 2 * 16 * S3_LD;    // floats per row warp
+// behind cfa: the row buffers (S3), then the nyquist and nyquist2 byte maps (S4..S6)
+constexpr size_t kSmemTotal = kSmemBytes + 2 * HALF;
+static_assert(16 * S3_ROW_WARPS >= TS - 8 && S3_ROW_WARPS * S3_BUF * 4 <= 2 * HALF && kSmemTotal <= 227 * 1024 - 64,
+              "stage-3 row buffers and byte maps");
 
 // Lifetime map of the reference's planes onto the slab (F0..F5 full planes;
 // "a"/"b" = first/second half of a full plane):
@@ -75,7 +82,7 @@ constexpr size_t kSmemBytes = 2 * HALF * 4 + TS2 * 4;            // hvwt + pmwt 
 //   F3 hcdalt (S2..S3)   -> a Dgrb2h, b Dgrb2v (S6) -> a Dgrb1 (S9..S10)
 //   F4 dgintv (S2..S5)   -> a rbm, b rbp     (S8..S9)
 //   F5 dginth (S2..S5)
-//   SMEM: cfa (fill..S10), hvwt (S4..S10), pmwt (S8..S9)
+//   SMEM: cfa (fill..S10), hvwt (S4..S10), pmwt (S8..S9), nyquist maps (S4..S6)
 struct Slab {
   float *cfa, *vcd, *hcd, *vcdalt, *hcdalt, *dgintv, *dginth;
   float *rbm, *rbp, *rbint, *cddiffsq, *Dgrb0, *rgbg, *Dgrb2h, *Dgrb2v, *Dgrb1;
@@ -101,7 +108,7 @@ __device__ Slab make_slab(unsigned char* base, float* cfa_smem) {
   s.Dgrb2h = s.hcdalt;
   s.Dgrb2v = s.hcdalt + HALF;
   s.Dgrb1 = s.hcdalt;
-  s.nyquist = reinterpret_cast<unsigned char*>(F + kFull * TS2);
+  s.nyquist = reinterpret_cast<unsigned char*>(cfa_smem + TS2);
   s.nyquist2 = s.nyquist + HALF;
   return s;
 }
@@ -161,33 +168,23 @@ __device__ __forceinline__ float delhvsqsum_at(const float* cfa, int idx) {
 
 // Stage 3 (:1375-1398) after the step has chosen h (the stage-2 value or its
 // alternate): the clamp against the site's Gint and its two neighbours along
-// the chain direction.  A pure function of h, so both candidates can be
-// finished before the chain recurrence decides between them.
+// the chain direction.  Green and R/B sites run the same formulas with h's
+// sign turned over, and every case is formed and selected, not branched to: a
+// warp holds both colours and all cases, so branches ran every path one after
+// the other (880 cycles a step).  The reference's h for a green site is
+// -median + c, not -(median - c): they differ in the sign of a zero.
 __device__ __forceinline__ float s3_finish(float h, float c, float cm, float cp, bool green, float clip_pt) {
-  float Gint;
-  if (green) {
-    Gint = -h + c;
-    if (h > 0) {
-      if (3.f * h > (Gint + c)) {
-        h = -median3(Gint, cm, cp) + c;
-      } else {
-        const float wt2 = 1.f - 3.f * h / (eps + Gint + c);
-        h = wt2 * h + (1.f - wt2) * (-median3(Gint, cm, cp) + c);
-      }
-    }
-  } else {
-    Gint = h + c;
-    if (h < 0) {
-      if (3.f * h < -(Gint + c)) {
-        h = median3(Gint, cm, cp) - c;
-      } else {
-        const float wt2 = 1.f + 3.f * h / (eps + Gint + c);
-        h = wt2 * h + (1.f - wt2) * (median3(Gint, cm, cp) - c);
-      }
-    }
-  }
-  if (Gint > clip_pt) h = (float)(green ? -1 : 1) * (median3(Gint, cm, cp) - c);
-  return h;
+  const float u = green ? -h : h;
+  const float Gint = u + c;
+  const float med = median3(Gint, cm, cp);
+  const float t = (green ? c : med) - (green ? med : c);
+  const float u3 = 3.f * u;
+  const float wt2 = 1.f + u3 / (eps + Gint + c);
+  const float mix = wt2 * h + (1.f - wt2) * t;
+  float r = u < 0.f ? (u3 < -(Gint + c) ? t : mix) : h;
+  const float d = med - c;
+  if (Gint > clip_pt) r = green ? -d : d;
+  return r;
 }
 
 // Directional variance of three consecutive chain values (:1380-1381).
@@ -276,11 +273,11 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
   __shared__ int s_doNyq;
   float mg = 0.f;  // max G of this thread's interior outputs
 
-  for (;;) {
-    if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);
-    __syncthreads();
-    const int tile = A.tile_lo + s_tile;
-    if (tile >= A.tile_hi) break;
+  if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);
+  __syncthreads();
+  for (int tile = A.tile_lo + s_tile; tile < A.tile_hi;) {
+    __syncthreads();  // every thread has read s_tile
+    if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);  // the next tile
     const int top = -16 + (tile / A.n_left) * (TS - 32);
     const int left = -16 + (tile % A.n_left) * (TS - 32);
     const int bottom = min(top + TS, H + 16);
@@ -294,11 +291,19 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     const FDiv fdc(cc1), fd8(cc1 - 8), fd32(cc1 - 32);
 
     // ---- zero what this tile reads before writing (fresh-buffer semantics)
-    for (int i = tid; i < 2 * HALF / 16; i += nth)
-      reinterpret_cast<float4*>(S.nyquist)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = tid; i < rr1 * cc1; i += nth) {
-      const int rr = fdc.div(i), cc = i - rr * cc1;
-      if (rr >= 4 && rr < rr1 - 4 && cc >= 4 && cc < cc1 - 4) continue;
+    // the 4-px frame of the stage-2 planes: eight rows, then eight columns
+    for (int i = tid; i < 8 * (rr1 + cc1); i += nth) {
+      int rr, cc;
+      if (i < 8 * cc1) {
+        rr = fdc.div(i);
+        cc = i - rr * cc1;
+        if (rr >= 4) rr = rr1 - 8 + rr;
+      } else {
+        rr = (i - 8 * cc1) >> 3;
+        cc = (i - 8 * cc1) & 7;
+        if (cc >= 4) cc = cc1 - 8 + cc;
+      }
+      if (rr < 0 || cc < 0) continue;  // a tile narrower than the two bands
       const int idx = rr * TS + cc;
       S.vcd[idx] = 0.f;
       S.hcd[idx] = 0.f;
@@ -422,64 +427,123 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         }
       }
       __syncthreads();
-      const int nlh = rr1 - 8, nlv = cc1 - 8;
-      const int n_h = 2 * nlh, n_v = 2 * nlv;
-      for (int item = tid; item < n_h + n_v; item += nth) {
-        const bool horiz = item < n_h;
-        const int it = horiz ? item : item - n_h;
-        const int nl = horiz ? nlh : nlv;
-        // row chains: the two chains of a row on neighbouring lanes (their
-        // sites share cache lines); column chains: grouped by the parity of
-        // line + start, i.e. by CFA colour, so a warp's lanes take the same
-        // branches and read consecutive columns of one row
-        int line, par;
-        if (horiz) {
-          line = 4 + (it >> 1);
-          par = it & 1;
-        } else {
-          const int grp = it >= nl;
-          line = 4 + (grp ? it - nl : it);
-          par = grp ? 1 - (line & 1) : (line & 1);
-        }
-        const int stride = horiz ? 2 : v2;      // chain step in the flat tile
-        const int len = horiz ? cc1 : rr1;
-        float* d = horiz ? S.hcd : S.vcd;
-        const float* alt = horiz ? S.hcdalt : S.vcdalt;
-        const float* cf = horiz ? cfaT : cfa;   // cf[pos * TS + line] / cf[line + pos * TS]
+      const int warp = tid >> 5, lane = tid & 31;
+      constexpr int G = 8;  // sites of one chain per group
+      if (warp < S3_ROW_WARPS) {
+        // Row chains: a warp takes 16 rows, the two chains of a row on
+        // neighbouring lanes.  16 columns (8 sites of each chain) and two
+        // columns of look-ahead at a time go through a buffer of the warp's
+        // own, so global memory is read and written along rows; read chain by
+        // chain, every load touched 16 rows' cache lines and the L1 tag rate
+        // bounded the stage (91 k of a tile's cycles; 80 k this way, 60 k with
+        // the cases of s3_finish selected instead of branched to).
+        float* buf = smem + kSmemBytes / 4 + warp * S3_BUF;  // [2][16][S3_LD]
+        const int line0 = 4 + 16 * warp, line = line0 + (lane >> 1), par = lane & 1;
+        const bool on = line < rr1 - 4;
         const int pos0 = 4 + par;
-        if (pos0 >= len - 4) continue;
-        const bool green = (fc_rt(A, horiz ? line : pos0, horiz ? pos0 : line) & 1) != 0;
-        const int K = (len - 4 - pos0 + 1) / 2;  // sites pos0, pos0 + 2, ... < len - 4
-        int idx = horiz ? line * TS + pos0 : pos0 * TS + line;
-        int cidx = pos0 * TS + line;  // site in cf (both layouts: position-major)
-        float prev = d[idx - stride], altp = alt[idx - stride];
-        constexpr int G = 8;
-        for (int s0 = 0; s0 < K; s0 += G) {
-          const int g = min(G, K - s0);
-          float dv[G + 1], av[G + 1];
+        const bool green = (fc_rt(A, line, pos0) & 1) != 0;
+        float prev = 0.f, altp = 0.f;
+        if (on) {
+          prev = S.hcd[line * TS + pos0 - 2];
+          altp = S.hcdalt[line * TS + pos0 - 2];
+        }
+        // element k of a lane: row 2k + lane / 16, column lane % 16 (k < 8),
+        // and row lane / 2, column 16 + lane % 2 (k = 8)
+        float nd[9], na[9];
+        auto fetch = [&](int cb) {
 #pragma unroll
-          for (int k = 0; k <= G; k++) {
-            dv[k] = k <= g ? d[idx + k * stride] : 0.f;
-            av[k] = k <= g ? alt[idx + k * stride] : 0.f;
+          for (int k = 0; k < 9; k++) {
+            const int rr = line0 + (k < 8 ? 2 * k + (lane >> 4) : lane >> 1);
+            const int cc = cb + (k < 8 ? lane & 15 : 16 + (lane & 1));
+            const bool in = rr < rr1 - 4 && cc < cc1;
+            nd[k] = in ? S.hcd[rr * TS + cc] : 0.f;
+            na[k] = in ? S.hcdalt[rr * TS + cc] : 0.f;
           }
+        };
+        if (line0 < rr1 - 4) {
+          fetch(4);
+          for (int cb = 4; cb < cc1 - 4; cb += 2 * G) {
 #pragma unroll
-          for (int k = 0; k < G; k++) {
-            if (k < g) {
-              const int ci = cidx + k * v2;
-              const float altvar = s3_var(altp, av[k], av[k + 1]);
-              const float h0 = (altvar < s3_var(prev, dv[k], dv[k + 1])) ? av[k] : dv[k];
-              const float h = s3_finish(h0, cf[ci], cf[ci - TS], cf[ci + TS], green, A.clip_pt);
-              d[idx + k * stride] = h;
-              prev = h;
-              altp = av[k];
+            for (int k = 0; k < 9; k++) {
+              const int q = (k < 8 ? 2 * k + (lane >> 4) : lane >> 1) * S3_LD + (k < 8 ? lane & 15 : 16 + (lane & 1));
+              buf[q] = nd[k];
+              buf[16 * S3_LD + q] = na[k];
             }
+            __syncwarp();
+            if (cb + 2 * G < cc1 - 4) fetch(cb + 2 * G);
+            float* bd = buf + (lane >> 1) * S3_LD + par;
+            const float* ba = bd + 16 * S3_LD;
+            const int cidx = (cb + par) * TS + line;  // in cfaT
+            float dk = bd[0], ak = ba[0];
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+              const float dn = bd[2 * k + 2], an = ba[2 * k + 2];
+              if (on && cb + par + 2 * k < cc1 - 4) {
+                const int ci = cidx + k * v2;
+                const float altvar = s3_var(altp, ak, an);
+                const float h0 = (altvar < s3_var(prev, dk, dn)) ? ak : dk;
+                const float h = s3_finish(h0, cfaT[ci], cfaT[ci - TS], cfaT[ci + TS], green, A.clip_pt);
+                bd[2 * k] = h;
+                prev = h;
+                altp = ak;
+              }
+              dk = dn;
+              ak = an;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const int rr = line0 + 2 * k + (lane >> 4), cc = cb + (lane & 15);
+              if (rr < rr1 - 4 && cc < cc1 - 4) S.hcd[rr * TS + cc] = buf[(2 * k + (lane >> 4)) * S3_LD + (lane & 15)];
+            }
+            __syncwarp();
           }
-          idx += g * stride;
-          cidx += g * v2;
+        }
+      } else {
+        // Column chains, grouped by the parity of line + start, i.e. by CFA
+        // colour, so a warp's lanes take the same branches and read
+        // consecutive columns of one row.
+        const int nlv = cc1 - 8;
+        for (int it = tid - 32 * S3_ROW_WARPS; it < 2 * nlv; it += nth - 32 * S3_ROW_WARPS) {
+          const int grp = it >= nlv;
+          const int line = 4 + (grp ? it - nlv : it);
+          const int par = grp ? 1 - (line & 1) : (line & 1);
+          const int pos0 = 4 + par;
+          if (pos0 >= rr1 - 4) continue;
+          const bool green = (fc_rt(A, pos0, line) & 1) != 0;
+          const int K = (rr1 - 4 - pos0 + 1) / 2;  // sites pos0, pos0 + 2, ... < rr1 - 4
+          int idx = pos0 * TS + line;
+          float* d = S.vcd;
+          const float* alt = S.vcdalt;
+          float prev = d[idx - v2], altp = alt[idx - v2];
+          for (int s0 = 0; s0 < K; s0 += G) {
+            const int g = min(G, K - s0);
+            float dv[G + 1], av[G + 1];
+#pragma unroll
+            for (int k = 0; k <= G; k++) {
+              dv[k] = k <= g ? d[idx + k * v2] : 0.f;
+              av[k] = k <= g ? alt[idx + k * v2] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+              if (k < g) {
+                const int ci = idx + k * v2;
+                const float altvar = s3_var(altp, av[k], av[k + 1]);
+                const float h0 = (altvar < s3_var(prev, dv[k], dv[k + 1])) ? av[k] : dv[k];
+                const float h = s3_finish(h0, cfa[ci], cfa[ci - TS], cfa[ci + TS], green, A.clip_pt);
+                d[ci] = h;
+                prev = h;
+                altp = av[k];
+              }
+            }
+            idx += g * v2;
+          }
         }
       }
     }
     __syncthreads();
+    for (int i = tid; i < 2 * HALF / 16; i += nth)
+      reinterpret_cast<float4*>(S.nyquist)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // cddiffsq at R/B sites (read only there by stage 4/5), half-indexed
     auto rb_count = [&](int a) { return (cc1 - a - a + 1) / 2 + 1; };
     {
@@ -796,6 +860,16 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     }
     __syncthreads();
 
+    const int next_tile = A.tile_lo + s_tile;
+    if (next_tile < A.tile_hi && A.cstride == 1) {
+      // the next tile's samples on their way to L2 (rows of at most six lines)
+      const int ntop = -16 + (next_tile / A.n_left) * (TS - 32), nleft = -16 + (next_tile % A.n_left) * (TS - 32);
+      const int row = ntop + tid / 6, col = nleft + 32 * (tid % 6);
+      if (tid < 6 * TS && row >= 0 && row < H && col < nleft + TS + 31) {
+        const int c = min(max(col, 0), W - 1);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(A.raw + (size_t)row * W + c));
+      }
+    }
     // Dgrb1 initialisation (:1563-1569): move the B-row values to Dgrb1.
     {
       const int r0 = 13 - A.ey;
@@ -877,6 +951,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       if (row >= 4 && row < H - 4 && col >= 4 && col < W - 4) mg = fmaxf(mg, fmaxf(0.f, g));
     }
     __syncthreads();
+    tile = next_tile;
   }
   // every thread leaves the tile loop together (s_tile is shared)
   if (A.max_g) {
@@ -994,8 +1069,8 @@ lre_status launch_amaze_rows(Context* c, AmazeArgs A, int row_lo, int row_hi) {
   A.tile_counter = reinterpret_cast<int*>(c->ws.take(256));
   if (!A.scratch || !A.tile_counter) return fail(c, LRE_ERR_OUT_OF_MEMORY, "demosaic_bayer_amaze: workspace too small");
   LRE_CUDA_TRY(c, cudaMemsetAsync(A.tile_counter, 0, sizeof(int), c->stream));
-  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_amaze, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-  k_amaze<<<nblk, AMZ_THREADS, kSmemBytes, c->stream>>>(A);
+  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_amaze, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal));
+  k_amaze<<<nblk, AMZ_THREADS, kSmemTotal, c->stream>>>(A);
   count_launch(c);
   c->ws.rewind(mark);
   return check_launch(c, "demosaic_bayer_amaze");
