@@ -500,7 +500,7 @@ typedef struct lre_tuning {
   int lanes;         /* batch/server: concurrent per-image pipelines (streams) */
   int axial_strip;   /* guided-filter strip width (columns per CTA): 128 or 64 */
   int axial_rows;    /* guided-filter output rows per CTA: 128 or 64          */
-  int blur_tile;     /* defringe blur output tile edge: 32 or 64              */
+  int blur_tile;     /* defringe blur row chunks: 64 tall, 32 half as tall     */
 } lre_tuning;
 lre_status lre_set_tuning(lre_ctx* ctx, const lre_tuning* t);
 lre_status lre_get_tuning(const lre_ctx* ctx, lre_tuning* t);

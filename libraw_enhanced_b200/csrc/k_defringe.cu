@@ -15,8 +15,8 @@
 //   K5  line-linked support + solo seeds          -> lfs, srs, sbs
 //   K6  blur(srs), blur(sbs)                      -> srb, sbb
 //   K7  classification + correction (in-place safe)
-// Blurs stage a (T+2ks)^2 clamped halo tile in shared memory and run both
-// passes there; the line-link kernel stages a +-14 px clamped halo.
+// Blurs walk column strips (k_df_blur_strip); the line-link kernel stages a
+// +-14 px clamped halo.
 #include <algorithm>
 #include <cmath>
 
@@ -46,6 +46,7 @@ namespace {
 struct DfScalars {
   float max_guide_raw;  // max(0, G) over the image
   float max_edge;       // max Sobel magnitude (interior)
+  int nonfinite;        // a log ratio of the image is infinite or NaN
 };
 
 struct DfPlanes {
@@ -97,8 +98,11 @@ __global__ void __launch_bounds__(256) k_df_prep_tiled(const float* __restrict__
       const float* p = src + i * 3;
       float r = p[0], g = p[1], b = p[2];
       float gg = smax(g, 0.f);
-      lrg[i] = log_cr((smax(r, 0.f) + ratio_eps) / (gg + ratio_eps));
-      lbg[i] = log_cr((smax(b, 0.f) + ratio_eps) / (gg + ratio_eps));
+      const float lr = log_cr((smax(r, 0.f) + ratio_eps) / (gg + ratio_eps));
+      const float lb = log_cr((smax(b, 0.f) + ratio_eps) / (gg + ratio_eps));
+      lrg[i] = lr;
+      lbg[i] = lb;
+      if (!(isfinite(lr) && isfinite(lb))) sc->nonfinite = 1;
       float mag = 0.f;
       if (y >= 1 && y < limit_y && x >= 1 && x < limit_x) {
         const int cy = ty + 1, cx = tx + 1;
@@ -131,9 +135,21 @@ struct BlurJob {
   float* out[5];
   int mode[5];
   int np;
+  unsigned long long nz = 0x8000000080000000ull;  // {-0.f, -0.f} (f2_mul)
 };
 
 constexpr int BT = 32;  // output tile edge
+
+__device__ __forceinline__ void ld4(const float* p, float* o) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  o[0] = t.x;
+  o[1] = t.y;
+  o[2] = t.z;
+  o[3] = t.w;
+}
+__device__ __forceinline__ void st4(float* p, const float* o) {
+  *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+}
 
 // Element p of a small parameter array through constant indices only: a
 // run-time index into a kernel parameter would copy the whole parameter block
@@ -211,14 +227,7 @@ __global__ void __launch_bounds__(256) k_df_blur(BlurJob job, GaussTaps taps, in
   }
 }
 
-// Register-tiled blur for a compile-time tap radius KS and output tile edge
-// TB (32 or 64): planes are processed one after another through the same
-// shared memory (18 KB at TB = 32, so 8 CTAs fit on an SM; 50 KB at TB = 64,
-// with 1.7x instead of 2.6x halo reads), each thread produces 8 horizontal
-// or 4 vertical outputs from operands held in registers.  Tap order and
-// clamping are those of k_df_blur.
-// Two floats in one 64-bit register: a blur item carries the outputs of two
-// rows (horizontal pass) or two adjacent columns (vertical pass) together.
+// Two floats in one 64-bit register.
 __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -227,123 +236,201 @@ __device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
 __device__ __forceinline__ void f2_unpack(unsigned long long v, float& a, float& b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
-// acc + w * x per lane, the product and the sum each rounded to nearest
-// (the reference's order, no contraction): the two products as IEEE scalar
-// multiplies, the two sums as one packed add.rn.f32x2.  A packed multiply
-// feeding a packed add is not safe: ptxas contracts that pair into a fused
-// multiply-add (one rounding), which on the 51 MP workload flipped one
-// pixel's classification by 1.6e-3.  With scalar products between them
-// there is nothing to contract: a B200 probe of the 21-tap chain gave 0
-// differences from scalar multiply-then-add over 4.2 M outputs, and the
-// blurs need a quarter fewer FP instructions than in all-scalar form.
-__device__ __forceinline__ unsigned long long f2_madd(unsigned long long acc, unsigned long long w,
-                                                      unsigned long long x) {
-  float w0, w1, x0, x1;
-  f2_unpack(w, w0, w1);
-  f2_unpack(x, x0, x1);
-  const unsigned long long p = f2_pack(__fmul_rn(w0, x0), __fmul_rn(w1, x1));
+// The product of a tap per lane, rounded to nearest, and its sum: the
+// reference rounds every multiply and every add.  A packed multiply feeding a
+// packed add is not safe: ptxas contracts that pair into a fused multiply-add
+// (one rounding).  The product is therefore fma(w, x, nz) with nz = {-0, -0}
+// from a kernel parameter: adding -0 changes no product, not even a zero's
+// sign, the compiler cannot know the value, and a fused multiply-add followed
+// by an add has nothing left to contract.
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long w, unsigned long long x, unsigned long long nz) {
+  unsigned long long p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(w), "l"(x), "l"(nz));
+  return p;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
   unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(acc), "l"(p));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 
-// The two separable passes of one plane on the tile in shared memory.
-template <int KS, int TB>
-__device__ __forceinline__ void blur_passes(const float* s_in, float* s_h, const float (&w)[2 * KS + 1], float* out,
-                                            int x0, int y0, int W, int H) {
-  constexpr int E = TB + 2 * KS;
-  constexpr int LD = E + 1;
-  // horizontal: item = (halo rows 2jp, 2jp + 1; group of 8 output columns)
-  for (int item = threadIdx.x; item < (E / 2) * (TB / 8); item += blockDim.x) {
-    const int j = (item / (TB / 8)) * 2, k0 = (item % (TB / 8)) * 8;
-    unsigned long long x[8 + 2 * KS];
+// Separable blur of one plane for a compile-time tap radius KS, on strips of
+// 128 columns.  A thread owns two columns and walks down the strip in batches
+// of P = 2 KS + 1 rows:
+//   1. the next batch's rows are on their way to shared memory (cp.async)
+//      while this one is summed;
+//   2. the horizontal sums of the thread's two columns, packed, go to shared
+//      memory of the thread's own;
+//   3. the vertical sums: P accumulators in registers, one per output row in
+//      flight.  A new row is multiplied once by each of the KS + 1 distinct
+//      weights (the kernel is symmetric) and the products are added to the
+//      accumulators, each of which gets its taps in ascending order from 0,
+//      the reference's order.  Unrolled over P rows, the accumulators rotate
+//      by name.
+// What bounds it: the FP32 pipe.  A packed operation takes the pipe twice as
+// long as a scalar one, so it is the operations per output that count:
+// 4 KS + 2 horizontally and 3 KS + 2 vertically (74 at KS = 10) against 97 in
+// 64 x 64 tiles, whose halo the horizontal pass ran too.  One plane of 51 MP
+// takes 217 us (tiles: 263 us); the pipe's time is 102 us, and register moves that
+// line up the odd taps' pairs, chunk overlap and dependent adds take the rest.
+constexpr int BS_X = 128;  // output columns per strip
+constexpr int BS_THREADS = BS_X / 2;
+
+template <int KS>
+struct BlurStrip {
+  static constexpr int P = 2 * KS + 1;              // accumulators, rows per batch
+  static constexpr int PAD = (KS + 3) & ~3;         // staged columns left and right of the strip
+  static constexpr int C = BS_X + 2 * PAD;
+  static constexpr int IN = (P + 1) * C;            // floats of one staged batch (one row more is read)
+  static constexpr size_t SMEM = (size_t)(2 * IN + (P + 1) * BS_X) * sizeof(float);
+};
+
+__device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (bytes == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+template <int KS>
+__global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, GaussTaps taps, int W, int H, int batches,
+                                                              const DfScalars* sc) {
+  using B = BlurStrip<KS>;
+  constexpr int P = B::P, C = B::C, PAD = B::PAD;
+  extern __shared__ __align__(16) float sm_strip[];
+  float* s_h = sm_strip + 2 * B::IN;  // [P + 1 rows][BS_X]
+  const int tid = threadIdx.x;
+  const float* __restrict__ in = pick5(job.in, blockIdx.z);
+  float* __restrict__ out = pick5(job.out, blockIdx.z);
+  const int mode = pick5(job.mode, blockIdx.z);
+  const unsigned long long nz = job.nz;
+  const int rows = batches * P - 2 * KS;  // output rows per strip chunk
+  const int x0 = blockIdx.x * BS_X, y0 = blockIdx.y * rows, y1 = min(y0 + rows, H);
+  const int x = x0 + 2 * tid;
+  unsigned long long w[KS + 1];  // distinct weights, outermost first
 #pragma unroll
-    for (int i = 0; i < 8 + 2 * KS; i++) x[i] = f2_pack(s_in[j * LD + k0 + i], s_in[(j + 1) * LD + k0 + i]);
-    unsigned long long acc[8];
+  for (int t = 0; t <= KS; t++) w[t] = f2_pack(taps.w[t], taps.w[t]);
+  const int step = mode == BS_GUIDE_LINEAR ? 3 : 1;  // the guide is read out of the RGB image
+  const float* src = in + (mode == BS_GUIDE_LINEAR ? 1 : 0);
+  // 16-byte copies where the plane's rows are aligned and the strip with its
+  // halo lies inside the image; else sample by sample with the column clamped
+  const bool wide = step == 1 && (W & 3) == 0 && x0 >= PAD && x0 + BS_X + PAD <= W;
+  auto stage = [&](int b) {
+    float* dst = sm_strip + (b & 1) * B::IN;
+    const int yb = y0 - KS + b * P;
+    if (wide) {
+      for (int i = tid; i < P * (C / 4); i += BS_THREADS) {
+        const int r = i / (C / 4), q = i - r * (C / 4);
+        cp_async(dst + r * C + 4 * q, src + (size_t)min(max(yb + r, 0), H - 1) * W + x0 - PAD + 4 * q, 16);
+      }
+    } else {
 #pragma unroll
-    for (int o = 0; o < 8; o++) acc[o] = 0ull;  // {+0.f, +0.f}
-#pragma unroll
-    for (int t = 0; t <= 2 * KS; t++) {
-      const unsigned long long wt = f2_pack(w[t], w[t]);
-#pragma unroll
-      for (int o = 0; o < 8; o++) acc[o] = f2_madd(acc[o], wt, x[o + t]);
-    }
-#pragma unroll
-    for (int o = 0; o < 8; o++) f2_unpack(acc[o], s_h[j * TB + k0 + o], s_h[(j + 1) * TB + k0 + o]);
-  }
-  __syncthreads();
-  // vertical: item = (output columns 2kp, 2kp + 1; group of 4 output rows)
-  for (int item = threadIdx.x; item < (TB / 2) * (TB / 4); item += blockDim.x) {
-    const int k = (item % (TB / 2)) * 2, j0 = (item / (TB / 2)) * 4;
-    unsigned long long x[4 + 2 * KS];
-#pragma unroll
-    for (int i = 0; i < 4 + 2 * KS; i++) x[i] = *reinterpret_cast<const unsigned long long*>(&s_h[(j0 + i) * TB + k]);
-    unsigned long long acc[4];
-#pragma unroll
-    for (int o = 0; o < 4; o++) acc[o] = 0ull;
-#pragma unroll
-    for (int t = 0; t <= 2 * KS; t++) {
-      const unsigned long long wt = f2_pack(w[t], w[t]);
-#pragma unroll
-      for (int o = 0; o < 4; o++) acc[o] = f2_madd(acc[o], wt, x[o + t]);
-    }
-    const int gx = x0 + k;
-#pragma unroll
-    for (int o = 0; o < 4; o++) {
-      float a, b;
-      f2_unpack(acc[o], a, b);
-      const int gy = y0 + j0 + o;
-      if (gy < H) {
-        if (gx < W) out[(size_t)gy * W + gx] = a;
-        if (gx + 1 < W) out[(size_t)gy * W + gx + 1] = b;
+      for (int k = 0; k < (C + BS_THREADS - 1) / BS_THREADS; k++) {
+        const int q = tid + k * BS_THREADS;
+        const int gx = min(max(x0 - PAD + q, 0), W - 1) * step;
+        if (q < C)
+          for (int r = 0; r < P; r++)
+            cp_async(dst + r * C + q, src + (size_t)min(max(yb + r, 0), H - 1) * W * step + gx, 4);
       }
     }
-  }
-  __syncthreads();
-}
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const float inv = mode == BS_PLANE_EDGE_NORM ? 1.f / smax(sc->max_edge, 1e-6f) : 0.f;
+  const bool vec = (W & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
 
-template <int KS, int TB>
-__device__ __forceinline__ void blur_fast_body(const BlurJob& job, const GaussTaps& taps, int W, int H,
-                                               const DfScalars* sc) {
-  constexpr int E = TB + 2 * KS;
-  constexpr int LD = E + 1;  // odd row stride: conflict-light row reads
-  extern __shared__ __align__(16) float sm_fast[];
-  float* s_in = sm_fast;           // [E][LD]
-  float* s_h = sm_fast + E * LD;   // [E][TB]
-  const int x0 = blockIdx.x * TB, y0 = blockIdx.y * TB;
-  float w[2 * KS + 1];
+  unsigned long long acc[P];
 #pragma unroll
-  for (int t = 0; t <= 2 * KS; t++) w[t] = taps.w[t];
-  for (int p = 0; p < job.np; p++) {
-    const float* in = pick5(job.in, p);
-    const int mode = pick5(job.mode, p);
-    float* out = pick5(job.out, p);
-    for (int i = threadIdx.x; i < E * E; i += blockDim.x) {
-      const int r = i / E, q = i % E;
-      const int gy = min(max(y0 - KS + r, 0), H - 1);
-      const int gx = min(max(x0 - KS + q, 0), W - 1);
-      s_in[r * LD + q] = blur_src(in, mode, sc, gx, gy, W);
+  for (int j = 0; j < P; j++) acc[j] = 0ull;
+  stage(0);
+  for (int b = 0; b < batches; b++) {
+    const int yb = y0 - KS + b * P;  // image row of the batch's first row
+    if (yb - KS >= y1) break;
+    float* cur = sm_strip + (b & 1) * B::IN;
+    if (b + 1 < batches) {
+      stage(b + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    // Both passes run two outputs per item and accumulate every output's
-    // taps in the reference's order from 0.f, each product and each sum
-    // rounded to nearest (f2_madd).
-    blur_passes<KS, TB>(s_in, s_h, w, out, x0, y0, W, H);
+    if (mode != BS_PLANE) {
+      for (int i = tid; i < P * C; i += BS_THREADS) cur[i] = mode == BS_GUIDE_LINEAR ? smax(cur[i], 0.f) : cur[i] * inv;
+      __syncthreads();
+    }
+    // horizontal sums of rows j, j + 1 at columns 2 tid, 2 tid + 1 (row P, read
+    // with row P - 1, is not used)
+#pragma unroll 1
+    for (int j = 0; j < P; j += 2) {
+      unsigned long long h[2];
+      float e[2][P + 2];
+      constexpr int O = PAD - KS;  // the window starts O columns into the pair
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const float2* q = reinterpret_cast<const float2*>(cur + (j + k) * C + 2 * tid + (O & ~1));
+#pragma unroll
+        for (int i = 0; i < (P + 1 + (O & 1) + 1) / 2; i++) {
+          const float2 f = q[i];
+          if (2 * i - (O & 1) >= 0) e[k][2 * i - (O & 1)] = f.x;
+          if (2 * i + 1 - (O & 1) <= P) e[k][2 * i + 1 - (O & 1)] = f.y;
+        }
+        h[k] = 0ull;
+      }
+#pragma unroll
+      for (int t = 0; t < P; t++) {
+        const unsigned long long wt = w[t <= KS ? t : 2 * KS - t];
+#pragma unroll
+        for (int k = 0; k < 2; k++) h[k] = f2_add(h[k], f2_mul(wt, f2_pack(e[k][t], e[k][t + 1]), nz));
+      }
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        *reinterpret_cast<unsigned long long*>(&s_h[(j + k) * BS_X + 2 * tid]) = h[k];
+    }
+    // vertical sums (the thread reads only what it wrote)
+#pragma unroll
+    for (int s = 0; s < P; s++) {
+      const unsigned long long v = *reinterpret_cast<const unsigned long long*>(&s_h[s * BS_X + 2 * tid]);
+      unsigned long long m[KS + 1];
+#pragma unroll
+      for (int t = 0; t <= KS; t++) m[t] = f2_mul(w[t], v, nz);
+      // accumulator (s + j) % P belongs to the output row KS - j above this
+      // one and gets tap 2 KS - j; the last one starts here
+#pragma unroll
+      for (int j = 0; j < P; j++) {
+        const int t = 2 * KS - j;
+        unsigned long long& A = acc[(s + j) % P];
+        A = f2_add(j == 2 * KS ? 0ull : A, m[t <= KS ? t : 2 * KS - t]);
+      }
+      const int o = yb + s - KS;
+      if (o >= y0 && o < y1 && x < W) {
+        float a, c;
+        f2_unpack(acc[s], a, c);
+        float* d = out + (size_t)o * W + x;
+        if (vec) {
+          *reinterpret_cast<float2*>(d) = make_float2(a, c);
+        } else {
+          d[0] = a;
+          if (x + 1 < W) d[1] = c;
+        }
+      }
+    }
+    __syncthreads();  // every thread has read the batch before the next but one is staged over it
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <int KS, int TB>
-__global__ void __launch_bounds__(256) k_df_blur_fast(BlurJob job, GaussTaps taps, int W, int H, const DfScalars* sc) {
-  blur_fast_body<KS, TB>(job, taps, W, H, sc);
-}
-
-template <int TB>
-lre_status run_blur_fast(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc) {
-  constexpr int E = TB + 2 * 10;
-  const size_t smem = ((size_t)E * (E + 1) + (size_t)E * TB) * sizeof(float);
-  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_fast<10, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((W + TB - 1) / TB, (H + TB - 1) / TB);
-  k_df_blur_fast<10, TB><<<grid, 256, smem, c->stream>>>(job, taps, W, H, sc);
+template <int KS>
+lre_status run_blur_strip(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc) {
+  using B = BlurStrip<KS>;
+  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_strip<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::SMEM));
+  // Batches per chunk: a chunk's first 2 KS rows produce nothing, so tall
+  // chunks, halved while the grid has fewer than twelve CTAs per SM.
+  int batches = c->tune.blur_tile == 64 ? 32 : 16;
+  const int strips = (W + BS_X - 1) / BS_X;
+  auto chunks = [&](int n) { return (H + n * B::P - 2 * KS - 1) / (n * B::P - 2 * KS); };
+  while (batches > 2 && (long long)strips * chunks(batches) * job.np < 12LL * c->sm_count) batches /= 2;
+  const dim3 grid((unsigned)strips, (unsigned)chunks(batches), (unsigned)job.np);
+  k_df_blur_strip<KS><<<grid, BS_THREADS, B::SMEM, c->stream>>>(job, taps, W, H, batches, sc);
   count_launch(c);
   return check_launch(c, "defringe blur");
 }
@@ -396,45 +483,48 @@ __device__ __forceinline__ float support_at(const float* __restrict__ src, size_
   return c_edge * c_bright * c_hue * c_chroma * natural_guard * green_enable;
 }
 
-// Blur of the five first-stage planes with K3 fused after it: once a tile's
-// blurred planes are written, the same CTA computes the fringe-support seed
-// of the tile's pixels while those values are still in L2.
-template <int KS, int TB>
-__global__ void __launch_bounds__(256) k_df_blur_support(BlurJob job, GaussTaps taps, int W, int H,
-                                                         const DfScalars* sc, const float* __restrict__ src,
-                                                         DfPlanes P, DfConst k) {
-  blur_fast_body<KS, TB>(job, taps, W, H, sc);  // ends with a CTA barrier
+// K3 per pixel, four consecutive pixels per thread.  A pixel whose blurred
+// edge planes are at or below the lower smoothstep edges has an edge factor of
+// exactly 0 and so a seed of 0: where all four are such and every log ratio of
+// the image is finite (no factor is NaN), the other planes are not read.
+// At 51 MP 343 us; fused behind the blur of the five planes it had taken
+// about 880 us of that kernel's 2200.
+__global__ void __launch_bounds__(256) k_df_support(const float* __restrict__ src, size_t n, DfPlanes P, DfConst k,
+                                                    const DfScalars* sc) {
   const float sensitivity = sclamp(sqrtf(smax(k.strength, 1.0f)), 1.0f, 2.5f);
   const float inv_s = 1.0f / sensitivity;
   const bool enable_green = k.green != 0;
-  const int x0 = blockIdx.x * TB, y0 = blockIdx.y * TB;
-  for (int i = threadIdx.x; i < TB * TB; i += blockDim.x) {
-    const int gx = x0 + i % TB, gy = y0 + i / TB;
-    if (gx >= W || gy >= H) continue;
-    const size_t gi = (size_t)gy * W + gx;
-    P.fs[gi] = support_at(src, gi, P, k, inv_s, enable_green);
+  const float e0_edge = k.edge_thr * 0.35f * inv_s, e0_raw = 0.55f * inv_s;
+  const bool can_skip = sc->nonfinite == 0 && k.edge_thr > 0.f;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (n + 3) / 4; q += stride) {
+    const size_t i = q * 4;
+    float be[4], ber[4], fs[4];
+    if (i + 4 <= n) {
+      ld4(P.be + i, be);
+      ld4(P.ber + i, ber);
+    } else {
+      for (int t = 0; t < 4; t++) {
+        be[t] = i + t < n ? P.be[i + t] : 0.f;
+        ber[t] = i + t < n ? P.ber[i + t] : 0.f;
+      }
+    }
+    unsigned need = 0;
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      if (i + t < n && !(can_skip && (be[t] <= e0_edge || ber[t] <= e0_raw))) need |= 1u << t;
+#pragma unroll
+    for (int t = 0; t < 4; t++) fs[t] = 0.f;
+#pragma unroll
+    for (int t = 0; t < 4; t++)
+      if (need >> t & 1u) fs[t] = support_at(src, i + t, P, k, inv_s, enable_green);
+    if (i + 4 <= n) {
+      st4(P.fs + i, fs);
+    } else {
+      for (int t = 0; t < 4; t++)
+        if (i + t < n) P.fs[i + t] = fs[t];
+    }
   }
-}
-
-template <int TB>
-lre_status run_blur_support(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc,
-                            const float* src, const DfPlanes& P, const DfConst& k) {
-  constexpr int E = TB + 2 * 10;
-  const size_t smem = ((size_t)E * (E + 1) + (size_t)E * TB) * sizeof(float);
-  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_support<10, TB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((W + TB - 1) / TB, (H + TB - 1) / TB);
-  k_df_blur_support<10, TB><<<grid, 256, smem, c->stream>>>(job, taps, W, H, sc, src, P, k);
-  count_launch(c);
-  return check_launch(c, "defringe blur + support");
-}
-
-__global__ void k_df_support(const float* __restrict__ src, int W, int H, DfPlanes P, DfConst k) {
-  const float sensitivity = sclamp(sqrtf(smax(k.strength, 1.0f)), 1.0f, 2.5f);
-  const float inv_s = 1.0f / sensitivity;
-  const bool enable_green = k.green != 0;
-  size_t n = (size_t)W * H;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    P.fs[i] = support_at(src, i, P, k, inv_s, enable_green);
 }
 
 // ---------------------------------------------------------------- K5
@@ -853,17 +943,6 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
   }
 }
 
-__device__ __forceinline__ void ld4(const float* p, float* o) {
-  const float4 t = *reinterpret_cast<const float4*>(p);
-  o[0] = t.x;
-  o[1] = t.y;
-  o[2] = t.z;
-  o[3] = t.w;
-}
-__device__ __forceinline__ void st4(float* p, const float* o) {
-  *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
-}
-
 // Four consecutive pixels per thread and step, read and written as float4
 // (src/dst 16-byte aligned; the planes are 256-byte aligned), so every load
 // of a step is issued before the first use; the one-pixel loop was bound by
@@ -981,12 +1060,6 @@ __global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, fl
   }
 }
 
-__global__ void k_df_init(DfScalars* sc, const float* in_max_g, float* out_max_g) {
-  sc->max_guide_raw = in_max_g ? *in_max_g : 0.f;
-  sc->max_edge = 0.f;
-  if (out_max_g) *out_max_g = 0.f;
-}
-
 __global__ void k_df_maxg(const float* __restrict__ src, size_t n, DfScalars* sc) {
   float m = 0.f;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -995,9 +1068,25 @@ __global__ void k_df_maxg(const float* __restrict__ src, size_t n, DfScalars* sc
   if ((threadIdx.x & 31) == 0) atomic_max_float(&sc->max_guide_raw, m);
 }
 
+// Tap radii 3 to 15 run the strip kernel compiled for them, others the tile
+// kernel with the radius at run time (all eight planes of 26 MP at radius 7:
+// 2575 us in tiles, 792 us in strips).
+template <int KS>
+lre_status blur_for(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc, bool* done) {
+  if constexpr (KS >= 3) {
+    if (taps.ks == KS) {
+      *done = true;
+      return run_blur_strip<KS>(c, job, taps, W, H, sc);
+    }
+    return blur_for<KS - 1>(c, job, taps, W, H, sc, done);
+  }
+  return LRE_OK;
+}
+
 lre_status run_blur(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc) {
-  if (taps.ks == 10)  // radius 10 (the reference default): sigma 10/3, 21 taps
-    return c->tune.blur_tile == 64 ? run_blur_fast<64>(c, job, taps, W, H, sc) : run_blur_fast<32>(c, job, taps, W, H, sc);
+  bool done = false;
+  LRE_TRY(blur_for<15>(c, job, taps, W, H, sc, &done));
+  if (done) return LRE_OK;
   const int E = BT + 2 * taps.ks;
   size_t smem = ((size_t)job.np * E * E + (size_t)job.np * E * BT) * sizeof(float);
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1036,10 +1125,11 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   if (!sc) return fail(c, LRE_ERR_OUT_OF_MEMORY, "defringe: workspace too small");
   DfConst k{edge_thr, chroma_thr, strength, green_scale, green ? 1 : 0};
   const size_t n = w * h;
-  const unsigned gstream = grid_for(n, 256, c->sm_count * 8);
 
-  k_df_init<<<1, 1, 0, c->stream>>>(sc, in_max_g, out_max_g);
-  count_launch(c);
+  LRE_CUDA_TRY(c, cudaMemsetAsync(sc, 0, sizeof(DfScalars), c->stream));
+  if (out_max_g) LRE_CUDA_TRY(c, cudaMemsetAsync(out_max_g, 0, sizeof(float), c->stream));
+  if (in_max_g)
+    LRE_CUDA_TRY(c, cudaMemcpyAsync(&sc->max_guide_raw, in_max_g, sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
   if (!in_max_g) {
     k_df_maxg<<<grid_for(n, 256, c->sm_count * 4), 256, 0, c->stream>>>(in, n, sc);
     count_launch(c);
@@ -1057,15 +1147,10 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   j1.in[2] = P.lbg; j1.mode[2] = BS_PLANE;           j1.out[2] = P.blbg;
   j1.in[3] = P.er;  j1.mode[3] = BS_PLANE_EDGE_NORM; j1.out[3] = P.be;
   j1.in[4] = P.er;  j1.mode[4] = BS_PLANE;           j1.out[4] = P.ber;
-  if (taps.ks == 10) {  // radius 10: the register-tiled blur with K3 fused
-    LRE_TRY(c->tune.blur_tile == 64 ? run_blur_support<64>(c, j1, taps, W, H, sc, in, P, k)
-                                    : run_blur_support<32>(c, j1, taps, W, H, sc, in, P, k));
-  } else {
-    LRE_TRY(run_blur(c, j1, taps, W, H, sc));
-    k_df_support<<<gstream, 256, 0, c->stream>>>(in, W, H, P, k);
-    count_launch(c);
-    LRE_TRY(check_launch(c, "defringe support"));
-  }
+  LRE_TRY(run_blur(c, j1, taps, W, H, sc));
+  k_df_support<<<grid_for((n + 3) / 4, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, n, P, k, sc);
+  count_launch(c);
+  LRE_TRY(check_launch(c, "defringe support"));
 
   BlurJob j2{};
   j2.np = 1;

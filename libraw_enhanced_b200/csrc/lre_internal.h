@@ -57,7 +57,7 @@ struct WsPlan {
 struct Tuning {
   int axial_strip = 128;    // guided-filter strip width (columns per CTA): 128 or 64
   int axial_rows = 128;     // guided-filter output rows per CTA: 128 or 64
-  int blur_tile = 64;       // defringe register-tiled blur output tile edge: 64 or 32
+  int blur_tile = 64;       // defringe blur strips: 64 for tall row chunks, 32 for half as tall
 };
 
 struct Context {

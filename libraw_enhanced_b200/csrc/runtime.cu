@@ -388,7 +388,7 @@ lre_status autotune(Batch* b, const lre_image* im, size_t n, bool host_mode) {
       }
     }
   }
-  // defringe blur tile
+  // defringe blur chunk height
   if (st == LRE_OK) {
     float best_ms = 1e30f;
     for (int t : {32, 64}) {
