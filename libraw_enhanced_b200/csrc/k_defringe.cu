@@ -441,9 +441,55 @@ struct DfConst {
   int green;
 };
 
+// smoothstep with edges that are the same for every pixel.  The quotient
+// (x - e0) / d is formed from the reciprocal y = RN(1 / d), known before the
+// launch, by Markstein's scheme (IBM J. Res. Dev. 34, 1990): a product, then
+// two corrections by the exact residual, the last of which rounds the true
+// quotient: with y correctly rounded and q within an ulp, RN(q + r y) is the
+// correctly rounded quotient.  The numerator is clamped to [0, d] first, which
+// gives the same t as clamping the quotient to [0, 1] (NaN stays NaN), so
+// nothing overflows, and x - e0 is 0 or at least half an ulp of e0, so no
+// residual underflows.  12 instructions against about 22 with an IEEE
+// division.  FAST needs d and e0 in [2^-60, 2^60]; otherwise (a zero or
+// negative threshold) the division itself runs.
+struct DfEdge {
+  float e0, e1, d, y;
+};
+template <bool FAST>
+__device__ __forceinline__ float ss(const DfEdge& E, float x) {
+  if (!FAST) return ssmooth(E.e0, E.e1, x);
+  float n = x - E.e0;
+  asm("max.NaN.f32 %0, %0, 0f00000000;" : "+f"(n));
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(n) : "f"(E.d));
+  float q = n * E.y;
+  q = __fmaf_rn(__fmaf_rn(-E.d, q, n), E.y, q);
+  q = __fmaf_rn(__fmaf_rn(-E.d, q, n), E.y, q);
+  return q * q * (3.0f - 2.0f * q);
+}
+// Edges written as literals: the compiler folds d and y.
+__device__ __forceinline__ float ssl(float e0, float e1, float x) {
+  const float d = e1 - e0;
+  return ss<true>(DfEdge{e0, e1, d, 1.0f / d}, x);
+}
+
+// The edges that depend on the call's parameters, in the reference's
+// expressions (factor * threshold * inv_s), formed on the host.
+enum DfEdgeId : int {
+  DE_CORE, DE_CORE_RAW, DE_LOW, DE_LOW_RAW, DE_BRIGHT, DE_CHROMA, DE_HUE, DE_RP_HUE, DE_ABS, DE_LOWC, DE_SOFT, DE_GATE,
+  DE_PEAK, DE_HALO, DE_SOLO, DE_SEED_SOLO, DE_N
+};
+struct DfTab {
+  DfEdge e[DE_N];
+  float inv_s, mask_cutoff;
+  float soften;      // 1 - 0.86 smoothstep(0.22, 0.40, chroma_thr)
+  float solo_enable; // smoothstep(1.25, 3, strength)
+  float release, surface;  // smoothstep(2, 6, strength), smoothstep(3, 8, strength)
+};
+
 // Fringe-support seed of pixel i (core/cpu_accelerator.cpp:4158-4205).
-__device__ __forceinline__ float support_at(const float* __restrict__ src, size_t i, const DfPlanes& P, const DfConst& k,
-                                            float inv_s, bool enable_green) {
+template <bool FAST>
+__device__ __forceinline__ float support_at(const float* __restrict__ src, size_t i, const DfPlanes& P, const DfTab& T,
+                                            bool enable_green) {
   const float rg = P.lrg[i];
   const float bgr = P.lbg[i];
   const float dr = rg - P.blrg[i];
@@ -456,29 +502,29 @@ __device__ __forceinline__ float support_at(const float* __restrict__ src, size_
   const float purple_excess = smin(smax(0.f, dr), smax(0.f, db));
   const float denom_support = smax(blur_guide, 0.05f);
   const float g_over_min_support = smax(0.f, g0 - smin(r0, b0)) / denom_support;
-  const float green_dom_support = ssmooth(0.010f, 0.060f, g_over_min_support);
+  const float green_dom_support = ssl(0.010f, 0.060f, g_over_min_support);
   const float green_excess = smax(smax(0.f, -dr), smax(0.f, -db)) * green_dom_support;
   const bool is_purple = purple_excess >= green_excess;
   const float excess_support = is_purple ? purple_excess : green_excess;
   const float min_dir = is_purple ? smax(0.f, smin(rg, bgr)) : smax(0.f, smin(-rg, -bgr));
   const float max_dir = is_purple ? smax(1e-4f, smax(rg, bgr)) : smax(1e-4f, smax(-rg, -bgr));
   const float balance = min_dir / max_dir;
-  const float c_edge = ssmooth(k.edge_thr * 0.35f * inv_s, k.edge_thr * 1.50f * inv_s, P.be[i]) *
-                       ssmooth(0.55f * inv_s, 1.35f * inv_s, P.ber[i]);
-  const float c_bright = ssmooth(0.24f * inv_s, 0.52f * inv_s, blur_guide);
-  const float c_chroma = ssmooth(k.chroma_thr * 0.45f * inv_s, k.chroma_thr * 1.60f * inv_s, excess_support);
+  const float c_edge = ss<FAST>(T.e[DE_CORE], P.be[i]) *
+                       ss<FAST>(T.e[DE_CORE_RAW], P.ber[i]);
+  const float c_bright = ss<FAST>(T.e[DE_BRIGHT], blur_guide);
+  const float c_chroma = ss<FAST>(T.e[DE_CHROMA], excess_support);
   const float red_strength = smax(0.f, r0 - smax(g0, b0)) / smax(r0, 1e-4f);
   const float red_blue_balance = b0 / smax(r0, 1e-4f);
   const float blue_lift = smax(0.f, b0 - g0) / smax(r0 - g0, 1e-4f);
-  const float red_purple = smax(ssmooth(0.55f, 0.78f, red_blue_balance), ssmooth(0.16f, 0.34f, blue_lift));
-  const float red_purple_hue_signal = ssmooth(0.50f, 0.72f, red_blue_balance) * ssmooth(0.24f, 0.42f, blue_lift);
-  const float balanced_hue = ssmooth(0.06f * inv_s, 0.22f * inv_s, min_dir) * ssmooth(0.35f, 0.75f, balance);
+  const float red_purple = smax(ssl(0.55f, 0.78f, red_blue_balance), ssl(0.16f, 0.34f, blue_lift));
+  const float red_purple_hue_signal = ssl(0.50f, 0.72f, red_blue_balance) * ssl(0.24f, 0.42f, blue_lift);
+  const float balanced_hue = ss<FAST>(T.e[DE_HUE], min_dir) * ssl(0.35f, 0.75f, balance);
   const float red_purple_hue = is_purple ? smin(1.f, red_purple_hue_signal * 1.50f) *
-                                               ssmooth(0.035f * inv_s, 0.16f * inv_s, min_dir) *
-                                               ssmooth(0.18f, 0.58f, balance)
+                                               ss<FAST>(T.e[DE_RP_HUE], min_dir) *
+                                               ssl(0.18f, 0.58f, balance)
                                          : 0.f;
   const float c_hue = smax(balanced_hue, red_purple_hue);
-  const float natural_guard = 1.f - ssmooth(0.08f, 0.25f, red_strength) * (1.f - red_purple);
+  const float natural_guard = 1.f - ssl(0.08f, 0.25f, red_strength) * (1.f - red_purple);
   const float green_enable = (enable_green || is_purple) ? 1.f : 0.f;
   return c_edge * c_bright * c_hue * c_chroma * natural_guard * green_enable;
 }
@@ -489,12 +535,11 @@ __device__ __forceinline__ float support_at(const float* __restrict__ src, size_
 // the image is finite (no factor is NaN), the other planes are not read.
 // At 51 MP 343 us; fused behind the blur of the five planes it had taken
 // about 880 us of that kernel's 2200.
+template <bool FAST>
 __global__ void __launch_bounds__(256) k_df_support(const float* __restrict__ src, size_t n, DfPlanes P, DfConst k,
-                                                    const DfScalars* sc) {
-  const float sensitivity = sclamp(sqrtf(smax(k.strength, 1.0f)), 1.0f, 2.5f);
-  const float inv_s = 1.0f / sensitivity;
+                                                    DfTab T, const DfScalars* sc) {
   const bool enable_green = k.green != 0;
-  const float e0_edge = k.edge_thr * 0.35f * inv_s, e0_raw = 0.55f * inv_s;
+  const float e0_edge = T.e[DE_CORE].e0, e0_raw = T.e[DE_CORE_RAW].e0;
   const bool can_skip = sc->nonfinite == 0 && k.edge_thr > 0.f;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (n + 3) / 4; q += stride) {
@@ -517,7 +562,7 @@ __global__ void __launch_bounds__(256) k_df_support(const float* __restrict__ sr
     for (int t = 0; t < 4; t++) fs[t] = 0.f;
 #pragma unroll
     for (int t = 0; t < 4; t++)
-      if (need >> t & 1u) fs[t] = support_at(src, i + t, P, k, inv_s, enable_green);
+      if (need >> t & 1u) fs[t] = support_at<FAST>(src, i + t, P, T, enable_green);
     if (i + 4 <= n) {
       st4(P.fs + i, fs);
     } else {
@@ -558,7 +603,8 @@ __device__ __forceinline__ void line_dir(const float* s_ls, const float* s_fs, i
   best = smax(best, along * thin);
 }
 
-__global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfConst k) {
+template <bool FAST>
+__global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfTab T) {
   __shared__ float s_ls[LE * LE];
   __shared__ float s_fs[LE * LE];
   __shared__ int s_any;
@@ -581,8 +627,6 @@ __global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, 
   // a tile whose line sources are all zero has every `along` zero, so every
   // line-linked support value is exactly 0
   const bool tile_active = s_any != 0;
-  const float sensitivity = sclamp(sqrtf(smax(k.strength, 1.0f)), 1.0f, 2.5f);
-  const float inv_s = 1.0f / sensitivity;
   for (int i = threadIdx.x; i < LT * LT; i += blockDim.x) {
     int ly = i / LT, lx = i % LT;
     int y = y0 + ly, x = x0 + lx;
@@ -617,20 +661,20 @@ __global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, 
     const float target_b = g * exp_cr(blbg);
     const float solo_r = smax(0.f, s0 - target_r) / smax(blur_guide, 0.05f);
     const float solo_b = smax(0.f, s2 - target_b) / smax(blur_guide, 0.05f);
-    const float linked_fringe = ssmooth(0.004f, 0.045f, smax(bfs, best * 0.90f));
-    const float c_edge_solo = ssmooth(k.edge_thr * 0.35f * inv_s, k.edge_thr * 1.50f * inv_s, be) *
-                              ssmooth(0.55f * inv_s, 1.35f * inv_s, ber);
-    const float c_bright_solo = ssmooth(0.24f * inv_s, 0.52f * inv_s, blur_guide);
-    const float solo_enable = ssmooth(1.25f, 3.0f, k.strength);
+    const float linked_fringe = ssl(0.004f, 0.045f, smax(bfs, best * 0.90f));
+    const float c_edge_solo = ss<FAST>(T.e[DE_CORE], be) *
+                              ss<FAST>(T.e[DE_CORE_RAW], ber);
+    const float c_bright_solo = ss<FAST>(T.e[DE_BRIGHT], blur_guide);
+    const float solo_enable = T.solo_enable;
     const float r0 = smax(s0, 0.f);
     const float g0 = smax(s1, 0.f);
     const float b0 = smax(s2, 0.f);
     const float red_strength_solo = smax(0.f, r0 - smax(g0, b0)) / smax(r0, 1e-4f);
-    const float solo_red_guard = 1.f - 0.90f * ssmooth(0.12f, 0.32f, red_strength_solo);
+    const float solo_red_guard = 1.f - 0.90f * ssl(0.12f, 0.32f, red_strength_solo);
     P.srs[gi] = solo_enable * c_edge_solo * c_bright_solo * linked_fringe * solo_red_guard *
-                ssmooth(k.chroma_thr * 0.22f * inv_s, k.chroma_thr * 0.95f * inv_s, solo_r);
+                ss<FAST>(T.e[DE_SEED_SOLO], solo_r);
     P.sbs[gi] = solo_enable * c_edge_solo * c_bright_solo *
-                ssmooth(k.chroma_thr * 0.22f * inv_s, k.chroma_thr * 0.95f * inv_s, solo_b);
+                ss<FAST>(T.e[DE_SEED_SOLO], solo_b);
   }
 }
 
@@ -638,7 +682,7 @@ __global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, 
 // Constants of the main pass (core/cpu_accelerator.cpp:4376-4706), formed
 // once per thread.
 struct DfMainK {
-  float inv_s, mask_cutoff, scene_highlight_gate, edge_threshold, chroma_threshold, strength, green_strength_scale;
+  float mask_cutoff, scene_highlight_gate, strength, green_strength_scale;
   float e0_edge, e0_raw;
   bool enable_green, can_skip;
 };
@@ -659,13 +703,13 @@ __device__ __forceinline__ bool df_keeps_input(const DfMainK& K, float be, float
 }
 
 // The correction of one pixel (s0, s1, s2) -> (d0, d1, d2).
-__device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const DfPx& v, const DfMainK& K, float& d0,
+template <bool FAST>
+__device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const DfPx& v, const DfMainK& K, const DfTab& T, float& d0,
                                            float& d1, float& d2) {
-  const float inv_s = K.inv_s;
   const float mask_cutoff = K.mask_cutoff;
   const float scene_highlight_gate = K.scene_highlight_gate;
   const bool enable_green = K.enable_green;
-  const float edge_threshold = K.edge_threshold, chroma_threshold = K.chroma_threshold, strength = K.strength;
+  const float strength = K.strength;
   const float green_strength_scale = K.green_strength_scale;
   d0 = s0;
   d1 = s1;
@@ -691,30 +735,30 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
   const float purple_excess = smin(purple_r, purple_b);
   const float denom = smax(blur_guide, 0.05f);
   const float g_over_min = smax(0.f, g0 - smin(r0, b0)) / denom;
-  const float green_dom = ssmooth(0.010f, 0.060f, g_over_min);
+  const float green_dom = ssl(0.010f, 0.060f, g_over_min);
   const float green_excess = smax(green_r, green_b) * green_dom;
   const bool is_purple = purple_excess >= green_excess;
   const float excess = is_purple ? purple_excess : green_excess;
   const float min_dir = is_purple ? smax(0.f, smin(rg, bg)) : smax(0.f, smin(-rg, -bg));
   const float max_dir = is_purple ? smax(1e-4f, smax(rg, bg)) : smax(1e-4f, smax(-rg, -bg));
   const float balance = min_dir / max_dir;
-  const float c_edge_core = ssmooth(edge_threshold * 0.35f * inv_s, edge_threshold * 1.50f * inv_s, v.be) *
-                            ssmooth(0.55f * inv_s, 1.35f * inv_s, v.ber);
-  const float c_edge_low = ssmooth(edge_threshold * 0.10f * inv_s, edge_threshold * 0.80f * inv_s, v.be) *
-                           ssmooth(0.20f * inv_s, 0.90f * inv_s, v.ber);
-  const float linked_fringe = ssmooth(0.004f, 0.045f, smax(blur_fringe_support, line_support * 0.90f));
-  const float c_bright = ssmooth(0.24f * inv_s, 0.52f * inv_s, blur_guide);
-  const float c_chroma = ssmooth(chroma_threshold * 0.45f * inv_s, chroma_threshold * 1.60f * inv_s, excess);
+  const float c_edge_core = ss<FAST>(T.e[DE_CORE], v.be) *
+                            ss<FAST>(T.e[DE_CORE_RAW], v.ber);
+  const float c_edge_low = ss<FAST>(T.e[DE_LOW], v.be) *
+                           ss<FAST>(T.e[DE_LOW_RAW], v.ber);
+  const float linked_fringe = ssl(0.004f, 0.045f, smax(blur_fringe_support, line_support * 0.90f));
+  const float c_bright = ss<FAST>(T.e[DE_BRIGHT], blur_guide);
+  const float c_chroma = ss<FAST>(T.e[DE_CHROMA], excess);
   const float red_blue_balance_hue = b0 / smax(r0, 1e-4f);
   const float blue_lift_hue = smax(0.f, b0 - g0) / smax(r0 - g0, 1e-4f);
-  const float red_purple_hue_signal = ssmooth(0.50f, 0.72f, red_blue_balance_hue) * ssmooth(0.24f, 0.42f, blue_lift_hue);
-  const float balanced_hue = ssmooth(0.06f * inv_s, 0.22f * inv_s, min_dir) * ssmooth(0.35f, 0.75f, balance);
+  const float red_purple_hue_signal = ssl(0.50f, 0.72f, red_blue_balance_hue) * ssl(0.24f, 0.42f, blue_lift_hue);
+  const float balanced_hue = ss<FAST>(T.e[DE_HUE], min_dir) * ssl(0.35f, 0.75f, balance);
   const float red_purple_hue_gate = is_purple ? smin(1.f, red_purple_hue_signal * 1.50f) *
-                                                    ssmooth(0.035f * inv_s, 0.16f * inv_s, min_dir) *
-                                                    ssmooth(0.18f, 0.58f, balance)
+                                                    ss<FAST>(T.e[DE_RP_HUE], min_dir) *
+                                                    ssl(0.18f, 0.58f, balance)
                                               : 0.f;
   const float green_unbalanced_hue =
-      (enable_green && !is_purple) ? ssmooth(0.035f * inv_s, 0.16f * inv_s, max_dir) : 0.f;
+      (enable_green && !is_purple) ? ss<FAST>(T.e[DE_RP_HUE], max_dir) : 0.f;
   const float c_hue = smax(balanced_hue, smax(red_purple_hue_gate, green_unbalanced_hue));
   const float rb_avg = rb_avg_pre;
   const float purple_abs = smin(smax(0.f, r0 - g0), smax(0.f, b0 - g0)) / smax(blur_guide, 0.05f);
@@ -723,11 +767,11 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
   const float green_abs = smax(green_abs_base, 0.55f * green_abs_alt);
   const bool abs_is_purple = purple_abs >= green_abs;
   const float abs_excess = abs_is_purple ? purple_abs : green_abs;
-  const float c_abs = ssmooth(chroma_threshold * 0.35f * inv_s, chroma_threshold * 1.20f * inv_s, abs_excess);
+  const float c_abs = ss<FAST>(T.e[DE_ABS], abs_excess);
   const float low_contrast_color =
-      ssmooth(chroma_threshold * 1.20f * inv_s, chroma_threshold * 2.40f * inv_s, abs_excess);
+      ss<FAST>(T.e[DE_LOWC], abs_excess);
   const float green_soft_edge_boost =
-      (enable_green && !is_purple) ? c_edge_low * ssmooth(0.05f * inv_s, 0.20f * inv_s, max_dir) : 0.f;
+      (enable_green && !is_purple) ? c_edge_low * ss<FAST>(T.e[DE_SOFT], max_dir) : 0.f;
   const float c_edge = smax(c_edge_core, smax(c_edge_low * linked_fringe * 1.45f,
                                               smax(c_edge_low * low_contrast_color * 0.35f, green_soft_edge_boost)));
   const float ratio_mask = c_edge * c_bright * c_hue * c_chroma;
@@ -737,39 +781,39 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
   const bool correct_purple = use_direct ? abs_is_purple : is_purple;
   float local_gate = 0.f;
   if (correct_purple) {
-    local_gate = ssmooth(chroma_threshold * 0.10f * inv_s, chroma_threshold * 0.55f * inv_s, purple_abs);
+    local_gate = ss<FAST>(T.e[DE_GATE], purple_abs);
     mask *= local_gate;
   } else {
-    local_gate = ssmooth(chroma_threshold * 0.10f * inv_s, chroma_threshold * 0.55f * inv_s, green_abs);
+    local_gate = ss<FAST>(T.e[DE_GATE], green_abs);
     if (enable_green) {
       const float peak_chroma_signal =
-          ssmooth(chroma_threshold * 0.80f * inv_s, chroma_threshold * 2.50f * inv_s, green_abs);
-      const float peak_neighbourhood = ssmooth(0.005f, 0.030f, blur_fringe_support);
+          ss<FAST>(T.e[DE_PEAK], green_abs);
+      const float peak_neighbourhood = ssl(0.005f, 0.030f, blur_fringe_support);
       const float green_peak_mask = peak_chroma_signal * peak_neighbourhood * c_bright * c_hue;
       mask = smax(mask, green_peak_mask * scene_highlight_gate);
     }
-    const float green_highlight_protect = 1.f - 0.85f * ssmooth(0.62f, 0.88f, blur_guide);
+    const float green_highlight_protect = 1.f - 0.85f * ssl(0.62f, 0.88f, blur_guide);
     const float rb_to_green = rb_avg / smax(g0, 1e-4f);
-    const float natural_green_highlight = ssmooth(0.22f, 0.46f, rb_to_green) * ssmooth(0.30f, 0.55f, g0);
+    const float natural_green_highlight = ssl(0.22f, 0.46f, rb_to_green) * ssl(0.30f, 0.55f, g0);
     const float natural_green_suppress = 1.f - 0.99f * natural_green_highlight;
     const float natural_green_suppress_sq = natural_green_suppress * natural_green_suppress;
     const float green_halo_strength =
-        ssmooth(chroma_threshold * 0.55f * inv_s, chroma_threshold * 1.65f * inv_s, green_abs);
+        ss<FAST>(T.e[DE_HALO], green_abs);
     const float green_gain_base = enable_green ? 0.60f : 0.35f;
     const float green_gain_slope = enable_green ? 1.10f : 0.95f;
     const float green_gain = green_gain_base + green_gain_slope * green_halo_strength;
     const float min_ratio_ref = smin(blur_log_rg, blur_log_bg);
-    const float green_neighbour = ssmooth(0.02f, 0.10f, smax(0.f, -min_ratio_ref));
+    const float green_neighbour = ssl(0.02f, 0.10f, smax(0.f, -min_ratio_ref));
     const float src_max = smax(r0, smax(g0, b0));
     const float src_min = smin(r0, smin(g0, b0));
     const float src_chroma = src_max - src_min;
     const float src_sat = src_chroma / smax(src_max, 1e-4f);
-    const float whiteish = 1.f - ssmooth(0.05f, 0.13f, src_sat);
+    const float whiteish = 1.f - ssl(0.05f, 0.13f, src_sat);
     const float foliage_guard =
-        green_neighbour * whiteish * ssmooth(0.35f, 0.75f, blur_guide) * (1.f - green_halo_strength);
-    const float strength_release = enable_green ? ssmooth(2.0f, 6.0f, strength) : 0.f;
-    const float green_line_evidence = ssmooth(0.004f, 0.030f, line_support) *
-                                      ssmooth(0.20f, 0.55f, green_halo_strength) * ssmooth(0.05f, 0.15f, src_sat);
+        green_neighbour * whiteish * ssl(0.35f, 0.75f, blur_guide) * (1.f - green_halo_strength);
+    const float strength_release = enable_green ? T.release : 0.f;
+    const float green_line_evidence = ssl(0.004f, 0.030f, line_support) *
+                                      ssl(0.20f, 0.55f, green_halo_strength) * ssl(0.05f, 0.15f, src_sat);
     const float not_natural_green = 1.f - natural_green_highlight;
     const float guard_release = strength_release * green_line_evidence * not_natural_green;
     const float released_highlight_protect = green_highlight_protect + (1.f - green_highlight_protect) * guard_release;
@@ -778,7 +822,7 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
     const float foliage_term = 1.f - 0.999f * foliage_guard;
     const float released_foliage_term = foliage_term + (1.f - foliage_term) * guard_release;
     mask *= local_gate * green_gain * released_highlight_protect * released_natural_suppress * released_foliage_term;
-    const float line_kill_evidence = ssmooth(0.04f, 0.15f, line_support);
+    const float line_kill_evidence = ssl(0.04f, 0.15f, line_support);
     const float natural_blob =
         sqrtf(smax(0.f, natural_green_highlight)) * (1.f - line_kill_evidence) * green_neighbour;
     mask *= 1.f - 0.999f * natural_blob;
@@ -791,10 +835,10 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
     const float red_strength = smax(0.f, r0 - smax(g0, b0)) / smax(r0, 1e-4f);
     const float red_blue_balance = b0 / smax(r0, 1e-4f);
     const float blue_lift = smax(0.f, b0 - g0) / smax(r0 - g0, 1e-4f);
-    const float red_purple_balance = ssmooth(0.55f, 0.78f, red_blue_balance);
-    const float red_purple_lift = ssmooth(0.16f, 0.34f, blue_lift);
+    const float red_purple_balance = ssl(0.55f, 0.78f, red_blue_balance);
+    const float red_purple_lift = ssl(0.16f, 0.34f, blue_lift);
     const float red_purple = smax(red_purple_balance, red_purple_lift);
-    const float red_strength_guard = ssmooth(0.08f, 0.25f, red_strength);
+    const float red_strength_guard = ssl(0.08f, 0.25f, red_strength);
     float red_purple_context = 0.f;
     float contextual_red_purple = 0.f;
     float red_magenta_surface = 0.f;
@@ -802,23 +846,23 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
       red_purple_context = linked_fringe;
       contextual_red_purple = red_purple * red_purple_context;
       if (red_purple_context < 0.20f && red_strength_guard < 0.50f && red_purple > 0.50f) {
-        red_magenta_surface = ssmooth(0.02f, 0.12f, purple_abs) * (1.f - red_purple_context);
+        red_magenta_surface = ssl(0.02f, 0.12f, purple_abs) * (1.f - red_purple_context);
       }
     }
     float neutral_gray_surface = 0.f;
     if (strength > 3.f && red_purple_context > 0.80f && line_support > 0.012f && red_strength_guard < 0.98f &&
         blue_lift > 1.10f && red_blue_balance > 0.82f && purple_abs > 0.015f) {
-      const float neutral_gray_edge = ssmooth(1.10f, 1.80f, blue_lift) * ssmooth(0.82f, 1.05f, red_blue_balance) *
+      const float neutral_gray_edge = ssl(1.10f, 1.80f, blue_lift) * ssl(0.82f, 1.05f, red_blue_balance) *
                                       (1.f - red_strength_guard);
-      neutral_gray_surface = neutral_gray_edge * ssmooth(0.015f, 0.08f, purple_abs) * ssmooth(3.f, 8.f, strength);
+      neutral_gray_surface = neutral_gray_edge * ssl(0.015f, 0.08f, purple_abs) * T.surface;
     }
     const float red_object_strength = smax(red_strength_guard, red_magenta_surface);
     const float natural_warm_guard_base = 1.f - red_object_strength * (1.f - contextual_red_purple);
     const float natural_warm_guard_sq =
         natural_warm_guard_base * natural_warm_guard_base * natural_warm_guard_base * natural_warm_guard_base;
     const float natural_warm_guard = natural_warm_guard_sq * natural_warm_guard_sq;
-    const float line_purple_relief = ssmooth(0.012f, 0.06f, line_support) * ssmooth(0.10f, 0.24f, blue_lift);
-    const float red_object_guard = ssmooth(0.55f, 0.90f, red_object_strength);
+    const float line_purple_relief = ssl(0.012f, 0.06f, line_support) * ssl(0.10f, 0.24f, blue_lift);
+    const float red_object_guard = ssl(0.55f, 0.90f, red_object_strength);
     const float linked_override = linked_fringe * 1.05f * (1.f - 0.85f * red_object_guard);
     const float line_override = line_purple_relief * (1.f - 0.85f * red_object_guard);
     const bool force_warm_guard = (red_object_guard > 0.75f) && (linked_fringe < 0.65f) && (line_purple_relief < 0.45f);
@@ -827,22 +871,22 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
                                                        : smax(natural_warm_guard, smax(linked_override, line_override)))
                                    : 1.f;
     const float red_without_support =
-        ssmooth(0.22f, 0.45f, red_strength) * (1.f - ssmooth(0.02f, 0.12f, blur_fringe_support));
+        ssl(0.22f, 0.45f, red_strength) * (1.f - ssl(0.02f, 0.12f, blur_fringe_support));
     const float protect = correct_purple ? red_without_support : 0.f;
     const float smooth_mask = ssmooth(mask_cutoff, mask_cutoff * 5.0f, mask);
-    const float threshold_soften = 1.f - 0.86f * ssmooth(0.22f, 0.40f, chroma_threshold);
+    const float threshold_soften = T.soften;
     const float src_max = smax(r0, smax(g0, b0));
     const float src_min = smin(r0, smin(g0, b0));
     const float src_chroma = src_max - src_min;
     const float src_sat = src_chroma / smax(src_max, 1e-4f);
-    const float neutral_guard_base = ssmooth(0.008f, 0.030f, src_sat);
-    const float neutral_guard = 1.f - (1.f - neutral_guard_base) * ssmooth(0.35f, 0.80f, red_object_strength);
+    const float neutral_guard_base = ssl(0.008f, 0.030f, src_sat);
+    const float neutral_guard = 1.f - (1.f - neutral_guard_base) * ssl(0.35f, 0.80f, red_object_strength);
     float amount = sclamp(smooth_mask * strength * 1.90f * (1.f - protect) * warm_protect * neutral_guard *
                               threshold_soften,
                           0.f, 1.f);
-    const float warm_edge_surface = ssmooth(0.006f, 0.035f, purple_abs) * ssmooth(0.25f, 0.65f, red_purple) *
-                                    ssmooth(0.15f, 0.65f, red_purple_context) * (1.f - 0.55f * red_strength_guard) *
-                                    ssmooth(3.f, 8.f, strength);
+    const float warm_edge_surface = ssl(0.006f, 0.035f, purple_abs) * ssl(0.25f, 0.65f, red_purple) *
+                                    ssl(0.15f, 0.65f, red_purple_context) * (1.f - 0.55f * red_strength_guard) *
+                                    T.surface;
     const float safe_surface = smax(neutral_gray_surface, warm_edge_surface);
     if (correct_purple && safe_surface > 1e-4f) {
       const float safe_amount_cap = 1.f - 0.99f * safe_surface;
@@ -909,7 +953,7 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
   }
 
   if (!skip_rest) {
-    const float solo_enable = ssmooth(1.25f, 3.0f, strength);
+    const float solo_enable = T.solo_enable;
     if (solo_enable > 0.f) {
       const float g = smax(s1, 0.f);
       const float target_r = g * exp_cr(blur_log_rg);
@@ -917,17 +961,17 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
       const float solo_r = smax(0.f, s0 - target_r) / smax(blur_guide, 0.05f);
       const float solo_b = smax(0.f, s2 - target_b) / smax(blur_guide, 0.05f);
       const float local_solo_r =
-          ssmooth(chroma_threshold * 0.12f * inv_s, chroma_threshold * 0.65f * inv_s, solo_r);
+          ss<FAST>(T.e[DE_SOLO], solo_r);
       const float local_solo_b =
-          ssmooth(chroma_threshold * 0.12f * inv_s, chroma_threshold * 0.65f * inv_s, solo_b);
+          ss<FAST>(T.e[DE_SOLO], solo_b);
       const float rr0 = smax(s0, 0.f);
       const float gg0 = g;
       const float bb0 = smax(s2, 0.f);
       const float g_over_min2 = smax(0.f, gg0 - smin(rr0, bb0)) / smax(blur_guide, 0.05f);
-      const float green_dom2 = ssmooth(0.010f, 0.060f, g_over_min2);
+      const float green_dom2 = ssl(0.010f, 0.060f, g_over_min2);
       const float denom_solo = smax(blur_guide, 0.05f);
       const float purpleish =
-          ssmooth(0.010f, 0.060f, smax(smax(0.f, rr0 - gg0), smax(0.f, bb0 - gg0)) / denom_solo);
+          ssl(0.010f, 0.060f, smax(smax(0.f, rr0 - gg0), smax(0.f, bb0 - gg0)) / denom_solo);
       const float solo_allow = 1.f - green_dom2 * (1.f - purpleish);
       const float solo_r_mask = v.srb * local_solo_r * solo_allow;
       const float solo_b_mask = v.sbb * local_solo_b * solo_allow;
@@ -953,23 +997,20 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
 constexpr int DFM_THREADS = 128;
 constexpr int DFM_VALS = 14;  // s0 s1 s2 be ber srb sbb bg blrg blbg bfs lfs lrg lbg
 
+template <bool FAST>
 __global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, float* dst, int W, int H, DfPlanes P,
-                                                           DfConst k, const DfScalars* sc, float* out_max_g) {
+                                                           DfConst k, DfTab T, const DfScalars* sc, float* out_max_g) {
   __shared__ float S[DFM_VALS * 4][DFM_THREADS];
   DfMainK K;
-  const float sensitivity = sclamp(sqrtf(smax(k.strength, 1.0f)), 1.0f, 2.5f);
-  K.inv_s = 1.0f / sensitivity;
-  K.mask_cutoff = 0.02f * K.inv_s;
+  K.mask_cutoff = T.mask_cutoff;
   const float max_guide = df_max_guide(sc);
   K.scene_highlight_gate = ssmooth(0.55f, 0.75f, max_guide);
   K.enable_green = k.green != 0;
-  K.edge_threshold = k.edge_thr;
-  K.chroma_threshold = k.chroma_thr;
   K.strength = k.strength;
   K.green_strength_scale = sclamp(k.green_scale, 0.f, 1.f);
-  K.e0_edge = K.edge_threshold * 0.10f * K.inv_s;
-  K.e0_raw = 0.20f * K.inv_s;
-  K.can_skip = !K.enable_green && K.edge_threshold > 0.f;  // smoothstep edges strictly ordered
+  K.e0_edge = T.e[DE_LOW].e0;
+  K.e0_raw = T.e[DE_LOW_RAW].e0;
+  K.can_skip = !K.enable_green && k.edge_thr > 0.f;  // smoothstep edges strictly ordered
   const size_t n = (size_t)W * H;
   const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
   const size_t n4 = vec ? n / 4 : 0;
@@ -1024,7 +1065,7 @@ __global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, fl
                    S[7 * 4 + t][tid],  S[8 * 4 + t][tid],  S[9 * 4 + t][tid],  S[10 * 4 + t][tid],
                    S[11 * 4 + t][tid], S[12 * 4 + t][tid], S[13 * 4 + t][tid]};
       float r0, r1, r2;
-      df_main_px(S[0 * 4 + t][tid], S[1 * 4 + t][tid], S[2 * 4 + t][tid], v, K, r0, r1, r2);
+      df_main_px<FAST>(S[0 * 4 + t][tid], S[1 * 4 + t][tid], S[2 * 4 + t][tid], v, K, T, r0, r1, r2);
       S[0 * 4 + t][tid] = r0;
       S[1 * 4 + t][tid] = r1;
       S[2 * 4 + t][tid] = r2;
@@ -1047,7 +1088,7 @@ __global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, fl
     if (!df_keeps_input(K, P.be[i], P.ber[i], P.srb[i], P.sbb[i])) {
       const DfPx v{P.be[i], P.ber[i], P.srb[i], P.sbb[i], P.bg[i],  P.blrg[i],
                    P.blbg[i], P.bfs[i], P.lfs[i], P.lrg[i], P.lbg[i]};
-      df_main_px(s0, s1, s2, v, K, d0, d1, d2);
+      df_main_px<FAST>(s0, s1, s2, v, K, T, d0, d1, d2);
     }
     dst[i * 3 + 0] = d0;
     dst[i * 3 + 1] = d1;
@@ -1096,6 +1137,50 @@ lre_status run_blur(Context* c, const BlurJob& job, const GaussTaps& taps, int W
   return check_launch(c, "defringe blur");
 }
 
+float host_ssmooth(float e0, float e1, float x) {
+  float t = (x - e0) / (e1 - e0);
+  t = t < 0.0f ? 0.0f : (1.0f < t ? 1.0f : t);
+  return t * t * (3.0f - 2.0f * t);
+}
+
+// The table of a call, and whether every edge is in the range of ss<true>.
+bool make_tab(const DfConst& k, DfTab* T) {
+  const float st = k.strength < 1.0f ? 1.0f : k.strength;
+  const float root = std::sqrt(st);
+  const float sensitivity = root < 1.0f ? 1.0f : (2.5f < root ? 2.5f : root);
+  const float i = 1.0f / sensitivity, e = k.edge_thr, c = k.chroma_thr;
+  T->inv_s = i;
+  T->mask_cutoff = 0.02f * i;
+  T->soften = 1.f - 0.86f * host_ssmooth(0.22f, 0.40f, c);
+  T->solo_enable = host_ssmooth(1.25f, 3.0f, k.strength);
+  T->release = host_ssmooth(2.0f, 6.0f, k.strength);
+  T->surface = host_ssmooth(3.f, 8.f, k.strength);
+  bool fast = true;
+  auto set = [&](int id, float e0, float e1) {
+    const float d = e1 - e0;
+    T->e[id] = DfEdge{e0, e1, d, 1.0f / d};
+    const float lo = 8.6e-19f, hi = 1.1e18f;  // 2^-60, 2^60
+    fast = fast && e0 >= lo && e0 <= hi && d >= lo && d <= hi;
+  };
+  set(DE_CORE, e * 0.35f * i, e * 1.50f * i);
+  set(DE_CORE_RAW, 0.55f * i, 1.35f * i);
+  set(DE_LOW, e * 0.10f * i, e * 0.80f * i);
+  set(DE_LOW_RAW, 0.20f * i, 0.90f * i);
+  set(DE_BRIGHT, 0.24f * i, 0.52f * i);
+  set(DE_CHROMA, c * 0.45f * i, c * 1.60f * i);
+  set(DE_HUE, 0.06f * i, 0.22f * i);
+  set(DE_RP_HUE, 0.035f * i, 0.16f * i);
+  set(DE_ABS, c * 0.35f * i, c * 1.20f * i);
+  set(DE_LOWC, c * 1.20f * i, c * 2.40f * i);
+  set(DE_SOFT, 0.05f * i, 0.20f * i);
+  set(DE_GATE, c * 0.10f * i, c * 0.55f * i);
+  set(DE_PEAK, c * 0.80f * i, c * 2.50f * i);
+  set(DE_HALO, c * 0.55f * i, c * 1.65f * i);
+  set(DE_SOLO, c * 0.12f * i, c * 0.65f * i);
+  set(DE_SEED_SOLO, c * 0.22f * i, c * 0.95f * i);
+  return fast;
+}
+
 }  // namespace
 
 size_t ws_bytes_defringe(size_t w, size_t h, float radius) {
@@ -1124,6 +1209,8 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   DfScalars* sc = reinterpret_cast<DfScalars*>(c->ws.take(sizeof(DfScalars)));
   if (!sc) return fail(c, LRE_ERR_OUT_OF_MEMORY, "defringe: workspace too small");
   DfConst k{edge_thr, chroma_thr, strength, green_scale, green ? 1 : 0};
+  DfTab T;
+  const bool fast = make_tab(k, &T);
   const size_t n = w * h;
 
   LRE_CUDA_TRY(c, cudaMemsetAsync(sc, 0, sizeof(DfScalars), c->stream));
@@ -1148,7 +1235,8 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   j1.in[3] = P.er;  j1.mode[3] = BS_PLANE_EDGE_NORM; j1.out[3] = P.be;
   j1.in[4] = P.er;  j1.mode[4] = BS_PLANE;           j1.out[4] = P.ber;
   LRE_TRY(run_blur(c, j1, taps, W, H, sc));
-  k_df_support<<<grid_for((n + 3) / 4, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, n, P, k, sc);
+  auto support = fast ? k_df_support<true> : k_df_support<false>;
+  support<<<grid_for((n + 3) / 4, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, n, P, k, T, sc);
   count_launch(c);
   LRE_TRY(check_launch(c, "defringe support"));
 
@@ -1158,7 +1246,8 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   LRE_TRY(run_blur(c, j2, taps, W, H, sc));
 
   dim3 lgrid((W + LT - 1) / LT, (H + LT - 1) / LT);
-  k_df_line<<<lgrid, 256, 0, c->stream>>>(in, W, H, P, k);
+  auto line = fast ? k_df_line<true> : k_df_line<false>;
+  line<<<lgrid, 256, 0, c->stream>>>(in, W, H, P, T);
   count_launch(c);
   LRE_TRY(check_launch(c, "defringe line"));
 
@@ -1168,8 +1257,9 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   j3.in[1] = P.sbs; j3.mode[1] = BS_PLANE; j3.out[1] = P.sbb;
   LRE_TRY(run_blur(c, j3, taps, W, H, sc));
 
-  k_df_main<<<grid_for((n + 3) / 4, DFM_THREADS, c->sm_count * 6), DFM_THREADS, 0, c->stream>>>(in, out, W, H, P, k,
-                                                                                                sc, out_max_g);
+  auto main_pass = fast ? k_df_main<true> : k_df_main<false>;
+  main_pass<<<grid_for((n + 3) / 4, DFM_THREADS, c->sm_count * 6), DFM_THREADS, 0, c->stream>>>(in, out, W, H, P, k, T,
+                                                                                               sc, out_max_g);
   count_launch(c);
   return check_launch(c, "defringe main");
 }
