@@ -250,8 +250,11 @@ lre_status develop_device(Context* c, const float* mosaic, void* out, size_t w, 
   const bool float_out = p.output_bits == 32;
   c->ws.reset();
   LRE_CUDA_TRY(c, c->ws.reserve(develop_ws_bytes(p, w, h), c->stream));
+  // The chain starts in rgb_a and changes buffers once where the axial filter
+  // runs: the caller's buffer is the one it ends in.
   float* rgb_a = float_out ? reinterpret_cast<float*>(out) : reinterpret_cast<float*>(c->ws.take(rgb_bytes));
   float* rgb_b = reinterpret_cast<float*>(c->ws.take(rgb_bytes));
+  if (p.axial_ca_correction) std::swap(rgb_a, rgb_b);
   if (!rgb_a || !rgb_b) return fail(c, LRE_ERR_OUT_OF_MEMORY, "develop: workspace too small");
   float* res = nullptr;
   LRE_TRY(run_chain(c, mosaic, rgb_a, rgb_b, w, h, p, &res));
