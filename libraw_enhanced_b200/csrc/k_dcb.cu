@@ -24,8 +24,7 @@
 // (Three of these are OpenMP row-parallel loops in the reference, so with
 // more than one thread rows at chunk boundaries depend on timing; the
 // sequential order is the defined result and the one computed here.)
-// k_gs_sweep (sweep.cuh) evaluates them in exactly that order with one warp
-// per 32-row band walking the columns on a skewed wavefront.
+// sweep.cuh evaluates them in exactly that order.
 //
 // Arithmetic is the reference's, operation for operation (--fmad=false); the
 // result is bit-identical to the reference run single-threaded.
@@ -57,19 +56,21 @@ __global__ void k_dcb_init(const float* __restrict__ raw, int cs, float* __restr
     float v[3] = {0.0f, 0.0f, 0.0f};
     v[f] = raw_at(raw, cs, g, r, c);
     if (r >= 1 && r < g.H - 1 && c >= 1 && c < g.W - 1) {
-      for (unsigned ch = 0; ch < 3; ch++) {
-        if (ch == f) continue;
-        float sum = 0.0f;
-        int count = 0;
-        for (int dr = -1; dr <= 1; dr++)
-          for (int dc = -1; dc <= 1; dc++) {
-            if (dr == 0 && dc == 0) continue;
-            if (g.fc(r + dr, c + dc) == ch) {
-              sum += raw_at(raw, cs, g, r + dr, c + dc);
-              count++;
-            }
-          }
-        if (count > 0) v[ch] = sum / count;
+      // the 2x2 layout fixes which neighbours have which colour (asking each of
+      // the eight took 252 us at 24 MP, this 152); sums in row-major order from 0
+      auto at = [&](int dr, int dc, unsigned ch) {
+        const size_t i = g.at(r + dr, c + dc);
+        return cs == 1 ? raw[i] : raw[i * 3 + ch];
+      };
+      if (f != 1) {
+        v[1] = (0.0f + at(-1, 0, 1) + at(0, -1, 1) + at(0, 1, 1) + at(1, 0, 1)) / 4;
+        v[2 - f] = (0.0f + at(-1, -1, 2 - f) + at(-1, 1, 2 - f) + at(1, -1, 2 - f) + at(1, 1, 2 - f)) / 4;
+      } else {
+        const unsigned h = g.fc(r, c + 1);
+        const float hv = (0.0f + at(0, -1, h) + at(0, 1, h)) / 2;
+        const float vv = (0.0f + at(-1, 0, 2 - h) + at(1, 0, 2 - h)) / 2;
+        v[0] = h == 0 ? hv : vv;
+        v[2] = h == 0 ? vv : hv;
       }
     }
     const size_t i = g.at(r, c);
@@ -353,13 +354,24 @@ __global__ void k_dcb_chroma_g(const float* __restrict__ C0, const float* __rest
   }
 }
 
+// Planes to interleaved, four pixels per thread as float4 where the image is
+// aligned (the planes are): 24 MP 229 -> 129 us.
 __global__ void k_dcb_output(const float* __restrict__ R, const float* __restrict__ G, const float* __restrict__ B,
-                             float* __restrict__ rgb, Geo g) {
-  GS_FOR_PIXELS(g) {
-    const size_t i = g.at(r, c);
-    rgb[i * 3 + 0] = R[i] / g.maxv;
-    rgb[i * 3 + 1] = G[i] / g.maxv;
-    rgb[i * 3 + 2] = B[i] / g.maxv;
+                             float* __restrict__ rgb, size_t n, float maxv) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const size_t n4 = (reinterpret_cast<uintptr_t>(rgb) & 15) == 0 ? n / 4 : 0;
+  for (size_t q = t0; q < n4; q += stride) {
+    const float4 r = reinterpret_cast<const float4*>(R)[q], gr = reinterpret_cast<const float4*>(G)[q],
+                 b = reinterpret_cast<const float4*>(B)[q];
+    float4* o = reinterpret_cast<float4*>(rgb) + 3 * q;
+    o[0] = make_float4(r.x / maxv, gr.x / maxv, b.x / maxv, r.y / maxv);
+    o[1] = make_float4(gr.y / maxv, b.y / maxv, r.z / maxv, gr.z / maxv);
+    o[2] = make_float4(b.z / maxv, r.w / maxv, gr.w / maxv, b.w / maxv);
+  }
+  for (size_t i = 4 * n4 + t0; i < n; i += stride) {
+    rgb[i * 3 + 0] = R[i] / maxv;
+    rgb[i * 3 + 1] = G[i] / maxv;
+    rgb[i * 3 + 2] = B[i] / maxv;
   }
 }
 
@@ -587,7 +599,9 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     std::swap(R, P2);
     std::swap(B, P3);
   }
-  DCB_LAUNCH(k_dcb_output, R, G, B, rgb, g);
+  k_dcb_output<<<grid_for((w * h + 3) / 4, 256, c->sm_count * 8), 256, 0, s>>>(R, G, B, rgb, w * h, maximum_value);
+  count_launch(c);
+  LRE_TRY(check_launch(c, "demosaic_bayer_dcb"));
 #undef DCB_LAUNCH
   LRE_TRY(launch_border_interp(c, rgb, w, h, filters, 3));
   if (d_err) return LRE_OK;  // the caller reads the flag after its own synchronisation
