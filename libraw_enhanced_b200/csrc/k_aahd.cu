@@ -206,7 +206,7 @@ __global__ void k_aahd_hot_pretest(Aahd A) {
 struct OpHideHots {
   static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 3, BLK_PAIR = 2, BLK_ROWS = 64, BLK_COLS = 64;
-  static constexpr bool UNROLL = false, STEP2 = false;
+  static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = false;
   // padded coordinates; the 2x2 pattern makes the 4-px offset invisible
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   template <class T>
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(256) k_aahd_evaluate(Aahd A) {
 struct OpRefineDirs {
   static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
-  static constexpr bool UNROLL = true, STEP2 = true;
+  static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   // the walk acts at even image columns; rows two steps apart share their parity
   __device__ static bool site(int, int c, const Geo&) { return ((c - kMargin) & 1) == 0; }
   __device__ static int phase(int, const Geo&) { return kMargin & 1; }

@@ -1093,10 +1093,21 @@ lre_status launch_amaze_from_host(Context* c, const float* h_mosaic, float* d_mo
   AmazeArgs A = amaze_args(d_mosaic, 1, rgb, w, h, filters, cam_mul, maximum_value);
   A.max_g = max_g;
   if (max_g) LRE_CUDA_TRY(c, cudaMemsetAsync(max_g, 0, sizeof(float), c->stream));
-  const int bands = std::max(1, std::min(n_events, A.n_top / 4));
+  // Bands of tile rows that fill whole waves of CTAs: one wave twice, so the
+  // demosaic starts after little of the upload, then growing ones (the upload
+  // of a wave's rows takes less time than the wave).  Equal bands ended in a
+  // nearly empty wave each.
+  int edge[9] = {0}, bands = 0;
+  n_events = std::min(n_events, 8);
+  for (int row = 0, waves = 1; row < A.n_top; waves = bands < 2 ? 1 : waves + 1) {
+    const int fit = std::max(1, waves * c->sm_count / A.n_left);
+    const int left = A.n_top - row;
+    row += bands + 1 == n_events || left < 2 * fit ? left : fit;
+    edge[++bands] = row;
+  }
   size_t copied = 0;  // mosaic rows already queued for upload
   for (int b = 0; b < bands; b++) {
-    const int row_lo = A.n_top * b / bands, row_hi = A.n_top * (b + 1) / bands;
+    const int row_lo = edge[b], row_hi = edge[b + 1];
     // a tile row k reads mosaic rows [128k - 16, 128k + 144) (clamped)
     const size_t need = std::min(h, (size_t)std::max(0, -16 + (row_hi - 1) * (TS - 32) + TS));
     if (need > copied) {

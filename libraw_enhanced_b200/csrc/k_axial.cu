@@ -681,6 +681,356 @@ __global__ void __launch_bounds__(32, WS == 128 ? 16 : 20) k_ax_q(const float* _
   }
 }
 
+// ---------------------------------------------------------------------------
+// The two passes at radius 6 (the default), without shared memory.
+//
+// A warp covers 128 columns, four adjacent ones per lane, of which the middle
+// 112 are outputs, and walks down a chunk of rows.  Each lane keeps the
+// vertical window sums of its four columns in registers (add the row entering,
+// subtract the row leaving); a 13-column window is then the lane's own four
+// columns, all four of its two neighbours' and up to two of the lanes beyond,
+// so eight shuffled partial sums per quantity give all four windows.  The
+// |grad G| plane is written as the rows enter, from the last three of them.
+//
+// What bounds it: the two passes move 76 B/px (0.6 ms at 51 MP) and convert
+// every sample to double twice at a quarter of the issue rate.  The form with
+// window sums in shared memory read and rewrote 96 B and read 228 B of shared
+// memory per pixel and kept the L1 pipe 84% busy: at 51 MP 1290 + 1138 us,
+// this one 609 + 807 us.  Sums are formed in another order, in double as before.
+constexpr int A6_R = 6, A6_COLS = 112, A6_WARPS = 4;
+
+__device__ __forceinline__ double shfl_up_d(double v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
+__device__ __forceinline__ double shfl_dn_d(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
+
+// The sums of the 13 columns around each of the lane's four.
+__device__ __forceinline__ void a6_window(const double (&c)[4], double (&h)[4]) {
+  const double s1 = c[3], s2 = c[2] + s1, s3 = c[1] + s2, t = c[0] + s3;
+  const double p1 = c[0], p2 = c[0] + c[1], p3 = p2 + c[2];
+  const double l2_2 = shfl_up_d(s2, 2), l2_1 = shfl_up_d(s1, 2);
+  const double l1_3 = shfl_up_d(s3, 1), l1_4 = shfl_up_d(t, 1);
+  const double r1_3 = shfl_dn_d(p3, 1), r1_4 = shfl_dn_d(t, 1);
+  const double r2_1 = shfl_dn_d(p1, 2), r2_2 = shfl_dn_d(p2, 2);
+  h[0] = (l2_2 + l1_4) + (t + r1_3);
+  h[1] = (l2_1 + l1_4) + (t + r1_4);
+  h[2] = (l1_4 + t) + (r1_4 + r2_1);
+  h[3] = (l1_3 + t) + (r1_4 + r2_2);
+}
+
+// Four consecutive floats of a plane row whose start is 16-byte aligned.
+__device__ __forceinline__ void a6_ld4(const float* p, float* v) {
+  const float4 f = *reinterpret_cast<const float4*>(p);
+  v[0] = f.x;
+  v[1] = f.y;
+  v[2] = f.z;
+  v[3] = f.w;
+}
+
+struct A6Strip {
+  int x, y0, y1;  // the lane's first column; the chunk's rows
+  bool inside, vec, out;
+  __device__ __forceinline__ A6Strip(int W, int H, int HS, int yb0, bool aligned) {
+    const int strip = blockIdx.x * A6_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    x = strip * A6_COLS - 8 + 4 * lane;
+    y0 = (blockIdx.y + yb0) * HS;
+    y1 = min(y0 + HS, H);
+    inside = x >= 0 && x + 3 < W;
+    vec = aligned && inside;  // aligned: W is a multiple of four, and so is x
+    out = lane >= 2 && lane < 30 && x < W;
+  }
+};
+
+// RGB of the lane's four columns of row y (zeros outside the image).
+__device__ __forceinline__ void a6_rgb(const float* __restrict__ src, const A6Strip& S, int W, int H, int y, float (&v)[12]) {
+  if (y < 0 || y >= H) {
+#pragma unroll
+    for (int k = 0; k < 12; k++) v[k] = 0.f;
+    return;
+  }
+  const float* p = src + ((ptrdiff_t)y * W + S.x) * 3;
+  if (S.vec) {
+    a6_ld4(p, v);
+    a6_ld4(p + 4, v + 4);
+    a6_ld4(p + 8, v + 8);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 12; k++) v[k] = S.x + k / 3 >= 0 && S.x + k / 3 < W ? p[k] : 0.f;
+  }
+}
+
+__global__ void __launch_bounds__(32 * A6_WARPS, 3) k_ax6_ab(const float* __restrict__ src, int W, int H, int pitch,
+                                                         float eps, int HS, const float* __restrict__ d_maxg,
+                                                         float* __restrict__ planes, int yb0, bool aligned) {
+  const A6Strip S(W, H, HS, yb0, aligned);
+  const float inv_norm = 1.f / fmaxf(*d_maxg, 1e-6f);
+  const size_t n = (size_t)pitch * H;
+  double V[6][4];
+#pragma unroll
+  for (int q = 0; q < 6; q++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) V[q][k] = 0.0;
+  auto quantities = [&](const float (&v)[12], int k, double (&q)[6]) {
+    const float rr = v[3 * k] * inv_norm, g = v[3 * k + 1] * inv_norm, b = v[3 * k + 2] * inv_norm;
+    q[0] = (double)g;
+    q[1] = (double)(g * g);
+    q[2] = (double)rr;
+    q[3] = (double)(g * rr);
+    q[4] = (double)b;
+    q[5] = (double)(g * b);
+  };
+  float gp[4] = {0.f, 0.f, 0.f, 0.f}, gc[4] = {0.f, 0.f, 0.f, 0.f};  // G of the two rows entered last
+  // Row y enters: its sums, and |grad G| of the row above it.
+  auto enter = [&](const float (&v)[12], int y) {
+    float gn[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      double q[6];
+      quantities(v, k, q);
+      gn[k] = v[3 * k + 1] * inv_norm;
+#pragma unroll
+      for (int i = 0; i < 6; i++) V[i][k] += q[i];
+    }
+    const int r = y - 1;
+    const float gl = __shfl_up_sync(0xffffffffu, gc[3], 1), gr = __shfl_down_sync(0xffffffffu, gc[0], 1);
+    if (S.out && r >= S.y0 && r < S.y1) {
+      float e[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int x = S.x + k;
+        const float gx = (k < 3 ? gc[k + 1] : gr) - (k > 0 ? gc[k - 1] : gl), gy = gn[k] - gp[k];
+        e[k] = x >= 1 && x < W - 1 && r >= 1 && r < H - 1 ? sqrtf(gx * gx + gy * gy) : 0.f;
+      }
+      *reinterpret_cast<float4*>(planes + 4 * n + (size_t)r * pitch + S.x) = make_float4(e[0], e[1], e[2], e[3]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      gp[k] = gc[k];
+      gc[k] = gn[k];
+    }
+  };
+  float a[12], l[12];
+  for (int y = S.y0 - A6_R; y <= S.y0 + A6_R; y++) {
+    a6_rgb(src, S, W, H, y, a);
+    enter(a, y);
+  }
+  double inv_cx[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) inv_cx[k] = S.x + k >= 0 && S.x + k < W ? 1.0 / (double)win_count(S.x + k, A6_R, W) : 0.0;
+  for (int y = S.y0; y < S.y1; y++) {
+    if (y > S.y0) {
+      enter(a, y + A6_R);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        double q[6];
+        quantities(l, k, q);
+#pragma unroll
+        for (int i = 0; i < 6; i++) V[i][k] -= q[i];
+      }
+    }
+    if (y + 1 < S.y1) {  // the next row's samples, in flight while this row's outputs are formed
+      a6_rgb(src, S, W, H, y + 1 + A6_R, a);
+      a6_rgb(src, S, W, H, y - A6_R, l);
+    }
+    const double inv_cy = 1.0 / (double)win_count(y, A6_R, H);
+    double hs[4], mi[4], iv[4];
+    a6_window(V[0], hs);
+#pragma unroll
+    for (int k = 0; k < 4; k++) mi[k] = hs[k] * (inv_cx[k] * inv_cy);
+    a6_window(V[1], hs);
+#pragma unroll
+    for (int k = 0; k < 4; k++) iv[k] = 1.0 / ((hs[k] * (inv_cx[k] * inv_cy) - mi[k] * mi[k]) + (double)eps);
+#pragma unroll
+    for (int ch = 0; ch < 2; ch++) {
+      double hp[4];
+      a6_window(V[2 + 2 * ch], hp);
+      a6_window(V[3 + 2 * ch], hs);
+      float fa[4], fb[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const double ia = inv_cx[k] * inv_cy;
+        const double mp = hp[k] * ia;
+        const double av = (hs[k] * ia - mi[k] * mp) * iv[k];
+        fa[k] = (float)av;
+        fb[k] = (float)(mp - av * mi[k]);
+      }
+      if (S.out) {
+        const size_t o = (size_t)y * pitch + S.x;
+        *reinterpret_cast<float4*>(planes + (2 * ch) * n + o) = make_float4(fa[0], fa[1], fa[2], fa[3]);
+        *reinterpret_cast<float4*>(planes + (2 * ch + 1) * n + o) = make_float4(fb[0], fb[1], fb[2], fb[3]);
+      }
+    }
+  }
+}
+
+// codes (nullable): the result as 16-bit codes (the quantisation that follows
+// the filter, on the stored floats) instead of floats.
+__global__ void __launch_bounds__(32 * A6_WARPS, 3) k_ax6_q(const float* __restrict__ src, float* __restrict__ dst,
+                                                        uint16_t* __restrict__ codes, int W, int H, int pitch,
+                                                        float strength, int HS, const float* __restrict__ d_maxg,
+                                                        const float* __restrict__ planes, int yb0, bool tone,
+                                                        float tone_scale, bool aligned) {
+  const A6Strip S(W, H, HS, yb0, aligned);
+  const float norm_ref = fmaxf(*d_maxg, 1e-6f);
+  const float inv_norm = 1.f / norm_ref;
+  const size_t n = (size_t)pitch * H;
+  double V[5][4];
+#pragma unroll
+  for (int q = 0; q < 5; q++)
+#pragma unroll
+    for (int k = 0; k < 4; k++) V[q][k] = 0.0;
+  // The planes' rows are padded to four columns; the padding of the last
+  // group is written by the first pass and must not be summed.
+  auto load = [&](int y, float (&v)[5][4]) {
+    const bool on = y >= 0 && y < H && S.x >= 0 && S.x < W;
+#pragma unroll
+    for (int q = 0; q < 5; q++) {
+      if (on) {
+        a6_ld4(planes + q * n + (size_t)y * pitch + S.x, v[q]);
+#pragma unroll
+        for (int k = 1; k < 4; k++)
+          if (S.x + k >= W) v[q][k] = 0.f;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[q][k] = 0.f;
+      }
+    }
+  };
+  float a[5][4], l[5][4];
+  auto enter = [&]() {
+#pragma unroll
+    for (int q = 0; q < 5; q++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) V[q][k] += (double)a[q][k];
+  };
+  for (int y = S.y0 - A6_R; y <= S.y0 + A6_R; y++) {
+    load(y, a);
+    enter();
+  }
+  double inv_cx[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) inv_cx[k] = S.x + k >= 0 && S.x + k < W ? 1.0 / (double)win_count(S.x + k, A6_R, W) : 0.0;
+  for (int y = S.y0; y < S.y1; y++) {
+    if (y > S.y0) {
+      enter();
+#pragma unroll
+      for (int q = 0; q < 5; q++)
+#pragma unroll
+        for (int k = 0; k < 4; k++) V[q][k] -= (double)l[q][k];
+    }
+    float c[12];
+    a6_rgb(src, S, W, H, y, c);
+    if (y + 1 < S.y1) {
+      load(y + 1 + A6_R, a);
+      load(y - A6_R, l);
+    }
+    const double inv_cy = 1.0 / (double)win_count(y, A6_R, H);
+    double ha[4], hb[4];
+    float qv[2][4], w[4];
+#pragma unroll
+    for (int ch = 0; ch < 2; ch++) {
+      a6_window(V[2 * ch], ha);
+      a6_window(V[2 * ch + 1], hb);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const double ia = inv_cx[k] * inv_cy;
+        qv[ch][k] = (float)((ha[k] * ia) * (double)(c[3 * k + 1] * inv_norm) + hb[k] * ia);
+      }
+    }
+    a6_window(V[4], ha);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float tt = clampf(((float)(ha[k] * (inv_cx[k] * inv_cy)) - 0.01f) / 0.05f, 0.f, 1.f);
+      w[k] = strength * (tt * tt * (3.f - 2.f * tt));
+    }
+    if (!S.out) continue;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float R = c[3 * k] * inv_norm, B = c[3 * k + 2] * inv_norm;
+      c[3 * k] = (R * (1.f - w[k]) + qv[0][k] * w[k]) * norm_ref;
+      c[3 * k + 2] = (B * (1.f - w[k]) + qv[1][k] * w[k]) * norm_ref;
+    }
+    if (tone) {  // the ACES stage that follows, applied to the stored floats
+#pragma unroll
+      for (int k = 0; k < 12; k++) c[k] = aces(c[k]) * tone_scale;
+    }
+    const size_t o = ((size_t)y * W + S.x) * 3;
+    if (codes) {
+      unsigned short u[12];
+#pragma unroll
+      for (int k = 0; k < 12; k++) u[k] = (unsigned short)(clampf(c[k], 0.f, 1.f) * 65535.0f + 0.5f);
+      if (S.vec) {
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          *reinterpret_cast<ushort4*>(codes + o + 4 * k) = make_ushort4(u[4 * k], u[4 * k + 1], u[4 * k + 2], u[4 * k + 3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 12; k++)
+          if (S.x + k / 3 < W) codes[o + k] = u[k];
+      }
+    } else if (S.vec) {
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        *reinterpret_cast<float4*>(dst + o + 4 * k) = make_float4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 12; k++)
+        if (S.x + k / 3 < W) dst[o + k] = c[k];
+    }
+  }
+}
+
+// Row chunks [k0, k1) of either pass.
+struct A6Call {
+  const float* src;
+  float* out;
+  uint16_t* codes;
+  int W, H, pitch, HS;
+  float eps, strength;
+  const float* d_max;
+  float* planes;
+  float tone_scale;
+  bool aligned() const {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(src) | (codes ? reinterpret_cast<uintptr_t>(codes) << 1
+                                                                  : reinterpret_cast<uintptr_t>(out));
+    return (W & 3) == 0 && (p & 15) == 0;
+  }
+  dim3 grid(int chunks) const {
+    return dim3((unsigned)((W + A6_COLS * A6_WARPS - 1) / (A6_COLS * A6_WARPS)), (unsigned)chunks);
+  }
+  cudaError_t pass_a(int k0, int k1, cudaStream_t s) const {
+    if (k1 <= k0) return cudaSuccess;
+    k_ax6_ab<<<grid(k1 - k0), 32 * A6_WARPS, 0, s>>>(src, W, H, pitch, eps, HS, d_max, planes, k0, aligned());
+    return cudaPeekAtLastError();
+  }
+  cudaError_t pass_b(int k0, int k1, cudaStream_t s) const {
+    if (k1 <= k0) return cudaSuccess;
+    k_ax6_q<<<grid(k1 - k0), 32 * A6_WARPS, 0, s>>>(src, out, codes, W, H, pitch, strength, HS, d_max, planes, k0,
+                                                    tone_scale >= 0.f, tone_scale, aligned());
+    return cudaPeekAtLastError();
+  }
+};
+
+size_t a6_plane_floats(size_t w, size_t h) { return ((w + 3) & ~size_t(3)) * h; }
+
+// Rows per chunk: what takes the fewest row steps over all waves of CTAs
+// (three per SM).  13 rows enter before a chunk's first output, which favours
+// tall chunks; a last wave that is nearly empty costs as much as a full one
+// (51 MP, 128 rows: 897 CTAs on 444 places, the second pass 1013 us; 136 rows
+// spread over the waves evenly, 807 us).
+int a6_rows(int tall, size_t w, size_t h, int sms, int bands) {
+  const size_t groups = (w + A6_COLS * A6_WARPS - 1) / (A6_COLS * A6_WARPS), places = 3 * (size_t)sms;
+  int best = 8;
+  size_t least = SIZE_MAX;
+  for (int hs = 8; hs <= tall; hs += 8) {
+    const size_t chunks = ((h + hs - 1) / hs + bands - 1) / bands;
+    const size_t cost = (groups * chunks + places - 1) / places * bands * (size_t)(hs + 2 * A6_R + 1);
+    if (cost <= least) {
+      least = cost;
+      best = hs;
+    }
+  }
+  return best;
+}
+
 template <int WS>
 cudaError_t axial_stream(size_t w, size_t h, int HS, cudaStream_t s, const float* src, float* out, int r, float eps,
                          float strength, const float* d_max, float* planes, bool tone, float tone_scale) {
@@ -726,17 +1076,18 @@ size_t ws_bytes_axial(size_t w, size_t h, int radius) {
   // the four a/b planes and the edge plane between the two passes, plus an out-of-place copy
   // when the caller runs in place (pass B reads input rows below the rows it
   // writes).
-  return ((w * h * 5 * sizeof(float) + 255) & ~size_t(255)) + w * h * 3 * sizeof(float) + 256;
+  return ((a6_plane_floats(w, h) * 5 * sizeof(float) + 255) & ~size_t(255)) + w * h * 3 * sizeof(float) + 256;
 }
 
 lre_status launch_axial_ca_banded(Context* c, const float* in, float* out, size_t w, size_t h, int radius, float eps,
                                   float strength, const float* d_max_g, int bands,
-                                  const std::function<lre_status(size_t, size_t)>& rows_done, float tone_scale) {
+                                  const std::function<lre_status(size_t, size_t)>& rows_done, float tone_scale,
+                                  uint16_t* codes) {
   if (radius < 1) radius = 1;
   if (radius > 16) return fail(c, LRE_ERR_INVALID_ARGUMENT, "ca_axial_cleanup: radius > 16 is not supported");
   if (in == out) return fail(c, LRE_ERR_INVALID_ARGUMENT, "ca_axial_cleanup: banded form runs out of place");
   strength = fminf(fmaxf(strength, 0.f), 1.f);
-  float* planes = reinterpret_cast<float*>(c->ws.take(w * h * 5 * sizeof(float)));
+  float* planes = reinterpret_cast<float*>(c->ws.take(a6_plane_floats(w, h) * 5 * sizeof(float)));
   if (!planes) return fail(c, LRE_ERR_OUT_OF_MEMORY, "ca_axial_cleanup: workspace too small");
   const int WS = c->tune.axial_strip == 64 ? 64 : 128;
   const size_t strips_x = (w + WS - 1) / WS;
@@ -746,11 +1097,30 @@ lre_status launch_axial_ca_banded(Context* c, const float* in, float* out, size_
   bands = std::max(1, bands);
   int HS = c->tune.axial_rows == 128 ? 128 : 64;
   while (HS > 16 && strips_x * ((h + HS - 1) / HS) < want * (size_t)bands) HS /= 2;
+  const bool r6 = radius == A6_R;
+  if (r6) HS = a6_rows(c->tune.axial_rows == 128 ? 192 : 96, w, h, c->sm_count, bands);
   // pass B of a chunk reads pass A's planes up to `radius` (<= HS) rows below
   // it, so pass A runs one band ahead of pass B
   const int nch = (int)((h + HS - 1) / HS);
   bands = std::min(bands, nch);
   auto edge = [&](int b) { return (int)((long long)nch * b / bands); };
+  if (r6) {
+    A6Call call{in,  out,      codes,   (int)w, (int)h,  (int)((w + 3) & ~size_t(3)), HS,
+                eps, strength, d_max_g, planes, tone_scale};
+    LRE_CUDA_TRY(c, call.pass_a(0, edge(1), c->stream));
+    count_launch(c);
+    for (int b = 0; b < bands; b++) {
+      if (b + 1 < bands) {
+        LRE_CUDA_TRY(c, call.pass_a(edge(b + 1), edge(b + 2), c->stream));
+        count_launch(c);
+      }
+      LRE_CUDA_TRY(c, call.pass_b(edge(b), edge(b + 1), c->stream));
+      count_launch(c);
+      LRE_TRY(check_launch(c, "ca_axial_cleanup"));
+      LRE_TRY(rows_done(std::min(h, (size_t)edge(b) * HS), std::min(h, (size_t)edge(b + 1) * HS)));
+    }
+    return LRE_OK;
+  }
   auto pass_a = [&](int b) {
     return WS == 64 ? axial_pass_a<64>(w, h, HS, edge(b), edge(b + 1), c->stream, in, radius, eps, d_max_g, planes)
                     : axial_pass_a<128>(w, h, HS, edge(b), edge(b + 1), c->stream, in, radius, eps, d_max_g, planes);
@@ -770,17 +1140,18 @@ lre_status launch_axial_ca_banded(Context* c, const float* in, float* out, size_
     count_launch(c);
     LRE_TRY(check_launch(c, "ca_axial_cleanup"));
     const size_t r0 = std::min(h, (size_t)edge(b) * HS), r1 = std::min(h, (size_t)edge(b + 1) * HS);
+    if (codes) LRE_TRY(launch_quantize_u16(c, out + r0 * w * 3, codes + r0 * w * 3, (r1 - r0) * w * 3));
     LRE_TRY(rows_done(r0, r1));
   }
   return LRE_OK;
 }
 
 lre_status launch_axial_ca(Context* c, const float* in, float* out, size_t w, size_t h, int radius, float eps,
-                           float strength, const float* d_max_g, float tone_scale) {
+                           float strength, const float* d_max_g, float tone_scale, uint16_t* codes) {
   if (radius < 1) radius = 1;
   if (radius > 16) return fail(c, LRE_ERR_INVALID_ARGUMENT, "ca_axial_cleanup: radius > 16 is not supported");
   strength = fminf(fmaxf(strength, 0.f), 1.f);
-  float* planes = reinterpret_cast<float*>(c->ws.take(w * h * 5 * sizeof(float)));
+  float* planes = reinterpret_cast<float*>(c->ws.take(a6_plane_floats(w, h) * 5 * sizeof(float)));
   if (!planes) return fail(c, LRE_ERR_OUT_OF_MEMORY, "ca_axial_cleanup: workspace too small");
   const float* src = in;
   if (in == out) {
@@ -789,7 +1160,17 @@ lre_status launch_axial_ca(Context* c, const float* in, float* out, size_t w, si
     LRE_CUDA_TRY(c, cudaMemcpyAsync(tmp, in, w * h * 3 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
     src = tmp;
   }
-  // Strip width 128 (4 columns per lane) or 64 (2 per lane); strip height:
+  if (radius == A6_R) {
+    A6Call call{src, out, codes, (int)w, (int)h, (int)((w + 3) & ~size_t(3)),
+                a6_rows(c->tune.axial_rows == 128 ? 192 : 96, w, h, c->sm_count, 1),
+                eps, strength, d_max_g, planes, tone_scale};
+    const int chunks = (call.H + call.HS - 1) / call.HS;
+    LRE_CUDA_TRY(c, call.pass_a(0, chunks, c->stream));
+    LRE_CUDA_TRY(c, call.pass_b(0, chunks, c->stream));
+    count_launch(c, 2);
+    return check_launch(c, "ca_axial_cleanup");
+  }
+  // Other radii.  Strip width 128 (4 columns per lane) or 64 (2 per lane); strip height:
   // enough one-warp strips for at least 24 per SM (more than the 16-20 that
   // fit at once, so every SM stays full while the passes, which are
   // load-latency bound, drain), but at least 16 rows so the 2r + 1 row
@@ -805,7 +1186,8 @@ lre_status launch_axial_ca(Context* c, const float* in, float* out, size_t w, si
                            : axial_stream<128>(w, h, HS, c->stream, src, out, radius, eps, strength, d_max_g, planes,
                                                tone, tone_scale));
   count_launch(c, 2);
-  return check_launch(c, "ca_axial_cleanup");
+  LRE_TRY(check_launch(c, "ca_axial_cleanup"));
+  return codes ? launch_quantize_u16(c, out, codes, w * h * 3) : LRE_OK;
 }
 
 // ---------------------------------------------------------------------------

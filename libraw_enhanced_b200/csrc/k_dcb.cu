@@ -415,7 +415,7 @@ __global__ void k_dcb_pp_terms(const float* __restrict__ G, float* __restrict__ 
 struct OpNyquist {
   static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 1, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
-  static constexpr bool UNROLL = true, STEP2 = true;
+  static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   // sites with r + c of the non-green parity
   __device__ static int phase(int r0, const Geo& g) { return (r0 & 1) ^ (g.fc(0, 0) == 1); }
@@ -432,7 +432,7 @@ struct OpNyquist {
 struct OpPP {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
-  static constexpr bool UNROLL = true, STEP2 = false;
+  static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }
   __device__ static int phase(int, const Geo&) { return 0; }
   template <class T>
@@ -457,7 +457,7 @@ __device__ __forceinline__ void clamp8(const T& t, float v) {
 struct OpRefine {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
-  static constexpr bool UNROLL = true, STEP2 = true;
+  static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   // sites with r + c of the non-green parity
   __device__ static int phase(int r0, const Geo& g) { return (r0 & 1) ^ (g.fc(0, 0) == 1); }
@@ -472,7 +472,7 @@ struct OpRefine {
 struct OpColorFull {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
-  static constexpr bool UNROLL = true, STEP2 = false;
+  static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }
   __device__ static int phase(int, const Geo&) { return 0; }
   template <class T>

@@ -328,7 +328,7 @@ struct OpLoca {
 struct OpLocaBlk {
   static constexpr int NS = 2, NP = 3, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, BLK_WARPS = 6;
   static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
-  static constexpr bool UNROLL = false, STEP2 = false;
+  static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = true;
   __device__ static bool site(int, int, const Geo&) { return true; }
   template <class T>
   __device__ static void cell(const T& t, int, const Geo& g) {

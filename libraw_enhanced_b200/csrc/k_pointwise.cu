@@ -165,8 +165,18 @@ lre_status launch_channel_max(Context* c, const float* rgb, size_t n_px, int cha
 }
 
 // Output quantisation, core/python_bindings.cpp:241-256.
+// Eight samples per thread (two 16-byte loads, one 16-byte store) where both
+// buffers are aligned: 72 M samples 133 us before, 66 us of traffic.
 __global__ void k_quantize_u16(const float* __restrict__ in, uint16_t* __restrict__ out, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const size_t n8 = vec ? n / 8 : 0;
+  auto code = [](float x) { return (unsigned)(uint16_t)(clampf(x, 0.f, 1.f) * 65535.0f + 0.5f); };
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n8; q += (size_t)gridDim.x * blockDim.x) {
+    const float4 a = reinterpret_cast<const float4*>(in)[2 * q], b = reinterpret_cast<const float4*>(in)[2 * q + 1];
+    reinterpret_cast<uint4*>(out)[q] = make_uint4(code(a.x) | code(a.y) << 16, code(a.z) | code(a.w) << 16,
+                                                  code(b.x) | code(b.y) << 16, code(b.z) | code(b.w) << 16);
+  }
+  for (size_t i = n8 * 8 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     float v = clampf(in[i], 0.f, 1.f);
     out[i] = (uint16_t)(v * 65535.0f + 0.5f);
   }

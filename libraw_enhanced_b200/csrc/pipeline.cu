@@ -94,14 +94,23 @@ bool banded_tail(const lre_develop_params& p) {
   return p.stage_order == 1 && p.axial_ca_correction && p.tone_mapping != 2;
 }
 
+// The axial filter is the last stage but the pointwise ones that its own last
+// pass applies (the ACES tone map, the 16-bit codes).
+bool axial_quantizes(const lre_develop_params& p) {
+  return p.output_bits == 16 && p.axial_ca_correction &&
+         (p.stage_order == 1 ? p.tone_mapping != 2 : !p.defringe);
+}
+
 // h_mosaic (nullable): the mosaic is still in host memory and d_mosaic is
 // its destination; the AMaZE route overlaps the upload with the demosaic,
 // every other route uploads it first.
 // tail (nullable): when banded_tail(p), the axial filter and the tone map run
 // in row bands and each finished band is passed to *tail.
+// codes (nullable): where axial_quantizes(p), the last stage writes the 16-bit
+// result there itself.
 lre_status run_chain(Context* c, const float* d_mosaic, float* rgb_a, float* rgb_b, size_t w, size_t h,
                      const lre_develop_params& p, float** result, const float* h_mosaic = nullptr,
-                     const RowsReady* tail = nullptr) {
+                     const RowsReady* tail = nullptr, uint16_t* codes = nullptr) {
   float* cur = rgb_a;
   float* other = rgb_b;
   const size_t mark = c->ws.used();
@@ -196,10 +205,10 @@ lre_status run_chain(Context* c, const float* d_mosaic, float* rgb_a, float* rgb
       float* dst = other;
       LRE_TRY(lre::launch_axial_ca_banded(
           c, cur, dst, w, h, p.axial_ca_radius, p.axial_ca_epsilon, p.axial_ca_strength, dmax, 8,
-          [&](size_t r0, size_t r1) -> lre_status { return (*tail)(dst, r0, r1); }, tone_scale));
+          [&](size_t r0, size_t r1) -> lre_status { return (*tail)(dst, r0, r1); }, tone_scale, codes));
     } else {
       LRE_TRY(lre::launch_axial_ca(c, cur, other, w, h, p.axial_ca_radius, p.axial_ca_epsilon, p.axial_ca_strength,
-                                   dmax, tone_scale));
+                                   dmax, tone_scale, codes));
     }
     std::swap(cur, other);
     cur_max_g = nullptr;
@@ -257,10 +266,11 @@ lre_status develop_device(Context* c, const float* mosaic, void* out, size_t w, 
   if (p.axial_ca_correction) std::swap(rgb_a, rgb_b);
   if (!rgb_a || !rgb_b) return fail(c, LRE_ERR_OUT_OF_MEMORY, "develop: workspace too small");
   float* res = nullptr;
-  LRE_TRY(run_chain(c, mosaic, rgb_a, rgb_b, w, h, p, &res));
+  uint16_t* codes = axial_quantizes(p) ? reinterpret_cast<uint16_t*>(out) : nullptr;
+  LRE_TRY(run_chain(c, mosaic, rgb_a, rgb_b, w, h, p, &res, nullptr, nullptr, codes));
   if (float_out) {
     if (res != out) LRE_CUDA_TRY(c, cudaMemcpyAsync(out, res, w * h * 12, cudaMemcpyDeviceToDevice, c->stream));
-  } else {
+  } else if (!codes) {
     LRE_TRY(launch_quantize_u16(c, res, reinterpret_cast<uint16_t*>(out), w * h * 3));
   }
   return LRE_OK;
@@ -352,16 +362,13 @@ lre_status lre_develop(lre_ctx* ctx, const float* mosaic, void* out, size_t w, s
     const RowsReady tail = [&](const float* rgb, size_t r0, size_t r1) -> lre_status {
       if (nb >= 8) return lre::fail(c, LRE_ERR_INVALID_ARGUMENT, "develop: internal: more than 8 row bands");
       const void* src = rgb + r0 * w * 3;
-      if (p.output_bits == 16) {
-        uint16_t* q = reinterpret_cast<uint16_t*>(c->d_out) + r0 * w * 3;
-        LRE_TRY(lre::launch_quantize_u16(c, rgb + r0 * w * 3, q, (r1 - r0) * w * 3));
-        src = q;
-      }
+      if (p.output_bits == 16) src = reinterpret_cast<uint16_t*>(c->d_out) + r0 * w * 3;  // axial_quantizes(p)
       LRE_CUDA_TRY(c, cudaEventRecord(c->tail_ev[nb], c->stream));
       bands[nb++] = {src, r0, r1};
       return LRE_OK;
     };
-    LRE_TRY(run_chain(c, reinterpret_cast<const float*>(c->d_in), rgb_a, rgb_b, w, h, p, &res, mosaic, &tail));
+    LRE_TRY(run_chain(c, reinterpret_cast<const float*>(c->d_in), rgb_a, rgb_b, w, h, p, &res, mosaic, &tail,
+                      p.output_bits == 16 ? reinterpret_cast<uint16_t*>(c->d_out) : nullptr));
     for (int b = 0; b < nb; b++) {
       LRE_CUDA_TRY(c, cudaStreamWaitEvent(c->copy_stream, c->tail_ev[b], 0));
       LRE_TRY(lre::copy_d2h(c, static_cast<char*>(out) + bands[b].r0 * w * px_bytes, bands[b].src,
@@ -369,9 +376,10 @@ lre_status lre_develop(lre_ctx* ctx, const float* mosaic, void* out, size_t w, s
     }
     LRE_CUDA_TRY(c, cudaStreamSynchronize(c->copy_stream));
   } else {
-    LRE_TRY(run_chain(c, reinterpret_cast<const float*>(c->d_in), rgb_a, rgb_b, w, h, p, &res, mosaic));
+    uint16_t* codes = axial_quantizes(p) ? reinterpret_cast<uint16_t*>(c->d_out) : nullptr;
+    LRE_TRY(run_chain(c, reinterpret_cast<const float*>(c->d_in), rgb_a, rgb_b, w, h, p, &res, mosaic, nullptr, codes));
     if (p.output_bits == 16) {
-      LRE_TRY(lre::launch_quantize_u16(c, res, reinterpret_cast<uint16_t*>(c->d_out), w * h * 3));
+      if (!codes) LRE_TRY(lre::launch_quantize_u16(c, res, reinterpret_cast<uint16_t*>(c->d_out), w * h * 3));
       LRE_TRY(lre::copy_d2h(c, out, c->d_out, out_bytes, c->stream));
     } else {
       LRE_TRY(lre::copy_d2h(c, out, res, out_bytes, c->stream));

@@ -28,7 +28,8 @@
 // columns, a power of two), BLK_WARPS (warps of a block), BLK_ROWS and
 // BLK_COLS (a block's overlap), BLK_SKEW and BLK_PAIR (a block's own skew),
 // UNROLL (whether a block's group of steps is unrolled), STEP2 (a block visits
-// every second step only, from phase(r0, g) on), site(r, c, g) (whether the
+// every second step only, from phase(r0, g) on), IDLE0 (sites whose inputs are
+// zero keep their values, so a group without others is skipped), site(r, c, g) (whether the
 // pass visits the site) and cell(t, c, g), which updates the site that the
 // accessor t stands on.
 #pragma once
@@ -514,12 +515,18 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
       for (int p = 0; p < NS; p++) sweep_smem[p * B::PLANE + (lrh + HALO) * B::PITCH + tr] = vh[p];
     }
   };
+  // Returns whether any input of the warp's group is non-zero.
   auto store_inputs = [&]() {
     const unsigned sl = B::INPUTS + lr8 * B::IPITCH + l8;
+    bool any = false;
 #pragma unroll
     for (int k = 0; k < 8; k++)
 #pragma unroll
-      for (int p = NS; p < NP; p++) sweep_smem[sl + (p - NS) * B::IPLANE + k * B::IPITCH] = v[k][p];
+      for (int p = NS; p < NP; p++) {
+        sweep_smem[sl + (p - NS) * B::IPLANE + k * B::IPITCH] = v[k][p];
+        any |= v[k][p] != 0.f;
+      }
+    return Op::IDLE0 ? __any_sync(0xffffffffu, any) != 0 : true;
   };
   const std::integral_constant<int, 0> z0{};
   const std::integral_constant<int, NS> zs{};
@@ -585,7 +592,7 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
     const int g = g_lo + k - warp;
     if (k >= warp && k - warp < ng) {
       store(g + 5);
-      store_inputs();
+      const bool busy = store_inputs();
       __syncwarp();
       load(g + 1, zs, zp);
       load(g + 6, z0, zs);
@@ -620,7 +627,7 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
         } else {
           if (ph) steps(no, f1); else steps(no, f0);
         }
-      } else {
+      } else if (busy) {
         const size_t px = (size_t)r * W + c0;
 #pragma unroll 1
         for (int s = 0; s < G; s++) {
