@@ -204,7 +204,7 @@ __global__ void k_aahd_hot_pretest(Aahd A) {
 // and r + 1 advance together, each row pair three columns behind the pair
 // above: (r - 2, c + 2) is then already rewritten and (r + 2, c - 2) not yet.
 struct OpHideHots {
-  static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 3, BLK_PAIR = 2, BLK_ROWS = 64, BLK_COLS = 64;
   static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = false;
   // padded coordinates; the 2x2 pattern makes the 4-px offset invisible
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(256) k_aahd_evaluate(Aahd A) {
 // image so the last odd column is reached.  Every neighbour read precedes or
 // follows the site exactly as in the row-major loops with skew 1.
 struct OpRefineDirs {
-  static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   // the walk acts at even image columns; rows two steps apart share their parity

@@ -413,7 +413,7 @@ __global__ void k_dcb_pp_terms(const float* __restrict__ G, float* __restrict__ 
 // R and B do not change across the nyquist passes).  A site reads rows r +- 2
 // only, so rows r and r + 1 advance together.
 struct OpNyquist {
-  static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 1, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
@@ -430,7 +430,7 @@ struct OpNyquist {
 // dcb_pp (:820-834), one channel (R or B) per warp: state the channel;
 // input K = G - mean8(G) (k_dcb_pp_terms; green does not change in the pass).
 struct OpPP {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
   static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }
@@ -455,7 +455,7 @@ __device__ __forceinline__ void clamp8(const T& t, float v) {
 
 // dcb_refinement's closing clamp (:992-994): state G; input the pre-clamp value.
 struct OpRefine {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
@@ -470,7 +470,7 @@ struct OpRefine {
 // dcb_color_full's last loop (:898-913), one channel per warp: state R or B;
 // input that channel's CLIP(chroma + G).
 struct OpColorFull {
-  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8;
+  static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
   static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
   static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }

@@ -48,7 +48,7 @@ struct HlParams {
 
 // Loop 1 per pixel (:1150-1191): mask, highlight flag, candidate flag.
 __global__ void k_hl_pass1(const float* __restrict__ in, size_t n, HlParams P, float* __restrict__ mask,
-                           uint8_t* __restrict__ flags, int* __restrict__ block_counts) {
+                           uint8_t* __restrict__ flags, int* __restrict__ block_counts, int* total) {
   const size_t i = (size_t)blockIdx.x * kHlBlock + threadIdx.x;
   int cand = 0;
   if (i < n) {
@@ -77,20 +77,33 @@ __global__ void k_hl_pass1(const float* __restrict__ in, size_t n, HlParams P, f
     flags[i] = f;
   }
   const int c = __syncthreads_count(cand);
-  if (threadIdx.x == 0) block_counts[blockIdx.x] = c;
+  if (threadIdx.x == 0) {
+    block_counts[blockIdx.x] = c;
+    if (c) atomicAdd(total, c);
+  }
 }
 
-// Exclusive scan of the per-block candidate counts (one CTA; the total goes
-// to block_off[nb]).
-__global__ void k_hl_scan(const int* __restrict__ counts, int nb, int* __restrict__ off) {
+// Exclusive scan of the per-block candidate counts (one CTA, eight counts per
+// thread and step; the total goes to block_off[nb]).
+__global__ void __launch_bounds__(1024) k_hl_scan(const int* __restrict__ counts, int nb, int* __restrict__ off,
+                                                   const int* __restrict__ total) {
+  if (*total == 0) {  // no terms: the usual case, as few highlights lie below 0.95
+    if (threadIdx.x == 0) off[nb] = 0;
+    return;
+  }
   __shared__ int warp_sums[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
-  for (int base = 0; base < nb; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int v = i < nb ? counts[i] : 0;
-    int x = v;
+  for (int base = 0; base < nb; base += 8192) {
+    const int i0 = base + 8 * threadIdx.x;
+    int v[8], t = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      v[k] = i0 + k < nb ? counts[i0 + k] : 0;
+      t += v[k];
+    }
+    int x = t;
     for (int d = 1; d < 32; d <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, d);
       if ((threadIdx.x & 31) >= d) x += y;
@@ -107,7 +120,12 @@ __global__ void k_hl_scan(const int* __restrict__ counts, int nb, int* __restric
     }
     __syncthreads();
     const int wp = (threadIdx.x >> 5) ? warp_sums[(threadIdx.x >> 5) - 1] : 0;
-    if (i < nb) off[i] = carry + wp + x - v;
+    int o = carry + wp + x - t;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      if (i0 + k < nb) off[i0 + k] = o;
+      o += v[k];
+    }
     __syncthreads();
     if (threadIdx.x == 1023) carry += wp + x;
     __syncthreads();
@@ -118,28 +136,33 @@ __global__ void k_hl_scan(const int* __restrict__ counts, int nb, int* __restric
 // The candidates' R/G and B/G terms, scattered in pixel order.
 __global__ void k_hl_compact(const float* __restrict__ in, size_t n, const uint8_t* __restrict__ flags,
                              const int* __restrict__ block_off, float* __restrict__ t_rg,
-                             float* __restrict__ t_bg) {
+                             float* __restrict__ t_bg, const int* __restrict__ total, int nb) {
   __shared__ int warp_base[kHlBlock / 32];
-  const size_t i = (size_t)blockIdx.x * kHlBlock + threadIdx.x;
-  const bool cand = i < n && flags[i] == 3;
-  const unsigned b = __ballot_sync(0xffffffffu, cand);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) warp_base[warp] = __popc(b);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s = 0;
-    for (int k = 0; k < kHlBlock / 32; k++) {
-      const int c = warp_base[k];
-      warp_base[k] = s;
-      s += c;
+  if (*total == 0) return;
+  for (int blk = blockIdx.x; blk < nb; blk += gridDim.x) {
+    if (block_off[blk + 1] == block_off[blk]) continue;  // none here
+    const size_t i = (size_t)blk * kHlBlock + threadIdx.x;
+    const bool cand = i < n && flags[i] == 3;
+    const unsigned b = __ballot_sync(0xffffffffu, cand);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) warp_base[warp] = __popc(b);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int s = 0;
+      for (int k = 0; k < kHlBlock / 32; k++) {
+        const int c = warp_base[k];
+        warp_base[k] = s;
+        s += c;
+      }
     }
-  }
-  __syncthreads();
-  if (cand) {
-    const int pos = block_off[blockIdx.x] + warp_base[warp] + __popc(b & ((1u << lane) - 1));
-    const float p0 = in[i * 3], p1 = in[i * 3 + 1], p2 = in[i * 3 + 2];
-    t_rg[pos] = p0 / p1;
-    t_bg[pos] = p2 / p1;
+    __syncthreads();
+    if (cand) {
+      const int pos = block_off[blk] + warp_base[warp] + __popc(b & ((1u << lane) - 1));
+      const float p0 = in[i * 3], p1 = in[i * 3 + 1], p2 = in[i * 3 + 2];
+      t_rg[pos] = p0 / p1;
+      t_bg[pos] = p2 / p1;
+    }
+    __syncthreads();
   }
 }
 
@@ -225,7 +248,6 @@ __global__ void k_hl_white(const float* __restrict__ R, const float* __restrict_
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     const int y = (int)(i / W), x = (int)(i % W);
     const float* src[3] = {R, G, B};
-    float* dst[3] = {R2, G2, B2};
     const bool white = (flags[i] & 4) && x > 0 && x < W - 1 && y > 0 && y < H - 1;
     float v[3];
 #pragma unroll
@@ -235,7 +257,6 @@ __global__ void k_hl_white(const float* __restrict__ R, const float* __restrict_
                            s[i + W + 1]) *
                               (1.f / 8.f)
                    : s[i];
-      dst[c][i] = v[c];
     }
     // Loop 4 changes a highlight pixel only from its own value, and only when
     // that value passes these two tests (:1307-1329), so they are decided
@@ -247,7 +268,13 @@ __global__ void k_hl_white(const float* __restrict__ R, const float* __restrict_
     out[i * 3] = v[0];
     out[i * 3 + 1] = v[1];
     out[i * 3 + 2] = v[2];
-    cand[i] = (flags[i] & 1) && !(l < thr * 0.90f) && !(rb <= v[1] * 1.04f) ? 1.f : 0.f;
+    const bool changes = (flags[i] & 1) && !(l < thr * 0.90f) && !(rb <= v[1] * 1.04f);
+    cand[i] = changes ? 1.f : 0.f;
+    if (changes) {  // loop 4 reads a candidate's own value while its result may already be in `out`
+      R2[i] = v[0];
+      G2[i] = v[1];
+      B2[i] = v[2];
+    }
   }
 }
 
@@ -274,11 +301,12 @@ __device__ __forceinline__ bool loca_lift(NL nl, RT ratio, float thr, float max_
   for (int dy = -2; dy <= 2; ++dy)
 #pragma unroll
     for (int dx = -2; dx <= 2; ++dx) {
+      // selected, not branched to: adding 0.0 changes neither sum
       const float q = ratio(dy, dx);
-      if (q == -1.f) continue;
+      const bool in = q != -1.f;
       const double w = 1.0 / (double)(1 + abs(dx) + abs(dy));
-      ratio_sum += q * w;
-      ratio_w += w;
+      ratio_sum += in ? (double)q * w : 0.0;
+      ratio_w += in ? w : 0.0;
     }
   const float local_ratio = (float)(ratio_w > 0.0 ? ratio_sum / ratio_w : 1.0);
   const float desired_g = rb * sclamp(local_ratio, 0.95f, 1.08f);
@@ -326,17 +354,17 @@ struct OpLoca {
 // from the planes where it is a candidate, and its result goes straight into
 // the interleaved image.
 struct OpLocaBlk {
-  static constexpr int NS = 2, NP = 3, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, BLK_WARPS = 6;
-  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr int NS = 2, NP = 3, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, BLK_WARPS = 4, BLK_PER_SM = 3;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 32, BLK_COLS = 96;
   static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = true;
   __device__ static bool site(int, int, const Geo&) { return true; }
   template <class T>
   __device__ static void cell(const T& t, int, const Geo& g) {
     if (t.input(2) == 0.f) return;
-    const float thr = g.aux[0];
+    const float thr = g.auxv[0];
     float p0 = __ldg(g.ex[0] + t.px), p1 = __ldg(g.ex[1] + t.px), p2 = __ldg(g.ex[2] + t.px);
     if (loca_lift([&](int dy, int dx) { return t.get(0, dy, dx); }, [&](int dy, int dx) { return t.get(1, dy, dx); },
-                  thr, g.aux[1], p0, p1, p2)) {
+                  thr, g.auxv[1], p0, p1, p2)) {
       const float n = smax(p0, smax(p1, p2));
       t.set(0, n);
       t.set(1, loca_ratio(p0, p1, p2, n, thr));
@@ -354,6 +382,19 @@ struct OpLocaBlk {
 __global__ void k_hl_aux(float* scal, float thr) {
   scal[3] = thr;
   scal[4] = scal[2];
+}
+
+// The planes of the in-order sweep at the pixels that loop 4 leaves alone
+// (`out` holds those; the candidates' are there), where it has to run.
+__global__ void k_hl_planes(const float* __restrict__ out, const float* __restrict__ cand, float* __restrict__ R,
+                            float* __restrict__ G, float* __restrict__ B, size_t n, const int* __restrict__ run_if) {
+  if (*run_if == 0) return;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    if (cand[i] != 0.f) continue;
+    R[i] = out[i * 3];
+    G[i] = out[i * 3 + 1];
+    B[i] = out[i * 3 + 2];
+  }
 }
 
 // The in-order sweep's planes into the result, where it had to run.
@@ -420,12 +461,14 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
     return check_launch(c, what);
   };
   LRE_CUDA_TRY(c, cudaMemsetAsync(scal, 0, 256, s));
-  k_hl_pass1<<<(unsigned)nb, kHlBlock, 0, s>>>(in, n, P, mask_out, flags, counts);
+  int* total = reinterpret_cast<int*>(scal + 8);  // terms of the ratio means
+  k_hl_pass1<<<(unsigned)nb, kHlBlock, 0, s>>>(in, n, P, mask_out, flags, counts, total);
   LRE_TRY(ck("recover_highlights"));
-  k_hl_scan<<<1, 1024, 0, s>>>(counts, (int)nb, offs);
+  k_hl_scan<<<1, 1024, 0, s>>>(counts, (int)nb, offs, total);
   LRE_TRY(ck("recover_highlights"));
   // the compacted terms live in R2/G2, which are free until loop 3
-  k_hl_compact<<<(unsigned)nb, kHlBlock, 0, s>>>(in, n, flags, offs, R2, G2);
+  k_hl_compact<<<(unsigned)std::min<size_t>(nb, (size_t)c->sm_count * 8), kHlBlock, 0, s>>>(in, n, flags, offs, R2, G2,
+                                                                                       total, (int)nb);
   LRE_TRY(ck("recover_highlights"));
   k_hl_ratio_sums<<<1, 32, 0, s>>>(R2, G2, offs + nb, scal);
   LRE_TRY(ck("recover_highlights"));
@@ -472,6 +515,8 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
     return LRE_OK;
   }
   LRE_TRY(blk_sweep<OpLocaBlk>(c, b, blk_ws, blk_len, &sa.run_if, "recover_highlights_loca"));
+  k_hl_planes<<<g1, 256, 0, s>>>(out, HL, R2, G2, B2, n, sa.run_if);
+  LRE_TRY(ck("recover_highlights"));
   LRE_TRY(sweep_in_order<OpLoca>(c, sa, sync, nb_max, "recover_highlights_loca"));
   k_hl_interleave<<<g1, 256, 0, s>>>(R2, G2, B2, out, n, sa.run_if);
   LRE_TRY(ck("recover_highlights"));

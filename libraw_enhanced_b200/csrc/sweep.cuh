@@ -25,7 +25,8 @@
 // An op supplies NS state planes + inputs (NP planes per warp), HALO, SKEW,
 // PAIR, NCH (independent channels run as separate warps), LAG (how many
 // columns behind its walk position a cell may still write), RING (ring
-// columns, a power of two), BLK_WARPS (warps of a block), BLK_ROWS and
+// columns, a power of two), BLK_WARPS (warps of a block), BLK_PER_SM (resident
+// blocks per SM), BLK_ROWS and
 // BLK_COLS (a block's overlap), BLK_SKEW and BLK_PAIR (a block's own skew),
 // UNROLL (whether a block's group of steps is unrolled), STEP2 (a block visits
 // every second step only, from phase(r0, g) on), IDLE0 (sites whose inputs are
@@ -54,6 +55,7 @@ struct Geo {
   const float* aux;  // optional device scalars an op reads (nullptr when unused)
   const float* ex[3];  // optional planes an op reads at its own sites only
   float* ex_out;       // and where it writes for the sites its block owns
+  float auxv[2];       // aux[0], aux[1], read once by a block
   __device__ __forceinline__ unsigned fc(int r, int c) const { return fcol3((unsigned)r, (unsigned)c, filters); }
   __device__ __forceinline__ size_t at(int r, int c) const { return (size_t)r * W + c; }
 };
@@ -381,6 +383,8 @@ struct Blk {
   static constexpr int NI = Op::NP - Op::NS, IPITCH = kBlkGroup + 1, IPLANE = ROWS * IPITCH;
   static constexpr int INPUTS = Op::NS * PLANE;  // where the input buffers start
   static constexpr size_t BYTES = (size_t)(INPUTS + NI * IPLANE) * sizeof(float);
+  static constexpr int PER_SM = Op::BLK_PER_SM;  // resident blocks, by shared memory and registers
+  static_assert(PER_SM * (BYTES + 1024) <= 227 * 1024, "blocks per SM");
   static constexpr int SKEW = Op::BLK_SKEW, PAIR = Op::BLK_PAIR;
   // skew of a row relative to the block's first one (floor division)
   __host__ __device__ static constexpr int skew(int lr) { return SKEW * (PAIR == 2 ? (lr >> 1) : lr); }
@@ -434,7 +438,7 @@ struct BlkCellAny {
 };
 
 template <class Op, bool REPAIR>
-__global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
+__global__ void __launch_bounds__(Blk<Op>::NW * 32, Blk<Op>::PER_SM) k_blk_sweep(BlkArgs a) {
   using B = Blk<Op>;
   constexpr int G = kBlkGroup, NP = Op::NP, NS = Op::NS, HALO = Op::HALO, NCH = Op::NCH, KR = Op::BLK_ROWS;
   if (a.skip_if_zero && *a.skip_if_zero == 0) return;
@@ -515,8 +519,8 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
       for (int p = 0; p < NS; p++) sweep_smem[p * B::PLANE + (lrh + HALO) * B::PITCH + tr] = vh[p];
     }
   };
-  // Returns whether any input of the warp's group is non-zero.
-  auto store_inputs = [&]() {
+  // Returns whether any input of the warp's group is non-zero (g: that group).
+  auto store_inputs = [&](int g) {
     const unsigned sl = B::INPUTS + lr8 * B::IPITCH + l8;
     bool any = false;
 #pragma unroll
@@ -525,6 +529,12 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
       for (int p = NS; p < NP; p++) {
         sweep_smem[sl + (p - NS) * B::IPLANE + k * B::IPITCH] = v[k][p];
         any |= v[k][p] != 0.f;
+        if (Op::IDLE0 && v[k][p] != 0.f) {
+          // what the op will read at this site, on its way to L1
+          const ptrdiff_t px = (ptrdiff_t)(r0 + lr8 + k) * W + g * G + l8 - B::skew(lr8 + k);
+#pragma unroll
+          for (int e = 0; e < 3; e++) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.g.ex[e] + px));
+        }
       }
     return Op::IDLE0 ? __any_sync(0xffffffffu, any) != 0 : true;
   };
@@ -585,6 +595,10 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
     flush(g_lo - 2);
     flush(g_lo - 1);
   }
+  if (a.g.aux) {
+    a.g.auxv[0] = a.g.aux[0];
+    a.g.auxv[1] = a.g.aux[1];
+  }
   const int lr = warp * 32 + lane, r = r0 + lr;
   const bool row_on = r >= a.r_lo && r <= a.r_hi && (!REPAIR || lr >= KR);
   const unsigned srow = (lr + HALO) * B::PITCH, irow = B::INPUTS + lr * B::IPITCH;
@@ -592,7 +606,7 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, 2) k_blk_sweep(BlkArgs a) {
     const int g = g_lo + k - warp;
     if (k >= warp && k - warp < ng) {
       store(g + 5);
-      const bool busy = store_inputs();
+      const bool busy = store_inputs(g);
       __syncwarp();
       load(g + 1, zs, zp);
       load(g + 6, z0, zs);
@@ -707,7 +721,7 @@ __global__ void k_blk_copy(BlkArgs a, const int* run_if, int back) {
 }
 
 // Owned steps per block: what takes the fewest phases over all waves of
-// blocks (two per SM).  A wide block spends less on overlap, a narrow one
+// blocks (PER_SM per SM, two for most ops).  A wide block spends less on overlap, a narrow one
 // fills the last wave: at 24 MP (21 rows of blocks) 512 gives one wave of 84
 // phases, 256 two of 52.
 constexpr int kBlkSms = 148;  // the grid shape is also planned without a device
@@ -719,7 +733,8 @@ void blk_grid(int W, int H, int* S, int* nbj, int* nbi) {
   long long best = LLONG_MAX;
   for (int t = 64; t <= 2048; t += 64) {
     const long long n = (long long)((steps + t - 1) / t) * *nbi * Op::NCH;
-    const long long cost = (n + 2 * kBlkSms - 1) / (2 * kBlkSms) * ((t + Op::BLK_COLS) / kBlkGroup + B::NW);
+    constexpr long long places = (long long)B::PER_SM * kBlkSms;
+    const long long cost = (n + places - 1) / places * ((t + Op::BLK_COLS) / kBlkGroup + B::NW);
     if (cost < best) {
       best = cost;
       *S = t;
