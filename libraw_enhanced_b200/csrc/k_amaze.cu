@@ -16,7 +16,8 @@
 //     pmwt -- that aliasing is reproduced explicitly below (dirwts1_eff).
 //
 // Device design: a persistent CTA per SM pulls the reference's tiles from a
-// counter and runs each one stage by stage.
+// counter and runs each one stage by stage; an image of fewer tiles than SMs
+// gives each tile a cluster of two to eight CTAs.
 //   * Scratch: one slab per CTA of 6 full planes (160x160 floats) plus one
 //     half plane; the reference's ~20 planes are mapped onto it by lifetime
 //     (a plane is reused once its last reader has run), the cheap gradient
@@ -259,6 +260,42 @@ __device__ __forceinline__ void weight_sweep(float* w, int a, int rr1, int cc1, 
   }
 }
 
+// Thread-block cluster: rank, split barrier, and a store into the same place of
+// every other CTA's shared memory.
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// (not .aligned: stage 6 arrives from different places of the code)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ unsigned cluster_map(const void* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_store(unsigned a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned a, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned a, unsigned char v) {
+  asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(a), "r"((unsigned)v) : "memory");
+}
+template <int CL, class T>
+__device__ __forceinline__ void put_remote(T* p, T v, int rank) {
+#pragma unroll
+  for (int d = 1; d < CL; d++) cluster_store(cluster_map(p, (rank + d) % CL), v);
+}
+
+// CL = 2, 4 or 8: the CTAs of a cluster share a tile.  Every loop over sites is
+// split over all their threads, the slab is common, and what lives in shared
+// memory (cfa, hvwt, pmwt, the nyquist maps) is kept whole in each of them: a
+// store goes to every copy (put).  Barriers are the cluster's.  The weight
+// sweeps run in each CTA on its own copy.
+template <int CL>
 __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
   const int v1 = TS, v2 = 2 * TS, v3 = 3 * TS, p1 = -TS + 1, p2 = -2 * TS + 2, p3 = -3 * TS + 3, m1 = TS + 1,
             m2 = 2 * TS + 2, m3 = 3 * TS + 3;
@@ -267,17 +304,32 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
   float* pmwt = smem + HALF;  // [HALF]
   float* cfa = smem + 2 * HALF;  // [TS2], read by nearly every stage
   const int tid = threadIdx.x, nth = blockDim.x;
+  const int rank = CL > 1 ? (int)cluster_rank() : 0;
+  const int gt = tid + rank * AMZ_THREADS, gn = CL * AMZ_THREADS;  // this thread among the tile's, and their number
+  auto bar = []() {
+    if (CL > 1) {
+      cluster_arrive();
+      cluster_wait();
+    } else {
+      __syncthreads();
+    }
+  };
+  auto put = [&](auto* p, auto v) {
+    *p = v;
+    if (CL > 1) put_remote<CL>(p, v, rank);
+  };
   const int W = A.W, H = A.H;
-  const Slab S = make_slab(A.scratch + (size_t)blockIdx.x * kSlabBytes, cfa);
+  const Slab S = make_slab(A.scratch + (size_t)(blockIdx.x / CL) * kSlabBytes, cfa);
   __shared__ int s_tile;
   __shared__ int s_doNyq;
   float mg = 0.f;  // max G of this thread's interior outputs
 
-  if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);
-  __syncthreads();
+  bar();  // every CTA of the cluster runs before another one stores into it
+  if (gt == 0) put(&s_tile, atomicAdd(A.tile_counter, 1));
+  bar();
   for (int tile = A.tile_lo + s_tile; tile < A.tile_hi;) {
-    __syncthreads();  // every thread has read s_tile
-    if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);  // the next tile
+    bar();  // every thread has read s_tile
+    if (gt == 0) put(&s_tile, atomicAdd(A.tile_counter, 1));  // the next tile
     const int top = -16 + (tile / A.n_left) * (TS - 32);
     const int left = -16 + (tile % A.n_left) * (TS - 32);
     const int bottom = min(top + TS, H + 16);
@@ -292,7 +344,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
 
     // ---- zero what this tile reads before writing (fresh-buffer semantics)
     // the 4-px frame of the stage-2 planes: eight rows, then eight columns
-    for (int i = tid; i < 8 * (rr1 + cc1); i += nth) {
+    for (int i = gt; i < 8 * (rr1 + cc1); i += gn) {
       int rr, cc;
       if (i < 8 * cc1) {
         rr = fdc.div(i);
@@ -312,20 +364,20 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     }
     if ((rrmin > 0 || rrmax < rr1) && (ccmin > 0 || ccmax < cc1)) {
       // unfilled 16x16 apron corners (:1326)
-      for (int i = tid; i < rr1 * cc1; i += nth) {
+      for (int i = gt; i < rr1 * cc1; i += gn) {
         const int rr = fdc.div(i), cc = i - rr * cc1;
         const bool rc = (rrmin > 0 && rr < 16) || (rrmax < rr1 && rr >= rrmax);
         const bool cc_ = (ccmin > 0 && cc < 16) || (ccmax < cc1 && cc >= ccmax);
-        if (rc && cc_) cfa[rr * TS + cc] = 0.f;
+        if (rc && cc_) put(&cfa[rr * TS + cc], 0.f);
       }
     }
-    __syncthreads();
+    bar();
 
     // ---- fill (:1254-1326); the right apron is written last, wrapping into
     // the next row when ccmax + 16 exceeds the tile width, as the reference's
     // flat buffer does
     const float scale = A.scale;
-    for (int i = tid; i < rr1 * cc1; i += nth) {
+    for (int i = gt; i < rr1 * cc1; i += gn) {
       const int rr = fdc.div(i), cc = i - rr * cc1;
       int srow = -1, scol = -1;
       if (rr >= rrmin && rr < rrmax && cc >= ccmin && cc < ccmax) {
@@ -344,22 +396,22 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         srow = min(max(top + rr, 0), H - 1);
         scol = min(max(W - (cc - ccmax) - 2, 0), W - 1);
       }
-      if (srow >= 0) cfa[rr * TS + cc] = raw_at(A, srow, scol) * scale;
+      if (srow >= 0) put(&cfa[rr * TS + cc], raw_at(A, srow, scol) * scale);
     }
     if (ccmax < cc1 && ccmax + 16 > TS) {
-      __syncthreads();
-      for (int i = tid; i < (rrmax - rrmin) * 16; i += nth) {
+      bar();
+      for (int i = gt; i < (rrmax - rrmin) * 16; i += gn) {
         const int rr = rrmin + i / 16, k = i % 16;
         if (ccmax + k < TS || rr + 1 >= TS) continue;
         const int srow = min(max(top + rr, 0), H - 1);
         const int scol = min(max(W - k - 2, 0), W - 1);
-        cfa[(rr + 1) * TS + (ccmax + k - TS)] = raw_at(A, srow, scol) * scale;
+        put(&cfa[(rr + 1) * TS + (ccmax + k - TS)], raw_at(A, srow, scol) * scale);
       }
     }
-    __syncthreads();
+    bar();
 
     // ---- S2 colour differences (:1341-1373); S1 planes recomputed
-    for (int i = tid; i < (rr1 - 8) * (cc1 - 8); i += nth) {
+    for (int i = gt; i < (rr1 - 8) * (cc1 - 8); i += gn) {
       const int q_ = fd8.div(i), rr = 4 + q_, cc = 4 + i - q_ * (cc1 - 8);
       const int idx = rr * TS + cc;
       const int sgn = (fc_rt(A, rr, cc) & 1) ? -1 : 1;
@@ -402,7 +454,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       S.dgintv[idx] = fminf(SQR(guha - gdha), SQR(guar - gdar));
       S.dginth[idx] = fminf(SQR(glha - grha), SQR(glar - grar));
     }
-    __syncthreads();
+    bar();
 
     // ---- S3 (:1375-1398): hcd chains along rows, vcd chains down columns,
     // each in the reference's scan order.  Every operand of a step except
@@ -426,10 +478,11 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
           }
         }
       }
-      __syncthreads();
+      bar();
       const int warp = tid >> 5, lane = tid & 31;
       constexpr int G = 8;  // sites of one chain per group
-      if (warp < S3_ROW_WARPS) {
+      const int cw = warp * CL + rank;  // chain warps, dealt over the tile's CTAs
+      if (cw < S3_ROW_WARPS) {
         // Row chains: a warp takes 16 rows, the two chains of a row on
         // neighbouring lanes.  16 columns (8 sites of each chain) and two
         // columns of look-ahead at a time go through a buffer of the warp's
@@ -438,7 +491,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         // bounded the stage (91 k of a tile's cycles; 80 k this way, 60 k with
         // the cases of s3_finish selected instead of branched to).
         float* buf = smem + kSmemBytes / 4 + warp * S3_BUF;  // [2][16][S3_LD]
-        const int line0 = 4 + 16 * warp, line = line0 + (lane >> 1), par = lane & 1;
+        const int line0 = 4 + 16 * cw, line = line0 + (lane >> 1), par = lane & 1;
         const bool on = line < rr1 - 4;
         const int pos0 = 4 + par;
         const bool green = (fc_rt(A, line, pos0) & 1) != 0;
@@ -504,7 +557,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         // colour, so a warp's lanes take the same branches and read
         // consecutive columns of one row.
         const int nlv = cc1 - 8;
-        for (int it = tid - 32 * S3_ROW_WARPS; it < 2 * nlv; it += nth - 32 * S3_ROW_WARPS) {
+        for (int it = 32 * (cw - S3_ROW_WARPS) + lane; it < 2 * nlv; it += gn - 32 * S3_ROW_WARPS) {
           const int grp = it >= nlv;
           const int line = 4 + (grp ? it - nlv : it);
           const int par = grp ? 1 - (line & 1) : (line & 1);
@@ -541,15 +594,15 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         }
       }
     }
-    __syncthreads();
-    for (int i = tid; i < 2 * HALF / 16; i += nth)
+    bar();
+    for (int i = tid; i < 2 * HALF / 16; i += nth)  // each CTA its own maps
       reinterpret_cast<float4*>(S.nyquist)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // cddiffsq at R/B sites (read only there by stage 4/5), half-indexed
     auto rb_count = [&](int a) { return (cc1 - a - a + 1) / 2 + 1; };
     {
       const int per_row = rb_count(4);
       const FDiv fdr(per_row);
-      for (int i = tid; i < (rr1 - 8) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 8) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = 4 + q_;
         const int cc = 4 + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - 4) continue;
@@ -558,14 +611,14 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       }
     }
     if (tid == 0) s_doNyq = 0;
-    __syncthreads();
+    bar();
 
     // ---- S4/5 directional variance + Nyquist test (:1400-1433)
     {
       const int a = 6;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -596,8 +649,8 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         const float hcdvar1 = epssq + hwt * Dgrbhvarr2 + (1.f - hwt) * Dgrbhvarl2;
         const float varwt = hcdvar / (vcdvar + hcdvar);
         const float diffwt = hcdvar1 / (vcdvar1 + hcdvar1);
-        hvwt[idx >> 1] =
-            ((0.5f - varwt) * (0.5f - diffwt) > 0.f && fabsf(0.5f - diffwt) < fabsf(0.5f - varwt)) ? varwt : diffwt;
+        put(&hvwt[idx >> 1],
+            ((0.5f - varwt) * (0.5f - diffwt) > 0.f && fabsf(0.5f - diffwt) < fabsf(0.5f - varwt)) ? varwt : diffwt);
         const float* cdd = S.cddiffsq;  // half-indexed; every tap is an R/B site
         auto dh = [&](int o) { return delhvsqsum_at(cfa, idx + o); };
         const float nt =
@@ -611,12 +664,12 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
                              dh(v2 - 1) + dh(v2 + 1)) +
              gaussgrad[5] * (dh(-m2) + dh(p2) + dh(-p2) + dh(m2)));
         if (nt > 0.f) {
-          S.nyquist[idx >> 1] = 1;
-          s_doNyq = 1;
+          put(&S.nyquist[idx >> 1], (unsigned char)1);
+          put(&s_doNyq, 1);
         }
       }
     }
-    __syncthreads();
+    bar();
     const bool doNyquist = s_doNyq != 0;
 
     // ---- S6 Nyquist refinement + green (:1435-1481)
@@ -624,7 +677,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       const int a = 8;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -632,10 +685,10 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         const unsigned char* nq = S.nyquist;
         const unsigned nqsum = nq[(idx - v2) >> 1] + nq[(idx - m1) >> 1] + nq[(idx + p1) >> 1] + nq[(idx - 2) >> 1] +
                                nq[(idx + 2) >> 1] + nq[(idx - p1) >> 1] + nq[(idx + m1) >> 1] + nq[(idx + v2) >> 1];
-        S.nyquist2[idx >> 1] = nqsum > 4 ? 1 : (nqsum < 4 ? 0 : nq[idx >> 1]);
+        put(&S.nyquist2[idx >> 1], (unsigned char)(nqsum > 4 ? 1 : (nqsum < 4 ? 0 : nq[idx >> 1])));
       }
-      __syncthreads();
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      bar();
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -660,9 +713,9 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         areawt = xdiv2f(areawt);
         const float hcdvar2 = epssq + fabsf(areawt * sumsqh - sumh * sumh);
         const float vcdvar2 = epssq + fabsf(areawt * sumsqv - sumv * sumv);
-        hvwt[idx >> 1] = hcdvar2 / (vcdvar2 + hcdvar2);
+        put(&hvwt[idx >> 1], hcdvar2 / (vcdvar2 + hcdvar2));
       }
-      __syncthreads();
+      bar();
     }
     // ---- S7/S8 diagonal R/B interpolation (:1483-1532); pmwt into SMEM.  The
     // R/B gradient planes of stage 7 are formed from cfa where they are read.
@@ -678,7 +731,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       auto delp = [&](int x) { return fabsf(cfa[x + p1] - cfa[x - p1]); };
       auto Dq1m = [&](int x) { return SQR(cfa[x] - cfa[x - m1]) + SQR(cfa[x] - cfa[x + m1]); };  // at G sites
       auto Dq1p = [&](int x) { return SQR(cfa[x] - cfa[x - p1]) + SQR(cfa[x] - cfa[x + p1]); };
-      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
+      for (int i = tid - 32 + rank * (AMZ_THREADS - 32); i < (rr1 - 2 * a) * per_row; i += CL * (AMZ_THREADS - 32)) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -727,20 +780,24 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
                      gausseven[1] * (Dq1p(idx - v2 - 1) + Dq1p(idx - v2 + 1) + Dq1p(idx - 2 - v1) +
                                      Dq1p(idx + 2 - v1) + Dq1p(idx - 2 + v1) + Dq1p(idx + 2 + v1) +
                                      Dq1p(idx + v2 - 1) + Dq1p(idx + v2 + 1)));
-        pmwt[idx1] = rbvarm / (rbvarp + rbvarm);
+        put(&pmwt[idx1], rbvarm / (rbvarp + rbvarm));
       }
     }
-    __syncthreads();
+    bar();
 
     // ---- S6 green / Dgrb2 per site from the swept hvwt, then the Nyquist
     // sites' green (:1456-1481), while warp 0 sweeps pmwt (:1534-1542)
+    // (a cluster's barrier counts every thread: warp 0 arrives at once and
+    // waits after its sweep)
     if (tid < 32) {
+      if (CL > 1 && doNyquist) cluster_arrive();
       weight_sweep(pmwt, 10, rr1, cc1, par0);
+      if (CL > 1 && doNyquist) cluster_wait();
     } else {
       const int a = 8;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
+      for (int i = tid - 32 + rank * (AMZ_THREADS - 32); i < (rr1 - 2 * a) * per_row; i += CL * (AMZ_THREADS - 32)) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -756,10 +813,15 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         S.Dgrb2v[idx >> 1] = nq2 ? SQR(g - xdiv2f(cfa[idx - v1] + cfa[idx + v1])) : 0.f;
       }
       if (doNyquist) {
-        asm volatile("bar.sync 1, %0;" ::"n"(AMZ_THREADS - 32) : "memory");
+        if (CL > 1) {
+          cluster_arrive();
+          cluster_wait();
+        } else {
+          asm volatile("bar.sync 1, %0;" ::"n"(AMZ_THREADS - 32) : "memory");
+        }
       const float* D2h = S.Dgrb2h;
       const float* D2v = S.Dgrb2v;
-      for (int i = tid - 32; i < (rr1 - 2 * a) * per_row; i += nth - 32) {
+      for (int i = tid - 32 + rank * (AMZ_THREADS - 32); i < (rr1 - 2 * a) * per_row; i += CL * (AMZ_THREADS - 32)) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -781,14 +843,14 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       }
     }
     }
-    __syncthreads();
+    bar();
 
     // ---- S9 (:1543-1592): rbint
     {
       const int a = 10;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -799,8 +861,8 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     }
     // Dgrb1 starts as zeros (its unwritten cells are read by the diagonal
     // step); it occupies Dgrb2h's half plane, dead after stage 6
-    for (int i = tid; i < HALF / 4; i += nth) reinterpret_cast<float4*>(S.Dgrb1)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
+    for (int i = gt; i < HALF / 4; i += gn) reinterpret_cast<float4*>(S.Dgrb1)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    bar();
     // dirwts1 as the reference reads it after pmwt was stored over it
     // (half index k of pmwt == float offset k of dirwts1).
     auto pm_written = [&](int p) -> bool {
@@ -816,7 +878,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
       const float* rbint = S.rbint;
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -858,14 +920,14 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         S.Dgrb0[idx1] = g - cfa[idx];
       }
     }
-    __syncthreads();
+    bar();
 
     const int next_tile = A.tile_lo + s_tile;
     if (next_tile < A.tile_hi && A.cstride == 1) {
       // the next tile's samples on their way to L2 (rows of at most six lines)
       const int ntop = -16 + (next_tile / A.n_left) * (TS - 32), nleft = -16 + (next_tile % A.n_left) * (TS - 32);
       const int row = ntop + tid / 6, col = nleft + 32 * (tid % 6);
-      if (tid < 6 * TS && row >= 0 && row < H && col < nleft + TS + 31) {
+      if (rank == 0 && tid < 6 * TS && row >= 0 && row < H && col < nleft + TS + 31) {
         const int c = min(max(col, 0), W - 1);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(A.raw + (size_t)row * W + c));
       }
@@ -875,7 +937,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       const int r0 = 13 - A.ey;
       const int nrows = (rr1 - 12 - r0 + 1) / 2;
       const int k0 = 13 - A.ex;
-      for (int i = tid; i < nrows * TSH; i += nth) {
+      for (int i = gt; i < nrows * TSH; i += gn) {
         const int rr = r0 + 2 * (i / TSH);
         if (rr >= rr1 - 12) continue;
         const int lo = (rr * TS + k0) >> 1, hi = (rr * TS + cc1 - 12) >> 1;
@@ -885,13 +947,13 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         S.Dgrb0[idx1] = 0;
       }
     }
-    __syncthreads();
+    bar();
     // Diagonal chroma interpolation (:1570-1587).
     {
       const int a = 14;
       const int per_row = rb_count(a);
       const FDiv fdr(per_row);
-      for (int i = tid; i < (rr1 - 2 * a) * per_row; i += nth) {
+      for (int i = gt; i < (rr1 - 2 * a) * per_row; i += gn) {
         const int q_ = fdr.div(i), rr = a + q_;
         const int cc = a + (fc_rt(A, rr, 2) & 1) + 2 * (i - q_ * per_row);
         if (cc >= cc1 - a) continue;
@@ -914,10 +976,10 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
             (wtnw + wtne + wtsw + wtse);
       }
     }
-    __syncthreads();
+    bar();
 
     // ---- S10 output (:1594-1625)
-    for (int i = tid; i < (rr1 - 32) * (cc1 - 32); i += nth) {
+    for (int i = gt; i < (rr1 - 32) * (cc1 - 32); i += gn) {
       const int q_ = fd32.div(i), rr = 16 + q_, cc = 16 + i - q_ * (cc1 - 32);
       const int row = rr + top, col = cc + left;
       if (row < 0 || row >= H || col < 0 || col >= W) continue;
@@ -950,7 +1012,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
       __stcs(o + 2, fmaxf(0.f, b));
       if (row >= 4 && row < H - 4 && col >= 4 && col < W - 4) mg = fmaxf(mg, fmaxf(0.f, g));
     }
-    __syncthreads();
+    bar();
     tile = next_tile;
   }
   // every thread leaves the tile loop together (s_tile is shared)
@@ -1062,15 +1124,40 @@ lre_status launch_amaze_rows(Context* c, AmazeArgs A, int row_lo, int row_hi) {
   A.tile_hi = row_hi * A.n_left;
   const int tiles = A.tile_hi - A.tile_lo;
   if (tiles <= 0) return LRE_OK;
-  int nblk = std::min(tiles, c->sm_count);
-  if (nblk < 1) nblk = 1;
+  // CTAs per tile: what takes the least time over all rounds.  One tile at a
+  // time takes 270 us with one CTA, 190 with two, 137 with four, 117 with
+  // eight (511x341 to 1536x1024); clusters of four and eight lie inside a GPC,
+  // which leaves 32 and 16 places.
+  const int sms = c->sm_count;
+  constexpr int cls[4] = {1, 2, 4, 8}, cost[4] = {100, 70, 51, 43};
+  const int places[4] = {sms, sms / 2, sms * 32 / 148, sms * 16 / 148};
+  int pick = 0;
+  for (int j = 1; j < 4; j++) {
+    auto rounds = [&](int q) { return (tiles + places[q] - 1) / places[q] * cost[q]; };
+    if (places[j] > 0 && rounds(j) < rounds(pick)) pick = j;
+  }
+  const int cl = cls[pick];
+  const int nblk = std::min(tiles, std::max(1, places[pick]));  // tiles in work at a time
   const size_t mark = c->ws.used();
   A.scratch = reinterpret_cast<unsigned char*>(c->ws.take((size_t)nblk * kSlabBytes));
   A.tile_counter = reinterpret_cast<int*>(c->ws.take(256));
   if (!A.scratch || !A.tile_counter) return fail(c, LRE_ERR_OUT_OF_MEMORY, "demosaic_bayer_amaze: workspace too small");
   LRE_CUDA_TRY(c, cudaMemsetAsync(A.tile_counter, 0, sizeof(int), c->stream));
-  LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_amaze, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal));
-  k_amaze<<<nblk, AMZ_THREADS, kSmemTotal, c->stream>>>(A);
+  auto kernel = cl == 1 ? k_amaze<1> : (cl == 2 ? k_amaze<2> : (cl == 4 ? k_amaze<4> : k_amaze<8>));
+  LRE_CUDA_TRY(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemTotal));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nblk * cl));
+  cfg.blockDim = dim3(AMZ_THREADS);
+  cfg.dynamicSmemBytes = kSmemTotal;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cl;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cl > 1 ? 1 : 0;
+  LRE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kernel, A));
   count_launch(c);
   c->ws.rewind(mark);
   return check_launch(c, "demosaic_bayer_amaze");
