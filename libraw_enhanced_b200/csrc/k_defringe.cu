@@ -424,11 +424,29 @@ lre_status run_blur_strip(Context* c, const BlurJob& job, const GaussTaps& taps,
   using B = BlurStrip<KS>;
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_strip<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::SMEM));
   // Batches per chunk: a chunk's first 2 KS rows produce nothing, so tall
-  // chunks, halved while the grid has fewer than twelve CTAs per SM.
+  // chunks, halved while the grid has fewer than twelve CTAs per SM.  Where
+  // even halves leave fewer than that (six are resident, so at most two waves),
+  // what takes the fewest batch steps over all waves, a nearly empty last one
+  // counting as much as a full one: the three blurs of 1.9 MP took 104 us
+  // halved and 88 us so; of 24 and 51 MP 839 and 1732 us halved and 859 and
+  // 1774 us by waves, whose CTAs don't run in step when there are many.
   int batches = c->tune.blur_tile == 64 ? 32 : 16;
+  const int tallest = batches;
   const int strips = (W + BS_X - 1) / BS_X;
   auto chunks = [&](int n) { return (H + n * B::P - 2 * KS - 1) / (n * B::P - 2 * KS); };
-  while (batches > 2 && (long long)strips * chunks(batches) * job.np < 12LL * c->sm_count) batches /= 2;
+  auto ctas = [&](int n) { return (long long)strips * chunks(n) * job.np; };
+  const long long places = 6LL * c->sm_count;
+  while (batches > 2 && ctas(batches) < 2 * places) batches /= 2;
+  if (batches <= 4) {
+    double least = 1e300;
+    for (int n = 2; n <= tallest; n++) {
+      const double cost = (double)((ctas(n) + places - 1) / places) * (n + 0.5);
+      if (cost <= least) {
+        least = cost;
+        batches = n;
+      }
+    }
+  }
   const dim3 grid((unsigned)strips, (unsigned)chunks(batches), (unsigned)job.np);
   k_df_blur_strip<KS><<<grid, BS_THREADS, B::SMEM, c->stream>>>(job, taps, W, H, batches, sc);
   count_launch(c);
@@ -1257,9 +1275,12 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
   j3.in[1] = P.sbs; j3.mode[1] = BS_PLANE; j3.out[1] = P.sbb;
   LRE_TRY(run_blur(c, j3, taps, W, H, sc));
 
+  // Eight times the resident CTAs: the work of a pixel depends on what it shows,
+  // and CTAs that took a sixth of an SM's share each left SMs idle at the end
+  // (51 MP 1110 us with 6 per SM, 997 us with 48; 26 MP odd 1261 and 1183 us).
   auto main_pass = fast ? k_df_main<true> : k_df_main<false>;
-  main_pass<<<grid_for((n + 3) / 4, DFM_THREADS, c->sm_count * 6), DFM_THREADS, 0, c->stream>>>(in, out, W, H, P, k, T,
-                                                                                               sc, out_max_g);
+  main_pass<<<grid_for((n + 3) / 4, DFM_THREADS, c->sm_count * 48), DFM_THREADS, 0, c->stream>>>(in, out, W, H, P, k,
+                                                                                                T, sc, out_max_g);
   count_launch(c);
   return check_launch(c, "defringe main");
 }
