@@ -12,6 +12,13 @@
 // equations in double with warp shuffles, and thread 0 solves and broadcasts
 // the step, so all LK iterations of a cell stay on chip.  Gate + smoothing
 // run in one small kernel; the remap is a streaming kernel.
+//
+// The estimate waits for its nine loads of a pixel.  What bought time was more
+// of them in flight: four pixels per turn of the loop, five CTAs per SM, no
+// clamps where the whole displaced cell lies inside, the pixel's row by a
+// multiply-high, and the matrix summed in the first iteration only.  The three
+// levels of 26 MP: 945 us before, 682 us now; of 1.9 MP 89 us, 70 us.
+// (Three CTAs per SM with the same loop: 1135 us, the loads no longer hidden.)
 #include <algorithm>
 #include <cmath>
 
@@ -31,6 +38,59 @@ __global__ void k_split_planes(const float* __restrict__ rgb, float* __restrict_
     G[i] = rgb[i * 3 + 1];
     B[i] = rgb[i * 3 + 2];
   }
+}
+
+// Split and the first 2x box in one pass, a thread per 2x2 block (the last one
+// of an odd side holds one column or row, which has no box): the box no longer
+// reads the planes back.  Bound by its 27 B per pixel.  vec: rgb is 8-byte
+// aligned, so a row that starts at an even pixel moves in pairs of floats.
+// 26 MP: split and boxes 105 + 90 us before, 130 us.
+__global__ void __launch_bounds__(256) k_split_down(const float* __restrict__ rgb, float* __restrict__ R,
+                                                    float* __restrict__ G, float* __restrict__ B,
+                                                    float* __restrict__ r2, float* __restrict__ g2,
+                                                    float* __restrict__ b2, int W, int H, bool vec) {
+  const int W2 = W / 2, H2 = H / 2;
+  float* const out[3] = {R, G, B};
+  float* const box[3] = {r2, g2, b2};
+  for (int y = blockIdx.y * blockDim.y + threadIdx.y; y < H - H2; y += gridDim.y * blockDim.y)
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W - W2; x += gridDim.x * blockDim.x) {
+      const bool two_x = x < W2, two_y = y < H2;
+      float v[2][6];
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        if (r == 1 && !two_y) break;
+        const size_t i = (size_t)(2 * y + r) * W + 2 * x;
+        if (vec && two_x && (i & 1) == 0) {
+#pragma unroll
+          for (int q = 0; q < 3; q++) {
+            const float2 t = __ldg(reinterpret_cast<const float2*>(rgb + 3 * i) + q);
+            v[r][2 * q] = t.x;
+            v[r][2 * q + 1] = t.y;
+          }
+        } else {
+#pragma unroll
+          for (int q = 0; q < 6; q++) v[r][q] = q < 3 || two_x ? __ldg(rgb + 3 * i + q) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        if (r == 1 && !two_y) break;
+        const size_t i = (size_t)(2 * y + r) * W + 2 * x;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+          if (two_x && (i & 1) == 0) {
+            *reinterpret_cast<float2*>(out[q] + i) = make_float2(v[r][q], v[r][q + 3]);
+          } else {
+            out[q][i] = v[r][q];
+            if (two_x) out[q][i + 1] = v[r][q + 3];
+          }
+        }
+      }
+      if (two_x && two_y)
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+          box[q][(size_t)y * W2 + x] = 0.25f * (v[0][q] + v[0][q + 3] + v[1][q] + v[1][q + 3]);
+    }
 }
 
 struct Planes3 {
@@ -79,10 +139,10 @@ struct LkMaps {
 
 // One CTA per (cell, channel).  blockIdx.x = cell, blockIdx.y = channel
 // (0: R, 1: B).
-__global__ void __launch_bounds__(LK_THREADS) k_lk_level(const float* __restrict__ G, const float* __restrict__ Rt,
-                                                         const float* __restrict__ Bt, int W, int H, int map_w,
-                                                         int map_h, int max_iterations, float max_shift,
-                                                         float scale_down, float scale_up, LkMaps maps) {
+__global__ void __launch_bounds__(LK_THREADS, 5)
+    k_lk_level(const float* __restrict__ G, const float* __restrict__ Rt, const float* __restrict__ Bt, int W, int H,
+               int map_w, int map_h, int max_iterations, float max_shift, float scale_down, float scale_up,
+               LkMaps maps) {
   __shared__ double red[5][LK_THREADS / 32];
   __shared__ float s_acc[2];
   __shared__ int s_done;
@@ -112,29 +172,66 @@ __global__ void __launch_bounds__(LK_THREADS) k_lk_level(const float* __restrict
   }
   const int iw = (int)(x1 - x0) - 2, ih = (int)(y1 - y0) - 2;  // interior extent
   const int npx = iw * ih;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // k / iw by a multiply-high: exact while npx * iw < 2^32, which holds for
+  // every cell whose sides are below 1600 px (beyond, the division itself)
+  const unsigned iw_m = 0xFFFFFFFFu / (unsigned)iw + 1u;
+  const bool small = iw > 1 && iw < 1600 && ih < 1600;
   float min_eig_final = 0.f;
+  // The matrix of the normal equations depends on G alone, so the first
+  // iteration forms it for all (a lane's sums of later ones would be the same,
+  // bit for bit); later iterations sum the right-hand side only.
+  double A00 = 0.0, A01 = 0.0, A11 = 0.0;
   for (int iter = 0; iter < max_iterations; iter++) {
-    double A00 = 0.0, A01 = 0.0, A11 = 0.0, bx = 0.0, by = 0.0;
-    for (int k = threadIdx.x; k < npx; k += blockDim.x) {
-      const int y = (int)y0 + 1 + k / iw;
-      const int x = (int)x0 + 1 + k % iw;
-      const size_t i = (size_t)y * W + x;
-      const float gx = G[i + 1] - G[i - 1];
-      const float gy = G[i + W] - G[i - W];
-      const float t_warp = bilinear_plane(T, W, H, (float)x + accum_dx, (float)y + accum_dy);
-      const float err = t_warp - G[i];
-      A00 += (double)gx * gx;
-      A01 += (double)gx * gy;
-      A11 += (double)gy * gy;
-      bx -= (double)gx * err;
-      by -= (double)gy * err;
+    double bx = 0.0, by = 0.0;
+    // A pixel whose whole displaced cell lies inside the image needs no clamps.
+    const bool inside = (float)x0 + accum_dx >= 0.f && (float)(x1 + 1) + accum_dx < (float)W &&
+                        (float)y0 + accum_dy >= 0.f && (float)(y1 + 1) + accum_dy < (float)H;
+    auto sweep = [&](auto in, auto first) {
+      constexpr bool IN = decltype(in)::value, FIRST = decltype(first)::value;
+#pragma unroll 4
+      for (int k = threadIdx.x; k < npx; k += LK_THREADS) {
+        const int yy = small ? (int)__umulhi((unsigned)k, iw_m) : k / iw;
+        const int x = (int)x0 + 1 + k - yy * iw, y = (int)y0 + 1 + yy;
+        const size_t i = (size_t)y * W + x;
+        const float gc = G[i];
+        const float gx = G[i + 1] - G[i - 1];
+        const float gy = G[i + W] - G[i - W];
+        const float tx = (float)x + accum_dx, ty = (float)y + accum_dy;
+        float t_warp;
+        if (IN) {
+          const int xi = (int)tx, yi = (int)ty;
+          const float fx = tx - (float)xi, fy = ty - (float)yi;
+          const float* q = T + ((size_t)yi * W + xi);
+          t_warp = (q[0] * (1.f - fx) + q[1] * fx) * (1.f - fy) + (q[W] * (1.f - fx) + q[W + 1] * fx) * fy;
+        } else {
+          t_warp = bilinear_plane(T, W, H, tx, ty);
+        }
+        const float err = t_warp - gc;
+        const double dx = (double)gx, dy = (double)gy, de = (double)err;
+        if (FIRST) {
+          A00 += dx * dx;
+          A01 += dx * dy;
+          A11 += dy * dy;
+        }
+        bx -= dx * de;
+        by -= dy * de;
+      }
+    };
+    const std::true_type yes{};
+    const std::false_type no{};
+    if (inside) {
+      if (iter == 0) sweep(yes, yes); else sweep(yes, no);
+    } else {
+      if (iter == 0) sweep(no, yes); else sweep(no, no);
     }
-    A00 = warp_sum_d(A00);
-    A01 = warp_sum_d(A01);
-    A11 = warp_sum_d(A11);
+    if (iter == 0) {
+      A00 = warp_sum_d(A00);
+      A01 = warp_sum_d(A01);
+      A11 = warp_sum_d(A11);
+    }
     bx = warp_sum_d(bx);
     by = warp_sum_d(by);
-    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
       red[0][wid] = A00;
       red[1][wid] = A01;
@@ -239,46 +336,114 @@ struct ShiftMaps {
   const float* dy;
 };
 
-__device__ __forceinline__ void sample_shift(ShiftMaps m, int map_w, int map_h, float cell, float clamp_shift, float px,
-                                             float py, float& out_dx, float& out_dy) {
-  const float gx_f = (px / cell) - 0.5f;
-  const float gy_f = (py / cell) - 0.5f;
-  int gx0 = (int)floorf(gx_f);
-  int gy0 = (int)floorf(gy_f);
-  if (gx0 < 0) gx0 = 0;
-  if (gy0 < 0) gy0 = 0;
-  if (gx0 >= map_w - 1) gx0 = map_w - 2;
-  if (gy0 >= map_h - 1) gy0 = map_h - 2;
-  if (gx0 < 0) gx0 = 0;
-  if (gy0 < 0) gy0 = 0;
-  const float fx = sclamp(gx_f - gx0, 0.f, 1.f);
-  const float fy = sclamp(gy_f - gy0, 0.f, 1.f);
-  const int gx1 = min(gx0 + 1, map_w - 1);
-  const int gy1 = min(gy0 + 1, map_h - 1);
-  const float dx = (m.dx[gy0 * map_w + gx0] * (1.f - fx) + m.dx[gy0 * map_w + gx1] * fx) * (1.f - fy) +
-                   (m.dx[gy1 * map_w + gx0] * (1.f - fx) + m.dx[gy1 * map_w + gx1] * fx) * fy;
-  const float dy = (m.dy[gy0 * map_w + gx0] * (1.f - fx) + m.dy[gy0 * map_w + gx1] * fx) * (1.f - fy) +
-                   (m.dy[gy1 * map_w + gx0] * (1.f - fx) + m.dy[gy1 * map_w + gx1] * fx) * fy;
-  out_dx = sclamp(dx, -clamp_shift, clamp_shift);
-  out_dy = sclamp(dy, -clamp_shift, clamp_shift);
+// The two map cells around a coordinate, and how far between them it lies.
+__device__ __forceinline__ void map_place(float p, float cell, int n, int& g0, int& g1, float& f) {
+  const float g_f = (p / cell) - 0.5f;
+  g0 = (int)floorf(g_f);
+  if (g0 < 0) g0 = 0;
+  if (g0 >= n - 1) g0 = n - 2;
+  if (g0 < 0) g0 = 0;
+  f = sclamp(g_f - g0, 0.f, 1.f);
+  g1 = min(g0 + 1, n - 1);
 }
 
-__global__ void k_lk_remap(const float* __restrict__ R0, const float* __restrict__ G0, const float* __restrict__ B0,
-                           float* __restrict__ dst, int W, int H, ShiftMaps mr, ShiftMaps mb, int map_w, int map_h,
-                           float cell, float clamp_shift) {
-  // (32 x 8) threads, 2D grid-stride: no 64-bit index division per pixel
-  for (int y = blockIdx.y * blockDim.y + threadIdx.y; y < H; y += gridDim.y * blockDim.y)
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < W; x += gridDim.x * blockDim.x) {
-    const size_t i = (size_t)y * W + x;
-    float drx, dry, dbx, dby;
-    sample_shift(mr, map_w, map_h, cell, clamp_shift, (float)x, (float)y, drx, dry);
-    sample_shift(mb, map_w, map_h, cell, clamp_shift, (float)x, (float)y, dbx, dby);
-    const float r_new = bilinear_plane(R0, W, H, (float)x + drx, (float)y + dry);
-    const float b_new = bilinear_plane(B0, W, H, (float)x + dbx, (float)y + dby);
-    dst[i * 3 + 0] = r_new;
-    dst[i * 3 + 1] = G0[i];
-    dst[i * 3 + 2] = b_new;
-  }
+constexpr int RM_ROWS = 16;  // rows of a thread's column
+constexpr int RM_B = 4;      // rows in flight
+
+// A warp's 32 columns over RM_ROWS rows.  The shift is bilinear in the map, so
+// its two horizontal means (of either map row, for four maps) stay in registers
+// while the rows stay between the same two map rows, and a pixel costs the
+// vertical mean alone, not 16 map loads and two divisions each way; the rows'
+// divisions are one, a row to a lane.  Four rows are sampled together without
+// clamps or branches where all their samples lie inside (a warp's vote): what
+// bounds the pass is the wait for its loads.  The interleaved rows go out
+// through shared memory, in whole sectors.
+// 26 MP: 288 us before, 177 us; its 24 B per pixel take 95 us.  (One row at a
+// time 287 us; three CTAs per SM 206 us, five, which spill, 201 us.)
+__global__ void __launch_bounds__(256, 4)
+    k_lk_remap(const float* __restrict__ R0, const float* __restrict__ G0, const float* __restrict__ B0,
+               float* __restrict__ dst, int W, int H, ShiftMaps mr, ShiftMaps mb, int map_w, int map_h, float cell,
+               float clamp_shift) {
+  __shared__ float stage[8][RM_B][96];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const float* const m[4] = {mr.dx, mr.dy, mb.dx, mb.dy};
+  const float xe = (float)(W - 1), ye = (float)(H - 1);
+  for (int yb = (blockIdx.y * 8 + wid) * RM_ROWS; yb < H; yb += gridDim.y * 8 * RM_ROWS)
+    for (int xb = blockIdx.x * 32; xb < W; xb += gridDim.x * 32) {
+      const int x = min(xb + lane, W - 1), live = min(32, W - xb) * 3;
+      int gx0, gx1, ly0, ly1, held = -1;
+      float fx, lfy, up[4], dn[4];
+      map_place((float)x, cell, map_w, gx0, gx1, fx);
+      map_place((float)(yb + lane), cell, map_h, ly0, ly1, lfy);
+      const int y_end = min(yb + RM_ROWS, H);
+      for (int y0 = yb; y0 < y_end; y0 += RM_B) {
+        float sx[RM_B][2], sy[RM_B][2];
+        bool in = true;
+#pragma unroll
+        for (int j = 0; j < RM_B; j++) {
+          const int y = min(y0 + j, y_end - 1);
+          const int gy0 = __shfl_sync(~0u, ly0, y - yb);
+          const float fy = __shfl_sync(~0u, lfy, y - yb);
+          if (gy0 != held) {
+            held = gy0;
+            const int gy1 = min(gy0 + 1, map_h - 1);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              up[q] = m[q][gy0 * map_w + gx0] * (1.f - fx) + m[q][gy0 * map_w + gx1] * fx;
+              dn[q] = m[q][gy1 * map_w + gx0] * (1.f - fx) + m[q][gy1 * map_w + gx1] * fx;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            sx[j][q] = (float)x + sclamp(up[2 * q] * (1.f - fy) + dn[2 * q] * fy, -clamp_shift, clamp_shift);
+            sy[j][q] = (float)y + sclamp(up[2 * q + 1] * (1.f - fy) + dn[2 * q + 1] * fy, -clamp_shift, clamp_shift);
+            in = in && sx[j][q] >= 0.f && sy[j][q] >= 0.f && sx[j][q] < xe && sy[j][q] < ye;
+          }
+        }
+        const float* const src[2] = {R0, B0};
+        if (__all_sync(~0u, in)) {
+          float v[RM_B][2][4], g[RM_B];
+#pragma unroll
+          for (int j = 0; j < RM_B; j++) {
+            g[j] = G0[(size_t)min(y0 + j, y_end - 1) * W + x];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+              const float* p = src[q] + ((size_t)(int)sy[j][q] * W + (int)sx[j][q]);
+              v[j][q][0] = p[0];
+              v[j][q][1] = p[1];
+              v[j][q][2] = p[W];
+              v[j][q][3] = p[W + 1];
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < RM_B; j++) {
+            stage[wid][j][lane * 3 + 1] = g[j];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+              const float tx = sx[j][q] - (float)(int)sx[j][q], ty = sy[j][q] - (float)(int)sy[j][q];
+              stage[wid][j][lane * 3 + 2 * q] = (v[j][q][0] * (1.f - tx) + v[j][q][1] * tx) * (1.f - ty) +
+                                                (v[j][q][2] * (1.f - tx) + v[j][q][3] * tx) * ty;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < RM_B; j++) {
+            stage[wid][j][lane * 3 + 1] = G0[(size_t)min(y0 + j, y_end - 1) * W + x];
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+              stage[wid][j][lane * 3 + 2 * q] = bilinear_plane(src[q], W, H, sx[j][q], sy[j][q]);
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < RM_B; j++)
+#pragma unroll
+          for (int k = 0; k < 3; k++)
+            if (y0 + j < y_end && lane + 32 * k < live)
+              dst[((size_t)(y0 + j) * W + xb) * 3 + lane + 32 * k] = stage[wid][j][lane + 32 * k];
+        __syncwarp();
+      }
+    }
 }
 
 __global__ void k_zero(float* p, size_t n) {
@@ -344,10 +509,16 @@ lre_status launch_lateral_ca(Context* c, const float* in, float* out, size_t w, 
   maps.conf[1] = mapmem + 5 * ncell;
   float* tmp = mapmem + 6 * ncell;
 
-  k_split_planes<<<grid_for(w * h, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, Rl[0], Gl[0], Bl[0], w * h);
+  if (eff > 1) {
+    const dim3 g((unsigned)std::min<size_t>((w + 63) / 64, 1024), (unsigned)std::min<size_t>((h + 15) / 16, 8192));
+    k_split_down<<<g, dim3(32, 8), 0, c->stream>>>(in, Rl[0], Gl[0], Bl[0], Rl[1], Gl[1], Bl[1], (int)w, (int)h,
+                                                   reinterpret_cast<uintptr_t>(in) % 8 == 0);
+  } else {
+    k_split_planes<<<grid_for(w * h, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, Rl[0], Gl[0], Bl[0], w * h);
+  }
   k_zero<<<grid_for(6 * ncell, 256, 64), 256, 0, c->stream>>>(mapmem, 6 * ncell);
   count_launch(c, 2);
-  for (int l = 1; l < eff; l++) {
+  for (int l = 2; l < eff; l++) {
     Planes3 p{{Rl[l - 1], Gl[l - 1], Bl[l - 1]}, {Rl[l], Gl[l], Bl[l]}};
     k_downsample3<<<grid_for((size_t)Wl[l] * Hl[l], 256, c->sm_count * 8), 256, 0, c->stream>>>(p, Wl[l - 1], Hl[l - 1],
                                                                                                 Wl[l], Hl[l]);
@@ -364,8 +535,9 @@ lre_status launch_lateral_ca(Context* c, const float* in, float* out, size_t w, 
   }
   k_lk_gate_smooth<<<1, 1024, 0, c->stream>>>(maps, map_w, map_h, min_conf, tmp);
   const float clamp_shift = max_shift * (float)(1 << (eff - 1));
-  k_lk_remap<<<dim3((unsigned)std::min<size_t>((w + 31) / 32, 1024), (unsigned)std::min<size_t>((h + 7) / 8, 8192)),
-               dim3(32, 8), 0, c->stream>>>(
+  const dim3 rg((unsigned)std::min<size_t>((w + 31) / 32, 1024),
+                (unsigned)std::min<size_t>((h + 8 * RM_ROWS - 1) / (8 * RM_ROWS), 8192));
+  k_lk_remap<<<rg, 256, 0, c->stream>>>(
       Rl[0], Gl[0], Bl[0], out, (int)w, (int)h, ShiftMaps{maps.dx[0], maps.dy[0]}, ShiftMaps{maps.dx[1], maps.dy[1]},
       map_w, map_h, (float)cell, clamp_shift);
   count_launch(c, 2);
