@@ -53,6 +53,7 @@ struct XtArgs {
   int n_top, n_left;
   unsigned char* scratch;
   int* tile_counter;
+  int refill;  // clear and refill the plane for each direction (plane-resident kernel)
   XtParams P;
 };
 
@@ -108,13 +109,6 @@ __device__ __forceinline__ float xraw_hex(const XtArgs& A, int row, int col, int
     v = A.raw[pos * 3 + xfc(A.P, r, c)];
   }
   return v / A.maximum;
-}
-
-// The same samples from the dense normalised mosaic (k_xt_normalize): the
-// value at (row, col), and at a linear offset from it.
-__device__ __forceinline__ float xn(const XtArgs& A, int row, int col) { return A.norm[(size_t)row * A.W + col]; }
-__device__ __forceinline__ float xn_hex(const XtArgs& A, int row, int col, int hex) {
-  return A.norm[(long long)row * A.W + col + hex];
 }
 
 // n / d by a multiply-high, exact while n * d < 2^32 (every loop here); the
@@ -700,24 +694,62 @@ __global__ void __launch_bounds__(XT_THREADS, kXtCtasPerSm) k_xtrans_3pass(XtArg
 // plane k through pass 0, whose derivatives (g) and RGB then go to the CTA's
 // global scratch, and on in place as plane k + 4 through passes 1 and 2.  The
 // green min/max table stays in shared memory for the whole tile.  The
-// homogeneity steps read the eight derivative planes back from the scratch
+// homogeneity steps stage the eight derivative planes back from the scratch
 // and keep their byte maps in shared memory, and the final average reads the
 // RGB planes back.  Every step visits each site of its class once and reads
 // no value that the same step writes (xt_sites_ok replays the reference's
 // scans), so each step runs one site per thread; sites stay in fresh-buffer
 // semantics (zeros where a tile computes nothing).
+//
+// What bounds the kernel is the issue of instructions around a few shared
+// loads per site, with 32 warps on the SM and a barrier after every step.  So:
+// * A class of sites is one (row mod 3, column mod 3) of the tile, at most four
+//   classes to a step.  256 threads take a class and a thread takes six of its
+//   38 x 38 sites, whose places within the 3x3 blocks are the same for every
+//   step: they stay in registers, and the class's hexagon offsets, directions
+//   and strides are the same for a whole warp.  (A list of the sites in shared
+//   memory, with the class looked up at each site in each step: twice the
+//   instructions and four dependent loads ahead of the first sample.)
+// * A step loads the samples of three sites before it stores one.
+// * The plane is cleared once per tile, not once per plane: a slot that no step
+//   writes stays zero, and one that a step writes is written before it is read
+//   (xt_fresh_once looks at the pattern for that; any other is cleared for each
+//   plane).
+// * (g) walks along its direction and forms each pixel's luma and chroma once,
+//   not three times; a pixel's own sample is the same in every plane, so two
+//   floats per pixel of the tile's outputs go to the scratch, not three per
+//   pixel of the tile (1.0 MB per CTA and tile, not 1.6).
+// * The homogeneity counts read staged rows, and the 5x5 sums add four byte
+//   columns per word.
+// 26 MP: 4614 us before, 2805 us.  A tile takes about 295,000 cycles: (c) to (f)
+// 84,000, (g) and the scratch's stores 61,000, (b) 20,000, (h) 49,000, (j) 11,000,
+// (l) 45,000, of which most waits for the chosen samples: the CTAs' scratches
+// together (142 MB) are more than L2 holds.  (Fetching them ahead, and stores
+// that leave L2 first, moved that wait to other steps.)
 constexpr int XS_THREADS = 1024;
 constexpr int kXsMaxCtas = 148;
 constexpr int XDN = XTS - 10;  // derivative plane edge
+constexpr int XBS = XTS / 3;   // 3x3 blocks across a tile
+constexpr int XS_CLS = 4;      // site classes of a step, at most
+constexpr int XS_S = 6;        // sites per thread and class
+constexpr int XS_B = 3;        // sites in flight
+constexpr int XS_SAFE = 8 * XTS + 8;  // a site of every tile, for the mosaic loads of slots without one
 constexpr size_t kPlaneFloats = (size_t)XTS * XTS * 3;
-constexpr size_t kPlaneBytes = kPlaneFloats * 4;            // 155,952
-// site lists: 4 of every 3x3 sites per class (the replay's bound), 38 x 38
-// such blocks in a tile
-constexpr int kXsListCap = (XTS / 3) * (XTS / 3) * 4;  // 5,776
-constexpr size_t kXsSmemBytes = kPlaneBytes + kGmmBytes + 2 * kXsListCap * 2 + 2 * XTS;  // 231,268
-constexpr size_t kXsSpillBytes = ((kRgbBytes + kDrvBytes + 255) / 256) * 256;
-static_assert(2 * kHomoBytes <= kPlaneBytes + kGmmBytes, "the homogeneity maps reuse the plane and table memory");
-static_assert(kPlaneBytes % 16 == 0 && kHomoBytes % 16 == 0, "float4 fills");
+constexpr size_t kPlaneBytes = kPlaneFloats * 4;  // 155,952
+// Samples of a site at the plane's edge may lie before the plane (they are
+// loaded and not used): up to four rows and four columns, (c).
+constexpr size_t kXsPad = ((4 * XTS + 5) * 12 + 15) / 16 * 16;
+constexpr int XHS = 116;                          // byte-map row, whole words
+constexpr size_t kXsMapBytes = (size_t)NDIR * XTS * XHS;
+constexpr int XH_R = 13;  // rows of a homogeneity strip, XH_R + 2 staged
+constexpr size_t kXsStageFloats = (size_t)NDIR * (XH_R + 2) * XDN;
+constexpr size_t kXsOwn = (kXsPad + kPlaneBytes + kGmmBytes + 15) / 16 * 16;  // the own colours lie behind
+constexpr size_t kXsSmemBytes = kXsOwn + (size_t)XTS * XTS;  // 226,468
+constexpr size_t kXsSpillBytes = (((size_t)NDIR * XTS * XTS * 8 + kDrvBytes + 255) / 256) * 256;
+static_assert(XTS % 3 == 0 && XBS == 38 && XS_S % XS_B == 0, "xs_site; five fields of site bits in a word");
+static_assert(2 * kXsMapBytes <= kXsOwn, "byte maps");
+static_assert(kXsMapBytes + 2 * kXsStageFloats * 4 + (size_t)XH_R * XDN * 4 <= kXsOwn, "homogeneity strips");
+static_assert(kPlaneBytes % 16 == 0 && kXsMapBytes % 16 == 0 && XDN % 4 == 0 && XHS % 4 == 0, "vector accesses");
 
 // raw / maximum for every mosaic site, in the reference's IEEE division
 // (xraw), once per image: the plane-resident kernel reads each sample in
@@ -728,57 +760,157 @@ __global__ void k_xt_normalize(XtArgs A, float* norm) {
     norm[i] = A.cstride == 1 ? A.raw[i] / A.maximum : xraw(A, (int)(i / A.W), (int)(i % A.W));
 }
 
-// (g) YPbPr derivatives of one finished direction plane D (:2346-2405),
-// yuv recomputed at the three taps, and the plane's RGB, into the CTA's
-// scratch.  Reads the plane only.
-__device__ __forceinline__ void xs_plane_out(const float* pl, float* srgb, float* sdrv, int D, int nr, int nc) {
+__device__ __forceinline__ void xs_cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ float2 xs_load_if(const float2* p, bool on) {
+  float2 v = make_float2(0.f, 0.f);
+  asm volatile("{.reg .pred q; setp.ne.s32 q, %3, 0; @q ld.global.v2.f32 {%0, %1}, [%2];}"
+               : "+f"(v.x), "+f"(v.y)
+               : "l"(p), "r"((int)on));
+  return v;
+}
+
+struct XsPixel {
+  float r, g, b, y, u, v;
+  __device__ __forceinline__ void of(const float* p) {
+    r = p[0];
+    g = p[1];
+    b = p[2];
+    y = 0.2627f * r + 0.6780f * g + 0.0593f * b;
+    u = (b - y) * 0.56433f;
+    v = (r - y) * 0.67815f;
+  }
+};
+__device__ __forceinline__ float xs_second(float m, float o, float p) { return SQRf(2 * o - p - m); }
+// The two samples of a pixel that its own colour is not.
+__device__ __forceinline__ float2 xs_two(float r, float g, float b, int own) {
+  return make_float2(own == 0 ? g : r, own == 2 ? g : b);
+}
+
+// Block corner of slot s of a thread (of the 256 of its class), -1 where there
+// is none.  Floats of neighbouring blocks lie 9 banks apart along a row and 2
+// along a column, so a warp takes 32 blocks of one row, and the six columns left
+// over four rows at a time, picked so that no two lanes meet in a bank: rows
+// r, r + 1, r + 4, r + 5.  (Blocks in running order: two wavefronts to most
+// loads, as a row ends within the warp.)
+__device__ __forceinline__ int xs_site(int slot_warp, int lane) {
+  if (slot_warp < XBS) return 3 * (slot_warp * XTS + lane);
+  const int g = slot_warp - XBS, r = lane / 6;
+  const int i = (g >> 1) * 8 + (g & 1) * 2 + (r & 1) + (r & 2) * 2, j = 32 + lane - 6 * r;
+  return r < 4 && i < XBS ? 3 * (i * XTS + j) : -1;
+}
+
+struct XsTile {
+  int nr, nc;          // computed extent
+  int r0, r1, c0, c1;  // outputs
+};
+
+// (g) YPbPr derivatives of one finished direction plane D (:2346-2405) and
+// the two interpolated samples of its outputs, into the CTA's scratch.  Reads
+// the plane only.  ALONG: the direction's column step per row (0, 1, -1), or 2
+// for the direction along the row.
+template <int ALONG>
+__device__ __forceinline__ void xs_derivatives(const float* pl, const unsigned char* own, float2* two, float* out,
+                                               const XsTile& T) {
   constexpr int ts = XTS;
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const int rows = nr - 10, cols = nc - 10;
-  if (rows > 0 && cols > 0) {
-    const int dv = D & 3;
-    // direction steps 1, ts, ts + 1, ts - 1 of directions 0..3 (and 4..7)
-    int f = dv == 0 ? 1 : (dv == 1 ? ts : (dv == 2 ? ts + 1 : ts - 1));
-    f = f == 1 ? 1 : f - 8;
-    // yuv buffer offset f (width ts - 8) -> tile offset
-    const int fr = (f == 1) ? 0 : 1, fc = (f == 1) ? 1 : (f - (XTS - 8));
-    const int step = (fr * ts + fc) * 3;
-    float* out = sdrv + (size_t)D * XDN * XDN;
-    const XDiv fd(cols);
-    for (int i = tid; i < rows * cols; i += nth) {
-      const int q = fd.div(i), row = 5 + q, col = 5 + i - q * cols;
-      const float* p = pl + (row * ts + col) * 3;
-      auto yuv = [](const float* s, float& y, float& u, float& v) {
-        y = 0.2627f * s[0] + 0.6780f * s[1] + 0.0593f * s[2];
-        u = (s[2] - y) * 0.56433f;
-        v = (s[0] - y) * 0.67815f;
-      };
-      float y0, u0, v0, yp, up, vp, ym, um, vm;
-      yuv(p, y0, u0, v0);
-      yuv(p + step, yp, up, vp);
-      yuv(p - step, ym, um, vm);
-      out[(row - 5) * XDN + (col - 5)] = SQRf(2 * y0 - yp - ym) + SQRf(2 * u0 - up - um) + SQRf(2 * v0 - vp - vm);
+  const int rows = T.nr - 10, cols = T.nc - 10;
+  static_assert(XDN + XH_R - 1 <= 128 && XDN <= 8 * XH_R && XDN <= 4 * 30, "four warps across, eight walks down");
+  // A thread's pixels, from (row0, col0) in steps of (DR, DC): which of them have
+  // a derivative and which are outputs, a bit each.
+  constexpr int DR = ALONG == 2 ? 8 : 1, DC = ALONG == 2 ? 0 : ALONG;
+  constexpr int OUT = ALONG == 1 || ALONG == -1 ? XH_R - 1 : 0;
+  const int lane = threadIdx.x & 31, across = threadIdx.x & 127, down = threadIdx.x >> 7;
+  const int row0 = 5 + (ALONG == 2 ? down : down * XH_R);
+  const int col0 = ALONG == 2 ? 4 + 30 * (across >> 5) + lane : 5 + across - (ALONG == 1 ? OUT : 0);
+  const int own_at = row0 * ts + col0;
+  const float* p = pl + own_at * 3;
+  auto bits = [&](int ra, int rb, int ca, int cb) {  // of the t with ra <= row < rb and ca <= col < cb
+    int lo = row0 < ra ? (ra - row0 + DR - 1) / DR : 0, hi = min(XH_R, row0 < rb ? (rb - row0 + DR - 1) / DR : 0);
+    if (DC == 0) {
+      if (col0 < ca || col0 >= cb) hi = 0;
+    } else if (DC == 1) {
+      lo = max(lo, ca - col0);
+      hi = min(hi, cb - col0);
+    } else {
+      lo = max(lo, col0 - cb + 1);
+      hi = min(hi, col0 - ca + 1);
+    }
+    return hi > lo ? (1u << hi) - (1u << lo) : 0u;
+  };
+  unsigned m_d = bits(5, 5 + rows, 5, 5 + cols), m_o = m_d & bits(T.r0, T.r1, T.c0, T.c1);
+  if (ALONG == 2 && (lane == 0 || lane == 31)) m_d = m_o = 0;
+  out += (row0 - 5) * XDN + col0 - 5;
+  two += own_at;
+  auto emit = [&](int t, const XsPixel& o, float d) {
+    if (m_d >> t & 1) out[t * (DR * XDN + DC)] = d;
+    if (m_o >> t & 1) two[t * (DR * ts + DC)] = xs_two(o.r, o.g, o.b, own[own_at + t * (DR * ts + DC)]);
+  };
+  if (ALONG == 2) {
+    // a warp per 30 pixels of a row; the neighbours' luma and chroma by shuffle
+#pragma unroll
+    for (int t = 0; t < XH_R; t++) {
+      if (row0 + t * DR >= 5 + rows) break;
+      XsPixel o;
+      o.of(p + t * DR * ts * 3);
+      const float d = xs_second(__shfl_up_sync(~0u, o.y, 1), o.y, __shfl_down_sync(~0u, o.y, 1)) +
+                      xs_second(__shfl_up_sync(~0u, o.u, 1), o.u, __shfl_down_sync(~0u, o.u, 1)) +
+                      xs_second(__shfl_up_sync(~0u, o.v, 1), o.v, __shfl_down_sync(~0u, o.v, 1));
+      emit(t, o, d);
+    }
+  } else {
+    // a thread walks XH_R rows; on a diagonal the columns shift with the rows,
+    // so walks start up to XH_R - 1 columns outside (those pixels lie in the
+    // rows above or below: read, not stored)
+    if (m_d == 0) return;
+    constexpr int STEP = (ts + ALONG) * 3;
+    XsPixel m, o, nx;
+    m.of(p - STEP);
+    o.of(p);
+#pragma unroll
+    for (int t = 0; t < XH_R; t++) {
+      if (row0 + t >= 5 + rows) break;
+      nx.of(p + (t + 1) * STEP);
+      emit(t, o, xs_second(m.y, o.y, nx.y) + xs_second(m.u, o.u, nx.u) + xs_second(m.v, o.v, nx.v));
+      m = o;
+      o = nx;
     }
   }
-  const float4* s4 = reinterpret_cast<const float4*>(pl);
-  float4* d4 = reinterpret_cast<float4*>(srgb + (size_t)D * kPlaneFloats);
-  for (int i = tid; i < (int)(kPlaneBytes / 16); i += nth) d4[i] = s4[i];
+}
+
+__device__ __forceinline__ void xs_plane_out(const float* pl, const unsigned char* own, float2* srgb, float* sdrv, int D,
+                                             const XsTile& T) {
+  float2* two = srgb + (size_t)D * XTS * XTS;
+  float* out = sdrv + (size_t)D * XDN * XDN;
+  // direction steps 1, ts, ts + 1, ts - 1 of directions 0..3 (and 4..7)
+  switch (D & 3) {
+    case 0: xs_derivatives<2>(pl, own, two, out, T); break;
+    case 1: xs_derivatives<0>(pl, own, two, out, T); break;
+    case 2: xs_derivatives<1>(pl, own, two, out, T); break;
+    default: xs_derivatives<-1>(pl, own, two, out, T); break;
+  }
+  // outputs beyond the derivatives: tiles at the image's border
+  if (T.r0 < 5 || T.c0 < 5 || T.r1 > T.nr - 5 || T.c1 > T.nc - 5) {
+    const XDiv fd(T.c1 - T.c0);
+    for (int i = threadIdx.x; i < (T.r1 - T.r0) * (T.c1 - T.c0); i += XS_THREADS) {
+      const int q = fd.div(i), row = T.r0 + q, col = T.c0 + i - q * (T.c1 - T.c0);
+      if (row >= 5 && row < T.nr - 5 && col >= 5 && col < T.nc - 5) continue;
+      const int e = row * XTS + col;
+      two[e] = xs_two(pl[e * 3], pl[e * 3 + 1], pl[e * 3 + 2], own[e]);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(XS_THREADS, 1) k_xtrans_3pass_planes(XtArgs Ain) {
   constexpr int ts = XTS;
   extern __shared__ __align__(16) unsigned char xs_smem[];
-  float* pl = reinterpret_cast<float*>(xs_smem);                   // [XTS][XTS][3]
-  float2* gmm = reinterpret_cast<float2*>(xs_smem + kPlaneBytes);  // [XTS][XTS/2] (min, max)
-  // the tile's non-green sites and 2x2-block greens, as row * XTS + column
-  unsigned short* lst_ng = reinterpret_cast<unsigned short*>(xs_smem + kPlaneBytes + kGmmBytes);
-  unsigned short* lst_gg = lst_ng + kXsListCap;
-  // per tile row / column: pattern phase (bits 0-2, mod 6), off the
-  // solitary-green class (bit 3), phase mod 3 (bits 4-5)
-  unsigned char* rinfo = reinterpret_cast<unsigned char*>(lst_gg + kXsListCap);
-  unsigned char* cinfo = rinfo + XTS;
-  __shared__ int s_n[2];
-  const int tid = threadIdx.x, nth = blockDim.x;
+  float* pl = reinterpret_cast<float*>(xs_smem + kXsPad);  // [XTS][XTS][3]
+  float2* gmm = reinterpret_cast<float2*>(xs_smem + kXsPad + kPlaneBytes);  // [XTS][XTS/2] (min, max)
+  unsigned char* own = xs_smem + kXsOwn;                           // [XTS][XTS] colour of the sample
+  __shared__ int s_tile, s_cls[2 * XS_CLS];
+  const int tid = threadIdx.x, nth = XS_THREADS;
   __shared__ XtArgs sA;
   {
     constexpr int NW = (int)(sizeof(XtArgs) / 4);
@@ -788,146 +920,215 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xtrans_3pass_planes(XtArgs Ai
     for (int k = 0; k < NW; k++)
       if (k % XS_THREADS == tid) to[k] = from[k];
   }
-  __syncthreads();
   const XtArgs& A = sA;
   const XtParams& P = A.P;
-  float* srgb = reinterpret_cast<float*>(A.scratch + (size_t)blockIdx.x * kXsSpillBytes);  // [NDIR][XTS][XTS][3]
-  float* sdrv = srgb + NDIR * kPlaneFloats;                                                // [NDIR][XDN][XDN]
-  __shared__ int s_tile;
-  const int W = A.W, H = A.H;
+  // the corners of this thread's blocks, for either class list
+  const int warp = tid >> 5, lane = tid & 31, nwarps = nth >> 5;
+  constexpr int CW = XS_THREADS / XS_CLS / 32;  // warps of a class
+  int e0[XS_S];
+#pragma unroll
+  for (int s = 0; s < XS_S; s++) e0[s] = xs_site((warp & (CW - 1)) + CW * s, lane);
+  // Opaque before each step: the addresses that the steps derive from them, kept
+  // over the loops by the compiler, would spill.
+  auto fresh = [&]() {
+#pragma unroll
+    for (int s = 0; s < XS_S; s++) asm volatile("" : "+r"(e0[s]));
+  };
+  const int my = warp / CW;  // this thread's class
 
+  if (tid == 0) s_tile = atomicAdd(Ain.tile_counter, 1);
+  __syncthreads();
   for (;;) {
-    if (tid == 0) s_tile = atomicAdd(A.tile_counter, 1);
-    __syncthreads();
     const int tile = s_tile;
-    __syncthreads();
     if (tile >= A.n_top * A.n_left) break;
+    const int W = A.W, H = A.H;
+    float2* srgb = reinterpret_cast<float2*>(A.scratch + (size_t)blockIdx.x * kXsSpillBytes);  // [NDIR][XTS][XTS]
+    float* sdrv = reinterpret_cast<float*>(srgb + (size_t)NDIR * ts * ts);                     // [NDIR][XDN][XDN]
     const int top = 3 + (tile / A.n_left) * (ts - 16);
     const int left = 3 + (tile % A.n_left) * (ts - 16);
     const int mrow_g = min(top + ts, H - 3);  // global row bound of the computations
     const int mcol_g = min(left + ts, W - 3);
-    const int nr = mrow_g - top, nc = mcol_g - left;
-    const int warp = tid >> 5, lane = tid & 31, nwarps = nth >> 5;
+    XsTile T;
+    const int nr = T.nr = mrow_g - top, nc = T.nc = mcol_g - left;
+    T.r0 = min(top, 8);
+    T.c0 = min(left, 8);
+    T.r1 = (H - top < ts + 4 ? H - top + 2 : nr) - 8;
+    T.c1 = (W - left < ts + 4 ? W - left + 2 : nc) - 8;
 
-    // site classes of the tile: line info, then the two site lists (their
-    // order is free: every step's sites are independent)
-    for (int i = tid; i < XTS; i += nth) {
-      const int r6 = (top + i) % 6, c6 = (left + i) % 6;
-      rinfo[i] = (unsigned char)(r6 | (((top + i - P.sgrow) % 3 != 0) << 3) | ((r6 % 3) << 4));
-      cinfo[i] = (unsigned char)(c6 | (((left + i - P.sgcol) % 3 != 0) << 3) | ((c6 % 3) << 4));
+    // the classes: non-green sites, and greens off the solitary ones' rows and
+    // columns, by their place in a 3x3 block of the tile
+    if (warp == 0) {
+      const int r = top + lane / 3, c = left + lane % 3;
+      const bool ng = lane < 9 && !(P.xt[r % 3][c % 3] & 1);
+      const bool gg = lane < 9 && (r - P.sgrow) % 3 != 0 && (c - P.sgcol) % 3 != 0;
+      const unsigned mn = __ballot_sync(~0u, ng), mg = __ballot_sync(~0u, gg), lt = (1u << lane) - 1;
+      if (lane < 2 * XS_CLS) s_cls[lane] = -1;
+      __syncwarp();
+      if (ng) s_cls[__popc(mn & lt)] = lane;
+      if (gg) s_cls[XS_CLS + __popc(mg & lt)] = lane;
     }
-    if (tid == 0) s_n[0] = s_n[1] = 0;
     __syncthreads();
-    for (int lr = warp; lr < nr; lr += nwarps) {
-      const int ri = rinfo[lr];
-      for (int c0 = 0; c0 < nc; c0 += 32) {
-        const int lc = c0 + lane;
-        const int ci = lc < nc ? cinfo[lc] : 0;
-        const bool ng = lc < nc && !(P.xt[ri >> 4][ci >> 4] & 1);
-        const bool gg = lc < nc && (ri & 8) && (ci & 8);
-        const unsigned mng = __ballot_sync(0xffffffffu, ng), mgg = __ballot_sync(0xffffffffu, gg);
-        int bng = 0, bgg = 0;
-        if (lane == 0) {
-          bng = atomicAdd(&s_n[0], __popc(mng));
-          bgg = atomicAdd(&s_n[1], __popc(mgg));
+    if (tid == 0) s_tile = atomicAdd(Ain.tile_counter, 1);  // the next one, read after this tile's barriers
+    const int qn = s_cls[my], qg = s_cls[XS_CLS + my];
+    const int an = qn < 0 ? 0 : qn / 3, bn = qn < 0 ? 0 : qn % 3, ag = qg < 0 ? 0 : qg / 3, bg = qg < 0 ? 0 : qg % 3;
+    const int on = an * ts + bn, og = ag * ts + bg;
+    const int r3 = (top + an) % 3, c3 = (left + bn) % 3;
+    const int flip = P.right_shift[r3] == 1 ? 0 : 1;
+    // six sites' bits each: in the tile, two and three off its edge, the own
+    // colour being blue; two off the edge in the other list
+    unsigned bits = 0;
+    {
+      unsigned blue = 0;  // by the parities of the block's row and column
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        blue |= (P.xt[(top + an + 3 * (q >> 1)) % 6][(left + bn + 3 * (q & 1)) % 6] == 2 ? 1u : 0u) << q;
+#pragma unroll
+      for (int s = 0; s < XS_S; s++) {
+        if (e0[s] < 0) continue;
+        const int i = e0[s] / ts, j = e0[s] - i * ts;  // multiples of three
+        auto edge = [&](int r, int c) { return min(min(r, nr - 1 - r), min(c, nc - 1 - c)); };
+        if (qn >= 0) {
+          const int d = edge(i + an, j + bn);
+          if (d >= 0) bits |= 1u << s;
+          if (d >= 2) bits |= 1u << (s + XS_S);
+          if (d >= 3) bits |= 1u << (s + 2 * XS_S);
+          bits |= (blue >> ((i & 1) * 2 + (j & 1)) & 1) << (s + 3 * XS_S);
         }
-        bng = __shfl_sync(0xffffffffu, bng, 0);
-        bgg = __shfl_sync(0xffffffffu, bgg, 0);
-        const unsigned lt = (1u << lane) - 1u;
-        if (ng) lst_ng[bng + __popc(mng & lt)] = (unsigned short)(lr * XTS + lc);
-        if (gg) lst_gg[bgg + __popc(mgg & lt)] = (unsigned short)(lr * XTS + lc);
+        if (qg >= 0 && edge(i + ag, j + bg) >= 2) bits |= 1u << (s + 4 * XS_S);
       }
     }
-    __syncthreads();
-    const int n_ng = s_n[0], n_gg = s_n[1];
+    const float* tb = A.norm + (size_t)top * W + left;
 
     // (a) green min / max (:1968-2053).  The scan stores a site's hexagon
     // min/max at its half-column slot; on rows with adjacent non-green pairs
     // it stores the first site's values at both sites' slots and computes
     // none for the second.
-    for (int j = tid; j < n_ng; j += nth) {
-      const int e = lst_ng[j], lr = e / XTS, lc = e - lr * XTS;
-      const int r3 = rinfo[lr] >> 4;
-      if (lc > 0 && !(P.xt[r3][cinfo[lc - 1] >> 4] & 1)) continue;  // second of a pair
-      const int row = top + lr, col = left + lc;
-      const short* hex = P.allhex0[r3][cinfo[lc] >> 4];
-      float minval = FLT_MAX, maxval = 0.f;
-      for (int c = 0; c < 6; c++) {
-        const float val = xn_hex(A, row, col, hex[c]);
-        minval = minval < val ? minval : val;
-        maxval = maxval > val ? maxval : val;
+    {
+      const bool second = !(P.xt[r3][(c3 + 2) % 3] & 1), first = !(P.xt[r3][(c3 + 1) % 3] & 1);
+      int hex[6];
+#pragma unroll
+      for (int c = 0; c < 6; c++) hex[c] = P.allhex0[r3][c3][c];
+      fresh();
+#pragma unroll
+      for (int s = 0; s < XS_S; s++) {
+        const bool in = bits >> s & 1;
+        const int e = in ? e0[s] + on : XS_SAFE, lr = e / ts, lc = e - lr * ts;
+        const float* q = tb + ((size_t)lr * W + lc);
+        float minval = FLT_MAX, maxval = 0.f;
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+          const float val = __ldg(q + hex[c]);
+          minval = minval < val ? minval : val;
+          maxval = maxval > val ? maxval : val;
+        }
+        if (in && !(second && lc > 0)) {
+          const float2 v = make_float2(minval, maxval);
+          gmm[e >> 1] = v;  // = row * (ts / 2) + column / 2: ts is even
+          if (first && lc + 1 < nc) gmm[(e + 1) >> 1] = v;
+        }
       }
-      const float2 v = make_float2(minval, maxval);
-      float2* g = gmm + (size_t)lr * (ts / 2);
-      g[lc >> 1] = v;
-      if (lc + 1 < nc && !(P.xt[r3][cinfo[lc + 1] >> 4] & 1)) g[(lc + 1) >> 1] = v;
+    }
+    // the solitary greens of (d), a site per thread and round, with their first
+    // colour; -1: none
+    int ed[2];
+    {
+      const int sgstartcol = (left - P.sgcol + 4) / 3 * 3 + P.sgcol;
+      const int row0 = (top - P.sgrow + 4) / 3 * 3 + P.sgrow;
+      const int nrow = row0 < mrow_g - 2 ? (mrow_g - 2 - row0 + 2) / 3 : 0;
+      const int ncol = sgstartcol < mcol_g - 2 ? (mcol_g - 2 - sgstartcol + 2) / 3 : 0;
+      const XDiv fd(ncol);
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const int item = tid + q * nth;
+        ed[q] = -1;
+        if (item < nrow * ncol) {
+          const int i = fd.div(item), row = row0 + 3 * i, kk = item - i * ncol;
+          const int h0 = xfc(P, row, sgstartcol + 1) ^ ((kk & 1) << 1);
+          ed[q] = ((row - top) * ts + (sgstartcol + 3 * kk - left)) | h0 << 16;
+        }
+      }
     }
 
     for (int k = 0; k < 4; k++) {
-      // fresh plane k: zeros, the native samples (:2055-2061; planes 1..3 are
-      // copies of plane 0 without its last float, :2067-2069) and (b) the
-      // green of direction k at every non-green site (:2071-2127)
-      {
-        float4* z = reinterpret_cast<float4*>(pl);
-        for (int i = tid; i < (int)(kPlaneBytes / 16); i += nth) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      __syncthreads();
-      for (int lr = warp; lr < nr; lr += nwarps) {
-        const int r6 = rinfo[lr] & 7;
-        const float* src = A.norm + (size_t)(top + lr) * W + left;
-        float* prow = pl + lr * ts * 3;
-        for (int lc = lane; lc < nc; lc += 32) {
-          const int fcv = P.xt[r6][cinfo[lc] & 7];
-          if (k == 0 || lr * ts + lc != ts * ts - 1 || fcv != 2) prow[lc * 3 + fcv] = src[lc];
+      // the plane's zeros and native samples (:2055-2061)
+      if (k == 0 || A.refill) {
+        for (int lc = lane; lc < ts; lc += 32) {
+          const int c6 = (left + lc) % 6;
+#pragma unroll
+          for (int j = 0; j < (ts + 31) / 32; j++) {
+            const int lr = warp + j * nwarps;
+            if (lr >= ts) break;
+            const int f = P.xt[(top + lr) % 6][c6];
+            const float v = lr < nr && lc < nc ? __ldg(tb + (size_t)lr * W + lc) : 0.f;
+            float* o = pl + (lr * ts + lc) * 3;
+            o[0] = f == 0 ? v : 0.f;
+            o[1] = f == 1 ? v : 0.f;
+            o[2] = f == 2 ? v : 0.f;
+            own[lr * ts + lc] = (unsigned char)f;
+          }
         }
+        __syncthreads();
       }
-      for (int j = tid; j < n_ng; j += nth) {
-        const int e = lst_ng[j], lr = e / XTS, lc = e - lr * XTS;
-        const int row = top + lr, col = left + lc;
-        const int r3 = rinfo[lr] >> 4;
-        const short* hex = P.allhex0[r3][cinfo[lc] >> 4];
-        const int cdir = k ^ (P.right_shift[r3] == 1 ? 0 : 1);
-        float color;
+      // planes 1..3 are copies of plane 0 without its last float (:2067-2069)
+      if (k && tid == 0) pl[kPlaneFloats - 1] = 0.f;
+      // (b) the green of direction k at every non-green site (:2071-2127)
+      {
+        const int cdir = k ^ flip;
+        const short* hex = P.allhex0[r3][c3];
+        fresh();
+        auto green = [&](auto color) {
+#pragma unroll
+          for (int s = 0; s < XS_S; s++) {
+            const bool in = bits >> s & 1;
+            const int e = in ? e0[s] + on : XS_SAFE, lr = e / ts, lc = e - lr * ts;
+            const float v = color(tb + ((size_t)lr * W + lc));
+            const float2 mmv = gmm[e >> 1];
+            if (in) pl[e * 3 + 1] = LIMf(v, mmv.x, mmv.y);
+          }
+        };
         if (cdir == 0) {
-          color = 0.6796875f * (xn_hex(A, row, col, hex[1]) + xn_hex(A, row, col, hex[0])) -
-                  0.1796875f * (xn_hex(A, row, col, 2 * hex[1]) + xn_hex(A, row, col, 2 * hex[0]));
+          const int h0 = hex[0], h1 = hex[1];
+          green([&](const float* q) {
+            return 0.6796875f * (__ldg(q + h1) + __ldg(q + h0)) - 0.1796875f * (__ldg(q + 2 * h1) + __ldg(q + 2 * h0));
+          });
         } else if (cdir == 1) {
-          color = 0.87109375f * xn_hex(A, row, col, hex[3]) + xn_hex(A, row, col, hex[2]) * 0.12890625f +
-                  0.359375f * (xn_hex(A, row, col, 0) - xn_hex(A, row, col, -hex[2]));
+          const int h2 = hex[2], h3 = hex[3];
+          green([&](const float* q) {
+            return 0.87109375f * __ldg(q + h3) + __ldg(q + h2) * 0.12890625f + 0.359375f * (__ldg(q) - __ldg(q - h2));
+          });
         } else {
           const int h4 = hex[cdir + 2];
-          color = 0.640625f * xn_hex(A, row, col, h4) + 0.359375f * xn_hex(A, row, col, -2 * h4) +
-                  0.12890625f * (2.f * xn_hex(A, row, col, 0) - xn_hex(A, row, col, 3 * h4) -
-                                 xn_hex(A, row, col, -3 * h4));
+          green([&](const float* q) {
+            return 0.640625f * __ldg(q + h4) + 0.359375f * __ldg(q - 2 * h4) +
+                   0.12890625f * (2.f * __ldg(q) - __ldg(q + 3 * h4) - __ldg(q - 3 * h4));
+          });
         }
-        const float2 mmv = gmm[(size_t)lr * (ts / 2) + (lc >> 1)];
-        pl[e * 3 + 1] = LIMf(color, mmv.x, mmv.y);
       }
       __syncthreads();
 
       for (int pass = 0; pass < 3; pass++) {
-        if (pass == 1) {
-          // plane k is final: (g) its derivatives and its RGB go to the
-          // scratch, and the plane continues in place as plane k + 4
-          xs_plane_out(pl, srgb, sdrv, k, nr, nc);
-          __syncthreads();
-        }
         // (c) recalculate green from closer pixels (:2138-2183): direction
         // d = 3..5 updates plane (d - 2) ^ flip, reading green sites only
         if (pass) {
-          for (int j = tid; j < n_ng; j += nth) {
-            const int e = lst_ng[j], lr = e / XTS, lc = e - lr * XTS;
-            if (lr < 2 || lr >= nr - 2 || lc < 2 || lc >= nc - 2) continue;
-            const int ri = rinfo[lr], ci = cinfo[lc];
-            const int dd = k ^ (P.right_shift[ri >> 4] == 1 ? 0 : 1);
-            if (dd == 0) continue;
-            const int f = P.xt[ri & 7][ci & 7];
-            const int hx = P.allhex1[ri >> 4][ci >> 4][dd + 2];
-            float* rix = pl + e * 3;
-            const int o1 = hx * 3, o2 = -2 * hx * 3;
-            const float val = 0.33333333f * (rix[o2 + 1] + 2 * (rix[o1 + 1] - rix[o1 + f]) - rix[o2 + f]) + rix[f];
-            const float2 mmv = gmm[(size_t)lr * (ts / 2) + (lc >> 1)];
-            rix[1] = LIMf(val, mmv.x, mmv.y);
+          const int dd = k ^ flip;
+          if (dd) {
+            const int hx = P.allhex1[r3][c3][dd + 2] * 3;
+            fresh();
+#pragma unroll
+            for (int s0 = 0; s0 < XS_S; s0 += XS_B) {
+              float val[XS_B];
+#pragma unroll
+              for (int j = 0; j < XS_B; j++) {
+                const int s = s0 + j, e = e0[s] + on;
+                const float *p = pl + e * 3, *p1 = p + hx, *p2 = p1 - 3 * hx;
+                const int f = bits >> (s + 3 * XS_S) & 1 ? 2 : 0;
+                const float2 mmv = gmm[e >> 1];
+                val[j] = LIMf(0.33333333f * (p2[1] + 2 * (p1[1] - p1[f]) - p2[f]) + p[f], mmv.x, mmv.y);
+              }
+#pragma unroll
+              for (int j = 0; j < XS_B; j++)
+                if (bits >> (s0 + j + XS_S) & 1) pl[(e0[s0 + j] + on) * 3 + 1] = val[j];
+            }
           }
           __syncthreads();
         }
@@ -936,45 +1137,33 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xtrans_3pass_planes(XtArgs Ai
         // the second of a pair falling back to the first where its
         // difference is larger
         {
-          const int sgstartcol = (left - P.sgcol + 4) / 3 * 3 + P.sgcol;
-          const int row0 = (top - P.sgrow + 4) / 3 * 3 + P.sgrow;
-          const int nrow = row0 < mrow_g - 2 ? (mrow_g - 2 - row0 + 2) / 3 : 0;
-          const int ncol = sgstartcol < mcol_g - 2 ? (mcol_g - 2 - sgstartcol + 2) / 3 : 0;
-          const int d_lo = k < 2 ? k : 2 * k - 2, nd = k < 2 ? 1 : 2;
-          for (int item = tid; item < nrow * ncol; item += nth) {
-            const int row = row0 + 3 * (item / ncol), kk = item % ncol;
-            const int col = sgstartcol + 3 * kk;
-            float* rix = pl + ((row - top) * ts + (col - left)) * 3;
-            const int h0 = xfc(P, row, sgstartcol + 1) ^ ((kk & 1) << 1);
-            float cr0 = 0.f, cb0 = 0.f, df0 = 0.f, r = 0.f, b = 0.f, df1 = 0.f;
+          // along i (1 or ts), the colour h at distance 1 and h ^ 2 at 2
+          auto along = [&](const float* rix, int i, int h, float& r, float& b) {
+            const float g1 = rix[1] + rix[1];
+            const float p1 = rix[3 * i + 1], m1 = rix[-3 * i + 1], ph = rix[3 * i + h], mh = rix[-3 * i + h];
+            const int h2 = h ^ 2;
+            const float p2 = rix[6 * i + 1], m2 = rix[-6 * i + 1], qh = rix[6 * i + h2], nh = rix[-6 * i + h2];
+            const float ga = g1 - p1 - m1, gb = g1 - p2 - m2;
+            const float va = ga + ph + mh, vb = gb + qh + nh;
+            r = h == 0 ? va : vb;
+            b = h == 0 ? vb : va;
+            float df = 0.f;
+            df += SQRf(p1 - m1 - ph + mh) + SQRf(ga);
+            df += SQRf(p2 - m2 - qh + nh) + SQRf(gb);
+            return df;
+          };
 #pragma unroll
-            for (int j = 0; j < 2; j++) {
-              if (j >= nd) break;
-              const int d = d_lo + j;
-              const int i = (d & 1) ? ts : 1;
-              int h = h0 ^ ((d & 1) << 1);
-              float df = 0.f, cr = 0.f, cb = 0.f;
-#pragma unroll
-              for (int c = 0; c < 2; c++, h ^= 2) {
-                const int op = i * (1 << c) * 3, om = -i * (1 << c) * 3;
-                const float g = rix[1] + rix[1] - rix[op + 1] - rix[om + 1];
-                const float v = g + rix[op + h] + rix[om + h];
-                if (h == 0) cr = v;
-                else cb = v;
-                if (d > 1) df += SQRf(rix[op + 1] - rix[om + 1] - rix[op + h] + rix[om + h]) + SQRf(g);
-              }
-              if (j == 0) {
-                cr0 = cr;
-                cb0 = cb;
-                df0 = df;
-              }
-              r = cr;
-              b = cb;
-              df1 = df;
-            }
-            if (nd == 2 && df0 < df1) {
-              r = cr0;
-              b = cb0;
+          for (int q = 0; q < 2; q++) {
+            if (ed[q] < 0) continue;
+            float* rix = pl + (ed[q] & 0xffff) * 3;
+            const int h0 = ed[q] >> 16;
+            float r, b;
+            if (k < 2) {
+              along(rix, k ? ts : 1, k ? h0 ^ 2 : h0, r, b);
+            } else {
+              float r1, b1;
+              const float d0 = along(rix, 1, h0, r, b), d1 = along(rix, ts, h0 ^ 2, r1, b1);
+              if (!(d0 < d1)) r = r1, b = b1;
             }
             rix[0] = 0.5f * r;
             rix[2] = 0.5f * b;
@@ -984,137 +1173,260 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xtrans_3pass_planes(XtArgs Ai
         // (e) red for blue pixels and vice versa (:2224-2264): every non-green
         // site writes its other colour f = 2 - own
         {
-          for (int j = tid; j < n_ng; j += nth) {
-            const int e = lst_ng[j], lr = e / XTS, lc = e - lr * XTS;
-            if (lr < 3 || lr >= nr - 3 || lc < 3 || lc >= nc - 3) continue;
-            const int ri = rinfo[lr];
-            const int c = (ri & 8) ? ts : 1;  // (row - sgrow) % 3 != 0
-            const int h = 3 * (c ^ ts ^ 1);
-            const int f = 2 - P.xt[ri & 7][cinfo[lc] & 7];
-            float* rix = pl + e * 3;
-            const float g0 = rix[1];
-            const bool use_c = k > 1 || ((k ^ c) & 1) ||
-                               ((fabsf(g0 - rix[c * 3 + 1]) + fabsf(g0 - rix[-c * 3 + 1])) <
-                                2.f * (fabsf(g0 - rix[h * 3 + 1]) + fabsf(g0 - rix[-h * 3 + 1])));
-            const int s = use_c ? c : h;
-            rix[f] = g0 + 0.5f * (rix[s * 3 + f] + rix[-s * 3 + f] - rix[s * 3 + 1] - rix[-s * 3 + 1]);
+          const bool off = (top + an - P.sgrow) % 3 != 0;
+          const bool ask = !(k > 1 || ((k ^ (off ? ts : 1)) & 1));
+          fresh();
+          auto sites = [&](auto c_, auto h_) {
+            constexpr int c = decltype(c_)::value, h = decltype(h_)::value;  // steps, as floats; h = 0: not asked for
+#pragma unroll
+            for (int s0 = 0; s0 < XS_S; s0 += XS_B) {
+              float val[XS_B];
+#pragma unroll
+              for (int j = 0; j < XS_B; j++) {
+                const int s = s0 + j;
+                const float *p = pl + (e0[s] + on) * 3, *pf = p + (bits >> (s + 3 * XS_S) & 1 ? 0 : 2);
+                const float g0 = p[1];
+                float gp = p[c + 1], gm = p[1 - c], fp = pf[c], fm = pf[-c];
+                if (h) {
+                  const float hp = p[h + 1], hm = p[1 - h], qp = pf[h], qm = pf[-h];
+                  if (!((fabsf(g0 - gp) + fabsf(g0 - gm)) < 2.f * (fabsf(g0 - hp) + fabsf(g0 - hm)))) {
+                    gp = hp;
+                    gm = hm;
+                    fp = qp;
+                    fm = qm;
+                  }
+                }
+                val[j] = g0 + 0.5f * (fp + fm - gp - gm);
+              }
+#pragma unroll
+              for (int j = 0; j < XS_B; j++) {
+                const int s = s0 + j;
+                if (bits >> (s + 2 * XS_S) & 1) pl[(e0[s] + on) * 3 + (bits >> (s + 3 * XS_S) & 1 ? 0 : 2)] = val[j];
+              }
+            }
+          };
+          using Row = std::integral_constant<int, 3 * ts>;
+          using Col = std::integral_constant<int, 3>;
+          using Row3 = std::integral_constant<int, 9 * ts>;
+          using Col3 = std::integral_constant<int, 9>;
+          using None = std::integral_constant<int, 0>;
+          if (off) {
+            if (ask) sites(Row{}, Col3{});
+            else sites(Row{}, None{});
+          } else {
+            if (ask) sites(Col{}, Row3{});
+            else sites(Col{}, None{});
           }
         }
         __syncthreads();
         // (f) R and B for 2x2 green blocks (:2266-2310): greens off the
         // solitary-green row and column classes, hexagon allhex1
         {
-          for (int j = tid; j < n_gg; j += nth) {
-            const int e = lst_gg[j], lr = e / XTS, lc = e - lr * XTS;
-            if (lr < 2 || lr >= nr - 2 || lc < 2 || lc >= nc - 2) continue;
-            float* rix = pl + e * 3;
-            const short* hex = P.allhex1[rinfo[lr] >> 4][cinfo[lc] >> 4];
-            const int o0 = hex[2 * k] * 3, o1 = hex[2 * k + 1] * 3;
-            const float v1 = rix[1], a1 = rix[o0 + 1], b1 = rix[o1 + 1];
-            const float a0 = rix[o0], b0 = rix[o1], a2 = rix[o0 + 2], b2 = rix[o1 + 2];
-            if (hex[2 * k] + hex[2 * k + 1]) {
-              const float g = 3 * v1 - 2 * a1 - b1;
-              rix[0] = (g + 2 * a0 + b0) * 0.33333333f;
-              rix[2] = (g + 2 * a2 + b2) * 0.33333333f;
-            } else {
-              const float g = 2 * v1 - a1 - b1;
-              rix[0] = (g + a0 + b0) * 0.5f;
-              rix[2] = (g + a2 + b2) * 0.5f;
+          const short* hex = P.allhex1[(top + ag) % 3][(left + bg) % 3];
+          const int o0 = hex[2 * k] * 3, o1 = hex[2 * k + 1] * 3;
+          const bool two = o0 + o1 != 0;
+          const float wv = two ? 3.f : 2.f, wa = two ? 2.f : 1.f, wo = two ? 0.33333333f : 0.5f;
+          fresh();
+#pragma unroll
+          for (int s0 = 0; s0 < XS_S; s0 += XS_B) {
+            float v0[XS_B], v2[XS_B];
+#pragma unroll
+            for (int j = 0; j < XS_B; j++) {
+              const float *p = pl + (e0[s0 + j] + og) * 3, *pa = p + o0, *pb = p + o1;
+              // a factor of one leaves a value as it is: one form for both
+              const float g = wv * p[1] - wa * pa[1] - pb[1];
+              v0[j] = (g + wa * pa[0] + pb[0]) * wo;
+              v2[j] = (g + wa * pa[2] + pb[2]) * wo;
             }
+#pragma unroll
+            for (int j = 0; j < XS_B; j++)
+              if (bits >> (s0 + j + 4 * XS_S) & 1) {
+                pl[(e0[s0 + j] + og) * 3] = v0[j];
+                pl[(e0[s0 + j] + og) * 3 + 2] = v2[j];
+              }
           }
         }
         __syncthreads();
+        // plane k, and after passes 1 and 2 plane k + 4, is final: (g) its
+        // derivatives and its RGB go to the scratch; it continues in place
+        if (pass != 1) {
+          xs_plane_out(pl, own, srgb, sdrv, pass ? k + 4 : k, T);
+          __syncthreads();
+        }
       }
-      xs_plane_out(pl, srgb, sdrv, k + 4, nr, nc);
-      __syncthreads();
     }
 
-    // (h) homogeneity maps (:2407-2496) from the derivative planes
-    unsigned char* homo = xs_smem;             // [NDIR][XTS][XTS]
-    unsigned char* hs5 = xs_smem + kHomoBytes;  // [NDIR][XTS][XTS]
+    // (h) homogeneity maps (:2407-2496) from the derivative planes, in strips of
+    // XH_R rows staged a strip ahead
+    unsigned char* homo = xs_smem;                 // [NDIR][XTS][XHS]
+    unsigned char* hs5 = xs_smem + kXsMapBytes;    // [NDIR][XTS][XHS], after the strips
+    float* stage = reinterpret_cast<float*>(hs5);  // 2 x [NDIR][XH_R + 2][XDN]
+    float* tr = stage + 2 * kXsStageFloats;        // [XH_R][XDN]
     {
+      const int rows = nr - 12, cols = nc - 12;  // >= 5: a tile computes 17 rows and columns at least
+      const int strips = (rows + XH_R - 1) / XH_R;
+      // the last strip begins early enough to be whole, if there are rows for it
+      auto first = [&](int st) { return max(0, min(st * XH_R, rows - XH_R)); };
+      auto fetch = [&](int st) {
+        const int n = min(XH_R + 2, rows + 2) * (XDN / 4);
+        float* to = stage + (st & 1) * kXsStageFloats;
+        const float* from = sdrv + (size_t)first(st) * XDN;
+        const XDiv fd(n);
+        for (int i = tid; i < NDIR * n; i += nth) {
+          const int d = fd.div(i), o = (i - d * n) * 4;
+          xs_cp16(to + (size_t)d * (XH_R + 2) * XDN + o, from + (size_t)d * XDN * XDN + o);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      fetch(0);
       float4* z = reinterpret_cast<float4*>(homo);
-      for (int i = tid; i < (int)(kHomoBytes / 16); i += nth) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
-    {
-      const int rows = nr - 12, cols = nc - 12;
-      if (rows > 0 && cols > 0) {
-        const XDiv fd(cols);
-        for (int i = tid; i < rows * cols; i += nth) {
-          const int q = fd.div(i), row = 6 + q, col = 6 + i - q * cols;
-          const float* dp = sdrv + (row - 5) * XDN + (col - 5);
-          float tr = dp[0] < dp[XDN * XDN] ? dp[0] : dp[XDN * XDN];
-          for (int d = 2; d < NDIR; d++) tr = (dp[d * XDN * XDN] < tr ? dp[d * XDN * XDN] : tr);
-          tr *= 8;
-          unsigned char temp[NDIR];
+      for (int i = tid; i < (int)(kXsMapBytes / 16); i += nth) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      const XDiv fd(cols);
+      for (int st = 0; st < strips; st++) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // this strip is here; the last one's buffer and thresholds are free
+        if (st + 1 < strips) fetch(st + 1);
+        const float* b = stage + (st & 1) * kXsStageFloats;
+        const int n = min(XH_R, rows);
+        constexpr int DP = (XH_R + 2) * XDN;
+        for (int i = tid; i < n * (XDN / 2); i += nth) {
+          const int q = i / (XDN / 2), c = (i - q * (XDN / 2)) * 2;
+          const float* dp = b + (q + 1) * XDN + c;
+          float2 v[NDIR];
 #pragma unroll
-          for (int d = 0; d < NDIR; d++) {
-            temp[d] = 0;
-            for (int v = -1; v <= 1; v++)
-              for (int h = -1; h <= 1; h++) temp[d] += (dp[d * XDN * XDN + v * XDN + h] <= tr ? 1 : 0);
+          for (int d = 0; d < NDIR; d++) v[d] = *reinterpret_cast<const float2*>(dp + d * DP);
+          float x = v[0].x < v[1].x ? v[0].x : v[1].x, y = v[0].y < v[1].y ? v[0].y : v[1].y;
+#pragma unroll
+          for (int d = 2; d < NDIR; d++) {
+            x = v[d].x < x ? v[d].x : x;
+            y = v[d].y < y ? v[d].y : y;
           }
-#pragma unroll
-          for (int d = 0; d < NDIR; d++) homo[(d * ts + row) * ts + col] = temp[d];
+          *reinterpret_cast<float2*>(tr + q * XDN + c) = make_float2(x * 8, y * 8);
         }
-      }
-    }
-    __syncthreads();
-    int mrow = nr, mcol = nc;
-    if (H - top < ts + 4) mrow = H - top + 2;
-    if (W - left < ts + 4) mcol = W - left + 2;
-    // (j) 5x5 homogeneity sums (:2504-2612), separably: row 5-sums first
-    const int r0 = min(top, 8), c0 = min(left, 8);
-    {
-      const int rows = mrow - 8 - r0 + 4, cols = mcol - 8 - c0;
-      if (rows > 0 && cols > 0) {
-        const XDiv fdr(rows * cols), fdc(cols);
-        for (int i = tid; i < NDIR * rows * cols; i += nth) {
-          const int d = fdr.div(i), rem = i - d * (rows * cols);
-          const int q = fdc.div(rem), row = r0 - 2 + q, col = c0 + rem - q * cols;
-          const unsigned char* hp = homo + (d * ts + row) * ts + col;
-          hs5[(d * ts + row) * ts + col] = (unsigned char)(hp[-2] + hp[-1] + hp[0] + hp[1] + hp[2]);
-        }
-      }
-    }
-    __syncthreads();
-    // (j) column sums and their max, then (l) the average of the most
-    // homogeneous directions (:2614-2650), one output pixel per thread
-    {
-      const int rows = mrow - 8 - r0, cols = mcol - 8 - c0;
-      if (rows > 0 && cols > 0) {
-        const XDiv fd(cols);
-        for (int i = tid; i < rows * cols; i += nth) {
-          const int q = fd.div(i), row = r0 + q, col = c0 + i - q * cols;
-          unsigned char hm[NDIR];
-          unsigned char maxval = 0;
+        __syncthreads();
+        for (int i = tid; i < NDIR * cols; i += nth) {
+          const int d = fd.div(i), c = i - d * cols;
+          const float* dp = b + d * DP + c;
+          unsigned char* o = homo + (d * ts + 6 + first(st)) * XHS + 6 + c;
+          float w[3][3];
 #pragma unroll
-          for (int d = 0; d < NDIR; d++) {
-            int s = 0;
-            for (int v = -2; v <= 2; v++) s += hs5[(d * ts + row + v) * ts + col];
-            hm[d] = (unsigned char)s;
-            if (d == 0 || maxval < hm[d]) maxval = hm[d];
-          }
-          maxval -= maxval >> 3;
+          for (int v = 0; v < 2; v++)
 #pragma unroll
-          for (int d = 4; d < NDIR; d++) {
-            if (hm[d - 4] < hm[d]) hm[d - 4] = 0;
-            else if (hm[d - 4] > hm[d]) hm[d] = 0;
-          }
-          float avg[4] = {0.f, 0.f, 0.f, 0.f};
-          const float* px = srgb + (size_t)(row * ts + col) * 3;
+            for (int h = 0; h < 3; h++) w[v + 1][h] = dp[v * XDN + h];
 #pragma unroll
-          for (int d = 0; d < NDIR; d++)
-            if (hm[d] >= maxval) {
-              const float* p = px + d * kPlaneFloats;
-              for (int c = 0; c < 3; c++) avg[c] += p[c];
-              avg[3] += 1.f;
+          for (int r = 0; r < XH_R; r++) {
+            if (r >= n) break;
+#pragma unroll
+            for (int h = 0; h < 3; h++) {
+              w[0][h] = w[1][h];
+              w[1][h] = w[2][h];
+              w[2][h] = dp[(r + 2) * XDN + h];
             }
-          float* o = A.rgb_out + ((size_t)(row + top) * W + (col + left)) * 3;
-          o[0] = fmaxf(0.f, avg[0] / avg[3]);
-          o[1] = fmaxf(0.f, avg[1] / avg[3]);
-          o[2] = fmaxf(0.f, avg[2] / avg[3]);
+            const float t = tr[r * XDN + c + 1];
+            // counted in a float's low bits: the adds go to another pipe than
+            // the comparisons
+            float count = 8388608.f;
+#pragma unroll
+            for (int v = 0; v < 3; v++)
+#pragma unroll
+              for (int h = 0; h < 3; h++)
+                if (w[v][h] <= t) count += 1.f;
+            o[r * XHS] = (unsigned char)__float_as_int(count);
+          }
         }
+      }
+    }
+    __syncthreads();
+    // (j) 5x5 homogeneity sums (:2504-2612), separably and four columns per
+    // word: a byte counts to 9, its row sum to 45 and the whole to 225, so no
+    // byte carries into the next (bytes beyond the outputs may; they carry
+    // away from them).  Row sums first:
+    const int rows = T.r1 - T.r0, cols = T.c1 - T.c0;
+    const int q0 = T.c0 >> 2, nq = ((T.c1 - 1) >> 2) - q0 + 1;
+    if (rows > 0 && cols > 0) {
+      const XDiv fq(nq), fr(rows + 4);
+      for (int i = tid; i < NDIR * (rows + 4) * nq; i += nth) {
+        const int line = fq.div(i), d = fr.div(line);
+        const int at = (d * ts + T.r0 - 2 + line - d * (rows + 4)) * XHS + (q0 + i - line * nq) * 4;
+        const unsigned* hp = reinterpret_cast<const unsigned*>(homo + at);
+        const unsigned w0 = hp[-1], w1 = hp[0], w2 = hp[1];
+        *reinterpret_cast<unsigned*>(hs5 + at) = __funnelshift_r(w0, w1, 16) + __funnelshift_r(w0, w1, 24) + w1 +
+                                                 __funnelshift_r(w1, w2, 8) + __funnelshift_r(w1, w2, 16);
+      }
+    }
+    __syncthreads();
+    // then columns, a thread down a quarter of them, over the counts' memory
+    if (rows > 0 && cols > 0) {
+      const XDiv fq(nq);
+      const int seg = (rows + 3) / 4;
+      for (int i = tid; i < NDIR * 4 * nq; i += nth) {
+        const int line = fq.div(i), d = line >> 2, ra = T.r0 + (line & 3) * seg, rb = min(ra + seg, T.r1);
+        const int at = d * ts * XHS + (q0 + i - line * nq) * 4;
+        auto in = [&](int r) { return *reinterpret_cast<const unsigned*>(hs5 + at + r * XHS); };
+        if (ra >= rb) continue;
+        unsigned sum = in(ra - 2) + in(ra - 1) + in(ra) + in(ra + 1);
+#pragma unroll 2
+        for (int r = ra; r < rb; r++) {
+          sum += in(r + 2);
+          *reinterpret_cast<unsigned*>(homo + at + r * XHS) = sum;
+          sum -= in(r - 2);
+        }
+      }
+    }
+    __syncthreads();
+    // their max, and (l) the average of the most homogeneous directions
+    // (:2614-2650), one output pixel per thread: which directions first, a bit
+    // each over the row sums' memory, so that the second loop's loads wait for
+    // one byte only
+    if (rows > 0 && cols > 0) {
+      const XDiv fd(cols);
+      unsigned char* chosen = hs5;
+#pragma unroll 2
+      for (int i = tid; i < rows * cols; i += nth) {
+        const int q = fd.div(i);
+        const unsigned char* hp = homo + (T.r0 + q) * XHS + T.c0 + i - q * cols;
+        int hm[NDIR], maxval = 0;
+#pragma unroll
+        for (int d = 0; d < NDIR; d++) {
+          hm[d] = hp[d * ts * XHS];
+          maxval = max(maxval, hm[d]);
+        }
+        maxval -= maxval >> 3;
+        unsigned m = 0;
+#pragma unroll
+        for (int d = 0; d < NDIR / 2; d++) {
+          // the lesser of a pair counts as zero
+          if ((hm[d] < hm[d + 4] ? 0 : hm[d]) >= maxval) m |= 1u << d;
+          if ((hm[d] > hm[d + 4] ? 0 : hm[d + 4]) >= maxval) m |= 16u << d;
+        }
+        chosen[i] = (unsigned char)m;
+      }
+      // (own writes: this thread's pixels)
+#pragma unroll 2
+      for (int i = tid; i < rows * cols; i += nth) {
+        const int q = fd.div(i), row = T.r0 + q, col = T.c0 + i - q * cols;
+        const unsigned m = chosen[i];
+        const float nat = __ldg(tb + (size_t)row * W + col);
+        const int f = own[row * ts + col];
+        const float2* px = srgb + (row * ts + col);
+        float2 p[NDIR];
+#pragma unroll
+        for (int d = 0; d < NDIR; d++) p[d] = xs_load_if(px + d * ts * ts, m & 1u << d);
+        float ax = 0.f, ay = 0.f, an_ = 0.f;
+#pragma unroll
+        for (int d = 0; d < NDIR; d++) {
+          ax += p[d].x;  // (a zero added changes no sum)
+          ay += p[d].y;
+          if (m & 1u << d) an_ += nat;
+        }
+        const float n = (float)__popc(m);
+        ax = fmaxf(0.f, ax / n);
+        ay = fmaxf(0.f, ay / n);
+        an_ = fmaxf(0.f, an_ / n);
+        float* o = A.rgb_out + ((size_t)(row + top) * W + (col + left)) * 3;
+        o[0] = f == 0 ? an_ : ax;
+        o[1] = f == 0 ? ax : (f == 1 ? an_ : ay);
+        o[2] = f == 2 ? an_ : ay;
       }
     }
     __syncthreads();
@@ -1278,6 +1590,47 @@ bool xt_sites_ok(const XtParams& P) {
   return true;
 }
 
+// Whether a plane may keep the last one's values: every slot that a step of
+// pass 0 reads is then native, never written, or written by an earlier step of
+// the same plane ((b) greens, (d) solitary greens, (e) non-green sites).  True
+// for the X-Trans layouts and their shifts.
+bool xt_fresh_once(const XtParams& P) {
+  auto fc = [&](int r, int c) { return (int)P.xt[(r + 12) % 6][(c + 12) % 6]; };
+  auto isg = [&](int r, int c) { return P.xt[(r + 12) % 3][(c + 12) % 3] & 1; };
+  auto sol = [&](int r, int c) { return (r + 12 - P.sgrow) % 3 == 0 && (c + 12 - P.sgcol) % 3 == 0; };
+  for (int r = 0; r < 6; r++)
+    for (int c = 0; c < 6; c++) {
+      if ((fc(r, c) == 1) != (isg(r, c) != 0)) return false;
+      if (sol(r, c)) {
+        // (d): the colour at distance 1 along the row, the other at 2, and the
+        // other way round along the column
+        const int h = fc(r, c + 1);
+        if (h == 1 || !isg(r, c)) return false;
+        for (int s = -1; s <= 1; s += 2)
+          if (fc(r, c + s) != h || fc(r, c + 2 * s) != (h ^ 2) || fc(r + s, c) != (h ^ 2) || fc(r + 2 * s, c) != h)
+            return false;
+      } else if (!isg(r, c)) {
+        // (e): its other colour at distance 1 across or along, and 3
+        const int f = 2 - fc(r, c);
+        const bool off = (r + 12 - P.sgrow) % 3 != 0;
+        for (int s = -3; s <= 3; s += 2) {
+          const bool down = off == (s == 1 || s == -1);
+          const int rr = down ? r + s : r, cc = down ? c : c + s;
+          if (fc(rr, cc) != f && !sol(rr, cc)) return false;
+        }
+      } else {
+        // (f): its hexagon holds no site of its own step
+        for (int d = 0; d < 8; d++)
+          for (int v = -2; v <= 2; v++) {
+            const int h = P.allhex1[r % 3][c % 3][d] - v * XTS;
+            if (h < -2 || h > 2) continue;
+            if (isg(r + v, c + h) && !sol(r + v, c + h)) return false;
+          }
+      }
+    }
+  return true;
+}
+
 // The plane-resident kernel runs where the replay accepts the pattern,
 // unless LRE_XTRANS_ROWSCAN=1 asks for the row-scan kernel (a test hook:
 // it keeps the fallback path covered on the X-Trans layouts).
@@ -1311,6 +1664,7 @@ lre_status launch_xtrans(Context* c, const float* raw, int cstride, float* rgb, 
   if (2 * w + 2 > 32767 && passes != 1)
     return fail(c, LRE_ERR_INVALID_ARGUMENT, "demosaic_xtrans_3pass: width above 16382 overflows the hexagon offsets");
   A.P = make_xt_params(xtrans, (int)w);
+  A.refill = !xt_fresh_once(A.P);
   if (passes == 1) {
     // border (1 px) first, then the interior (:2681-2760)
     k_xtrans_border<<<grid_for(4 * (w + h), 256, c->sm_count * 2), 256, 0, c->stream>>>(A, 1);
