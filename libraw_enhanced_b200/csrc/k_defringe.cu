@@ -595,23 +595,14 @@ constexpr int LT = 32;   // line-link output tile
 constexpr int LH = 14;   // max step along a line
 constexpr int LE = LT + 2 * LH;
 
-// Running max of a line's samples.  `along` starts at 0 and the samples are
-// finite or NaN: std::max(along, v) then equals fmaxf(along, v) (neither ever
-// yields NaN), so the single-instruction form is exact here.
-template <int TX, int TY, int STEPS>
-__device__ __forceinline__ float line_along(const float* s_ls, int c) {
-  float along = 0.f;
-#pragma unroll
-  for (int step = 1; step <= STEPS; step++) {
-    along = fmaxf(along, s_ls[c + (TY * LE + TX) * step]);
-    along = fmaxf(along, s_ls[c - (TY * LE + TX) * step]);
-  }
-  return along;
-}
+constexpr int LN_THREADS = 320;
+static_assert(LE % (LN_THREADS / 32) == 0 && LE <= 64, "whole rows, two columns to a lane");
+constexpr int LPAD = 16;  // floats around the sources: runs that begin or end beside the tile read up to 4 beyond
 
-template <int TX, int TY, int STEPS>
-__device__ __forceinline__ void line_dir(const float* s_ls, const float* s_fs, int c, float& best) {
-  const float along = line_along<TX, TY, STEPS>(s_ls, c);
+// A direction's share of a pixel's line support, from the largest source along
+// the line on either side.
+template <int TX, int TY>
+__device__ __forceinline__ void line_dir(const float* s_fs, int c, float along, float& best) {
   // along == 0 contributes 0 * thin (thin in [0, 1], or NaN which
   // std::max ignores) to a running max that is already >= 0
   if (along == 0.f) return;
@@ -621,57 +612,151 @@ __device__ __forceinline__ void line_dir(const float* s_ls, const float* s_fs, i
   best = smax(best, along * thin);
 }
 
+// Four neighbouring pixels of a line share most of their windows: v holds the
+// line from STEPS before the first to STEPS behind the last.  The maximum starts
+// at 0 and the samples are finite or NaN: std::max(along, v) then equals
+// fmaxf(along, v) (neither ever yields NaN) in whatever order.
+template <int STEPS>
+__device__ __forceinline__ void line_windows(const float (&v)[2 * STEPS + 4], float (&along)[4]) {
+  float back = 0.f, ahead = 0.f;
+#pragma unroll
+  for (int k = 3; k < STEPS; k++) back = fmaxf(back, v[k]);
+#pragma unroll
+  for (int k = STEPS + 4; k <= 2 * STEPS; k++) ahead = fmaxf(ahead, v[k]);
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    float a = fmaxf(back, ahead);
+#pragma unroll
+    for (int k = j; k < 3; k++) a = fmaxf(a, fmaxf(v[k], v[k + STEPS + 1]));
+#pragma unroll
+    for (int k = 0; k < j; k++) a = fmaxf(a, fmaxf(v[STEPS + k], v[2 * STEPS + 1 + k]));
+    along[j] = a;
+  }
+}
+
+// One direction over the tile, a thread per run of four pixels along it,
+// (x + DX j, y + DY j); (TX, TY) is the reference's sense of the direction.
+// Runs that leave the tile sideways hold fewer pixels of it.
+template <int DX, int DY, int STEPS, int TX, int TY>
+__device__ __forceinline__ void line_runs(const float* s_ls, const float* s_fs, float* s_best) {
+  constexpr int AX = DX < 0 ? -DX : DX, NS = LT + 3 * AX, STEP = DY * LE + DX;
+  for (int i = threadIdx.x; i < 8 * NS; i += LN_THREADS) {
+    const int g = i / NS, x = i - g * NS - (DX > 0 ? 3 * AX : 0);
+    const int y = DY == 1 ? 4 * g : 8 * (g >> 1) + (g & 1);
+    const int c = (y + LH) * LE + x + LH;
+    float v[2 * STEPS + 4], along[4];
+#pragma unroll
+    for (int k = 0; k < 2 * STEPS + 4; k++) v[k] = s_ls[c + (k - STEPS) * STEP];
+    line_windows<STEPS>(v, along);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (AX && (unsigned)(x + DX * j) >= (unsigned)LT) continue;
+      float& best = s_best[(y + DY * j) * LT + x + DX * j];
+      line_dir<TX, TY>(s_fs, c + j * STEP, along[j], best);
+    }
+  }
+  __syncthreads();
+}
+
+// K5: line-linked support, then the solo seeds.  Bound by instructions and, a
+// little, by the wait for the staged rows:
+// * the eight directions' maxima are formed for four pixels of a line at a time
+//   (of a pixel each: 160 loads and 160 maxima), with enough threads that every
+//   direction's runs, up to 304 of a tile, take one turn;
+// * a warp stages whole rows, all of its loads in flight (an element's place by
+//   two divisions and four clamps, two in flight: about 105 instructions a pixel);
+// * a pixel whose blurred edge planes are at or below the lower smoothstep edges
+//   has solo seeds of exactly 0 where every log ratio of the image is finite
+//   (K3's rule), without the two exponentials in double.
+// 51 MP: 1223 us before, 768 us; 26 MP odd 664 and 470 us; 1.9 MP 55 and 45 us.
+// (256 threads 926 us at 51 MP; two rows in flight 853 us; five CTAs per SM, which
+// spill, 769 us.)
 template <bool FAST>
-__global__ void __launch_bounds__(256) k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfTab T) {
-  __shared__ float s_ls[LE * LE];
+__global__ void __launch_bounds__(LN_THREADS, 4) k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfConst k,
+                                                 DfTab T, const DfScalars* sc) {
+  __shared__ __align__(16) float s_src[LPAD + LE * LE + LPAD];
   __shared__ float s_fs[LE * LE];
+  __shared__ __align__(16) float s_best[LT * LT];
   __shared__ int s_any;
+  float* s_ls = s_src + LPAD;
   const int x0 = blockIdx.x * LT, y0 = blockIdx.y * LT;
   if (threadIdx.x == 0) s_any = 0;
   __syncthreads();
   int any = 0;
-  for (int i = threadIdx.x; i < LE * LE; i += blockDim.x) {
-    int gy = min(max(y0 - LH + i / LE, 0), H - 1);
-    int gx = min(max(x0 - LH + i % LE, 0), W - 1);
-    size_t gi = (size_t)gy * W + gx;
-    float f = P.fs[gi];
-    s_fs[i] = f;
-    const float ls = smax(f, P.bfs[gi] * 0.55f);
-    s_ls[i] = ls;
-    any |= ls != 0.f;
+  {
+    const int lane = threadIdx.x & 31, gx0 = min(max(x0 - LH + lane, 0), W - 1), gx1 = min(x0 - LH + lane + 32, W - 1);
+#pragma unroll
+    for (int r = threadIdx.x >> 5; r < LE; r += LN_THREADS / 32) {
+      const size_t gr = (size_t)min(max(y0 - LH + r, 0), H - 1) * W;
+      const float f0 = P.fs[gr + gx0], b0 = P.bfs[gr + gx0];
+      const float f1 = P.fs[gr + gx1], b1 = P.bfs[gr + gx1];
+      const float l0 = smax(f0, b0 * 0.55f), l1 = smax(f1, b1 * 0.55f);
+      s_fs[r * LE + lane] = f0;
+      s_ls[r * LE + lane] = l0;
+      any |= l0 != 0.f;
+      if (lane < LE - 32) {
+        s_fs[r * LE + lane + 32] = f1;
+        s_ls[r * LE + lane + 32] = l1;
+        any |= l1 != 0.f;
+      }
+    }
   }
   if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) s_any = 1;
   __syncthreads();
   // a tile whose line sources are all zero has every `along` zero, so every
   // line-linked support value is exactly 0
   const bool tile_active = s_any != 0;
+  if (tile_active) {
+    // directions and step counts of core/cpu_accelerator.cpp:4290-4318; along
+    // a row first, from vector loads, which sets every pixel's value
+    if (threadIdx.x < 256) {
+      const int y = threadIdx.x >> 3, x = (threadIdx.x & 7) * 4, c = (y + LH) * LE + x + LH;
+      float v[32], along[4], best[4];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const float4 t = *reinterpret_cast<const float4*>(s_ls + c - LH + 4 * q);
+        v[4 * q] = t.x;
+        v[4 * q + 1] = t.y;
+        v[4 * q + 2] = t.z;
+        v[4 * q + 3] = t.w;
+      }
+      line_windows<14>(v, along);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        best[j] = 0.f;
+        line_dir<1, 0>(s_fs, c + j, along[j], best[j]);
+      }
+      *reinterpret_cast<float4*>(s_best + y * LT + x) = make_float4(best[0], best[1], best[2], best[3]);
+    }
+    __syncthreads();
+    line_runs<0, 1, 14, 0, 1>(s_ls, s_fs, s_best);
+    line_runs<1, 1, 14, 1, 1>(s_ls, s_fs, s_best);
+    line_runs<-1, 1, 14, 1, -1>(s_ls, s_fs, s_best);
+    line_runs<2, 1, 6, 2, 1>(s_ls, s_fs, s_best);
+    line_runs<1, 2, 6, 1, 2>(s_ls, s_fs, s_best);
+    line_runs<-2, 1, 6, 2, -1>(s_ls, s_fs, s_best);
+    line_runs<-1, 2, 6, 1, -2>(s_ls, s_fs, s_best);
+  }
+  const float e0_edge = T.e[DE_CORE].e0, e0_raw = T.e[DE_CORE_RAW].e0;
+  const bool can_skip = sc->nonfinite == 0 && k.edge_thr > 0.f;
   for (int i = threadIdx.x; i < LT * LT; i += blockDim.x) {
     int ly = i / LT, lx = i % LT;
     int y = y0 + ly, x = x0 + lx;
     if (x >= W || y >= H) continue;
-    const int c = (ly + LH) * LE + (lx + LH);
     const size_t gi = (size_t)y * W + x;
-    // the solo-seed operands are loaded first, so their latency overlaps
-    // the line search (which reads shared memory only); loaded after the
-    // lfs store below, they would wait for it
+    const float best = tile_active ? s_best[i] : 0.f;
+    const float be = P.be[gi], ber = P.ber[gi];
+    P.lfs[gi] = best;
+    if (can_skip && (be <= e0_edge || ber <= e0_raw)) {
+      P.srs[gi] = 0.f;
+      P.sbs[gi] = 0.f;
+      continue;
+    }
     const float* s = src + gi * 3;
     const float s0 = s[0], s1 = s[1], s2 = s[2];
     const float blur_guide = P.bg[gi];
     const float blrg = P.blrg[gi], blbg = P.blbg[gi];
-    const float bfs = P.bfs[gi], be = P.be[gi], ber = P.ber[gi];
-    float best = 0.f;
-    if (tile_active) {
-      // directions and step counts of core/cpu_accelerator.cpp:4290-4318
-      line_dir<1, 0, 14>(s_ls, s_fs, c, best);
-      line_dir<0, 1, 14>(s_ls, s_fs, c, best);
-      line_dir<1, 1, 14>(s_ls, s_fs, c, best);
-      line_dir<1, -1, 14>(s_ls, s_fs, c, best);
-      line_dir<2, 1, 6>(s_ls, s_fs, c, best);
-      line_dir<1, 2, 6>(s_ls, s_fs, c, best);
-      line_dir<2, -1, 6>(s_ls, s_fs, c, best);
-      line_dir<1, -2, 6>(s_ls, s_fs, c, best);
-    }
-    P.lfs[gi] = best;
+    const float bfs = P.bfs[gi];
 
     // solo seeds (core/cpu_accelerator.cpp:4325-4374)
     const float g = smax(s1, 0.f);
@@ -1265,7 +1350,7 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
 
   dim3 lgrid((W + LT - 1) / LT, (H + LT - 1) / LT);
   auto line = fast ? k_df_line<true> : k_df_line<false>;
-  line<<<lgrid, 256, 0, c->stream>>>(in, W, H, P, T);
+  line<<<lgrid, LN_THREADS, 0, c->stream>>>(in, W, H, P, k, T, sc);
   count_launch(c);
   LRE_TRY(check_launch(c, "defringe line"));
 
