@@ -1097,13 +1097,19 @@ __device__ __forceinline__ void df_main_px(float s0, float s1, float s2, const D
 // only when a pixel of the group needs them.  The group's operands are then
 // staged in shared memory (one column per thread) and one copy of the
 // per-pixel code runs over the four pixels.
+// Bound by the instructions of the pixels that don't keep their input, in warps
+// where the others wait.  PACK: a warp lists its pixels with work and deals them
+// to its lanes (51 MP 1008 us without, 853 us with; 1.9 MP 72 and 59 us; seven
+// CTAs per SM, which spill more, 863 us).
 constexpr int DFM_THREADS = 128;
 constexpr int DFM_VALS = 14;  // s0 s1 s2 be ber srb sbb bg blrg blbg bfs lfs lrg lbg
 
-template <bool FAST>
-__global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, float* dst, int W, int H, DfPlanes P,
-                                                           DfConst k, DfTab T, const DfScalars* sc, float* out_max_g) {
+template <bool FAST, bool PACK>
+__global__ void __launch_bounds__(DFM_THREADS, 6)
+    k_df_main(const float* src, float* dst, int W, int H, DfPlanes P, DfConst k, DfTab T, const DfScalars* sc,
+              float* out_max_g) {
   __shared__ float S[DFM_VALS * 4][DFM_THREADS];
+  __shared__ unsigned char s_list[PACK ? 4 * DFM_THREADS : 1];
   DfMainK K;
   K.mask_cutoff = T.mask_cutoff;
   const float max_guide = df_max_guide(sc);
@@ -1120,70 +1126,104 @@ __global__ void __launch_bounds__(DFM_THREADS, 6) k_df_main(const float* src, fl
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const int tid = threadIdx.x;
   float mg = 0.f;  // max(0, G) of what this thread writes (fmaxf drops NaN)
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + tid; q < n4; q += stride) {
-    const size_t i = q * 4;
-    float s[12], be[4], ber[4], srb[4], sbb[4];
-    ld4(src + i * 3, s);
-    ld4(src + i * 3 + 4, s + 4);
-    ld4(src + i * 3 + 8, s + 8);
-    ld4(P.be + i, be);
-    ld4(P.ber + i, ber);
-    ld4(P.srb + i, srb);
-    ld4(P.sbb + i, sbb);
-    unsigned keep = 0;
+  const int lane = tid & 31, wb = tid - lane;
+  unsigned char* list = s_list + 4 * wb;
+  for (size_t q0 = blockIdx.x * (size_t)blockDim.x + wb; q0 < n4; q0 += stride) {
+    const size_t i = (q0 + lane) * 4;
+    unsigned keep = 0xFu;
+    if (q0 + lane < n4) {
+      float s[12], be[4], ber[4], srb[4], sbb[4];
+      ld4(src + i * 3, s);
+      ld4(src + i * 3 + 4, s + 4);
+      ld4(src + i * 3 + 8, s + 8);
+      ld4(P.be + i, be);
+      ld4(P.ber + i, ber);
+      ld4(P.srb + i, srb);
+      ld4(P.sbb + i, sbb);
+      keep = 0;
 #pragma unroll
-    for (int t = 0; t < 4; t++) keep |= df_keeps_input(K, be[t], ber[t], srb[t], sbb[t]) ? 1u << t : 0u;
-    if (keep == 0xFu) {
-      st4(dst + i * 3, s);
-      st4(dst + i * 3 + 4, s + 4);
-      st4(dst + i * 3 + 8, s + 8);
-      mg = fmaxf(mg, fmaxf(fmaxf(s[1], s[4]), fmaxf(s[7], s[10])));
-      continue;
+      for (int t = 0; t < 4; t++) keep |= df_keeps_input(K, be[t], ber[t], srb[t], sbb[t]) ? 1u << t : 0u;
+      if (keep == 0xFu) {
+        st4(dst + i * 3, s);
+        st4(dst + i * 3 + 4, s + 4);
+        st4(dst + i * 3 + 8, s + 8);
+        mg = fmaxf(mg, fmaxf(fmaxf(s[1], s[4]), fmaxf(s[7], s[10])));
+      } else {
+        float pl[7][4];
+        ld4(P.bg + i, pl[0]);
+        ld4(P.blrg + i, pl[1]);
+        ld4(P.blbg + i, pl[2]);
+        ld4(P.bfs + i, pl[3]);
+        ld4(P.lfs + i, pl[4]);
+        ld4(P.lrg + i, pl[5]);
+        ld4(P.lbg + i, pl[6]);
+        // S[v * 4 + t][tid]: value v of pixel t
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          S[0 * 4 + t][tid] = s[3 * t];
+          S[1 * 4 + t][tid] = s[3 * t + 1];
+          S[2 * 4 + t][tid] = s[3 * t + 2];
+          S[3 * 4 + t][tid] = be[t];
+          S[4 * 4 + t][tid] = ber[t];
+          S[5 * 4 + t][tid] = srb[t];
+          S[6 * 4 + t][tid] = sbb[t];
+#pragma unroll
+          for (int v = 0; v < 7; v++) S[(7 + v) * 4 + t][tid] = pl[v][t];
+        }
+      }
     }
-    float pl[7][4];
-    ld4(P.bg + i, pl[0]);
-    ld4(P.blrg + i, pl[1]);
-    ld4(P.blbg + i, pl[2]);
-    ld4(P.bfs + i, pl[3]);
-    ld4(P.lfs + i, pl[4]);
-    ld4(P.lrg + i, pl[5]);
-    ld4(P.lbg + i, pl[6]);
-    // S[v * 4 + t][tid]: value v of pixel t
+    if (PACK) {
+      // the warp's pixels with work, dealt to its lanes
+      int count = 0;
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      S[0 * 4 + t][tid] = s[3 * t];
-      S[1 * 4 + t][tid] = s[3 * t + 1];
-      S[2 * 4 + t][tid] = s[3 * t + 2];
-      S[3 * 4 + t][tid] = be[t];
-      S[4 * 4 + t][tid] = ber[t];
-      S[5 * 4 + t][tid] = srb[t];
-      S[6 * 4 + t][tid] = sbb[t];
-#pragma unroll
-      for (int v = 0; v < 7; v++) S[(7 + v) * 4 + t][tid] = pl[v][t];
-    }
+      for (int t = 0; t < 4; t++) {
+        const bool work = !(keep >> t & 1u);
+        const unsigned m = __ballot_sync(~0u, work);
+        if (work) list[count + __popc(m & ((1u << lane) - 1))] = (unsigned char)(t << 5 | lane);
+        count += __popc(m);
+      }
+      __syncwarp();
 #pragma unroll 1
-    for (int t = 0; t < 4; t++) {
-      if (keep >> t & 1u) continue;
-      const DfPx v{S[3 * 4 + t][tid],  S[4 * 4 + t][tid],  S[5 * 4 + t][tid],  S[6 * 4 + t][tid],
-                   S[7 * 4 + t][tid],  S[8 * 4 + t][tid],  S[9 * 4 + t][tid],  S[10 * 4 + t][tid],
-                   S[11 * 4 + t][tid], S[12 * 4 + t][tid], S[13 * 4 + t][tid]};
-      float r0, r1, r2;
-      df_main_px<FAST>(S[0 * 4 + t][tid], S[1 * 4 + t][tid], S[2 * 4 + t][tid], v, K, T, r0, r1, r2);
-      S[0 * 4 + t][tid] = r0;
-      S[1 * 4 + t][tid] = r1;
-      S[2 * 4 + t][tid] = r2;
+      for (int j = lane; j < count; j += 32) {
+        const int t = list[j] >> 5, x = wb + (list[j] & 31);
+        const DfPx v{S[3 * 4 + t][x],  S[4 * 4 + t][x],  S[5 * 4 + t][x],  S[6 * 4 + t][x],
+                     S[7 * 4 + t][x],  S[8 * 4 + t][x],  S[9 * 4 + t][x],  S[10 * 4 + t][x],
+                     S[11 * 4 + t][x], S[12 * 4 + t][x], S[13 * 4 + t][x]};
+        float r0, r1, r2;
+        df_main_px<FAST>(S[0 * 4 + t][x], S[1 * 4 + t][x], S[2 * 4 + t][x], v, K, T, r0, r1, r2);
+        S[0 * 4 + t][x] = r0;
+        S[1 * 4 + t][x] = r1;
+        S[2 * 4 + t][x] = r2;
+      }
+      __syncwarp();
+    } else {
+#pragma unroll 1
+      for (int t = 0; t < 4; t++) {
+        if (keep >> t & 1u) continue;
+        const DfPx v{S[3 * 4 + t][tid],  S[4 * 4 + t][tid],  S[5 * 4 + t][tid],  S[6 * 4 + t][tid],
+                     S[7 * 4 + t][tid],  S[8 * 4 + t][tid],  S[9 * 4 + t][tid],  S[10 * 4 + t][tid],
+                     S[11 * 4 + t][tid], S[12 * 4 + t][tid], S[13 * 4 + t][tid]};
+        float r0, r1, r2;
+        df_main_px<FAST>(S[0 * 4 + t][tid], S[1 * 4 + t][tid], S[2 * 4 + t][tid], v, K, T, r0, r1, r2);
+        S[0 * 4 + t][tid] = r0;
+        S[1 * 4 + t][tid] = r1;
+        S[2 * 4 + t][tid] = r2;
+      }
     }
-    float d[12];
+    if (keep != 0xFu) {
+      float d[12];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-      d[3 * t] = S[0 * 4 + t][tid];
-      d[3 * t + 1] = S[1 * 4 + t][tid];
-      d[3 * t + 2] = S[2 * 4 + t][tid];
+      for (int t = 0; t < 4; t++) {
+        d[3 * t] = S[0 * 4 + t][tid];
+        d[3 * t + 1] = S[1 * 4 + t][tid];
+        d[3 * t + 2] = S[2 * 4 + t][tid];
+      }
+      st4(dst + i * 3, d);
+      st4(dst + i * 3 + 4, d + 4);
+      st4(dst + i * 3 + 8, d + 8);
+      mg = fmaxf(mg, fmaxf(fmaxf(d[1], d[4]), fmaxf(d[7], d[10])));
     }
-    st4(dst + i * 3, d);
-    st4(dst + i * 3 + 4, d + 4);
-    st4(dst + i * 3 + 8, d + 8);
-    mg = fmaxf(mg, fmaxf(fmaxf(d[1], d[4]), fmaxf(d[7], d[10])));
+    if (PACK) __syncwarp();
   }
   for (size_t i = n4 * 4 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     const float s0 = src[i * 3 + 0], s1 = src[i * 3 + 1], s2 = src[i * 3 + 2];
@@ -1362,8 +1402,13 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
 
   // Eight times the resident CTAs: the work of a pixel depends on what it shows,
   // and CTAs that took a sixth of an SM's share each left SMs idle at the end
-  // (51 MP 1110 us with 6 per SM, 997 us with 48; 26 MP odd 1261 and 1183 us).
-  auto main_pass = fast ? k_df_main<true> : k_df_main<false>;
+  // (51 MP 1110 us with 6 per SM, 997 us with 48; 26 MP odd 1261 and 1183 us;
+  // before packing).
+  // Packing pays where pixels keep their input; with green correction none does
+  // (24 MP 589 us without, 485 us with it; 26 MP with green 1181 and 1279 us).
+  const bool pack = !k.green && k.edge_thr > 0.f;
+  auto main_pass = fast ? (pack ? k_df_main<true, true> : k_df_main<true, false>)
+                        : (pack ? k_df_main<false, true> : k_df_main<false, false>);
   main_pass<<<grid_for((n + 3) / 4, DFM_THREADS, c->sm_count * 48), DFM_THREADS, 0, c->stream>>>(in, out, W, H, P, k,
                                                                                                 T, sc, out_max_g);
   count_launch(c);

@@ -2,7 +2,8 @@
 its surroundings within the filter's reach only, so a crop that moves the tile
 grid over the picture leaves the pixels beyond that reach as they are, bit for
 bit.  Runs of four pixels leave the tile sideways by up to six, and begin in
-each of its rows and columns, as the grid moves."""
+each of its rows and columns, as the grid moves; the correction's warps pack
+other pixels together, and end within a group of four at odd widths."""
 import numpy as np
 import pytest
 
