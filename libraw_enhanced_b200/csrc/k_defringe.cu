@@ -62,68 +62,90 @@ __device__ __forceinline__ float guide_signal_at(const float* __restrict__ src, 
   return sqrtf(sclamp(gg / max_guide, 0.f, 1.f));
 }
 
-// K1 on 32 x 8 output tiles: the guide signal (a square root and a divide
-// per pixel) is staged once per pixel in shared memory with a 1-px halo and
-// the Sobel taps read it from there, instead of recomputing it for each of
-// the 8 neighbours that use it.
-constexpr int PT_X = 32, PT_Y = 8;
+// K1: log ratios and Sobel magnitude of the guide signal.  A warp walks up to
+// PW_ROWS rows of 30 columns (and one beside them on either side): the guide signal, a
+// square root and a divide, is formed once per pixel, its neighbours come from
+// the lanes beside and the two rows before, and the next two rows are on their
+// way meanwhile.  Bound by instructions: two logarithms in double, two divides
+// and the guide.  51 MP 438 us, 26 MP odd 234 us, 1.9 MP
+// 20 us; on 32 x 8 tiles with the guide in shared memory, a barrier before and after,
+// 783, 402 and 24 us, and with CUDA's log in double besides 856, 441 and 27 us.
+constexpr int PW_ROWS = 32, PW_COLS = 30;
 
-__global__ void __launch_bounds__(256) k_df_prep_tiled(const float* __restrict__ src, int W, int H, DfScalars* sc,
-                                                       float* __restrict__ lrg, float* __restrict__ lbg,
-                                                       float* __restrict__ er) {
-  __shared__ float s_g[PT_Y + 2][PT_X + 3];
+__global__ void __launch_bounds__(256) k_df_prep(const float* __restrict__ src, int W, int H, int rows, DfScalars* sc,
+                                                 float* __restrict__ lrg, float* __restrict__ lbg,
+                                                 float* __restrict__ er) {
+  __shared__ __align__(16) double2 s_log[LOG_TAB_N];
+  log_tab_fill(s_log);
+  __syncthreads();
   const float max_guide = df_max_guide(sc);
   const float ratio_eps = smax(max_guide * 1e-4f, 1e-6f);
   const int limit_y = (H > 1) ? H - 1 : 1;
   const int limit_x = (W > 1) ? W - 1 : 1;
-  const int tiles_x = (W + PT_X - 1) / PT_X;
-  const int n_tiles = tiles_x * ((H + PT_Y - 1) / PT_Y);
+  const int strips = (W + PW_COLS - 1) / PW_COLS;
+  const long long items = (long long)strips * ((H + rows - 1) / rows);
+  const int lane = threadIdx.x & 31;
+  auto guide = [&](float g) { return sqrtf(sclamp(smax(g, 0.f) / max_guide, 0.f, 1.f)); };
+  bool odd = false;
   float local_max = 0.f;
-  // a CTA walks several tiles, so the max-edge reduction costs one atomic
-  // per warp in total rather than one per tile
-  for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    const int x0 = (t % tiles_x) * PT_X, y0 = (t / tiles_x) * PT_Y;
-    __syncthreads();  // the previous tile's readers are done with s_g
-    for (int i = threadIdx.x; i < (PT_Y + 2) * (PT_X + 2); i += blockDim.x) {
-      const int r = i / (PT_X + 2), q = i % (PT_X + 2);
-      const int gy = min(max(y0 - 1 + r, 0), H - 1);
-      const int gx = min(max(x0 - 1 + q, 0), W - 1);
-      s_g[r][q] = guide_signal_at(src, gx, gy, W, max_guide);
-    }
-    __syncthreads();
-    const int tx = threadIdx.x % PT_X, ty = threadIdx.x / PT_X;
-    const int x = x0 + tx, y = y0 + ty;
-    if (x < W && y < H) {
-      const size_t i = (size_t)y * W + x;
-      const float* p = src + i * 3;
-      float r = p[0], g = p[1], b = p[2];
-      float gg = smax(g, 0.f);
-      const float lr = log_cr((smax(r, 0.f) + ratio_eps) / (gg + ratio_eps));
-      const float lb = log_cr((smax(b, 0.f) + ratio_eps) / (gg + ratio_eps));
-      lrg[i] = lr;
-      lbg[i] = lb;
-      if (!(isfinite(lr) && isfinite(lb))) sc->nonfinite = 1;
+  for (long long it = blockIdx.x * 8LL + (threadIdx.x >> 5); it < items; it += gridDim.x * 8LL) {
+    const int chunk = (int)(it / strips), x = (int)(it - (long long)chunk * strips) * PW_COLS + lane - 1;
+    const int y0 = chunk * rows, y1 = min(y0 + rows, H);
+    const float* col = src + (size_t)min(max(x, 0), W - 1) * 3;
+    auto row = [&](int y) { return col + (size_t)min(max(y, 0), H - 1) * W * 3; };
+    struct Px {
+      float r, g, b;
+    };
+    auto load = [&](int y) {
+      const float* p = row(y);
+      return Px{p[0], p[1], p[2]};
+    };
+    // a: the row above, b: this row, c: the row below; 0 left, 1 here, 2 right
+    auto across = [&](float v, float& l, float& r) {
+      l = __shfl_up_sync(~0u, v, 1);
+      r = __shfl_down_sync(~0u, v, 1);
+    };
+    Px cur = load(y0), nxt = load(y0 + 1);
+    float a00, a01 = guide(row(y0 - 1)[1]), a02, a10, a11 = guide(cur.g), a12, a20, a21, a22;
+    across(a01, a00, a02);
+    across(a11, a10, a12);
+    const bool mine = lane >= 1 && lane <= PW_COLS && x < W;
+    const bool inside = mine && x >= 1 && x < limit_x;
+#pragma unroll 2
+    for (int y = y0; y < y1; y++) {
+      const Px aft = load(y + 2);
+      a21 = guide(nxt.g);
+      across(a21, a20, a22);
+      const float gg = smax(cur.g, 0.f);
+      const float lr = log_tab(s_log, (smax(cur.r, 0.f) + ratio_eps) / (gg + ratio_eps));
+      const float lb = log_tab(s_log, (smax(cur.b, 0.f) + ratio_eps) / (gg + ratio_eps));
       float mag = 0.f;
-      if (y >= 1 && y < limit_y && x >= 1 && x < limit_x) {
-        const int cy = ty + 1, cx = tx + 1;
-        float a00 = s_g[cy - 1][cx - 1];
-        float a01 = s_g[cy - 1][cx];
-        float a02 = s_g[cy - 1][cx + 1];
-        float a10 = s_g[cy][cx - 1];
-        float a12 = s_g[cy][cx + 1];
-        float a20 = s_g[cy + 1][cx - 1];
-        float a21 = s_g[cy + 1][cx];
-        float a22 = s_g[cy + 1][cx + 1];
-        float gx = -a00 + a02 - 2.f * a10 + 2.f * a12 - a20 + a22;
-        float gy = -a00 - 2.f * a01 - a02 + a20 + 2.f * a21 + a22;
+      if (inside && y >= 1 && y < limit_y) {
+        const float gx = -a00 + a02 - 2.f * a10 + 2.f * a12 - a20 + a22;
+        const float gy = -a00 - 2.f * a01 - a02 + a20 + 2.f * a21 + a22;
         mag = sqrtf(gx * gx + gy * gy);
         local_max = smax(local_max, mag);
       }
-      er[i] = mag;
+      if (mine) {
+        const size_t i = (size_t)y * W + x;
+        odd |= !(isfinite(lr) && isfinite(lb));
+        lrg[i] = lr;
+        lbg[i] = lb;
+        er[i] = mag;
+      }
+      cur = nxt;
+      nxt = aft;
+      a00 = a10;
+      a01 = a11;
+      a02 = a12;
+      a10 = a20;
+      a11 = a21;
+      a12 = a22;
     }
   }
+  if (odd) sc->nonfinite = 1;
   local_max = warp_max(local_max);
-  if ((threadIdx.x & 31) == 0) atomic_max_float(&sc->max_edge, local_max);
+  if (lane == 0) atomic_max_float(&sc->max_edge, local_max);
 }
 
 // ---------------------------------------------------------------- blurs
@@ -1364,9 +1386,14 @@ lre_status launch_defringe(Context* c, const float* in, float* out, size_t w, si
     k_df_maxg<<<grid_for(n, 256, c->sm_count * 4), 256, 0, c->stream>>>(in, n, sc);
     count_launch(c);
   }
-  const size_t prep_tiles = (size_t)((W + PT_X - 1) / PT_X) * ((H + PT_Y - 1) / PT_Y);
-  k_df_prep_tiled<<<(unsigned)std::min<size_t>(prep_tiles, (size_t)c->sm_count * 8), 256, 0, c->stream>>>(
-      in, W, H, sc, P.lrg, P.lbg, P.er);
+  // Rows of a walk: 32, fewer while the SMs have less than 32 warps each (two
+  // rows beside a walk are formed for it alone).
+  const size_t prep_strips = (W + PW_COLS - 1) / PW_COLS;
+  int prep_rows = PW_ROWS;
+  while (prep_rows > 4 && prep_strips * ((H + prep_rows - 1) / prep_rows) < (size_t)c->sm_count * 32) prep_rows /= 2;
+  const size_t prep_blocks = (prep_strips * ((H + prep_rows - 1) / prep_rows) + 7) / 8;
+  k_df_prep<<<(unsigned)std::min<size_t>(prep_blocks, (size_t)c->sm_count * 24), 256, 0, c->stream>>>(
+      in, W, H, prep_rows, sc, P.lrg, P.lbg, P.er);
   count_launch(c);
   LRE_TRY(check_launch(c, "defringe prep"));
 
