@@ -39,10 +39,11 @@ __device__ __forceinline__ float aces_tm(float x) {
 // and quantity pair) beside 20 B/px of HBM traffic per pass.  The form before
 // (one thread per row, then one per column, each walking the whole image with
 // a running sum) left the GPU to H or W threads: 18.97 ms at 8256x5504; this
-// one takes 0.74 ms.  A sum restarts at every chunk (DT_ROWS rows) and every
-// four columns, so it carries the roundings of at most DT_ROWS + 2R additions
-// instead of the whole column's: the error against 64 bits is 2e-7 where
-// the whole-image running sums had 1.7e-6.
+// one takes 0.63 ms (0.74 ms with eight divisions a lane and row by the number of
+// samples, whose reciprocals a lane now keeps).  A sum restarts at every chunk of
+// rows and every four columns, so it carries the roundings of at most 256 + 2R
+// additions instead of the whole column's: the error against 64 bits is 2e-7
+// where the whole-image running sums had 1.7e-6.
 constexpr int DT_R = 12;               // box radius (core/libraw_wrapper.cpp:1424)
 constexpr int DT_X = 128;              // output columns per strip
 constexpr int DT_C = DT_X + 2 * DT_R;  // columns whose vertical sums a strip holds
@@ -98,6 +99,9 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_box(const float* rgb, const f
       s1 += PASS == 0 ? q0[k] * q0[k] : q1[k];
     }
   }
+  // 1 / (samples of a window) for the lane's four columns, formed anew where the
+  // number of rows changes
+  float inv[4], held = 0.f;
   float n0[DT_STEP], n1[DT_STEP];  // the next step's entering samples
 #pragma unroll
   for (int k = 0; k < DT_STEP; k++) fetch(y0 + DT_R + k, n0[k], n1[k]);
@@ -153,13 +157,17 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_box(const float* rgb, const f
       }
       const float cy = (float)(min(H - 1, oy + DT_R) - max(0, oy - DT_R) + 1);
       const int x = x0 + 4 * lane;
+      if (cy != held) {
+        held = cy;
+#pragma unroll
+        for (int k = 0; k < 4; k++) inv[k] = 1.0f / (cy * (float)(min(W - 1, x + k + DT_R) - max(0, x + k - DT_R) + 1));
+      }
       float o0[4], o1[4];
       if (PASS == 0) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          const float cnt = cy * (float)(min(W - 1, x + k + DT_R) - max(0, x + k - DT_R) + 1);
           // m0 = mean(guide), m1 = mean(guide^2)  (core/libraw_wrapper.cpp:1431-1436)
-          const float m0 = h0[k] / cnt, m1 = h1[k] / cnt;
+          const float m0 = h0[k] * inv[k], m1 = h1[k] * inv[k];
           const float var = smax(0.0f, m1 - m0 * m0);
           o0[k] = var / (var + eps);
           o1[k] = m0 * (1.0f - o0[k]);
@@ -189,12 +197,11 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_box(const float* rgb, const f
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-          const float cnt = cy * (float)(min(W - 1, x + k + DT_R) - max(0, x + k - DT_R) + 1);
           // m0 = mean(a), m1 = mean(b)  (core/libraw_wrapper.cpp:1442-1465)
-          const float m0 = h0[k] / cnt, m1 = h1[k] / cnt;
+          const float m0 = h0[k] * inv[k], m1 = h1[k] * inv[k];
           const float guide = dt_guide(c + 3 * k);
           const float base = smax(1e-6f, m0 * guide + m1);
-          float w = (base - edge0) / (edge1 - edge0);
+          float w = (base - edge0) * (1.0f / (edge1 - edge0));
           w = sclamp(w, 0.0f, 1.0f);
           w = w * w * (3.0f - 2.0f * w);
           if (w > 0.0f) {
