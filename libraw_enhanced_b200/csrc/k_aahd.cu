@@ -111,6 +111,30 @@ __global__ void k_aahd_stats_init(const float* __restrict__ raw, int cs, Aahd A)
   *A.hot = 0;
 }
 
+// Zeros in the margins of the sample plane and the six direction planes.  The
+// stages read up to two cells beyond the image; inside, every cell is written
+// before it is read (k_aahd_init the samples, in X and in their own channel,
+// k_aahd_greens the other greens, k_aahd_rb_hv and k_aahd_rb_last the rest).
+// 12 MP: 73 us for clearing the eight planes whole, 20 us for the margins and
+// the direction map.
+__global__ void __launch_bounds__(256) k_aahd_margins(float* base, size_t plane, int W, int H, int NW) {
+  float* p = base + blockIdx.y * plane;
+  const int rows = 2 * kMargin * NW, n = rows + 2 * kMargin * H;
+  for (int k = blockIdx.x * 256 + threadIdx.x; k < n; k += gridDim.x * 256) {
+    int i, j;
+    if (k < rows) {
+      i = k / NW;
+      j = k - i * NW;
+      if (i >= kMargin) i += H;
+    } else {
+      i = kMargin + (k - rows) / (2 * kMargin);
+      j = (k - rows) % (2 * kMargin);
+      if (j >= kMargin) j += W;
+    }
+    p[(size_t)i * NW + j] = 0.f;
+  }
+}
+
 // Constructor copy (:276-306): non-zero samples go to both direction images
 // and to the per-colour max/min (min starts from pixel 0's three channels).
 // Each thread keeps the extremes of its own samples, and a block settles them
@@ -123,12 +147,12 @@ __global__ void __launch_bounds__(256) k_aahd_init(const float* __restrict__ raw
   AAHD_FOR_PIXELS(A) {
     const unsigned c = A.fc(i, j);
     const size_t k = (size_t)i * A.W + j;
-    const float d = cs == 1 ? raw[k] : raw[k * 3 + c];
+    const float v = cs == 1 ? raw[k] : raw[k * 3 + c], d = v != 0 ? v : 0.f;
+    const size_t p = A.pi(i, j);
+    A.X[p] = d;
+    A.pl(0, c)[p] = d;
+    A.pl(1, c)[p] = d;
     if (d != 0) {
-      const size_t p = A.pi(i, j);
-      A.X[p] = d;
-      A.pl(0, c)[p] = d;
-      A.pl(1, c)[p] = d;
 #pragma unroll
       for (unsigned q = 0; q < 3; q++)
         if (c == q) {
@@ -486,7 +510,11 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
   A.stats = stats;
   A.hot = reinterpret_cast<int*>(stats + 8);
   cudaStream_t s = c->stream;
-  LRE_CUDA_TRY(c, cudaMemsetAsync(base, 0, 8 * pb, s));
+  // the direction map (plane 7) whole: hide_hots passes through it
+  LRE_CUDA_TRY(c, cudaMemsetAsync(base + 7 * pb, 0, pb, s));
+  const unsigned margin_blocks = (unsigned)std::min<size_t>((2 * kMargin * (A.NW + h) + 255) / 256, 64);
+  k_aahd_margins<<<dim3(margin_blocks, 7), 256, 0, s>>>(plane(0), pb / sizeof(float), A.W, A.H, A.NW);
+  count_launch(c);
   int* err = d_err ? d_err : sync + 1;
   if (!d_err) LRE_CUDA_TRY(c, cudaMemsetAsync(err, 0, sizeof(int), s));
   k_aahd_stats_init<<<1, 32, 0, s>>>(raw, raw_c_stride, A);
