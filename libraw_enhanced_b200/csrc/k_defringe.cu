@@ -279,10 +279,10 @@ __device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsig
 // Separable blur of one plane for a compile-time tap radius KS, on strips of
 // 128 columns.  A thread owns two columns and walks down the strip in batches
 // of P = 2 KS + 1 rows:
-//   1. the next batch's rows are on their way to shared memory (cp.async)
-//      while this one is summed;
-//   2. the horizontal sums of the thread's two columns, packed, go to shared
+//   1. the horizontal sums of the thread's two columns, packed, go to shared
 //      memory of the thread's own;
+//   2. the next batch's rows are on their way to shared memory (cp.async)
+//      over this one's;
 //   3. the vertical sums: P accumulators in registers, one per output row in
 //      flight.  A new row is multiplied once by each of the KS + 1 distinct
 //      weights (the kernel is symmetric) and the products are added to the
@@ -293,8 +293,12 @@ __device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsig
 // long as a scalar one, so it is the operations per output that count:
 // 4 KS + 2 horizontally and 3 KS + 2 vertically (74 at KS = 10) against 97 in
 // 64 x 64 tiles, whose halo the horizontal pass ran too.  One plane of 51 MP
-// takes 217 us (tiles: 263 us); the pipe's time is 102 us, and register moves that
+// takes 206 us (tiles: 263 us); the pipe's time is 102 us, and register moves that
 // line up the odd taps' pairs, chunk overlap and dependent adds take the rest.
+// One staged batch, seven CTAs per SM: with a second one, on its way from the
+// horizontal sums on, six fit, and the blurs of 51 MP took 1730 us, not 1647, of
+// 26 MP at radius 7 790 us, not 733.  (Eight CTAs 1650 and 740 us, nine, which
+// spill, 1607 and 764 us; 24 MP 790, 780 and 818 us.)
 constexpr int BS_X = 128;  // output columns per strip
 constexpr int BS_THREADS = BS_X / 2;
 
@@ -303,8 +307,8 @@ struct BlurStrip {
   static constexpr int P = 2 * KS + 1;              // accumulators, rows per batch
   static constexpr int PAD = (KS + 3) & ~3;         // staged columns left and right of the strip
   static constexpr int C = BS_X + 2 * PAD;
-  static constexpr int IN = (P + 1) * C;            // floats of one staged batch (one row more is read)
-  static constexpr size_t SMEM = (size_t)(2 * IN + (P + 1) * BS_X) * sizeof(float);
+  static constexpr int IN = (P + 1) * C;            // floats of the staged batch (one row more is read)
+  static constexpr size_t SMEM = (size_t)(IN + (P + 1) * BS_X) * sizeof(float);
 };
 
 __device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes) {
@@ -316,12 +320,12 @@ __device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes
 }
 
 template <int KS>
-__global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, GaussTaps taps, int W, int H, int batches,
+__global__ void __launch_bounds__(BS_THREADS, 7) k_df_blur_strip(BlurJob job, GaussTaps taps, int W, int H, int batches,
                                                               const DfScalars* sc) {
   using B = BlurStrip<KS>;
   constexpr int P = B::P, C = B::C, PAD = B::PAD;
   extern __shared__ __align__(16) float sm_strip[];
-  float* s_h = sm_strip + 2 * B::IN;  // [P + 1 rows][BS_X]
+  float* s_h = sm_strip + B::IN;  // [P + 1 rows][BS_X]
   const int tid = threadIdx.x;
   const float* __restrict__ in = pick5(job.in, blockIdx.z);
   float* __restrict__ out = pick5(job.out, blockIdx.z);
@@ -339,7 +343,7 @@ __global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, Ga
   // halo lies inside the image; else sample by sample with the column clamped
   const bool wide = step == 1 && (W & 3) == 0 && x0 >= PAD && x0 + BS_X + PAD <= W;
   auto stage = [&](int b) {
-    float* dst = sm_strip + (b & 1) * B::IN;
+    float* dst = sm_strip;
     const int yb = y0 - KS + b * P;
     if (wide) {
       for (int i = tid; i < P * (C / 4); i += BS_THREADS) {
@@ -368,13 +372,8 @@ __global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, Ga
   for (int b = 0; b < batches; b++) {
     const int yb = y0 - KS + b * P;  // image row of the batch's first row
     if (yb - KS >= y1) break;
-    float* cur = sm_strip + (b & 1) * B::IN;
-    if (b + 1 < batches) {
-      stage(b + 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+    float* cur = sm_strip;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     if (mode != BS_PLANE) {
       for (int i = tid; i < P * C; i += BS_THREADS) cur[i] = mode == BS_GUIDE_LINEAR ? smax(cur[i], 0.f) : cur[i] * inv;
@@ -408,6 +407,8 @@ __global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, Ga
       for (int k = 0; k < 2; k++)
         *reinterpret_cast<unsigned long long*>(&s_h[(j + k) * BS_X + 2 * tid]) = h[k];
     }
+    __syncthreads();  // every thread has read the batch
+    if (b + 1 < batches) stage(b + 1);
     // vertical sums (the thread reads only what it wrote)
 #pragma unroll
     for (int s = 0; s < P; s++) {
@@ -436,7 +437,6 @@ __global__ void __launch_bounds__(BS_THREADS, 6) k_df_blur_strip(BlurJob job, Ga
         }
       }
     }
-    __syncthreads();  // every thread has read the batch before the next but one is staged over it
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -446,18 +446,19 @@ lre_status run_blur_strip(Context* c, const BlurJob& job, const GaussTaps& taps,
   using B = BlurStrip<KS>;
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_strip<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::SMEM));
   // Batches per chunk: a chunk's first 2 KS rows produce nothing, so tall
-  // chunks, halved while the grid has fewer than twelve CTAs per SM.  Where
-  // even halves leave fewer than that (six are resident, so at most two waves),
+  // chunks, halved while the grid has fewer than fourteen CTAs per SM.  Where
+  // even halves leave fewer than that (seven are resident, so at most two waves),
   // what takes the fewest batch steps over all waves, a nearly empty last one
-  // counting as much as a full one: the three blurs of 1.9 MP took 104 us
-  // halved and 88 us so; of 24 and 51 MP 839 and 1732 us halved and 859 and
-  // 1774 us by waves, whose CTAs don't run in step when there are many.
+  // counting as much as a full one.  With six CTAs per SM the three blurs of
+  // 1.9 MP took 104 us halved and 88 us so (82 us with seven); those of 24 and
+  // 51 MP 839 and 1732 us halved and 859 and 1774 us by waves, whose CTAs don't
+  // run in step when there are many.
   int batches = c->tune.blur_tile == 64 ? 32 : 16;
   const int tallest = batches;
   const int strips = (W + BS_X - 1) / BS_X;
   auto chunks = [&](int n) { return (H + n * B::P - 2 * KS - 1) / (n * B::P - 2 * KS); };
   auto ctas = [&](int n) { return (long long)strips * chunks(n) * job.np; };
-  const long long places = 6LL * c->sm_count;
+  const long long places = 7LL * c->sm_count;
   while (batches > 2 && ctas(batches) < 2 * places) batches /= 2;
   if (batches <= 4) {
     double least = 1e300;
@@ -1295,7 +1296,7 @@ __global__ void __launch_bounds__(256) k_df_maxg(const float* __restrict__ src, 
 
 // Tap radii 3 to 15 run the strip kernel compiled for them, others the tile
 // kernel with the radius at run time (all eight planes of 26 MP at radius 7:
-// 2575 us in tiles, 792 us in strips).
+// 2575 us in tiles, 733 us in strips).
 template <int KS>
 lre_status blur_for(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc, bool* done) {
   if constexpr (KS >= 3) {
