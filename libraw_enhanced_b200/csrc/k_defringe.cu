@@ -56,20 +56,14 @@ struct DfPlanes {
 __device__ __forceinline__ float df_max_guide(const DfScalars* s) { return smax(s->max_guide_raw, 1e-6f); }
 
 // ---------------------------------------------------------------- K1
-__device__ __forceinline__ float guide_signal_at(const float* __restrict__ src, int x, int y, int W, float max_guide) {
-  float g = src[((size_t)y * W + x) * 3 + 1];
-  float gg = smax(g, 0.f);
-  return sqrtf(sclamp(gg / max_guide, 0.f, 1.f));
-}
-
 // K1: log ratios and Sobel magnitude of the guide signal.  A warp walks up to
-// PW_ROWS rows of 30 columns (and one beside them on either side): the guide signal, a
-// square root and a divide, is formed once per pixel, its neighbours come from
-// the lanes beside and the two rows before, and the next two rows are on their
-// way meanwhile.  Bound by instructions: two logarithms in double, two divides
-// and the guide.  51 MP 438 us, 26 MP odd 234 us, 1.9 MP
-// 20 us; on 32 x 8 tiles with the guide in shared memory, a barrier before and after,
-// 783, 402 and 24 us, and with CUDA's log in double besides 856, 441 and 27 us.
+// PW_ROWS rows of 30 columns (and one beside them on either side): the guide
+// signal, a square root and a divide, is formed once per pixel, its neighbours
+// come from the lanes beside and the two rows before, and the next two rows are
+// on their way meanwhile.  Bound by instructions: two logarithms in double, two
+// divides and the guide.  51 MP 438 us, 26 MP odd 234 us, 1.9 MP 20 us; on 32 x 8
+// tiles with the guide in shared memory, a barrier before and after, 783, 402 and
+// 24 us, and with CUDA's log in double besides 856, 441 and 27 us.
 constexpr int PW_ROWS = 32, PW_COLS = 30;
 
 __global__ void __launch_bounds__(256) k_df_prep(const float* __restrict__ src, int W, int H, int rows, DfScalars* sc,
@@ -695,8 +689,8 @@ __device__ __forceinline__ void line_runs(const float* s_ls, const float* s_fs, 
 // (256 threads 926 us at 51 MP; two rows in flight 853 us; five CTAs per SM, which
 // spill, 769 us.)
 template <bool FAST>
-__global__ void __launch_bounds__(LN_THREADS, 4) k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfConst k,
-                                                 DfTab T, const DfScalars* sc) {
+__global__ void __launch_bounds__(LN_THREADS, 4)
+    k_df_line(const float* __restrict__ src, int W, int H, DfPlanes P, DfConst k, DfTab T, const DfScalars* sc) {
   __shared__ __align__(16) float s_src[LPAD + LE * LE + LPAD];
   __shared__ float s_fs[LE * LE];
   __shared__ __align__(16) float s_best[LT * LT];

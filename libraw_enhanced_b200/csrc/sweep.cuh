@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
 // leaves most SMs waiting; a sweep of 24 MP took 1.9 to 2.8 ms (44 ms for the
 // LoCA lift) whatever its arithmetic.  Blocks at 24 MP: nyquist 1930 -> 252 us,
 // pp 2810 -> 324, refinement 2360 -> 186, color_full 2800 -> 378, LoCA 44470
-// -> 1420 (with its terms as state); direction refinement at 12 MP 2210 ->
+// -> 1270 (with its terms as state, three blocks of four warps per SM); direction refinement at 12 MP 2210 ->
 // 104, hot pixels 2000 -> 205.  Staging through registers and keeping the
 // inputs in one group's buffer (two blocks per SM instead of one) was worth
 // 1.9x; 4-byte cp.async into a full ring of every plane had given 620 us for
