@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     const int ccmin = (left < 0) ? 16 : 0;
     const int rrmax = (bottom > H) ? H - top : rr1;
     const int ccmax = (right > W) ? W - left : cc1;
-    const FDiv fdc(cc1), fd8(cc1 - 8), fd32(cc1 - 32);
+    const FDiv fdc(cc1), fd8(cc1 - 8);
 
     // ---- zero what this tile reads before writing (fresh-buffer semantics)
     // the 4-px frame of the stage-2 planes: eight rows, then eight columns
@@ -377,6 +377,27 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     // the next row when ccmax + 16 exceeds the tile width, as the reference's
     // flat buffer does
     const float scale = A.scale;
+    if (CL == 1 && rrmin == 0 && ccmin == 0 && rrmax == TS && ccmax == TS) {
+      // a whole tile inside the image: a warp's rows, all samples in flight
+      // (20,000 cycles of a tile's 457,000 with a sample at a time)
+      const int lane = tid & 31, gw = gt >> 5;
+      constexpr int NW = AMZ_THREADS / 32, NR = (TS + NW - 1) / NW;
+      float v[NR][TS / 32];
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+#pragma unroll
+        for (int k = 0; k < TS / 32; k++) {
+          const int rr = gw + j * NW;
+          v[j][k] = rr < TS ? raw_at(A, rr + top, 32 * k + lane + left) : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < NR; j++)
+#pragma unroll
+        for (int k = 0; k < TS / 32; k++) {
+          const int rr = gw + j * NW;
+          if (rr < TS) put(&cfa[rr * TS + 32 * k + lane], v[j][k] * scale);
+        }
+    } else {
     for (int i = gt; i < rr1 * cc1; i += gn) {
       const int rr = fdc.div(i), cc = i - rr * cc1;
       int srow = -1, scol = -1;
@@ -397,6 +418,7 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
         scol = min(max(W - (cc - ccmax) - 2, 0), W - 1);
       }
       if (srow >= 0) put(&cfa[rr * TS + cc], raw_at(A, srow, scol) * scale);
+    }
     }
     if (ccmax < cc1 && ccmax + 16 > TS) {
       bar();
@@ -979,38 +1001,70 @@ __global__ void __launch_bounds__(AMZ_THREADS, 1) k_amaze(AmazeArgs A) {
     bar();
 
     // ---- S10 output (:1594-1625)
-    for (int i = gt; i < (rr1 - 32) * (cc1 - 32); i += gn) {
-      const int q_ = fd32.div(i), rr = 16 + q_, cc = 16 + i - q_ * (cc1 - 32);
-      const int row = rr + top, col = cc + left;
-      if (row < 0 || row >= H || col < 0 || col >= W) continue;
-      const int t = rr * TS + cc;
-      float r, g, b;
+    // One CTA per tile: a thread takes two neighbours, one green and one not, as a
+    // warp over single pixels runs both branches for each of them.  Clusters have
+    // threads to spare and keep single pixels (511 x 341: 108 us, 110 in pairs).
+    // 51 MP: 5000 us with single pixels and the fill in turn, 4952 in pairs, 4770
+    // with the whole fill in flight besides.
+    {
       const float* D0 = S.Dgrb0;
       const float* D1 = S.Dgrb1;
-      if (fc_rt(A, row, col) == 1) {
-        g = cfa[t];
-        const float wsum_inv =
-            1.0f / (hvwt[(t - v1) >> 1] + 2.f - hvwt[(t + 1) >> 1] - hvwt[(t - 1) >> 1] + hvwt[(t + v1) >> 1]);
-        const float r_diff = (hvwt[(t - v1) >> 1] * D0[(t - v1) >> 1] + (1.f - hvwt[(t + 1) >> 1]) * D0[(t + 1) >> 1] +
-                              (1.f - hvwt[(t - 1) >> 1]) * D0[(t - 1) >> 1] + hvwt[(t + v1) >> 1] * D0[(t + v1) >> 1]) *
+      struct Rgb {
+        float r, g, b;
+      };
+      auto green_px = [&](int t) {
+        const float g = cfa[t];
+        const float hn = hvwt[(t - v1) >> 1], hs = hvwt[(t + v1) >> 1], he = hvwt[(t + 1) >> 1], hw = hvwt[(t - 1) >> 1];
+        const float wsum_inv = 1.0f / (hn + 2.f - he - hw + hs);
+        const float r_diff = (hn * D0[(t - v1) >> 1] + (1.f - he) * D0[(t + 1) >> 1] + (1.f - hw) * D0[(t - 1) >> 1] +
+                              hs * D0[(t + v1) >> 1]) *
                              wsum_inv;
-        const float b_diff = (hvwt[(t - v1) >> 1] * D1[(t - v1) >> 1] + (1.f - hvwt[(t + 1) >> 1]) * D1[(t + 1) >> 1] +
-                              (1.f - hvwt[(t - 1) >> 1]) * D1[(t - 1) >> 1] + hvwt[(t + v1) >> 1] * D1[(t + v1) >> 1]) *
+        const float b_diff = (hn * D1[(t - v1) >> 1] + (1.f - he) * D1[(t + 1) >> 1] + (1.f - hw) * D1[(t - 1) >> 1] +
+                              hs * D1[(t + v1) >> 1]) *
                              wsum_inv;
-        r = g - r_diff;
-        b = g - b_diff;
-      } else {
-        g = S.rgbg[t >> 1];
-        r = g - D0[t >> 1];
-        b = g - D1[t >> 1];
-      }
+        return Rgb{g - r_diff, g, g - b_diff};
+      };
+      auto other_px = [&](int t) {
+        const float g = S.rgbg[t >> 1];
+        return Rgb{g - D0[t >> 1], g, g - D1[t >> 1]};
+      };
       // streaming stores: the output is not re-read by this kernel, so it
       // should not evict the slab planes from L2
-      float* o = A.rgb + ((size_t)row * W + col) * 3;
-      __stcs(o + 0, fmaxf(0.f, r));
-      __stcs(o + 1, fmaxf(0.f, g));
-      __stcs(o + 2, fmaxf(0.f, b));
-      if (row >= 4 && row < H - 4 && col >= 4 && col < W - 4) mg = fmaxf(mg, fmaxf(0.f, g));
+      auto store = [&](int row, int col, const Rgb& v) {
+        float* o = A.rgb + ((size_t)row * W + col) * 3;
+        __stcs(o + 0, fmaxf(0.f, v.r));
+        __stcs(o + 1, fmaxf(0.f, v.g));
+        __stcs(o + 2, fmaxf(0.f, v.b));
+        if (row >= 4 && row < H - 4 && col >= 4 && col < W - 4) mg = fmaxf(mg, fmaxf(0.f, v.g));
+      };
+      if (CL == 1) {
+        const int pairs = (cc1 - 31) / 2;
+        const FDiv fdp(pairs);
+        for (int i = gt; i < (rr1 - 32) * pairs; i += gn) {
+          const int q_ = fdp.div(i), rr = 16 + q_, cc = 16 + 2 * (i - q_ * pairs);
+          const int row = rr + top, col = cc + left;
+          if (row < 0 || row >= H || col < 0 || col >= W) continue;
+          const int t = rr * TS + cc;
+          const bool two = cc + 1 < cc1 - 16 && col + 1 < W;
+          const bool first = fc_rt(A, row, col) == 1;
+          if (first != (fc_rt(A, row, col + 1) == 1)) {
+            const Rgb g = green_px(first ? t : t + 1), o = other_px(first ? t + 1 : t);
+            if (first || two) store(row, first ? col : col + 1, g);
+            if (!first || two) store(row, first ? col + 1 : col, o);
+          } else {
+            for (int k = 0; k < (two ? 2 : 1); k++) store(row, col + k, first ? green_px(t + k) : other_px(t + k));
+          }
+        }
+      } else {
+        const FDiv fd32(cc1 - 32);
+        for (int i = gt; i < (rr1 - 32) * (cc1 - 32); i += gn) {
+          const int q_ = fd32.div(i), rr = 16 + q_, cc = 16 + i - q_ * (cc1 - 32);
+          const int row = rr + top, col = cc + left;
+          if (row < 0 || row >= H || col < 0 || col >= W) continue;
+          const int t = rr * TS + cc;
+          store(row, col, fc_rt(A, row, col) == 1 ? green_px(t) : other_px(t));
+        }
+      }
     }
     bar();
     tile = next_tile;
