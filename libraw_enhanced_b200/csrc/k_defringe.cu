@@ -196,50 +196,43 @@ __device__ __forceinline__ float blur_src(const float* in, int mode, const DfSca
   }
 }
 
-// One CTA = BT x BT outputs of every plane in the job; the clamped input halo
-// and the horizontal-pass rows live in shared memory.
+// One CTA = BT x BT outputs of one plane of the job (blockIdx.z); the clamped
+// input halo and the horizontal-pass rows live in shared memory, 48 KB at the
+// largest tap radius.  (With the job's five planes in one CTA it was 222 KB at
+// tap radius 30 and more than a CTA may have at 31 and 32.)
 __global__ void __launch_bounds__(256) k_df_blur(BlurJob job, GaussTaps taps, int W, int H, const DfScalars* sc) {
   extern __shared__ __align__(16) float sm[];
   const int ks = taps.ks;
   const int E = BT + 2 * ks;  // halo tile edge
   const int x0 = blockIdx.x * BT, y0 = blockIdx.y * BT;
-  float* s_in = sm;                       // [np][E][E]
-  float* s_h = sm + (size_t)job.np * E * E;  // [np][E][BT]
-  for (int p = 0; p < job.np; p++) {
-    const float* in = pick5(job.in, p);
-    const int mode = pick5(job.mode, p);
-    for (int i = threadIdx.x; i < E * E; i += blockDim.x) {
-      int gy = min(max(y0 - ks + i / E, 0), H - 1);
-      int gx = min(max(x0 - ks + i % E, 0), W - 1);
-      s_in[(size_t)p * E * E + i] = blur_src(in, mode, sc, gx, gy, W);
-    }
+  float* s_in = sm;         // [E][E]
+  float* s_h = sm + E * E;  // [E][BT]
+  const float* in = pick5(job.in, blockIdx.z);
+  const int mode = pick5(job.mode, blockIdx.z);
+  for (int i = threadIdx.x; i < E * E; i += blockDim.x) {
+    int gy = min(max(y0 - ks + i / E, 0), H - 1);
+    int gx = min(max(x0 - ks + i % E, 0), W - 1);
+    s_in[i] = blur_src(in, mode, sc, gx, gy, W);
   }
   __syncthreads();
   // horizontal pass over all E halo rows (rows are the clamped image rows)
-  for (int p = 0; p < job.np; p++) {
-    const float* si = s_in + (size_t)p * E * E;
-    float* sh = s_h + (size_t)p * E * BT;
-    for (int i = threadIdx.x; i < E * BT; i += blockDim.x) {
-      int j = i / BT, k = i % BT;
-      const float* row = si + j * E + k;
-      float acc = 0.f;
-      for (int t = 0; t <= 2 * ks; t++) acc += taps.w[t] * row[t];
-      sh[i] = acc;
-    }
+  for (int i = threadIdx.x; i < E * BT; i += blockDim.x) {
+    int j = i / BT, k = i % BT;
+    const float* row = s_in + j * E + k;
+    float acc = 0.f;
+    for (int t = 0; t <= 2 * ks; t++) acc += taps.w[t] * row[t];
+    s_h[i] = acc;
   }
   __syncthreads();
   // vertical pass
-  for (int p = 0; p < job.np; p++) {
-    const float* sh = s_h + (size_t)p * E * BT;
-    float* out = pick5(job.out, p);
-    for (int i = threadIdx.x; i < BT * BT; i += blockDim.x) {
-      int j = i / BT, k = i % BT;
-      int gy = y0 + j, gx = x0 + k;
-      if (gx >= W || gy >= H) continue;
-      float acc = 0.f;
-      for (int t = 0; t <= 2 * ks; t++) acc += taps.w[t] * sh[(j + t) * BT + k];
-      out[(size_t)gy * W + gx] = acc;
-    }
+  float* out = pick5(job.out, blockIdx.z);
+  for (int i = threadIdx.x; i < BT * BT; i += blockDim.x) {
+    int j = i / BT, k = i % BT;
+    int gy = y0 + j, gx = x0 + k;
+    if (gx >= W || gy >= H) continue;
+    float acc = 0.f;
+    for (int t = 0; t <= 2 * ks; t++) acc += taps.w[t] * s_h[(j + t) * BT + k];
+    out[(size_t)gy * W + gx] = acc;
   }
 }
 
@@ -1308,9 +1301,9 @@ lre_status run_blur(Context* c, const BlurJob& job, const GaussTaps& taps, int W
   LRE_TRY(blur_for<15>(c, job, taps, W, H, sc, &done));
   if (done) return LRE_OK;
   const int E = BT + 2 * taps.ks;
-  size_t smem = ((size_t)job.np * E * E + (size_t)job.np * E * BT) * sizeof(float);
+  const size_t smem = ((size_t)E * E + (size_t)E * BT) * sizeof(float);
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((W + BT - 1) / BT, (H + BT - 1) / BT);
+  const dim3 grid((W + BT - 1) / BT, (H + BT - 1) / BT, job.np);
   k_df_blur<<<grid, 256, smem, c->stream>>>(job, taps, W, H, sc);
   count_launch(c);
   return check_launch(c, "defringe blur");
