@@ -229,9 +229,10 @@ __global__ void __launch_bounds__(DT_THREADS) k_dt_box(const float* rgb, const f
 
 // The same tone map with the reference's own running sums, one thread per
 // row, then per column, in its scan order: last bit for last bit the
-// reference's floats.  It serves the develops where a difference in the last
-// bits could become a visible one: 16-bit codes, and defringe or lateral CA
-// after the tone map, which decide by thresholds.
+// reference's floats.  It serves the develops, where a difference in the last
+// bits could become a visible one (16-bit codes, and the thresholds of defringe
+// and lateral CA after the tone map) and where 16 bits are to be the quantised
+// 32 of the same chain; 18.97 ms at 8256x5504 against 0.63 of the strips.
 // Horizontal running box sums of two planes at once.  mode 0: the planes are
 // derived from RGB (guide = max(0, maxRGB), guide^2); mode 1: plain planes.
 __global__ void k_box_rows2(const float* __restrict__ rgb, const float* __restrict__ p0, const float* __restrict__ p1,

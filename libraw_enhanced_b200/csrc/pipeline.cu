@@ -173,10 +173,10 @@ lre_status run_chain(Context* c, const float* d_mosaic, float* rgb_a, float* rgb
     if (p.tone_mapping) cur_max_g = nullptr;
     if (p.tone_mapping == 1) LRE_TRY(lre::launch_tone_mapping(c, cur, cur, w * h, p.tone_after_scale));
     if (p.tone_mapping == 2) {
-      // 16-bit codes and the threshold decisions of lateral CA and defringe
-      // keep the reference's last bits
-      const bool decides_later = p.stage_order != 1 && (p.defringe || p.lateral_ca_correction);
-      LRE_TRY(lre::launch_detail_tonemap(c, cur, cur, w, h, p.output_bits == 16 || decides_later));
+      // In the reference's order in every develop: its last bits decide 16-bit
+      // codes and the thresholds of lateral CA and defringe, and a 16-bit
+      // develop is the quantised 32-bit one, stage for stage.
+      LRE_TRY(lre::launch_detail_tonemap(c, cur, cur, w, h, true));
       c->ws.rewind(mark);
     }
     return LRE_OK;
