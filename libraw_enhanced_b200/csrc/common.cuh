@@ -97,11 +97,15 @@ __device__ __forceinline__ float pow_cr(float x, float y) { return (float)pow((d
 // log x = e log 2 + log c + log1p(m / c - 1).  The two intervals at 1 have c = 1,
 // so a small logarithm keeps its relative accuracy.  The series ends at r^7: its
 // error is below 2.3e-16 of the result for |r| < 2^-7.  In double throughout, and
-// rounded to float once, as log_cr: of all 2.1e9 positive normal floats one has
-// another result than log_cr, by one ulp.  About half its instructions (K1 of
-// defringe 856 us with log_cr, 783 us with this one at 51 MP); the table, two
+// rounded to float once, as log_cr.  The two doubles are at most five units in the
+// last place apart, so they round alike unless the middle of two floats lies that
+// near (LOG_TAB_NEAR is three times as far): there log_cr decides, and all 2.1e9
+// positive normal floats have log_cr's result (without that one of them was an ulp
+// off; K1 of defringe 438 us at 51 MP, 449 with it).  About half its instructions (K1 of
+// defringe, in tiles, 856 us with log_cr, 783 us with this one); the table, two
 // doubles an interval, is formed by each block with CUDA's log.
 constexpr int LOG_TAB_N = 128;
+constexpr unsigned LOG_TAB_NEAR = 16;
 __device__ __forceinline__ void log_tab_fill(double2* tab) {
   for (int j = threadIdx.x; j < LOG_TAB_N; j += blockDim.x) {
     const double a = __int_as_float(0x3f330000 + (j << 16)), b = __int_as_float(0x3f330000 + ((j + 1) << 16));
@@ -110,7 +114,6 @@ __device__ __forceinline__ void log_tab_fill(double2* tab) {
   }
 }
 __device__ __forceinline__ float log_tab(const double2* tab, float x) {
-  if (!(x >= 1.17549435e-38f && x <= 3.4028235e38f)) return log_cr(x);  // zero, subnormal, infinite, NaN
   const int bits = __float_as_int(x), t = bits - 0x3f330000;
   const double2 c = tab[t >> 16 & (LOG_TAB_N - 1)];
   const double r = fma((double)__int_as_float(bits - (t & 0xff800000)), c.x, -1.0);
@@ -119,7 +122,12 @@ __device__ __forceinline__ float log_tab(const double2* tab, float x) {
   q = fma(r, q, -1.0 / 4.0);
   q = fma(r, q, 1.0 / 3.0);
   q = fma(r, q, -1.0 / 2.0);
-  return (float)(fma((double)(t >> 23), 0.693147180559945309417, c.y) + fma(r * r, q, r));
+  const double d = fma((double)(t >> 23), 0.693147180559945309417, c.y) + fma(r * r, q, r);
+  // the 29 bits that the rounding to float drops, at the top of a word: how far
+  // from the middle of two floats
+  const unsigned off = 8u * (unsigned)__double2loint(d) + (0x80000000u + 8u * LOG_TAB_NEAR);
+  const bool normal = (unsigned)bits - 0x00800000u < 0x7f000000u;  // not zero, subnormal, negative, infinite or NaN
+  return normal && off > 16u * LOG_TAB_NEAR ? (float)d : log_cr(x);
 }
 
 }  // namespace lre
