@@ -84,6 +84,10 @@ struct Context {
   cudaEvent_t tail_ev[8] = {};  // rows of the final RGB ready for download
   std::mutex mu;               // one host-buffer call at a time per context
   int sm_count = 148;
+  // Contexts that work on the GPU at the same time, this one included, as far
+  // as their owner knows (the lanes of a batch or a server; else 1).  Bits do
+  // not depend on it: it weighs one image's latency against the lanes' work.
+  int sharers = 1;
   // Bound of each device-side wait of the in-order sweeps, in SM clock
   // cycles (0: the default, ~2 s), and a one-shot host-side fault injection:
   // the next sweep's band `sweep_hold_band` never reports its progress.

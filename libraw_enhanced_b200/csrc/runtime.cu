@@ -223,7 +223,12 @@ std::vector<unsigned char> batch_signature(const Batch* b, const lre_image* im, 
 lre_status enqueue_all(Batch* b, const lre_image* im, const std::vector<std::vector<size_t>>& plan, bool host_mode,
                        uint64_t* launches) {
   uint64_t before = 0;
-  for (auto& l : b->L) before += l.c->launches.load();
+  int busy = 0;
+  for (auto& p : plan) busy += !p.empty();
+  for (auto& l : b->L) {
+    before += l.c->launches.load();
+    l.c->sharers = std::max(1, busy);
+  }
   // round-robin over lanes so every stream receives work early
   size_t maxlen = 0;
   for (auto& p : plan) maxlen = std::max(maxlen, p.size());
@@ -597,6 +602,9 @@ void scheduler(Server* s) {
       r->lane = li;
       s->running[li] = r;
       admitted = true;
+      // lanes at work once the queue has been admitted as far as it goes
+      const size_t running = s->L.size() - std::count(s->running.begin(), s->running.end(), nullptr);
+      l.c->sharers = (int)std::min(s->L.size(), running + s->queue.size());
       lk.unlock();
       lre_status st = lane_fit(l, r->img, true);
       if (st == LRE_OK) st = lane_enqueue(l, r->img, true);
