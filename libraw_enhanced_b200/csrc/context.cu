@@ -1,4 +1,6 @@
 // context.cu -- context, workspace arena, errors and pinned host memory.
+#include <algorithm>
+#include <chrono>
 #include <cstdio>
 #include <cstring>
 
@@ -67,6 +69,31 @@ lre_status check_injection(Context* c) {
   return LRE_OK;
 }
 
+// By the clock: whether a context's last demosaic still runs, only its stream or
+// an event could tell, and neither may be asked while another thread captures a
+// graph.  Half a millisecond is about the longest that a demosaic of fewer tiles
+// than SMs, the only ones whose form depends on this, runs beside others.  An
+// entry that two contexts share counts them as one.
+namespace {
+constexpr int kWorkDevices = 16, kWorkSlots = 64;
+constexpr long long kWorkNs = 500000;
+std::atomic<long long> g_asked[kWorkDevices][kWorkSlots];
+}  // namespace
+
+int contexts_at_work(Context* c) {
+  const long long now =
+      std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now().time_since_epoch()).count();
+  std::atomic<long long>* const row = g_asked[c->device % kWorkDevices];
+  const int own = c->id % kWorkSlots;
+  int n = 1;
+  for (int k = 0; k < kWorkSlots; k++) {
+    const long long t = row[k].load(std::memory_order_relaxed);
+    n += k != own && t != 0 && now - t < kWorkNs;
+  }
+  row[own].store(now, std::memory_order_relaxed);
+  return std::max(n, c->sharers);
+}
+
 lre_status ensure_buffer(Context* c, void** p, size_t* cap, size_t bytes) {
   if (bytes <= *cap && *p) return LRE_OK;
   if (*p) {
@@ -120,6 +147,8 @@ lre_status lre_create(int device, lre_ctx** out) {
   if (cudaSetDevice(device) != cudaSuccess) return LRE_ERR_CUDA;
   Context* c = new Context();
   c->device = device;
+  static std::atomic<int> created{0};
+  c->id = created.fetch_add(1);
   c->sm_count = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;

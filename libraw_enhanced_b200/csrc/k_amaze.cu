@@ -1182,13 +1182,13 @@ lre_status launch_amaze_rows(Context* c, AmazeArgs A, int row_lo, int row_hi) {
   // time takes 270 us with one CTA, 190 with two, 137 with four, 117 with
   // eight (511x341 to 1536x1024); clusters of four and eight lie inside a GPC,
   // which leaves 32 and 16 places.  Where other contexts work beside this one
-  // (a batch's lanes, a server's) their tiles take places too, as many each:
+  // (a batch's or server's lanes, other threads') their tiles take places too, as many each:
   // a cluster of eight is the fastest for a thumbnail by itself, and takes 3.4
   // times the SM time of one CTA.
   const int sms = c->sm_count;
   constexpr int cls[4] = {1, 2, 4, 8}, cost[4] = {100, 70, 51, 43};
   const int places[4] = {sms, sms / 2, sms * 32 / 148, sms * 16 / 148};
-  const long long in_flight = (long long)tiles * c->sharers;
+  const long long in_flight = (long long)tiles * contexts_at_work(c);
   int pick = 0;
   for (int j = 1; j < 4; j++) {
     auto rounds = [&](int q) { return (in_flight + places[q] - 1) / places[q] * cost[q]; };

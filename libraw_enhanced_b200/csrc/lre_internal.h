@@ -86,8 +86,9 @@ struct Context {
   int sm_count = 148;
   // Contexts that work on the GPU at the same time, this one included, as far
   // as their owner knows (the lanes of a batch or a server; else 1).  Bits do
-  // not depend on it: it weighs one image's latency against the lanes' work.
+  // not depend on it: it weighs one image's latency against the others' work.
   int sharers = 1;
+  int id = 0;  // contexts of the process in order of creation (contexts_at_work)
   // Bound of each device-side wait of the in-order sweeps, in SM clock
   // cycles (0: the default, ~2 s), and a one-shot host-side fault injection:
   // the next sweep's band `sweep_hold_band` never reports its progress.
@@ -110,6 +111,10 @@ lre_status fail(Context* c, lre_status st, const std::string& msg);
 lre_status cuda_fail(Context* c, cudaError_t e, const char* what);
 lre_status check_launch(Context* c, const char* what);
 lre_status check_injection(Context* c);
+// Contexts of this process that enqueue demosaics on this context's device at
+// about the same time, this one included: the owner's number, or those that
+// asked this within the last half millisecond (context.cu).
+int contexts_at_work(Context* c);
 
 #define LRE_CUDA_TRY(ctx, call)                                        \
   do {                                                                 \

@@ -2,6 +2,7 @@
 clusters of CTAs, so lanes must leave room for one another.  Eight lanes take
 well under the time of one (with every image in clusters of eight they took 0.80
 of it), and the bits do not depend on the number of lanes."""
+import threading
 import time
 
 import pytest
@@ -47,3 +48,36 @@ def test_bits_do_not_depend_on_the_lanes(h, w):
         outs = run(lanes, h, w)[1]
         first = first or outs
         assert all(torch.equal(x, y) for x, y in zip(first, outs))
+
+
+def test_threads_share_the_gpu():
+    """The same for threads that keep a context each."""
+    h, w, n = 341, 511, 100
+
+    def took(threads):
+        accs = [lre.CudaAccelerator(0) for _ in range(threads)]
+        mos = [torch.from_numpy(scenes.bayer_scene(h, w, 120)).cuda() for _ in accs]
+        outs = [torch.empty((h, w, 3), device="cuda") for _ in accs]
+        torch.cuda.synchronize()
+
+        def work(i, n):
+            for _ in range(n):
+                accs[i].dev_develop(mos[i], outs[i], w, h, P)
+            accs[i].synchronize()
+
+        best = 1e9
+        for n_dev in (10, n, n, n, n):
+            ts = [threading.Thread(target=work, args=(i, n_dev)) for i in range(threads)]
+            t0 = time.perf_counter()
+            for t in ts:
+                t.start()
+            for t in ts:
+                t.join()
+            best = min(best, (time.perf_counter() - t0) / (n_dev * threads))
+        assert all(torch.equal(o, outs[0]) for o in outs)
+        for a in accs:
+            a.close()
+        return best
+
+    one, eight = took(1), took(8)
+    assert eight < 0.6 * one, f"an image on one thread {one * 1e6:.0f} us, on eight {eight * 1e6:.0f} us"
