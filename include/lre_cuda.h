@@ -99,6 +99,11 @@ lre_status lre_set_wait_limit(lre_ctx* ctx, long long cycles);
  * progress -- a message that is dropped -- so the band below it waits until
  * its bound runs out.  One-shot; band < 0 clears it.  No device fault. */
 void lre_inject_sweep_stall(lre_ctx* ctx, int band);
+/* How often, since the context was made, a block of these passes disagreed
+ * with its neighbours, and how often a pass then ran in order (passes that a
+ * wait limit or a stall sent in order are not counted).  Waits for the
+ * context's stream.  Either pointer may be null. */
+lre_status lre_sweep_counts(lre_ctx* ctx, unsigned* blocks_repeated, unsigned* passes_in_order);
 
 /* ------------------------------------------------ stages, host buffers */
 /* GPUAccelerator::demosaic_bayer_amaze (core/gpu_accelerator.h:35-39;

@@ -165,6 +165,13 @@ class CudaAccelerator:
         """Fault injection: in the next in-order sweep, `band` never reports progress."""
         self._lib.lre_inject_sweep_stall(self._h, int(band))
 
+    def sweep_counts(self):
+        """Blocks of DCB, AAHD and highlight recovery that disagreed with their
+        neighbours since the context was made, and passes that then ran in order."""
+        n = (C.c_uint(), C.c_uint())
+        self._check(self._lib.lre_sweep_counts(self._h, C.byref(n[0]), C.byref(n[1])))
+        return n[0].value, n[1].value
+
     # ------------------------------------------------------------ stages (host)
     def demosaic_bayer_amaze(self, raw_rgb, filters: int, cam_mul=(1.0, 1.0, 1.0, 1.0), maximum_value: float = 1.0):
         """AMaZE + 4-px border fill of the reference's sparse (H, W, 3) raw buffer."""

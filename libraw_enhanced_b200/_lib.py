@@ -196,6 +196,7 @@ SIGNATURES = {
     "lre_inject_fault": (None, [_p, _i]),
     "lre_set_wait_limit": (_st, [_p, C.c_longlong]),
     "lre_inject_sweep_stall": (None, [_p, _i]),
+    "lre_sweep_counts": (_st, [_p, C.POINTER(C.c_uint), C.POINTER(C.c_uint)]),
     "lre_demosaic_bayer_amaze": (_st, [_p, _p, _p, _sz, _sz, C.c_uint32, _p, _f]),
     "lre_demosaic_xtrans_1pass": (_st, [_p, _p, _p, _sz, _sz, _p, _p, _f]),
     "lre_demosaic_xtrans_3pass": (_st, [_p, _p, _p, _sz, _sz, _p, _p, _f]),

@@ -160,7 +160,8 @@ lre_status lre_create(int device, lre_ctx** out) {
     delete c;
     return LRE_ERR_OUT_OF_MEMORY;
   }
-  if (lre::aahd_upload_gamma(c) != LRE_OK) {
+  if (cudaMemset(lre::sweep_counts(c), 0, 2 * sizeof(unsigned)) != cudaSuccess ||
+      lre::aahd_upload_gamma(c) != LRE_OK) {
     cudaFree(c->d_scalars);
     cudaStreamDestroy(c->own_stream);
     delete c;
@@ -276,6 +277,17 @@ lre_status lre_set_wait_limit(lre_ctx* ctx, long long cycles) {
 void lre_inject_sweep_stall(lre_ctx* ctx, int band) {
   Context* c = reinterpret_cast<Context*>(ctx);
   if (c) c->sweep_hold_band = band >= 0 ? band : -1;
+}
+
+lre_status lre_sweep_counts(lre_ctx* ctx, unsigned* blocks_repeated, unsigned* passes_in_order) {
+  Context* c = reinterpret_cast<Context*>(ctx);
+  if (!c) return LRE_ERR_INVALID_ARGUMENT;
+  unsigned n[2] = {0, 0};
+  LRE_CUDA_TRY(c, cudaMemcpyAsync(n, lre::sweep_counts(c), sizeof(n), cudaMemcpyDeviceToHost, c->stream));
+  LRE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  if (blocks_repeated) *blocks_repeated = n[0];
+  if (passes_in_order) *passes_in_order = n[1];
+  return LRE_OK;
 }
 
 }  // extern "C"

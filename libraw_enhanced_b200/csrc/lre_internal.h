@@ -115,6 +115,8 @@ lre_status check_injection(Context* c);
 // about the same time, this one included: the owner's number, or those that
 // asked this within the last half millisecond (context.cu).
 int contexts_at_work(Context* c);
+// The context's two counters of the block sweeps, on the device (sweep.cuh).
+inline unsigned* sweep_counts(Context* c) { return reinterpret_cast<unsigned*>(c->d_scalars + 56); }
 
 #define LRE_CUDA_TRY(ctx, call)                                        \
   do {                                                                 \

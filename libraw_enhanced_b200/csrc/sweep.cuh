@@ -372,6 +372,7 @@ struct BlkArgs {
   int S, nbj, nbi;             // owned steps per block, blocks per row of blocks, rows of blocks
   float* side;                 // per block: the kept outside values
   int* bad;                    // [0], [1]: a block disagreed in the first / second check; [2..]: per block
+  unsigned* counts;            // of the context: blocks that disagreed, passes that gave way (lre_sweep_counts)
   const int* skip_if_zero;
 };
 
@@ -698,10 +699,15 @@ __global__ void __launch_bounds__(256) k_blk_check(BlkArgs a) {
   bad = __syncthreads_or(bad);
   if (threadIdx.x == 0) {
     if (ROUND == 0) a.bad[2 + blk] = bad;
-    if (bad) atomicExch(a.bad + ROUND, 1);
-    // an op that also writes behind its walk position is not repaired: a
-    // repair would update the last site of the block before it twice
-    if (bad && Op::LAG > 0) atomicExch(a.bad + 1, 1);
+    if (bad) {
+      if (ROUND == 0) {
+        atomicExch(a.bad, 1);
+        atomicAdd(a.counts, 1u);
+      }
+      // an op that also writes behind its walk position is not repaired: a
+      // repair would update the last site of the block before it twice
+      if ((ROUND == 1 || Op::LAG > 0) && atomicExch(a.bad + 1, 1) == 0) atomicAdd(a.counts + 1, 1u);
+    }
   }
 }
 
@@ -790,6 +796,7 @@ lre_status blk_sweep(Context* c, BlkArgs& b, void* ws, size_t ws_len, const int*
   if (n * B::side_floats(b.S) * sizeof(float) + (n + 2) * sizeof(int) > ws_len || b.nbi > 65535)
     return fail(c, LRE_ERR_CUDA, std::string(what) + ": block table too small");
   b.bad = reinterpret_cast<int*>(ws);
+  b.counts = sweep_counts(c);
   b.side = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + (((n + 2) * sizeof(int) + 255) & ~size_t(255)));
   *run_if = b.bad + 1;
   // fault injection and a wait limit are about the in-order sweep
