@@ -529,6 +529,8 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
   LRE_CUDA_TRY(c, cudaMemsetAsync(M, 0, w * h, s));
   int* err = d_err ? d_err : sync + 1;
   if (!d_err) LRE_CUDA_TRY(c, cudaMemsetAsync(err, 0, sizeof(int), s));
+  int* nyquist_gave_up = sync + 2;
+  LRE_CUDA_TRY(c, cudaMemsetAsync(nyquist_gave_up, 0, sizeof(int), s));
   DCB_LAUNCH(k_dcb_init, raw, raw_c_stride, R, G, B, g);
   DCB_LAUNCH(k_dcb_hv, G, P1, P2, g);
   DCB_LAUNCH(k_dcb_hvc, R, B, P1, P2, P3, P4, g);
@@ -552,7 +554,7 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     ny.plane[2] = P2;
     for (int k = 0; k < 3; k++) {
       ny.plane[0] = G;
-      LRE_TRY(sweep<OpNyquist>(c, ny, &P3, false, blk_ws, blk_len, sync, nb_max, "dcb_nyquist"));
+      LRE_TRY(sweep<OpNyquist>(c, ny, &P3, false, blk_ws, blk_len, sync, nb_max, "dcb_nyquist", nyquist_gave_up));
       std::swap(G, P3);
     }
     DCB_LAUNCH(k_dcb_map, G, M, g);

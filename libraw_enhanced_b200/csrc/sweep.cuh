@@ -130,6 +130,9 @@ __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// ints of a call's sync table before the per-band progress: [1] error flag,
+// [2] gave-up flag, the last one the ticket
+constexpr int kSyncInts = 64;
 constexpr long long kWaitCycles = 4000000000LL;  // default wait bound: ~2 s at 1.9 GHz
 
 __device__ __forceinline__ void cp_async4(float* s, const float* g) {
@@ -336,6 +339,18 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
 // repair), is checked again, and if that disagrees too the in-order sweep
 // below runs on the untouched input.  The result is the in-order one always.
 //
+// Which frames disagree: those with flat areas larger than the overlap, clipped
+// ones or synthetic ones, where a mean of equal values passes on a unit in the
+// last place for ever, and runs of sites that each decide the next one.  Such a
+// pass costs the blocks and the whole in-order sweep, so where a call runs the
+// same op several times (DCB's nyquist) one that gave way sends the later ones
+// in order at once (two iterations of DCB on clipped waves, 24, 1.5 and 0.17 MP:
+// 17.5, 4.0 and 1.9 ms without that, 15.0, 3.6 and 1.5 ms; before the blocks 16.1,
+// 3.2 and 1.2 ms).
+// (Mending the blocks one after another instead is slower: a chain of changes
+// passes through whole blocks, 250 us each, where the in-order sweep's links are
+// 32 rows by 16 columns: 25.5 ms against 11.6 for DCB of 24 MP of clipped waves.)
+//
 // Block geometry: BLK_WARPS warps of 32 rows walk the steps tau = c + SKEW *
 // (row / PAIR) of the block in groups of kBlkGroup, each warp one group behind
 // the warp above; a barrier per group.  The state planes live in a
@@ -359,8 +374,8 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_gs_sweep(SweepArgs a) {
 //
 // Overlap: an average of four updated neighbours passes on 3/7 of a change
 // per row and 1/1.5 per step (pp); from a difference of 2^18 ulps, 64 rows
-// and 96 steps leave fewer than 2^-20 ulps.  With 64 steps, one pp block in
-// about 2000 was repaired at 24 MP.
+// and 96 steps leave fewer than 2^-20 ulps.  The noisy 12 and 24 MP scenes of the
+// measured calls have no block that disagrees (lre_sweep_counts).
 constexpr int kBlkGroup = 8;    // steps per group
 constexpr int kBlkRing = 64;    // ring steps (power of two): groups g-2 .. g+5
 
@@ -373,6 +388,7 @@ struct BlkArgs {
   float* side;                 // per block: the kept outside values
   int* bad;                    // [0], [1]: a block disagreed in the first / second check; [2..]: per block
   unsigned* counts;            // of the context: blocks that disagreed, passes that gave way (lre_sweep_counts)
+  int* gave_up;                // optional: an earlier pass of the call gave way, and this one is to
   const int* skip_if_zero;
 };
 
@@ -445,6 +461,13 @@ __global__ void __launch_bounds__(Blk<Op>::NW * 32, Blk<Op>::PER_SM) k_blk_sweep
   if (a.skip_if_zero && *a.skip_if_zero == 0) return;
   const int ch = blockIdx.z, bi = blockIdx.y, bj = blockIdx.x;
   const int blk = (ch * a.nbi + bi) * a.nbj + bj;
+  if (a.gave_up && *a.gave_up != 0) {
+    if (!REPAIR && blk == 0 && threadIdx.x == 0) {
+      a.bad[1] = 1;
+      atomicAdd(a.counts + 1, 1u);
+    }
+    return;
+  }
   if (REPAIR && a.bad[2 + blk] == 0) return;
   const int W = a.g.W, H = a.g.H;
   const int own_r = bi * B::OWN, r0 = own_r - KR;
@@ -669,6 +692,7 @@ __global__ void __launch_bounds__(256) k_blk_check(BlkArgs a) {
   constexpr int NS = Op::NS, HALO = Op::HALO, NCH = Op::NCH;
   if (a.skip_if_zero && *a.skip_if_zero == 0) return;
   if (ROUND == 1 && a.bad[0] == 0) return;
+  if (a.gave_up && *a.gave_up != 0) return;
   const int ch = blockIdx.z, bi = blockIdx.y, bj = blockIdx.x;
   const int blk = (ch * a.nbi + bi) * a.nbj + bj;
   const int own_r = bi * B::OWN, r0 = own_r - Op::BLK_ROWS;
@@ -706,7 +730,10 @@ __global__ void __launch_bounds__(256) k_blk_check(BlkArgs a) {
       }
       // an op that also writes behind its walk position is not repaired: a
       // repair would update the last site of the block before it twice
-      if ((ROUND == 1 || Op::LAG > 0) && atomicExch(a.bad + 1, 1) == 0) atomicAdd(a.counts + 1, 1u);
+      if ((ROUND == 1 || Op::LAG > 0) && atomicExch(a.bad + 1, 1) == 0) {
+        atomicAdd(a.counts + 1, 1u);
+        if (a.gave_up) *a.gave_up = 1;
+      }
     }
   }
 }
@@ -771,15 +798,14 @@ lre_status sweep_in_order(Context* c, const SweepArgs& base, int* sync, int nb_m
   const int nb = (base.r_hi - base.r_lo + 32) / 32 * Op::NCH;
   if (nb > nb_max) return fail(c, LRE_ERR_CUDA, std::string(what) + ": band table too small");
   SweepArgs a = base;
-  a.ticket = sync;
-  a.progress = sync + 64;
+  a.ticket = sync + kSyncInts - 1;  // cleared together with the table
+  a.progress = sync + kSyncInts;
   a.wait_cycles = c->sweep_wait_cycles > 0 ? c->sweep_wait_cycles : kWaitCycles;
   // a held band (host-side fault injection, one sweep only) never reports
   // its progress, so the band below it waits until its bound runs out
   a.hold_ticket = c->sweep_hold_band >= 0 ? c->sweep_hold_band * Op::NCH : -1;
   c->sweep_hold_band = -1;
-  LRE_CUDA_TRY(c, cudaMemsetAsync(sync, 0, sizeof(int), c->stream));
-  LRE_CUDA_TRY(c, cudaMemsetAsync(a.progress, 0, (size_t)nb * sizeof(int), c->stream));
+  LRE_CUDA_TRY(c, cudaMemsetAsync(a.ticket, 0, (size_t)(nb + 1) * sizeof(int), c->stream));
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_gs_sweep<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::BYTES));
   k_gs_sweep<Op><<<nb, kSweepWarps * 32, R::BYTES, c->stream>>>(a);
   count_launch(c);
@@ -824,7 +850,7 @@ lre_status blk_sweep(Context* c, BlkArgs& b, void* ws, size_t ws_len, const int*
 // end in the input planes instead.  ws: blk_ws_bytes of the plane.
 template <class Op>
 lre_status sweep(Context* c, const SweepArgs& base, float* const* out, bool keep, void* ws, size_t ws_len, int* sync,
-                 int nb_max, const char* what) {
+                 int nb_max, const char* what, int* gave_up = nullptr) {
   constexpr int NPL = Op::NS * Op::NCH;
   if (base.r_hi < base.r_lo || base.c_hi < base.c_lo) {  // nothing to update
     if (!keep)
@@ -842,6 +868,7 @@ lre_status sweep(Context* c, const SweepArgs& base, float* const* out, bool keep
   b.c_lo = base.c_lo;
   b.c_hi = base.c_hi;
   b.skip_if_zero = base.skip_if_zero;
+  b.gave_up = gave_up;
   SweepArgs a = base;
   LRE_TRY(blk_sweep<Op>(c, b, ws, ws_len, &a.run_if, what));
   LRE_TRY(sweep_in_order<Op>(c, a, sync, nb_max, what));
@@ -866,9 +893,6 @@ bool bayer_2x2(uint32_t filters) {
   if (fcol3(0, 0, filters) == 1 && fcol3(1, 0, filters) == 1) return false;
   return n0 + n1 == 2 && n0 != n1;
 }
-
-constexpr int kSyncInts = 64;  // ticket, error flag, then per-band progress
-
 
 }  // namespace
 }  // namespace lre
