@@ -296,7 +296,11 @@ struct BlurStrip {
   static constexpr int C = BS_X + 2 * PAD;
   static constexpr int IN = (P + 1) * C;            // floats of the staged batch (one row more is read)
   static constexpr size_t SMEM = (size_t)(IN + (P + 1) * BS_X) * sizeof(float);
+  // resident CTAs per SM: what the registers are bounded for, fewer where shared
+  // memory (228 KB, 1 KB of it a CTA's own) holds fewer: six at tap radii 14 and 15
+  static constexpr int PER_SM = 228 * 1024 / (SMEM + 1024) < 7 ? (int)(228 * 1024 / (SMEM + 1024)) : 7;
 };
+static_assert(BlurStrip<13>::PER_SM == 7 && BlurStrip<14>::PER_SM == 6 && BlurStrip<15>::PER_SM == 6, "blocks per SM");
 
 __device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -307,7 +311,7 @@ __device__ __forceinline__ void cp_async(float* dst, const float* src, int bytes
 }
 
 template <int KS>
-__global__ void __launch_bounds__(BS_THREADS, 7) k_df_blur_strip(BlurJob job, GaussTaps taps, int W, int H, int batches,
+__global__ void __launch_bounds__(BS_THREADS, BlurStrip<KS>::PER_SM) k_df_blur_strip(BlurJob job, GaussTaps taps, int W, int H, int batches,
                                                               const DfScalars* sc) {
   using B = BlurStrip<KS>;
   constexpr int P = B::P, C = B::C, PAD = B::PAD;
@@ -433,8 +437,8 @@ lre_status run_blur_strip(Context* c, const BlurJob& job, const GaussTaps& taps,
   using B = BlurStrip<KS>;
   LRE_CUDA_TRY(c, cudaFuncSetAttribute(k_df_blur_strip<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B::SMEM));
   // Batches per chunk: a chunk's first 2 KS rows produce nothing, so tall
-  // chunks, halved while the grid has fewer than fourteen CTAs per SM.  Where
-  // even halves leave fewer than that (seven are resident, so at most two waves),
+  // chunks, halved while the grid has less than two waves of resident CTAs (seven
+  // per SM at most tap radii).  Where even halves leave fewer than that,
   // what takes the fewest batch steps over all waves, a nearly empty last one
   // counting as much as a full one.  With six CTAs per SM the three blurs of
   // 1.9 MP took 104 us halved and 88 us so (82 us with seven); those of 24 and
@@ -445,7 +449,7 @@ lre_status run_blur_strip(Context* c, const BlurJob& job, const GaussTaps& taps,
   const int strips = (W + BS_X - 1) / BS_X;
   auto chunks = [&](int n) { return (H + n * B::P - 2 * KS - 1) / (n * B::P - 2 * KS); };
   auto ctas = [&](int n) { return (long long)strips * chunks(n) * job.np; };
-  const long long places = 7LL * c->sm_count;
+  const long long places = (long long)B::PER_SM * c->sm_count;
   while (batches > 2 && ctas(batches) < 2 * places) batches /= 2;
   if (batches <= 4) {
     double least = 1e300;
