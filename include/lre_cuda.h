@@ -503,8 +503,10 @@ lre_status lre_dev_develop_raw(lre_ctx* ctx, const uint16_t* raw_image, const lr
 /* Kernel-shape choices that never change results, only speed. */
 typedef struct lre_tuning {
   int lanes;         /* batch/server: concurrent per-image pipelines (streams) */
-  int axial_strip;   /* guided-filter strip width (columns per CTA): 128 or 64 */
-  int axial_rows;    /* guided-filter output rows per CTA: 128 or 64          */
+  int axial_strip;   /* guided-filter strip width (columns per CTA): 128 or 64;
+                        not read at radius 6, whose strips have one width     */
+  int axial_rows;    /* guided-filter output rows per CTA: 128 or 64; at radius 6
+                        the most that a CTA may get, 192 or 96                */
   int blur_tile;     /* defringe blur row chunks: 64 tall, 32 half as tall     */
 } lre_tuning;
 lre_status lre_set_tuning(lre_ctx* ctx, const lre_tuning* t);

@@ -55,8 +55,8 @@ struct WsPlan {
 // Kernel-shape choices that do not change results (picked by the batch
 // autotuner, or set with lre_set_tuning).
 struct Tuning {
-  int axial_strip = 128;    // guided-filter strip width (columns per CTA): 128 or 64
-  int axial_rows = 128;     // guided-filter output rows per CTA: 128 or 64
+  int axial_strip = 128;    // guided-filter strip width (columns per CTA) at radii other than 6: 128 or 64
+  int axial_rows = 128;     // guided-filter output rows per CTA: 128 or 64 (at radius 6 at most 192 or 96)
   int blur_tile = 64;       // defringe blur strips: 64 for tall row chunks, 32 for half as tall
 };
 

@@ -370,12 +370,13 @@ lre_status autotune(Batch* b, const lre_image* im, size_t n, bool host_mode) {
   }
   const lre_develop_params& p = ref.params;
   Tuning best = b->tune;
-  // guided filter variants
+  // guided filter variants (at radius 6 the strip width is not read)
   {
     const int cand[4][2] = {{128, 128}, {128, 64}, {64, 128}, {64, 64}};
     float best_ms = 1e30f;
     float* dmax = c->d_scalars + 1;
     for (auto& v : cand) {
+      if (p.axial_ca_radius == 6 && v[0] != 128) continue;
       c->tune.axial_strip = v[0];
       c->tune.axial_rows = v[1];
       float ms = time_stream(c->stream, [&]() -> lre_status {
