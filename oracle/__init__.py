@@ -46,11 +46,19 @@ def _img(a):
     return a
 
 
+class Missing(FileNotFoundError):
+    """A library of the oracle has not been built."""
+
+
+def _load(path):
+    if not os.path.exists(path):
+        raise Missing(f"oracle library missing: {path} (run `make -C oracle`)")
+    return C.CDLL(path)
+
+
 class _Lib:
     def __init__(self, path, sigs):
-        if not os.path.exists(path):
-            raise FileNotFoundError(f"oracle library missing: {path} (run `make -C oracle`)")
-        self.lib = C.CDLL(path)
+        self.lib = _load(path)
         for name, (res, args) in sigs.items():
             fn = getattr(self.lib, name)
             fn.restype = res
@@ -224,9 +232,7 @@ def ref_detail_tonemap(img):
     oracle/_ref/liblre_ref_dt.so.  Returns the tone-mapped copy."""
     global _ref_dt
     if _ref_dt is None:
-        if not os.path.exists(REF_DT_SO):
-            raise FileNotFoundError(f"oracle library missing: {REF_DT_SO} (run `make -C oracle ref`)")
-        _ref_dt = C.CDLL(REF_DT_SO)
+        _ref_dt = _load(REF_DT_SO)
         _ref_dt.ref_detail_tonemap.restype = C.c_int
         _ref_dt.ref_detail_tonemap.argtypes = [_p, _sz, _sz]
     a = _img(img).copy()
@@ -239,7 +245,7 @@ def recover_highlights(rgb, saturation_threshold, want_mask=False, wb_rgb=None):
     compiled from those lines alone.  Returns (recovered copy, mask or None)."""
     global _ref_hl
     if _ref_hl is None:
-        _ref_hl = C.CDLL(REF_HL_SO)
+        _ref_hl = _load(REF_HL_SO)
         _ref_hl.ref_recover_highlights.restype = C.c_int
         _ref_hl.ref_recover_highlights.argtypes = [_p, _sz, _sz, _f, _p, _p]
     img = np.ascontiguousarray(rgb, dtype=np.float32).copy()
