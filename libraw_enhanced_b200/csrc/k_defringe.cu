@@ -563,8 +563,10 @@ __device__ __forceinline__ float support_at(const float* __restrict__ src, size_
 
 // K3 per pixel, four consecutive pixels per thread.  A pixel whose blurred
 // edge planes are at or below the lower smoothstep edges has an edge factor of
-// exactly 0 and so a seed of 0: where all four are such and every log ratio of
-// the image is finite (no factor is NaN), the other planes are not read.
+// exactly 0 and so a seed of 0: where all four are such, every log ratio of the
+// image is finite and every pair of edges is apart (FAST; a chroma threshold of 0
+// makes 0 / 0 of a pixel without excess), so no factor is NaN, the other planes
+// are not read.
 // At 51 MP 343 us; fused behind the blur of the five planes it had taken
 // about 880 us of that kernel's 2200.
 template <bool FAST>
@@ -572,7 +574,7 @@ __global__ void __launch_bounds__(256) k_df_support(const float* __restrict__ sr
                                                     DfTab T, const DfScalars* sc) {
   const bool enable_green = k.green != 0;
   const float e0_edge = T.e[DE_CORE].e0, e0_raw = T.e[DE_CORE_RAW].e0;
-  const bool can_skip = sc->nonfinite == 0 && k.edge_thr > 0.f;
+  const bool can_skip = FAST && sc->nonfinite == 0 && k.edge_thr > 0.f;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < (n + 3) / 4; q += stride) {
     const size_t i = q * 4;
@@ -680,8 +682,8 @@ __device__ __forceinline__ void line_runs(const float* s_ls, const float* s_fs, 
 // * a warp stages whole rows, all of its loads in flight (an element's place by
 //   two divisions and four clamps, two in flight: about 105 instructions a pixel);
 // * a pixel whose blurred edge planes are at or below the lower smoothstep edges
-//   has solo seeds of exactly 0 where every log ratio of the image is finite
-//   (K3's rule), without the two exponentials in double.
+//   has solo seeds of exactly 0 where no factor is NaN (K3's rule), without the
+//   two exponentials in double.
 // 51 MP: 1223 us before, 768 us; 26 MP odd 664 and 470 us; 1.9 MP 55 and 45 us.
 // (256 threads 926 us at 51 MP; two rows in flight 853 us; five CTAs per SM, which
 // spill, 769 us.)
@@ -753,7 +755,7 @@ __global__ void __launch_bounds__(LN_THREADS, 4)
     line_runs<-1, 2, 6, 1, -2>(s_ls, s_fs, s_best);
   }
   const float e0_edge = T.e[DE_CORE].e0, e0_raw = T.e[DE_CORE_RAW].e0;
-  const bool can_skip = sc->nonfinite == 0 && k.edge_thr > 0.f;
+  const bool can_skip = FAST && sc->nonfinite == 0 && k.edge_thr > 0.f;
   for (int i = threadIdx.x; i < LT * LT; i += blockDim.x) {
     int ly = i / LT, lx = i % LT;
     int y = y0 + ly, x = x0 + lx;
