@@ -44,8 +44,8 @@ METRIC = "develop MP/s on 1 B200 (51 MP Bayer: AMaZE->defringe->axial CA->tone m
 STAGE_BYTES = {"amaze": 16.0, "defringe": 24.0, "axial": 24.0, "tone": 24.0}
 # From one ncu capture of k_amaze at 4096x3072: DRAM read+write bytes and
 # executed warp-instructions per output pixel.
-AMAZE_DRAM_BYTES_PER_PX = (124.060416e6 + 909.380352e6) / (4096 * 3072)
-AMAZE_WARP_INST_PER_PX = 925190063 / (4096 * 3072)
+AMAZE_DRAM_BYTES_PER_PX = (91.017728e6 + 682.944e6) / (4096 * 3072)
+AMAZE_WARP_INST_PER_PX = 809979366 / (4096 * 3072)
 # issue roofline: 148 SMs x 4 schedulers x 1.965 GHz, one warp-instruction per cycle each
 ISSUE_PEAK_G = 148 * 4 * 1.965
 

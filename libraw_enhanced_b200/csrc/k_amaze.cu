@@ -1179,8 +1179,8 @@ lre_status launch_amaze_rows(Context* c, AmazeArgs A, int row_lo, int row_hi) {
   const int tiles = A.tile_hi - A.tile_lo;
   if (tiles <= 0) return LRE_OK;
   // CTAs per tile: what takes the least time over all rounds.  One tile at a
-  // time takes 270 us with one CTA, 190 with two, 137 with four, 117 with
-  // eight (511x341 to 1536x1024); clusters of four and eight lie inside a GPC,
+  // time takes 262 us with one CTA, 177 with two, 126 with four, 105 with
+  // eight (1536x1024, 1024x768, 700x600, 511x341); clusters of four and eight lie inside a GPC,
   // which leaves 32 and 16 places.  Where other contexts work beside this one
   // (a batch's or server's lanes, other threads') their tiles take places too, as many each:
   // a cluster of eight is the fastest for a thumbnail by itself, and takes 3.4

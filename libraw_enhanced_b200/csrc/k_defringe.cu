@@ -61,7 +61,7 @@ __device__ __forceinline__ float df_max_guide(const DfScalars* s) { return smax(
 // signal, a square root and a divide, is formed once per pixel, its neighbours
 // come from the lanes beside and the two rows before, and the next two rows are
 // on their way meanwhile.  Bound by instructions: two logarithms in double, two
-// divides and the guide.  51 MP 438 us, 26 MP odd 234 us, 1.9 MP 20 us; on 32 x 8
+// divides and the guide.  51 MP 448 us, 26 MP odd 237 us, 1.9 MP 20 us; on 32 x 8
 // tiles with the guide in shared memory, a barrier before and after, 783, 402 and
 // 24 us, and with CUDA's log in double besides 856, 441 and 27 us.
 constexpr int PW_ROWS = 32, PW_COLS = 30;
@@ -567,7 +567,7 @@ __device__ __forceinline__ float support_at(const float* __restrict__ src, size_
 // image is finite and every pair of edges is apart (FAST; a chroma threshold of 0
 // makes 0 / 0 of a pixel without excess), so no factor is NaN, the other planes
 // are not read.
-// At 51 MP 343 us; fused behind the blur of the five planes it had taken
+// At 51 MP 258 us; fused behind the blur of the five planes it had taken
 // about 880 us of that kernel's 2200.
 template <bool FAST>
 __global__ void __launch_bounds__(256) k_df_support(const float* __restrict__ src, size_t n, DfPlanes P, DfConst k,
@@ -1288,8 +1288,9 @@ __global__ void __launch_bounds__(256) k_df_maxg(const float* __restrict__ src, 
 }
 
 // Tap radii 3 to 15 run the strip kernel compiled for them, others the tile
-// kernel with the radius at run time (all eight planes of 26 MP at radius 7:
-// 2575 us in tiles, 733 us in strips).
+// kernel with the radius at run time (all eight planes of 12 MP: radius 3 253 us
+// and 15 634 us in strips, 2 678 us and 15.5 2257 us in tiles).  The strips'
+// 2 KS + 1 accumulators take two registers each: 62 of 168 at 15.
 template <int KS>
 lre_status blur_for(Context* c, const BlurJob& job, const GaussTaps& taps, int W, int H, const DfScalars* sc, bool* done) {
   if constexpr (KS >= 3) {

@@ -41,9 +41,13 @@ __device__ __forceinline__ float aces_tm(float x) {
 // a running sum) left the GPU to H or W threads: 18.97 ms at 8256x5504; this
 // one takes 0.63 ms (0.74 ms with eight divisions a lane and row by the number of
 // samples, whose reciprocals a lane now keeps).  A sum restarts at every chunk of
-// rows and every four columns, so it carries the roundings of at most 256 + 2R
-// additions instead of the whole column's: the error against 64 bits is 2e-7
-// where the whole-image running sums had 1.7e-6.
+// rows and every four columns, so a vertical sum carries the roundings of at most
+// 2 * 256 + 2R additions and subtractions (a row enters and one leaves), not of
+// the whole column's; 24 more form a window's, and a product with a rounded
+// reciprocal its mean.  Measured against 64 bits: 2e-7, where the whole-image
+// running sums had 1.7e-6.  Samples above 1.8e19, whose squares are infinite,
+// spoil the sums of their window and, behind them, of the chunk (there the whole
+// column).
 constexpr int DT_R = 12;               // box radius (core/libraw_wrapper.cpp:1424)
 constexpr int DT_X = 128;              // output columns per strip
 constexpr int DT_C = DT_X + 2 * DT_R;  // columns whose vertical sums a strip holds
