@@ -229,7 +229,7 @@ __global__ void k_aahd_hot_pretest(Aahd A) {
 // above: (r - 2, c + 2) is then already rewritten and (r + 2, c - 2) not yet.
 struct OpHideHots {
   static constexpr int NS = 1, NP = 1, HALO = 2, SKEW = 3, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 3, BLK_PAIR = 2, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 2, BLK_ROWS = 64, BLK_COLS = 64, BLK_FROM = 800;
   static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = false;
   // padded coordinates; the 2x2 pattern makes the 4-px offset invisible
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(256) k_aahd_evaluate(Aahd A) {
 // follows the site exactly as in the row-major loops with skew 1.
 struct OpRefineDirs {
   static constexpr int NS = 1, NP = 1, HALO = 1, SKEW = 1, PAIR = 1, NCH = 1, LAG = 1, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64, BLK_FROM = 950;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   // the walk acts at even image columns; rows two steps apart share their parity
   __device__ static bool site(int, int c, const Geo&) { return ((c - kMargin) & 1) == 0; }
@@ -536,6 +536,7 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
   count_launch(c);
   LRE_TRY(check_launch(c, "demosaic_bayer_aahd"));
   AAHD_LAUNCH(k_aahd_hot_pretest, A);
+  bool moved = false;
   SweepArgs sa{};
   sa.g = Geo{A.NW, (int)h + 2 * kMargin, filters, maximum_value};
   sa.err = err;
@@ -549,7 +550,7 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
     hh.skip_if_zero = A.hot;
     // through the direction plane (unused so far, its margin zero like X's)
     // and back: without hot sites nothing runs and X stays as it is
-    LRE_TRY(sweep<OpHideHots>(c, hh, &A.ND, true, blk_ws, blk_len, sync, nb_max, "aahd_hide_hots"));
+    LRE_TRY(sweep<OpHideHots>(c, hh, &A.ND, true, blk_ws, blk_len, sync, nb_max, "aahd_hide_hots", &moved));
   }
   AAHD_LAUNCH(k_aahd_greens, A);
   AAHD_LAUNCH(k_aahd_rb_hv, A);
@@ -564,8 +565,8 @@ lre_status launch_aahd(Context* c, const float* raw, int raw_c_stride, float* rg
     rd.r_hi = (int)h + kMargin - 1;
     rd.c_lo = kMargin;
     rd.c_hi = (int)w + kMargin;  // one past the image: the last odd column
-    LRE_TRY(sweep<OpRefineDirs>(c, rd, &A.X, false, blk_ws, blk_len, sync, nb_max, "aahd_refine_dirs"));
-    std::swap(A.ND, A.X);  // the samples are no longer needed
+    LRE_TRY(sweep<OpRefineDirs>(c, rd, &A.X, false, blk_ws, blk_len, sync, nb_max, "aahd_refine_dirs", &moved));
+    if (moved) std::swap(A.ND, A.X);  // the samples are no longer needed
   }
   AAHD_LAUNCH(k_aahd_combine, A, rgb);
 #undef AAHD_LAUNCH

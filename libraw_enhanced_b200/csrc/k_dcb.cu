@@ -414,7 +414,7 @@ __global__ void k_dcb_pp_terms(const float* __restrict__ G, float* __restrict__ 
 // only, so rows r and r + 1 advance together.
 struct OpNyquist {
   static constexpr int NS = 1, NP = 3, HALO = 2, SKEW = 1, PAIR = 2, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 1, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr int BLK_SKEW = 1, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96, BLK_FROM = 1000;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   // sites with r + c of the non-green parity
@@ -431,7 +431,7 @@ struct OpNyquist {
 // input K = G - mean8(G) (k_dcb_pp_terms; green does not change in the pass).
 struct OpPP {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96, BLK_FROM = 1000;
   static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }
   __device__ static int phase(int, const Geo&) { return 0; }
@@ -456,7 +456,7 @@ __device__ __forceinline__ void clamp8(const T& t, float v) {
 // dcb_refinement's closing clamp (:992-994): state G; input the pre-clamp value.
 struct OpRefine {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 1, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 96, BLK_FROM = 1000;
   static constexpr bool UNROLL = true, STEP2 = true, IDLE0 = false;
   __device__ static bool site(int r, int c, const Geo& g) { return g.fc(r, c) != 1; }
   // sites with r + c of the non-green parity
@@ -471,7 +471,7 @@ struct OpRefine {
 // input that channel's CLIP(chroma + G).
 struct OpColorFull {
   static constexpr int NS = 1, NP = 2, HALO = 1, SKEW = 2, PAIR = 1, NCH = 2, LAG = 0, RING = kRing, BLK_WARPS = 8, BLK_PER_SM = 2;
-  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64;
+  static constexpr int BLK_SKEW = 2, BLK_PAIR = 1, BLK_ROWS = 64, BLK_COLS = 64, BLK_FROM = 1000;
   static constexpr bool UNROLL = true, STEP2 = false, IDLE0 = false;
   __device__ static bool site(int, int, const Geo&) { return true; }
   __device__ static int phase(int, const Geo&) { return 0; }
@@ -547,6 +547,7 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     x.c_hi = W - 1 - m;
     return x;
   };
+  bool moved = false;  // a sweep's result is in the plane it was given beside the input
   if (iterations > 0) DCB_LAUNCH(k_dcb_nyq_terms, R, B, P1, P2, g);
   for (int it = 1; it <= iterations; it++) {
     SweepArgs ny = rect(sa, 2);
@@ -554,8 +555,9 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     ny.plane[2] = P2;
     for (int k = 0; k < 3; k++) {
       ny.plane[0] = G;
-      LRE_TRY(sweep<OpNyquist>(c, ny, &P3, false, blk_ws, blk_len, sync, nb_max, "dcb_nyquist", nyquist_gave_up));
-      std::swap(G, P3);
+      LRE_TRY(sweep<OpNyquist>(c, ny, &P3, false, blk_ws, blk_len, sync, nb_max, "dcb_nyquist", &moved,
+                               nyquist_gave_up));
+      if (moved) std::swap(G, P3);
     }
     DCB_LAUNCH(k_dcb_map, G, M, g);
     DCB_LAUNCH(k_dcb_correction, G, M, g);
@@ -569,9 +571,11 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     pp.plane[2] = P1;
     pp.plane[3] = P1;
     float* const out[2] = {P2, P3};
-    LRE_TRY(sweep<OpPP>(c, pp, out, false, blk_ws, blk_len, sync, nb_max, "dcb_pp"));
-    std::swap(R, P2);
-    std::swap(B, P3);
+    LRE_TRY(sweep<OpPP>(c, pp, out, false, blk_ws, blk_len, sync, nb_max, "dcb_pp", &moved));
+    if (moved) {
+      std::swap(R, P2);
+      std::swap(B, P3);
+    }
   }
   DCB_LAUNCH(k_dcb_map, G, M, g);
   DCB_LAUNCH(k_dcb_correction2, G, R, B, M, g);
@@ -586,8 +590,8 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     SweepArgs rf = rect(sa, 4);
     rf.plane[0] = G;
     rf.plane[1] = P1;
-    LRE_TRY(sweep<OpRefine>(c, rf, &P2, false, blk_ws, blk_len, sync, nb_max, "dcb_refinement"));
-    std::swap(G, P2);
+    LRE_TRY(sweep<OpRefine>(c, rf, &P2, false, blk_ws, blk_len, sync, nb_max, "dcb_refinement", &moved));
+    if (moved) std::swap(G, P2);
     DCB_LAUNCH(k_dcb_chroma_native, R, B, G, P4, g);
     DCB_LAUNCH(k_dcb_chroma, P4, P2, P3, g);
     DCB_LAUNCH(k_dcb_chroma_g, P2, P3, G, P1, P4, g);
@@ -597,9 +601,11 @@ lre_status launch_dcb(Context* c, const float* raw, int raw_c_stride, float* rgb
     cf.plane[2] = P1;
     cf.plane[3] = P4;
     float* const out[2] = {P2, P3};
-    LRE_TRY(sweep<OpColorFull>(c, cf, out, false, blk_ws, blk_len, sync, nb_max, "dcb_color_full"));
-    std::swap(R, P2);
-    std::swap(B, P3);
+    LRE_TRY(sweep<OpColorFull>(c, cf, out, false, blk_ws, blk_len, sync, nb_max, "dcb_color_full", &moved));
+    if (moved) {
+      std::swap(R, P2);
+      std::swap(B, P3);
+    }
   }
   k_dcb_output<<<grid_for((w * h + 3) / 4, 256, c->sm_count * 8), 256, 0, s>>>(R, G, B, rgb, w * h, maximum_value);
   count_launch(c);

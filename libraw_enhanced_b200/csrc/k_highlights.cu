@@ -355,7 +355,7 @@ struct OpLoca {
 // the interleaved image.
 struct OpLocaBlk {
   static constexpr int NS = 2, NP = 3, HALO = 2, SKEW = 3, PAIR = 1, NCH = 1, LAG = 0, BLK_WARPS = 4, BLK_PER_SM = 3;
-  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 32, BLK_COLS = 96;
+  static constexpr int BLK_SKEW = 3, BLK_PAIR = 1, BLK_ROWS = 32, BLK_COLS = 96, BLK_FROM = 0;
   static constexpr bool UNROLL = false, STEP2 = false, IDLE0 = true;
   __device__ static bool site(int, int, const Geo&) { return true; }
   template <class T>
@@ -388,7 +388,7 @@ __global__ void k_hl_aux(float* scal, float thr) {
 // (`out` holds those; the candidates' are there), where it has to run.
 __global__ void k_hl_planes(const float* __restrict__ out, const float* __restrict__ cand, float* __restrict__ R,
                             float* __restrict__ G, float* __restrict__ B, size_t n, const int* __restrict__ run_if) {
-  if (*run_if == 0) return;
+  if (run_if && *run_if == 0) return;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     if (cand[i] != 0.f) continue;
     R[i] = out[i * 3];
@@ -401,7 +401,7 @@ __global__ void k_hl_planes(const float* __restrict__ out, const float* __restri
 __global__ void k_hl_interleave(const float* __restrict__ R, const float* __restrict__ G,
                                 const float* __restrict__ B, float* __restrict__ out, size_t n,
                                 const int* __restrict__ run_if) {
-  if (*run_if == 0) return;
+  if (run_if && *run_if == 0) return;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     out[i * 3] = R[i];
     out[i * 3 + 1] = G[i];
@@ -514,7 +514,8 @@ lre_status launch_recover_highlights(Context* c, const float* in, float* out, si
     if (!d_err) LRE_CUDA_TRY(c, cudaStreamSynchronize(s));
     return LRE_OK;
   }
-  LRE_TRY(blk_sweep<OpLocaBlk>(c, b, blk_ws, blk_len, &sa.run_if, "recover_highlights_loca"));
+  if (!sweeps_in_order<OpLocaBlk>(c, (int)w, (int)h))
+    LRE_TRY(blk_sweep<OpLocaBlk>(c, b, blk_ws, blk_len, &sa.run_if, "recover_highlights_loca"));
   k_hl_planes<<<g1, 256, 0, s>>>(out, HL, R2, G2, B2, n, sa.run_if);
   LRE_TRY(ck("recover_highlights"));
   LRE_TRY(sweep_in_order<OpLoca>(c, sa, sync, nb_max, "recover_highlights_loca"));

@@ -26,8 +26,8 @@
 // PAIR, NCH (independent channels run as separate warps), LAG (how many
 // columns behind its walk position a cell may still write), RING (ring
 // columns, a power of two), BLK_WARPS (warps of a block), BLK_PER_SM (resident
-// blocks per SM), BLK_ROWS and
-// BLK_COLS (a block's overlap), BLK_SKEW and BLK_PAIR (a block's own skew),
+// blocks per SM), BLK_ROWS and BLK_COLS (a block's overlap), BLK_FROM (how large a
+// plane has to be for blocks, sweeps_in_order), BLK_SKEW and BLK_PAIR (a block's own skew),
 // UNROLL (whether a block's group of steps is unrolled), STEP2 (a block visits
 // every second step only, from phase(r0, g) on), IDLE0 (sites whose inputs are
 // zero keep their values, so a group without others is skipped), site(r, c, g) (whether the
@@ -825,10 +825,7 @@ lre_status blk_sweep(Context* c, BlkArgs& b, void* ws, size_t ws_len, const int*
   b.counts = sweep_counts(c);
   b.side = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + (((n + 2) * sizeof(int) + 255) & ~size_t(255)));
   *run_if = b.bad + 1;
-  // fault injection and a wait limit are about the in-order sweep
-  const bool held = c->sweep_hold_band >= 0 || c->sweep_wait_cycles > 0;
-  LRE_CUDA_TRY(c, cudaMemsetAsync(b.bad, held ? 1 : 0, 2 * sizeof(int), c->stream));
-  if (held) return LRE_OK;
+  LRE_CUDA_TRY(c, cudaMemsetAsync(b.bad, 0, 2 * sizeof(int), c->stream));
   const dim3 grid((unsigned)b.nbj, (unsigned)b.nbi, Op::NCH);
   auto k0 = k_blk_sweep<Op, false>;
   auto k1 = k_blk_sweep<Op, true>;
@@ -845,20 +842,30 @@ lre_status blk_sweep(Context* c, BlkArgs& b, void* ws, size_t ws_len, const int*
   return check_launch(c, what);
 }
 
-// The sweep of base.plane[0 .. NS * NCH) into out[0 .. NS * NCH) (whole
-// planes; the input planes are scratch afterwards).  keep: the result is to
-// end in the input planes instead.  ws: blk_ws_bytes of the plane.
+// Whether a pass runs in order without trying blocks: where a wait limit or an
+// injected stall asks for it, and on planes so small that the blocks' latency (43
+// to 52 us a pass, whatever the size) is more than that of the few bands, which
+// grows with the width and 2.5 times the height.  Blocks and in order, us: DCB (one
+// iteration, six passes) 64x64 496 and 285, 128x128 507 and 440, 256x128 508 and
+// 524; AAHD without hot pixels 64x64 136 and 110, 128x128 147 and 146, with them
+// 64x128 213 and 219.  LoCA's blocks are the faster ones from 48x48 on.
+template <class Op>
+bool sweeps_in_order(Context* c, int W, int H) {
+  return c->sweep_hold_band >= 0 || c->sweep_wait_cycles > 0 || 2 * W + 5 * H < Op::BLK_FROM;
+}
+
+// The sweep of base.plane[0 .. NS * NCH).  The result is in out[0 .. NS * NCH)
+// (whole planes; the input planes are then scratch) if *moved says so, else where
+// the input was.  keep: it is to end in the input planes.  ws: blk_ws_bytes of the
+// plane.
 template <class Op>
 lre_status sweep(Context* c, const SweepArgs& base, float* const* out, bool keep, void* ws, size_t ws_len, int* sync,
-                 int nb_max, const char* what, int* gave_up = nullptr) {
+                 int nb_max, const char* what, bool* moved, int* gave_up = nullptr) {
   constexpr int NPL = Op::NS * Op::NCH;
-  if (base.r_hi < base.r_lo || base.c_hi < base.c_lo) {  // nothing to update
-    if (!keep)
-      for (int p = 0; p < NPL; p++)
-        LRE_CUDA_TRY(c, cudaMemcpyAsync(out[p], base.plane[p], (size_t)base.g.W * base.g.H * sizeof(float),
-                                        cudaMemcpyDeviceToDevice, c->stream));
-    return LRE_OK;
-  }
+  *moved = false;
+  if (base.r_hi < base.r_lo || base.c_hi < base.c_lo) return LRE_OK;  // nothing to update
+  if (sweeps_in_order<Op>(c, base.g.W, base.g.H)) return sweep_in_order<Op>(c, base, sync, nb_max, what);
+  *moved = !keep;
   BlkArgs b{};
   for (int p = 0; p < 4; p++) b.in[p] = base.plane[p];
   for (int p = 0; p < NPL; p++) b.out[p] = out[p];
