@@ -139,7 +139,10 @@ struct LkMaps {
 
 // One CTA per (cell, channel).  blockIdx.x = cell, blockIdx.y = channel
 // (0: R, 1: B).
-__global__ void __launch_bounds__(LK_THREADS, 5)
+// PER_SM: resident CTAs that the registers are bounded for, five where there are
+// CTAs enough, two where not (a CTA is then the faster by itself).
+template <int PER_SM>
+__global__ void __launch_bounds__(LK_THREADS, PER_SM)
     k_lk_level(const float* __restrict__ G, const float* __restrict__ Rt, const float* __restrict__ Bt, int W, int H,
                int map_w, int map_h, int max_iterations, float max_shift, float scale_down, float scale_up,
                LkMaps maps) {
@@ -347,10 +350,9 @@ __device__ __forceinline__ void map_place(float p, float cell, int n, int& g0, i
   g1 = min(g0 + 1, n - 1);
 }
 
-constexpr int RM_ROWS = 16;  // rows of a thread's column
-constexpr int RM_B = 4;      // rows in flight
+constexpr int RM_B = 4;  // rows in flight
 
-// A warp's 32 columns over RM_ROWS rows.  The shift is bilinear in the map, so
+// A warp's 32 columns over ROWS rows.  The shift is bilinear in the map, so
 // its two horizontal means (of either map row, for four maps) stay in registers
 // while the rows stay between the same two map rows, and a pixel costs the
 // vertical mean alone, not 16 map loads and two divisions each way; the rows'
@@ -360,6 +362,7 @@ constexpr int RM_B = 4;      // rows in flight
 // through shared memory, in whole sectors.
 // 26 MP: 288 us before, 177 us; its 24 B per pixel take 95 us.  (One row at a
 // time 287 us; three CTAs per SM 206 us, five, which spill, 201 us.)
+template <int ROWS>
 __global__ void __launch_bounds__(256, 4)
     k_lk_remap(const float* __restrict__ R0, const float* __restrict__ G0, const float* __restrict__ B0,
                float* __restrict__ dst, int W, int H, ShiftMaps mr, ShiftMaps mb, int map_w, int map_h, float cell,
@@ -368,14 +371,14 @@ __global__ void __launch_bounds__(256, 4)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const float* const m[4] = {mr.dx, mr.dy, mb.dx, mb.dy};
   const float xe = (float)(W - 1), ye = (float)(H - 1);
-  for (int yb = (blockIdx.y * 8 + wid) * RM_ROWS; yb < H; yb += gridDim.y * 8 * RM_ROWS)
+  for (int yb = (blockIdx.y * 8 + wid) * ROWS; yb < H; yb += gridDim.y * 8 * ROWS)
     for (int xb = blockIdx.x * 32; xb < W; xb += gridDim.x * 32) {
       const int x = min(xb + lane, W - 1), live = min(32, W - xb) * 3;
       int gx0, gx1, ly0, ly1, held = -1;
       float fx, lfy, up[4], dn[4];
       map_place((float)x, cell, map_w, gx0, gx1, fx);
       map_place((float)(yb + lane), cell, map_h, ly0, ly1, lfy);
-      const int y_end = min(yb + RM_ROWS, H);
+      const int y_end = min(yb + ROWS, H);
       for (int y0 = yb; y0 < y_end; y0 += RM_B) {
         float sx[RM_B][2], sy[RM_B][2];
         bool in = true;
@@ -524,20 +527,31 @@ lre_status launch_lateral_ca(Context* c, const float* in, float* out, size_t w, 
                                                                                                 Wl[l], Hl[l]);
     count_launch(c);
   }
+  // Up to two CTAs per SM, or five of large cells, the form for few CTAs: 511x341,
+  // cell 96 (48 CTAs) 36 us, 44 with the other; 1200x800 (234) 53 and 59; 1536x1024
+  // (352) 83 and 73; cells of 400 at 26 MP (352) 1066 and 1522, of 200 at 12 MP (600)
+  // 408 and 420, at 26 MP (1344) 819 and 803.
+  const bool few = 2 * ncell <= (size_t)c->sm_count * (cell >= 160 ? 5 : 2);
   for (int L = eff - 1; L >= 0; L--) {
     const float scale_down = 1.f / (float)(1 << L);
     const float level_max_shift = max_shift * scale_down + (float)(1 << L) * 0.5f;
     const float scale_up = (float)(1 << L);
     dim3 grid((unsigned)ncell, 2);
-    k_lk_level<<<grid, LK_THREADS, 0, c->stream>>>(Gl[L], Rl[L], Bl[L], Wl[L], Hl[L], map_w, map_h, iters,
-                                                   level_max_shift, scale_down, scale_up, maps);
+    auto level = few ? k_lk_level<2> : k_lk_level<5>;
+    level<<<grid, LK_THREADS, 0, c->stream>>>(Gl[L], Rl[L], Bl[L], Wl[L], Hl[L], map_w, map_h, iters, level_max_shift,
+                                              scale_down, scale_up, maps);
     count_launch(c);
   }
   k_lk_gate_smooth<<<1, 1024, 0, c->stream>>>(maps, map_w, map_h, min_conf, tmp);
   const float clamp_shift = max_shift * (float)(1 << (eff - 1));
-  const dim3 rg((unsigned)std::min<size_t>((w + 31) / 32, 1024),
-                (unsigned)std::min<size_t>((h + 8 * RM_ROWS - 1) / (8 * RM_ROWS), 8192));
-  k_lk_remap<<<rg, 256, 0, c->stream>>>(
+  // Sixteen rows a thread where that leaves eight CTAs per SM, else four: 0.2 MP 4.4
+  // us, 10.0 with sixteen; 3 MP 24.8 and 26.2; 6 MP 46.8 and 46.4; 26 MP 193 and 177.
+  const size_t strips = (w + 31) / 32;
+  const bool tall = strips * ((h + 127) / 128) >= (size_t)c->sm_count * 8;
+  const int rows = tall ? 16 : 4;
+  const dim3 rg((unsigned)std::min<size_t>(strips, 1024), (unsigned)std::min<size_t>((h + 8 * rows - 1) / (8 * rows), 8192));
+  auto remap = tall ? k_lk_remap<16> : k_lk_remap<4>;
+  remap<<<rg, 256, 0, c->stream>>>(
       Rl[0], Gl[0], Bl[0], out, (int)w, (int)h, ShiftMaps{maps.dx[0], maps.dy[0]}, ShiftMaps{maps.dx[1], maps.dy[1]},
       map_w, map_h, (float)cell, clamp_shift);
   count_launch(c, 2);
