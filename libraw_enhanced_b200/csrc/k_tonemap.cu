@@ -352,15 +352,15 @@ __global__ void k_box_cols2(const float* __restrict__ t0, const float* __restric
 // Local mean and standard deviation of one channel: the 81-tap sums of v and
 // v^2, each product and each sum rounded, in (ky, kx) order from 0.
 //
-// A thread owns one column of a 32-column strip of one channel and walks down
-// MC_ROWS rows; nine accumulator pairs (v and v^2 packed in one 64-bit
+// A thread owns one column of a 64-column strip of one channel and walks down
+// a chunk of rows; nine accumulator pairs (v and v^2 packed in one 64-bit
 // register) are in flight, one per output row.  A staged sample is multiplied
 // once per distinct |ky| (five packed products for nine rows) and the row's
 // nine samples are taken in kx order, so every accumulator gets its taps in
 // the reference's order.  The accumulators rotate by name over nine rows.
 // What bounds it: the FP32 pipe.  Per channel and pixel 2 x (45 + 81)
 // operations against 2 x 162 + 81 with every tap multiplied (and v squared)
-// on its own.  4032x3024: 407 us (620 before);
+// on its own.  4032x3024: 384 us (611 with tiles);
 // the pipe's time is 290 us.
 constexpr int MC_R = 4;
 constexpr int MC_X = 64;                  // output columns per CTA
@@ -380,11 +380,12 @@ __device__ __forceinline__ unsigned long long mc_pack(float a, float b) {
   return r;
 }
 
-__global__ void __launch_bounds__(MC_THREADS) k_mc_stats(const float* __restrict__ in, int W, int H, int batches,
+__global__ void __launch_bounds__(MC_THREADS) k_mc_stats(const float* __restrict__ in, int W, int H, int periods,
                                                          McTaps taps, float* __restrict__ mean3,
                                                          float* __restrict__ std3, float* d_max) {
   __shared__ __align__(16) float s[2][MC_B][MC_C * 3];
-  const int x0 = blockIdx.x * MC_X, rows = batches * MC_B - 2 * MC_R;
+  const int x0 = blockIdx.x * MC_X, rows = periods * MC_P - 2 * MC_R;
+  const int batches = (periods + 1) / 2;
   const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, H);
   const int tid = threadIdx.x, ch = tid % 3, col = tid / 3, x = x0 + col;
   const unsigned long long nz = taps.nz;
@@ -400,10 +401,12 @@ __global__ void __launch_bounds__(MC_THREADS) k_mc_stats(const float* __restrict
   };
   auto stage = [&](int b) {
     const int yb = y0 - MC_R + b * MC_B;
+    const int n = (periods - 2 * b) * MC_P;  // rows of the chunk from yb
     for (int i = tid; i < MC_C * 3; i += MC_THREADS) {
       const int gx = min(max(x0 - MC_R + i / 3, 0), W - 1), c = i % 3;
 #pragma unroll
       for (int r = 0; r < MC_B; r++) {
+        if (r == MC_P && n == MC_P) break;
         const float* g = in + ((size_t)min(max(yb + r, 0), H - 1) * W + gx) * 3 + c;
         const unsigned d = (unsigned)__cvta_generic_to_shared(&s[b & 1][r][i]);
         asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(g) : "memory");
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(MC_THREADS) k_mc_stats(const float* __restrict
     }
     __syncthreads();
 #pragma unroll 1
-    for (int half = 0; half < 2; half++)
+    for (int half = 0; half < min(2, periods - 2 * b); half++)
 #pragma unroll
     for (int r = 0; r < MC_P; r++) {
       const float* row = &s[b & 1][half * MC_P + r][col * 3 + ch];
@@ -600,14 +603,24 @@ lre_status launch_micro_contrast(Context* c, const float* in, float* out, size_t
   if (!mean3 || !std3 || !dmax) return fail(c, LRE_ERR_OUT_OF_MEMORY, "enhance_micro_contrast: workspace too small");
   static const McTaps taps = make_mc_taps();
   LRE_CUDA_TRY(c, cudaMemsetAsync(dmax, 0, sizeof(float), c->stream));
-  // chunks of up to 8 batches of 18 rows (a chunk reads 8 rows more than it
-  // writes), fewer while the grid has fewer than eight CTAs per SM
+  // A chunk of n periods of nine rows writes 9n - 8 of them.  n by the time that the
+  // fullest SM takes: its CTAs share the FP32 pipe, a quarter of a microsecond each
+  // per row of theirs, and one alone waits for its own chain besides (0.42 us a row
+  // with one CTA on the SM, 0.67 with two, 1.17 with four); more than one batch
+  // begins with the loads of two.  Up to eight batches.
+  // 530x530 19.1 us, 1536x1024 62.8, 4032x3024 384; halving from eight batches until
+  // there were eight CTAs per SM 21.2, 81.0, 398; a tile per CTA 18.7, 87.1, 611.
   const int strips = (W + MC_X - 1) / MC_X;
-  int batches = 8;
-  auto chunks = [&](int n) { return (H + n * MC_B - 2 * MC_R - 1) / (n * MC_B - 2 * MC_R); };
-  while (batches > 1 && (long long)strips * chunks(batches) < 8LL * c->sm_count) batches /= 2;
-  const dim3 grid((unsigned)strips, (unsigned)chunks(batches));
-  k_mc_stats<<<grid, MC_THREADS, 0, c->stream>>>(in, W, H, batches, taps, mean3, std3, dmax);
+  auto chunks = [&](int n) { return (H + n * MC_P - 2 * MC_R - 1) / (n * MC_P - 2 * MC_R); };
+  auto cost = [&](int n) {
+    const long long ctas = (long long)strips * chunks(n);
+    return n * (2 + 3 * ((ctas + c->sm_count - 1) / c->sm_count)) + (n > 2 ? 2 : 0);
+  };
+  int periods = 2;
+  for (int n = 3; n <= 16; n++)
+    if (cost(n) < cost(periods)) periods = n;
+  const dim3 grid((unsigned)strips, (unsigned)chunks(periods));
+  k_mc_stats<<<grid, MC_THREADS, 0, c->stream>>>(in, W, H, periods, taps, mean3, std3, dmax);
   k_mc_apply<<<grid_for(w * h, 256, c->sm_count * 8), 256, 0, c->stream>>>(in, out, mean3, std3, mask, w * h,
                                                                             threshold, strength, target, dmax);
   count_launch(c, 2);
